@@ -334,8 +334,9 @@ sevc_status sevc_set_graphs(sevc_handle *h, int on);
 /* Launch-shape autotuner (no counterpart in the reference): times `steps`
  * steps from the current state for each candidate block size of the
  * vertex pass (128/256/512) and of the per-boundary passes, each side
- * count from which grains get a warp each (9..12), and the resident blocks
- * per SM of the thread-per-grain grain pass (4, 5, 6, 8), one parameter at a
+ * count from which grains get a warp each in the grain pass (9..11; 12: none
+ * below 32), and the grain pass's block shape (4, 5: 64 grains a block; 6,
+ * 8: 32), one parameter at a
  * time, keeps the fastest and restores the state.  chosen (4 ints, may be
  * NULL) receives them in that order.  Results never depend on these
  * shapes. */

@@ -251,20 +251,6 @@ template <> struct InvSplit<6> { static constexpr double hi = 0x1.5555555555555p
 template <> struct InvSplit<7> { static constexpr double hi = 0x1.2492492492492p-3, lo = 0x1.2492492492492p-57; };
 template <> struct InvSplit<9> { static constexpr double hi = 0x1.c71c71c71c71cp-4, lo = 0x1.c71c71c71c71cp-58; };
 template <> struct InvSplit<10> { static constexpr double hi = 0x1.999999999999ap-4, lo = -0x1.999999999999ap-58; };
-template <int N> __device__ __forceinline__ double div_small(double x)
-{
-    if constexpr (N == 4) {
-        return dscale_down<2>(x);
-    } else if constexpr (N == 8) {
-        return dscale_down<3>(x);
-    } else {
-        unsigned long long b = mag2(x);
-        if (b >= (0x07B0000000000000ULL << 1) && b < (0x7830000000000000ULL << 1))
-            return __fma_rn(x, InvSplit<N>::hi, __dmul_rn(x, InvSplit<N>::lo));
-        return ddiv_slow(x, (double)N);
-    }
-}
-
 __device__ __forceinline__ double wrapd(double dest, double orig, double D) /* wrap_dist :147 */
 {
     double d = dest - orig;

@@ -215,8 +215,8 @@ bool alloc_device(sevc_handle *h)
         { (void **)&x.extra, I * EXTRA_CAP * 4 }, { (void **)&x.threadfail, I * grid * 4 },
         { (void **)&x.block_area, I * h->p.n_blocks * 8 }, { (void **)&x.counters, I * CTR_COUNT * 4 },
         { (void **)&x.rng, nrng * sizeof(curandState) }, { (void **)&x.rng_saved, nrng * sizeof(curandState) },
-        { (void **)&x.nucl_buf, I * 96 * 4 }, { (void **)&x.vbucket, 64 * 4 }, { (void **)&x.perm, G * 4 },
-        { (void **)&x.n_perm, 4 }, { (void **)&m.nlist, G * 4 }, { (void **)&m.nnlist, I * 4 }, { (void **)&m.pos0, V * 16 },
+        { (void **)&x.nucl_buf, I * 96 * 4 }, { (void **)&x.reserved64, 64 * 4 }, { (void **)&x.three, G * 4 },
+        { (void **)&x.n_three, 4 }, { (void **)&m.nlist, G * 4 }, { (void **)&m.nnlist, I * 4 }, { (void **)&m.pos0, V * 16 },
         { (void **)&m.vel0, V * 16 }, { (void **)&m.bv0, B * 8 }, { (void **)&m.vstamp, V * 4 },
         { (void **)&m.bstamp, B * 4 }, { (void **)&m.stamp, 4 }, { (void **)&m.bexact, B }, { (void **)&m.gexact, G },
         { (void **)&m.bmark, B }, { (void **)&m.lastblk, 8 * 4 },
@@ -233,6 +233,10 @@ bool alloc_device(sevc_handle *h)
     h->dblock = base;
     h->dbytes = total;
     for (auto &q : r) { *q.p = base; base += align256(q.bytes); }
+    /* the count of 3-sided grains is zero between steps; the first word of
+     * its 256 bytes held another count in earlier checkpoint files, so it
+     * takes the second */
+    x.n_three += 1;
     /* reservation keys start above every key an event writes */
     if (!cuda_ok(cudaMemsetAsync(x.vown, 0xFF, V * 8, h->stream), "memset") ||
         !cuda_ok(cudaMemsetAsync(x.bown, 0xFF, B * 8, h->stream), "memset"))
@@ -493,27 +497,23 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
         { Prof pr(h, "nucleation"); launch_nucleation(m, x, h->p, s); }
         if (h->tape.after_nucleation) h->tape.after_nucleation(s);
     }
-    /* From here three branches that share no written data run concurrently
-     * (side streams, graph branches when captured):
-     *   main   side-count order, thread-per-grain grain pass
-     *   side0  boundary arclengths and energies (:124-130 / :171-181)
-     *   side1  warp-per-grain grain pass of the widest grains; the first
-     *          2x3 count (:228), which depends only on the topology that
-     *          nothing changes before that loop; the device-side decision
-     *          whether this step computes every output-only value
-     * and join before the vertex pass, which reads all of them.  After it,
-     * dA/dt of the 3-sided grains (side0) runs beside the t_ext labels.
+    /* From here branches that share no written data run concurrently (side
+     * streams, graph branches when captured):
+     *   main   grain pass (:127,:203), vertex pass, t_ext labels
+     *   side0  boundary arclengths and energies (:124-130 / :171-181), which
+     *          the vertex pass reads; then dA/dt of the 3-sided grains beside
+     *          the t_ext labels
+     *   side1  beside the vertex pass: the first 2x3 count (:228), which
+     *          depends only on the topology that nothing changes before that
+     *          loop, from the 3-sided grains the grain pass listed; the
+     *          device-side decision whether this step computes every
+     *          output-only value
      * While profiling everything stays on the main stream, in order. */
     /* every boundary energy this step is 1 * 1 exactly (k_boundary_geometry) */
     const bool unit_gamma = o.GB_eps == 0.0 && o.GB_scaling == 1.0;
     if (h->profiling) {
         { Prof pr(h, "boundary_geometry"); launch_boundary_geometry(m, o.GB_eps, o.GB_scaling, h->p.shape, s); }
-        {
-            Prof pr(h, "grain_fd");
-            launch_grain_sort(m, x, s);
-            launch_grain_fd_wide(m, x, h->p.shape, s);
-            launch_grain_fd_sorted(m, x, h->p.shape, s);
-        }
+        { Prof pr(h, "grain_fd"); launch_grain_pass(m, x, h->p.shape, s); }
         { Prof pr(h, "two_three_count"); launch_two_three_first(m, x, x.list_b, x.n_b, s); }
         launch_full_flag(m, x, s);
         { Prof pr(h, "vertex_fd"); launch_vertex_fd(m, h->p.mu, unit_gamma, h->p.shape, s); }
@@ -527,22 +527,22 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
         cudaStreamWaitEvent(s0, ev[0], 0);
         launch_boundary_geometry(m, o.GB_eps, o.GB_scaling, h->p.shape, s0);          /* :124-130, :171-181 */
         cudaEventRecord(ev[1], s0);
-        launch_grain_sort(m, x, s);
+        launch_grain_pass(m, x, h->p.shape, s);                                        /* :127,:203 */
         cudaEventRecord(ev[2], s);
         cudaStreamWaitEvent(s1, ev[2], 0);
-        launch_grain_fd_wide(m, x, h->p.shape, s1);                                    /* :127,:203 */
         launch_two_three_first(m, x, x.list_b, x.n_b, s1);                             /* :228 */
         launch_full_flag(m, x, s1);
         cudaEventRecord(ev[3], s1);
-        launch_grain_fd_sorted(m, x, h->p.shape, s);                                   /* :127,:203 */
         cudaStreamWaitEvent(s, ev[1], 0);
-        cudaStreamWaitEvent(s, ev[3], 0);
         launch_vertex_fd(m, h->p.mu, unit_gamma, h->p.shape, s);                       /* :133,:203 */
+        cudaStreamWaitEvent(s, ev[3], 0);
         cudaEventRecord(ev[4], s);
         cudaStreamWaitEvent(s0, ev[4], 0);
         launch_grain_dadt(m, x, s0);                                                   /* :206 */
         cudaEventRecord(ev[5], s0);
+        sevc_pdl_skip = 1;       /* two predecessors */
         launch_text_label(m, x, o.dt, h->p.shape, s);                                  /* :212-216 */
+        sevc_pdl_skip = 0;
         launch_compact(m, x, CK_CAND, x.list_a, x.n_a, s);
         cudaStreamWaitEvent(s, ev[5], 0);
     }

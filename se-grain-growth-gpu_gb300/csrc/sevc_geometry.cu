@@ -15,7 +15,9 @@
  */
 #include "sevc_internal.h"
 
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 
 namespace {
 
@@ -45,198 +47,98 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
     if (j >= 0) m.contrib[3 * v + j] = make_double2(se * (dabs(Ax) - absA), se * (dabs(Ay) - absA));
 }
 
-/* Grain pass for a grain of N sides (compile-time), polygon in registers.
+/* ------------------------------------------------------------------ */
+/* grain pass                                                          */
+/* ------------------------------------------------------------------ */
+/* Every grain's area and the areas with each list vertex moved by +eps in
+ * x and in y (compute_area of the polygon with vertex p moved, src/
+ * geometry.h:757, :908), bit for bit.
  *
- * compute_area of the polygon with vertex p moved (src/geometry.h:757,
- * :908) differs from the unmoved one only from vertex p on: the unwrapped
- * coordinates of vertices 0..p-1 and the partial shoelace sum of terms
- * 0..p-2 are the same operations on the same values, so they are taken
- * from the unmoved pass; the moved component's unwrapped chain and the
- * terms from p-1 on are recomputed in the reference's order.  The other
- * component is unchanged (its dom_mod is the identity; if it is not, the
- * slot falls back to a full recomputation). */
-/* Area of the polygon with vertex p moved along component C (0 = x,
- * 1 = y).  R/A0/DD are the moved component's raw positions, unwrapped
- * coordinates and wrapped deltas, Ro/B0 the other component's. */
-__device__ __noinline__ double area_stream_slow(const int *__restrict__ L, int n, const double2 *__restrict__ pos,
-                                                int ps, double2 pp, double D)
+ * Certificate.  Let u be the ulp of a grain's smallest coordinate along an
+ * axis, Rmin.  When every coordinate lies in [Rmin, 1.75 Rmin] (and below
+ * Dlim, and no coordinate + eps leaves its binade), all coordinates are
+ * multiples of u, no wrap occurs, and every wrapped delta, unwrapped
+ * coordinate and moved coordinate the reference forms is a multiple of u
+ * below 2^53 u: each of those additions and subtractions is exact.  So the
+ * unwrapped coordinate of vertex k is R[k] - R[0] in one subtraction; the
+ * moved vertex's is A[p] + d_p and, for p = 0, every later one A[k] - d_0,
+ * where d_p = RN(R[p] + eps) - R[p] depends on R[p]'s exponent only (the
+ * multiple of ulp(R[p]) nearest to eps; eps is never halfway); and the moved
+ * chain is back on the unmoved values from p + 1 on.  Only the products,
+ * the shoelace terms and their running sum round, and those are formed in
+ * the reference's order.  On 1M grains (domain 1000) about 0.4% of the
+ * grains fail the certificate (next to an axis, where ulps are finer, or
+ * across the wrap); they are walked vertex by vertex as written.
+ *
+ * What bounds it: the FP64 pipe (2 thread-operations per clock and SM, of
+ * which independent chains reach 84%).  The certificate leaves 136 FP64
+ * operations per grain (234 when the chains are recomputed), and the
+ * integer pipe, otherwise idle, forms the exact differences.
+ *
+ * Layout.  A block takes GPB consecutive grains, orders them by falling
+ * side count in shared memory (no order over the whole mesh is needed), and
+ * works on chunks of 32 of them in loops over shared memory:
+ *   per slot            position and grain-slot loads;
+ *   per grain, axis     certificate;
+ *   per slot, axis      coordinates relative to vertex 0, and to vertex 0
+ *                       moved;
+ *   per slot, polygon   shoelace products and terms (the unmoved polygon
+ *                       and the two with vertex 0 moved);
+ *   per grain, polygon  running sum, area;
+ *   per slot, axis      the area with its vertex moved: the slots in falling
+ *                       number s = n - 2 - p of terms behind them (those of
+ *                       one s are a prefix of the order), so that the lanes
+ *                       of a warp run the same operations.
+ * Afterwards a warp per grain takes the rest, vertex by vertex: grains of
+ * `wide` or more sides or of fewer than 3, and the few whose moved chain
+ * does not rejoin.
+ *
+ * Measured (GB300): 1M grains 0.446 ms, FP64 pipe active 68-73% of the
+ * cycles, 23.5 of 32 lanes per FP64 instruction (slots of different s or p in
+ * one warp); 2,000 grains 25 us.  The form before it (a grain per thread,
+ * polygon in registers, one unrolled body per side count, side-count order
+ * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
+ * took 0.50 ms and 95 us: on a small mesh each unrolled body runs once and
+ * its instruction fetch is the time. */
+constexpr int GP_NMAX = 32;              /* side counts below this may take the ordered path (bits of AxisCert::up, lanes) */
+constexpr int GP_E0 = 1023 - 20, GP_E1 = 1023 + 20;   /* biased exponents of certified coordinates */
+
+/* significand of eps = 1e-8 = GP_EPS_M 2^(GP_EPS_E - 1075) */
+#define GP_EPS_M 0x15798ee2308c3aLL
+#define GP_EPS_E (1023 - 27)
+
+/* 1/n as a pair (hi, lo) for the division below; 4 and 8 are exact */
+#define INV_SPLIT(n) { InvSplit<n>::hi, InvSplit<n>::lo }
+__constant__ double2 c_inv_split[11] = { { 0, 0 }, { 0, 0 }, { 0, 0 }, INV_SPLIT(3), { 0.25, 0.0 }, INV_SPLIT(5),
+                                         INV_SPLIT(6), INV_SPLIT(7), { 0.125, 0.0 }, INV_SPLIT(9), INV_SPLIT(10) };
+
+/* x / n for a side count n: a multiplication and an fma where the bound of
+ * InvSplit holds, else the division */
+__device__ __forceinline__ double div_sides(double x, int n)
 {
-    return area_stream(L, n, pos, ps, pp, D);
+    unsigned long long b = mag2(x);
+    if (n >= 3 && n <= 10 && b >= (0x07B0000000000000ULL << 1) && b < (0x7830000000000000ULL << 1)) {
+        double2 z = c_inv_split[n];
+        return __fma_rn(x, z.x, __dmul_rn(x, z.y));
+    }
+    return ddiv_slow(x, (double)n);
 }
 
-/* shoelace term k of the moved component C: P = its unwrapped
- * coordinates k and k+1, B = the other component's */
-template <int C>
-__device__ __forceinline__ double moved_term(double pk, double bk, double pk1, double bk1)
+/* x - y for x, y >= 0, on the integer pipe when both lie in one binade and
+ * differ by less than 2^31 ulps (the difference is then exact: an integer
+ * below 2^31 times the ulp) */
+__device__ __forceinline__ double diff_near(double x, double y)
 {
-    return C == 0 ? pk * bk1 - bk * pk1 : bk * pk1 - pk * bk1;
-}
-
-/* Moving vertex p (0 < p < N-1) changes the unwrapped chain at p, then
- * at p+1 by the wrapped deltas into and out of the moved point.  When the
- * moved chain arrives at p+1 on the unmoved value (bit for bit: the two
- * deltas cancel exactly, which they do unless a wrap or a tiny coordinate
- * makes a difference inexact), every later coordinate is the same
- * operation on the same values as in the unmoved pass, so terms p+1.. are
- * the unmoved terms T[k] and only the running sum is redone.  Otherwise
- * the polygon is recomputed from memory. */
-template <int N, int C>
-__device__ __forceinline__ double moved_area_mid(const DevMesh &m, const int *__restrict__ L, int p, double moved,
-                                                 double other, const double (&R)[N], const double (&A0)[N],
-                                                 const double (&B0)[N], const double (&S)[N], const double (&T)[N])
-{
-    const double D = m.D;
-    double pp = p == 1 ? zero_plus(wrapd(moved, R[0], D)) : A0[p - 1] + wrapd(moved, R[p - 1], D);
-    double pn = pp + wrapd(R[p + 1], moved, D);
-    if (dbits(pn) != dbits(A0[p + 1])) {
-        double2 q = C == 0 ? make_double2(moved, other) : make_double2(other, moved);
-        return area_stream_slow(L, N, m.pos, p, q, D);
-    }
-    /* terms p-1 and p (the products that involve only unmoved
-     * coordinates are the unmoved pass's; the compiler shares them) */
-    double a = 0;
-    if (p >= 2) {
-        double t = moved_term<C>(A0[p - 1], B0[p - 1], pp, B0[p]);
-        a = p == 2 ? zero_plus(t) : S[p - 2] + t;
-    }
-    double t = moved_term<C>(pp, B0[p], A0[p + 1], B0[p + 1]);
-    a = p == 1 ? zero_plus(t) : a + t;
-#pragma unroll
-    for (int k = 2; k < N - 1; k++)
-        if (k > p) a = a + T[k];
-    a = C == 0 ? add_closing_term(a, A0[N - 1], B0[N - 1]) : add_closing_term(a, B0[N - 1], A0[N - 1]);
-    return dscale_down<1>(a);
-}
-
-template <int N, int C>
-__device__ __forceinline__ double moved_area(const DevMesh &m, const int *__restrict__ L, int p, const double (&R)[N],
-                                             const double (&Ro)[N], const double (&A0)[N], const double (&B0)[N],
-                                             const double (&DD)[N], const double (&S)[N], const double (&T)[N])
-{
-    const double D = m.D;
-    double moved = dmod(R[p] + SEVC_GRAD_EPS_D, D);
-    double other = dmod(Ro[p], D);
-    if (dbits(other) != dbits(Ro[p])) {
-        double2 pp = C == 0 ? make_double2(moved, other) : make_double2(other, moved);
-        return area_stream(L, N, m.pos, p, pp, D);
-    }
-    if (p > 0 && p < N - 1) return moved_area_mid<N, C>(m, L, p, moved, other, R, A0, B0, S, T);
-    double Pm[N];
-    Pm[0] = 0;
-#pragma unroll
-    for (int k = 1; k < N; k++) {
-        if (k < p) Pm[k] = A0[k];
-        else if (k == 1) Pm[k] = zero_plus(k == p ? wrapd(moved, R[0], D) : wrapd(R[1], moved, D));   /* +0 + w */
-        else if (k == p) Pm[k] = A0[k - 1] + wrapd(moved, R[k - 1], D);
-        else if (k == p + 1) Pm[k] = Pm[k - 1] + wrapd(R[k], moved, D);
-        else Pm[k] = Pm[k - 1] + DD[k];
-    }
-    double a = (p >= 2) ? S[p - 2] : 0.0;  /* S[0] = +0: term 0 never changes the sum */
-#pragma unroll
-    for (int k = 1; k < N - 1; k++) {
-        if (k < p - 1) continue;
-        double term = C == 0 ? Pm[k] * B0[k + 1] - B0[k] * Pm[k + 1] : B0[k] * Pm[k + 1] - Pm[k] * B0[k + 1];
-        a = (k == 1 && p <= 2) ? zero_plus(term) : a + term;   /* the sum is still +0 */
-    }
-    a = C == 0 ? add_closing_term(a, Pm[N - 1], B0[N - 1]) : add_closing_term(a, B0[N - 1], Pm[N - 1]);
-    return dscale_down<1>(a);
-}
-
-template <int N>
-__device__ __forceinline__ void grain_fd_fixed(const DevMesh &m, int g, const int *__restrict__ L)
-{
-    const double D = m.D;
-    int V[N];
-    double RX[N], RY[N], AX[N], AY[N], DX[N], DY[N], S[N], T[N];
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        V[k] = L[k];
-        double2 q = m.pos[V[k]];
-        RX[k] = q.x;
-        RY[k] = q.y;
-    }
-    AX[0] = 0; AY[0] = 0; DX[0] = 0; DY[0] = 0;
-#pragma unroll
-    for (int k = 1; k < N; k++) {
-        DX[k] = wrapd(RX[k], RX[k - 1], D);
-        DY[k] = wrapd(RY[k], RY[k - 1], D);
-        AX[k] = k == 1 ? zero_plus(DX[k]) : AX[k - 1] + DX[k];   /* AX[0] = +0 */
-        AY[k] = k == 1 ? zero_plus(DY[k]) : AY[k - 1] + DY[k];
-    }
-    double acc = 0;                    /* terms 0 and N-1 involve the origin */
-    S[0] = 0;
-    T[0] = 0;
-#pragma unroll
-    for (int k = 1; k < N - 1; k++) {
-        double term = AX[k] * AY[k + 1] - AY[k] * AX[k + 1];
-        T[k] = term;
-        acc = k == 1 ? zero_plus(term) : acc + term;
-        S[k] = acc;
-    }
-    T[N - 1] = 0;
-    acc = add_closing_term(acc, AX[N - 1], AY[N - 1]);
-    S[N - 1] = acc;
-    double A = dscale_down<1>(acc);
-    m.garea[g] = A;
-    double se = m.gse[g];
-    m.gq[g] = div_small<N>(se * A);
-    double absA = dabs(A);
-#pragma unroll
-    for (int p = 0; p < N; p++) {
-        double ax = moved_area<N, 0>(m, L, p, RX, RY, AX, AY, DX, S, T);
-        double ay = moved_area<N, 1>(m, L, p, RY, RX, AY, AX, DY, S, T);
-        put_contrib(m, g, V[p], se, absA, ax, ay);
-    }
-}
-
-/* Grain pass, any side count: each polygon streamed from memory. */
-__device__ __noinline__ void grain_fd_generic(const DevMesh &m, int g, const int *__restrict__ L, int n)
-{
-    double2 none = make_double2(0, 0);
-    double A = area_stream(L, n, m.pos, -1, none, m.D);
-    m.garea[g] = A;
-    double se = m.gse[g];
-    m.gq[g] = se * A / n;
-    double absA = dabs(A);
-    for (int p = 0; p < n; p++) {
-        int v = L[p];
-        double2 q = m.pos[v];
-        double2 px = make_double2(dmod(q.x + SEVC_GRAD_EPS_D, m.D), dmod(q.y, m.D));
-        double2 py = make_double2(dmod(q.x, m.D), dmod(q.y + SEVC_GRAD_EPS_D, m.D));
-        double Ax = area_stream(L, n, m.pos, p, px, m.D);
-        double Ay = area_stream(L, n, m.pos, p, py, m.D);
-        put_contrib(m, g, v, se, absA, Ax, Ay);
-    }
-}
-
-/* grain pass over the grains of fewer than `wide` sides (11 by default), ordered by
- * side count (warps see one N), most sides first so that the longest
- * blocks start in the first wave.  The pass is FP64 bound and waits on
- * FP64 results: OCC resident blocks of 128 per SM (4: 128 registers, 5:
- * 96, 6: 80, 8: 64) trades registers (and spills) for warps to hide that
- * latency; the launch-shape autotuner picks it (6 on the 1M-grain mesh).
- * Capping registers at 128 measured 9% faster than the compiler's
- * 218-register choice. */
-template <int OCC>
-__global__ void __launch_bounds__(128, OCC) k_grain_fd_sorted(DevMesh m, const int *perm, const int *vbucket, int wide)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int total = vbucket[VB_START(wide)];
-    if (i >= total) return;
-    int g = perm[total - 1 - i];
-    const int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    switch (n) {
-    case 3: grain_fd_fixed<3>(m, g, L); break;
-    case 4: grain_fd_fixed<4>(m, g, L); break;
-    case 5: grain_fd_fixed<5>(m, g, L); break;
-    case 6: grain_fd_fixed<6>(m, g, L); break;
-    case 7: grain_fd_fixed<7>(m, g, L); break;
-    case 8: grain_fd_fixed<8>(m, g, L); break;
-    case 9: grain_fd_fixed<9>(m, g, L); break;
-    case 10: grain_fd_fixed<10>(m, g, L); break;
-    default: grain_fd_generic(m, g, L, n); break;
-    }
+    long long bx = dbits(x), by = dbits(y), k = bx - by;
+    int E = (int)(by >> 52);
+    if ((int)(bx >> 52) != E || k != (long long)(int)k || E <= 64 || E >= 2047 || (int)k == INT_MIN)
+        return dsub_slow(x, y);
+    unsigned a = (unsigned)((int)k < 0 ? -(int)k : (int)k);
+    if (a == 0) return 0.0;
+    int lz = __clz((int)a);
+    unsigned mt = (a << lz) << 1;                      /* the bits below the leading one, left-aligned */
+    unsigned hi = ((unsigned)k & 0x80000000u) | ((unsigned)(E - 52 + 31 - lz) << 20) | (mt >> 12);
+    return __hiloint2double((int)hi, (int)(mt << 20));
 }
 
 /* area_stream over a polygon staged in shared memory (raw positions P[k]
@@ -259,87 +161,371 @@ __device__ __forceinline__ double area_shared(const double2 *P, int n, int ps, d
     return dscale_down<1>(area);
 }
 
-/* grain pass over the grains of `wide` or more sides (the tail of the
- * side-count order): one warp per grain, polygon staged in shared memory.
- * The 2n+1 areas of a grain (vertex p moved along x: task 2p, along y:
- * task 2p+1, unmoved: task 2n) are spread over the lanes, so a grain of
- * up to 15 sides costs one polygon walk per lane.  A thread per grain
- * would walk 2n+1 polygons of n dependent loads each and hold up the
- * whole pass. */
-constexpr int WIDE_WARPS = 4;
-__global__ void __launch_bounds__(32 * WIDE_WARPS) k_grain_fd_wide(DevMesh m, const int *perm, const int *vbucket,
-                                                                  const int *total, int wide)
+/* grain g by one warp, polygon staged in shared memory.  The 2n+1
+ * areas (vertex p moved along x: task 2p, along y: task 2p+1, unmoved:
+ * task 2n) are spread over the lanes, so a grain of up to 15 sides costs one
+ * polygon walk per lane. */
+__device__ __noinline__ void grain_by_warp(const DevMesh &m, int g, double2 *P, double *R, int lane)
 {
-    __shared__ double2 poly[WIDE_WARPS][SEVC_MAXV];
-    __shared__ double area[WIDE_WARPS][2 * SEVC_MAXV + 1];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double2 *P = poly[w];
-    double *R = area[w];
-    int first = vbucket[VB_START(wide)], end = *total;
-    int nwarps = gridDim.x * WIDE_WARPS;
     const double D = m.D;
-    for (int i = first + blockIdx.x * WIDE_WARPS + w; i < end; i += nwarps) {
-        int g = perm[i];
-        const int *L = m.glist + (size_t)SEVC_MAXV * g;
-        int n = m.gvlen[g];
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) P[k] = m.pos[L[k]];
-        __syncwarp();
-        for (int t = lane; t <= 2 * n; t += 32) {
-            int p = t >> 1;
-            double2 pp = make_double2(0, 0);
-            if (t < 2 * n) {
-                double2 q = P[p];
-                pp = (t & 1) ? make_double2(dmod(q.x, D), dmod(q.y + SEVC_GRAD_EPS_D, D))
-                             : make_double2(dmod(q.x + SEVC_GRAD_EPS_D, D), dmod(q.y, D));
-            } else {
-                p = -1;
-            }
-            R[t] = area_shared(P, n, p, pp, D);
+    const int *L = m.glist + (size_t)SEVC_MAXV * g;
+    int n = m.gvlen[g];
+    for (int k = lane; k < n; k += 32) P[k] = m.pos[L[k]];
+    __syncwarp();
+    for (int t = lane; t <= 2 * n; t += 32) {
+        int p = t >> 1;
+        double2 pp = make_double2(0, 0);
+        if (t < 2 * n) {
+            double2 q = P[p];
+            pp = (t & 1) ? make_double2(dmod(q.x, D), dmod(q.y + SEVC_GRAD_EPS_D, D))
+                         : make_double2(dmod(q.x + SEVC_GRAD_EPS_D, D), dmod(q.y, D));
+        } else {
+            p = -1;
         }
-        __syncwarp();
-        double A = R[2 * n];
-        double se = m.gse[g];
-        if (lane == 0) {
-            m.garea[g] = A;
-            m.gq[g] = se * A / n;
-        }
-        double absA = dabs(A);
-        for (int p = lane; p < n; p += 32) put_contrib(m, g, L[p], se, absA, R[2 * p], R[2 * p + 1]);
+        R[t] = area_shared(P, n, p, pp, D);
     }
+    __syncwarp();
+    double A = R[2 * n];
+    double se = m.gse[g];
+    if (lane == 0) {
+        m.garea[g] = A;
+        m.gq[g] = se * A / n;
+    }
+    double absA = dabs(A);
+    for (int p = lane; p < n; p += 32) put_contrib(m, g, L[p], se, absA, R[2 * p], R[2 * p + 1]);
+    __syncwarp();
 }
 
-/* counting sort of the enabled grains by side count (16 buckets, the last
- * one for 15 or more sides) */
-constexpr int NBUCKET = 16;
-/* Side-count histogram of the enabled grains into cnt[0..15]; the last
- * block to finish turns it into cursor[16..31] (bucket starts, advanced by
- * the scatter), start[32..47] and count[48..63] (kept for later passes
- * over one bucket) and leaves cnt[0..15] zero for the next step. */
-__global__ void k_vlen_hist(DevMesh m, int *cnt, int *cursor, int *total)
+/* one axis of a grain: the exponent of its smallest coordinate (index into
+ * the tables) and the mask of the vertices one binade above it */
+struct AxisCert { int e; unsigned up; };
+enum { GP_REST = 0, GP_CERT = 1, GP_CHAIN = 2 };
+
+constexpr int GP_CHUNK = 32, GP_SLOTS = 9 * GP_CHUNK;
+struct GrainChunk {
+    static constexpr int SLOTS = GP_SLOTS;
+    double R[2][SLOTS];                        /* raw coordinates; then the terms k of the polygons with vertex 0 moved */
+    double A[2][SLOTS];                        /* unwrapped coordinates */
+    double M[2][SLOTS];                        /* the same with vertex 0 moved along the axis; then M[0]: sum of T up to k */
+    double Q[2][SLOTS], T[SLOTS];              /* A[0][k] A[1][k+1], A[1][k] A[0][k+1], their difference */
+    int dest[SLOTS];                           /* 3 v + grain slot */
+    unsigned short moved[SLOTS], inner[SLOTS]; /* the slots in the order they are worked on */
+    unsigned char owner[SLOTS];
+    double se[GP_CHUNK], absA[GP_CHUNK], sum0[2][GP_CHUNK];   /* sum0: twice the areas with vertex 0 moved */
+    int sg[GP_CHUNK];
+    unsigned short off[GP_CHUNK];              /* first slot */
+    unsigned char n[GP_CHUNK];
+    int ok[2][GP_CHUNK];                       /* GP_* of each axis */
+    AxisCert c[2][GP_CHUNK];
+    __device__ int state(int i) const          /* certified, walked as a chain, or left to the rest */
+    {
+        int x = ok[0][i], y = ok[1][i];
+        return x && y ? (x > y ? x : y) : GP_REST;
+    }
+};
+struct GrainRest { double2 P[SEVC_MAXV]; double R[2 * SEVC_MAXV + 1]; };   /* one per warp */
+#define GRAIN_SMEM(NT) (sizeof(GrainChunk) > sizeof(GrainRest) * ((NT) / 32) ? sizeof(GrainChunk) : sizeof(GrainRest) * ((NT) / 32))
+/* a - b for positive binary64 patterns whose exponents are e or e + 1 and
+ * whose difference is a multiple of 2^(e - 1075) below 2^53 of them (hence
+ * exact), on the integer pipe */
+__device__ __forceinline__ double sub_exact(long long a, long long b, int e)
 {
-    __shared__ int h[NBUCKET];
-    if (threadIdx.x < NBUCKET) h[threadIdx.x] = 0;
-    __syncthreads();
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < m.ng && m.gen[g]) atomicAdd(&h[min(m.gvlen[g], NBUCKET - 1)], 1);
-    __syncthreads();
-    if (threadIdx.x < NBUCKET && h[threadIdx.x]) atomicAdd(&cnt[threadIdx.x], h[threadIdx.x]);
-    bool last = last_block(m.lastblk + 1);
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        int acc = 0;
-        for (int b = 0; b < NBUCKET; b++) {
-            int c = __ldcg(cnt + b);
-            cursor[b] = acc;
-            cnt[2 * NBUCKET + b] = acc;
-            cnt[3 * NBUCKET + b] = c;
-            acc += c;
-            cnt[b] = 0;
-        }
-        *total = acc;
+    const long long M = 0x000FFFFFFFFFFFFFLL, H = 1LL << 52;
+    long long ma = (a & M) | H, mb = (b & M) | H;
+    ma <<= (int)(a >> 52) - e;
+    mb <<= (int)(b >> 52) - e;
+    const long long d = ma - mb;
+    const unsigned long long u = (unsigned long long)(d < 0 ? -d : d);
+    const int sh = __clzll((long long)u) - 11;
+    const unsigned long long r = ((unsigned long long)(e - 1 - sh) << 52) + (u << sh);
+    return d == 0 ? 0.0 : __longlong_as_double((long long)(r | ((unsigned long long)d & 0x8000000000000000ULL)));
+}
+
+/* certificate of one axis over the raw coordinates r[0..n); that no
+ * coordinate + eps leaves its binade is checked slot by slot.  A grain
+ * with a coordinate outside [0, D) takes the rest's path. */
+__device__ __forceinline__ int certify_axis(const double *r, int n, double D, long long dlim, AxisCert &c)
+{
+    long long lo = dbits(r[0]), hi = lo;
+    for (int k = 1; k < n; k++) {
+        long long b = dbits(r[k]);
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+    }
+    int e = (int)(lo >> 52), e1 = (int)(hi >> 52);
+    c.e = e - GP_E0;
+    c.up = 0;
+    if (lo < 0 || hi >= dbits(D)) return GP_REST;
+    if (e < GP_E0 || e1 > GP_E1 || e1 > e + 1 || hi >= dlim) return GP_CHAIN;
+    long long ml = (lo & 0x000FFFFFFFFFFFFFLL) | (1LL << 52), mh = ((hi & 0x000FFFFFFFFFFFFFLL) | (1LL << 52)) << (e1 - e);
+    return mh - ml <= (ml >> 1) + (ml >> 2) ? GP_CERT : GP_CHAIN;
+}
+
+/* One axis of an uncertified grain: the unwrapped chain a of its raw
+ * coordinates r, and the chain u with vertex 0 moved, each addition as the
+ * reference makes it */
+__device__ __noinline__ void chain_axis(const double *r, double *a, double *u, int n, double D)
+{
+    double r0 = r[0], m0 = dmod(r0 + SEVC_GRAD_EPS_D, D), x = 0, y = 0, prev = r0;
+    a[0] = 0;
+    u[0] = 0;
+    for (int k = 1; k < n; k++) {
+        double rk = r[k], d = wrapd(rk, prev, D);
+        x = k == 1 ? zero_plus(d) : x + d;
+        y = k == 1 ? zero_plus(wrapd(rk, m0, D)) : y + d;
+        a[k] = x;
+        u[k] = y;
+        prev = rk;
     }
 }
+/* The unwrapped coordinate of the moved vertex p > 0 of an uncertified
+ * grain (raw coordinates: its own r, the neighbours' rm and rp; a the
+ * unwrapped chain).  NaN (no certified value is one) when the chain does
+ * not come back to the unmoved value at p + 1, bit for bit: the grain is
+ * then walked vertex by vertex. */
+__device__ __noinline__ double chain_moved(const double *a, int p, int n, double r, double rm, double rp, double D)
+{
+    double mv = dmod(r + SEVC_GRAD_EPS_D, D), w = wrapd(mv, rm, D);
+    double x = p == 1 ? zero_plus(w) : a[p - 1] + w;
+    if (p < n - 1 && dbits(x + wrapd(rp, mv, D)) != dbits(a[p + 1])) return __longlong_as_double(0x7FF8000000000000LL);
+    return x;
+}
+
+template <int GPB, int NT>
+__global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n_three, int wide, long long dlim)
+{
+    __shared__ __align__(16) unsigned char smem[GRAIN_SMEM(NT)];
+    GrainChunk &B = *reinterpret_cast<GrainChunk *>(smem);
+    __shared__ int order[GPB];                 /* the block's grains by falling side count */
+    __shared__ unsigned char sides[GPB];
+    __shared__ int cnt[GP_NMAX], start[GP_NMAX];
+    __shared__ int first[GP_NMAX];             /* first[j]: first entry of B.moved (and B.inner) with s + 2 = j */
+    __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved;
+    __shared__ long long ntab[GP_E1 - GP_E0 + 1];
+    __shared__ double dtab[GP_E1 - GP_E0 + 1];
+    constexpr int W = NT / 32;
+    static_assert(GPB <= NT, "a thread per grain orders them");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = blockIdx.x * GPB + tid;
+    bool on = tid < GPB && g < m.ng;
+    int n = 0, r = 0;
+    if (on) {
+        uint8_t en = m.gen[g];
+        n = m.gvlen[g];
+        on = en;
+    }
+    if (tid < GP_NMAX) cnt[tid] = 0;
+    if (tid == 0) nrest = 0;
+    for (int t = tid; t <= GP_E1 - GP_E0; t += NT) {
+        /* RN(eps / ulp) for coordinates of this exponent, and that multiple
+         * of the ulp as a double (below 2^46 ulps: exact) */
+        int d = t + GP_E0 - GP_EPS_E;
+        long long nk = (GP_EPS_M + (1LL << (d - 1))) >> d;
+        int lz = __clzll(nk) - 11;
+        ntab[t] = nk;
+        dtab[t] = __longlong_as_double(((long long)(t + GP_E0 - 1 - lz) << 52) + (nk << lz));
+    }
+    __syncthreads();
+    /* the block's grains by falling side count */
+    if (on) {
+        if (n == 3) three[atomicAdd(n_three, 1)] = g;
+        if (n < 3 || n >= wide || n >= GP_NMAX) {
+            rest[atomicAdd(&nrest, 1)] = g;
+            on = false;
+        } else {
+            r = atomicAdd(&cnt[n], 1);
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int k = GP_NMAX - 1 - lane, c = cnt[k];
+        int a = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(0xffffffffu, a, o);
+            if (lane >= o) a += y;
+        }
+        start[k] = a - c;                      /* grains of more than k sides */
+        if (k == 0) listed = a;
+    }
+    __syncthreads();
+    if (on) {
+        order[start[n] + r] = g;
+        sides[start[n] + r] = (unsigned char)n;
+    }
+    __syncthreads();
+    /* chunks of up to 32 grains (and GP_SLOTS slots) of the order */
+    for (int c0 = 0; c0 < listed; c0 += chunk) {
+    if (warp == 0) {
+        const int i = c0 + lane, k = i < listed ? sides[i] : 0;
+        int o = k;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            int y = __shfl_up_sync(0xffffffffu, o, d);
+            if (lane >= d) o += y;
+        }
+        const bool in = k > 0 && o <= GP_SLOTS;
+        const int c = __popc(__ballot_sync(0xffffffffu, in));
+        o -= k;
+        if (in) {
+            const int gi = order[i];
+            B.sg[lane] = gi;
+            B.n[lane] = (unsigned char)k;
+            B.off[lane] = (unsigned short)o;
+            for (int j = 0; j < k; j++) B.owner[o + j] = (unsigned char)lane;
+            if (lane == c - 1) { slots = o + k; chunk = c; }
+        }
+        /* class of s = q - 3: one slot of each grain of q or more sides */
+        const int q = GP_NMAX - 1 - lane;
+        int ge = (q > 0 ? start[q - 1] : listed) - c0;
+        ge = ge < 0 ? 0 : (ge < c ? ge : c);
+        int f = ge;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            int y = __shfl_up_sync(0xffffffffu, f, d);
+            if (lane >= d) f += y;
+        }
+        f -= ge;
+        if (q >= 1) first[q - 1] = f;          /* j = s + 2 = q - 1; q = 2, 1: p = n - 1 and p = 0, every grain */
+        else nmoved = f;
+    } else if (warp == W - 1) {
+        if (c0 + lane < listed) B.se[lane] = m.gse[order[c0 + lane]];
+    }
+    __syncthreads();
+    const int total = chunk;
+    /* per slot: position, where the vertex keeps this grain's terms, places
+     * in the work orders */
+#pragma unroll 2
+    for (int q = tid; q < slots; q += NT) {
+        const int i = B.owner[q], k = q - B.off[i], nn = B.n[i], gi = B.sg[i];
+        const int v = m.glist[(size_t)SEVC_MAXV * gi + k];
+        const double2 p = m.pos[v];
+        const int4 sv = m.vg[v];
+        B.moved[first[k == 0 ? 0 : nn - k] + i] = (unsigned short)q;
+        if (k > 0 && k < nn - 1) B.inner[first[k + 1] + i] = (unsigned short)q;
+        const int w = sv.x == gi ? 0 : (sv.y == gi ? 1 : (sv.z == gi ? 2 : -1));
+        B.R[0][q] = p.x;
+        B.R[1][q] = p.y;
+        B.dest[q] = w >= 0 ? 3 * v + w : -1;
+    }
+    __syncthreads();
+    /* per grain and axis: certificate */
+    for (int t = tid; t < 2 * total; t += NT) {
+        const int x = t >= total, i = x ? t - total : t;
+        B.ok[x][i] = certify_axis(B.R[x] + B.off[i], B.n[i], m.D, dlim, B.c[x][i]);
+    }
+    __syncthreads();
+    /* per slot and axis: coordinate relative to vertex 0, and to vertex 0
+     * moved; the first slot of an uncertified grain walks its chains */
+    for (int t = tid; t < 2 * slots; t += NT) {
+        const int x = t >= slots, q = x ? t - slots : t, i = B.owner[q], o = B.off[i], st = B.state(i);
+        if (B.dest[q] < 0) B.ok[0][i] = GP_REST;
+        if (st == GP_CERT) {
+            const int e = B.c[x][i].e;
+            const long long b = dbits(B.R[x][q]), b0 = dbits(B.R[x][o]);
+            const int u = (int)(b >> 52) - GP_E0;
+            if (((b + ntab[u]) ^ b) >> 52) B.ok[0][i] = GP_REST;
+            if (u != e) atomicOr(&B.c[x][i].up, 1u << (q - o));
+            B.A[x][q] = sub_exact(b, b0, e + GP_E0);
+            B.M[x][q] = sub_exact(b, b0 + ntab[(int)(b0 >> 52) - GP_E0], e + GP_E0);
+        } else if (st == GP_CHAIN && q == o) {
+            chain_axis(B.R[x] + o, B.A[x] + o, B.M[x] + o, B.n[i], m.D);
+        }
+    }
+    __syncthreads();
+    /* per slot 0 < k < n - 1 (by falling k, those of one k a prefix of the
+     * order) and polygon (unmoved, vertex 0 moved along x, along y): the
+     * shoelace products and their difference.  Along y the difference has
+     * the opposite sign: only magnitudes of moved areas are used. */
+    const int ninner = first[1];
+    for (int t = tid; t < 3 * ninner; t += NT) {
+        const int c = t >= 2 * ninner ? 2 : (t >= ninner ? 1 : 0), q = B.inner[t - c * ninner];
+        const double *F = c == 0 ? B.A[0] : B.M[c - 1], *G = c == 2 ? B.A[0] : B.A[1];
+        const double q1 = F[q] * G[q + 1], q2 = G[q] * F[q + 1], d = q1 - q2;
+        if (c == 0) {
+            B.Q[0][q] = q1;
+            B.Q[1][q] = q2;
+            B.T[q] = d;
+        } else {
+            B.R[c - 1][q] = d;
+        }
+    }
+    __syncthreads();
+    /* per grain and polygon: the running sum; of the unmoved one, the area.
+     * (Sums that only a magnitude is taken of leave out the reference's
+     * 0.0 + first term and its closing +-0: those change the sign of a zero
+     * at most.) */
+    for (int t = tid; t < 3 * total; t += NT) {
+        const int c = t >= 2 * total ? 2 : (t >= total ? 1 : 0), i = t - c * total, o = B.off[i], nn = B.n[i];
+        if (B.state(i) == GP_REST) {
+            if (c == 0) rest[atomicAdd(&nrest, 1)] = B.sg[i];
+            continue;
+        }
+        const double *Z = c == 0 ? B.T : B.R[c - 1];
+        double acc = zero_plus(Z[o + 1]);
+        if (c == 0) B.M[0][o + 1] = acc;
+        for (int k = 2; k < nn - 1; k++) {
+            acc = acc + Z[o + k];
+            if (c == 0) B.M[0][o + k] = acc;
+        }
+        if (c == 0) {
+            acc = add_closing_term(acc, B.A[0][o + nn - 1], B.A[1][o + nn - 1]);
+            const double A = dscale_down<1>(acc);
+            B.absA[i] = dabs(A);
+            m.garea[B.sg[i]] = A;
+            m.gq[B.sg[i]] = div_sides(B.se[i] * A, nn);
+        } else {
+            B.sum0[c - 1][i] = acc;
+        }
+    }
+    __syncthreads();
+    /* per slot and axis: the area with its vertex moved along the axis.  With
+     * F the moved axis and G the other one, the terms p - 1 and p are
+     * F[p-1] G[p] - G[p-1] f and f G[p+1] - G[p] F[p+1] for x, minus those
+     * for y; along y the whole sum is formed with the opposite sign. */
+    for (int t = tid; t < 2 * nmoved; t += NT) {
+        const int x = t >= nmoved, q = B.moved[x ? t - nmoved : t], i = B.owner[q], o = B.off[i], p = q - o, nn = B.n[i];
+        const int st = B.state(i);
+        if (st == GP_REST) continue;
+        double a;         /* twice the moved area */
+        if (p == 0) {
+            a = B.sum0[x][i];
+        } else {
+            const double *F = B.A[x], *G = B.A[1 - x];
+            double f;
+            if (st == GP_CERT) {
+                f = F[q] + dtab[B.c[x][i].e + ((B.c[x][i].up >> p) & 1)];
+            } else {
+                const double2 rr = m.pos[B.dest[q] / 3], rm = m.pos[B.dest[q - 1] / 3];
+                const double2 rp = m.pos[B.dest[p < nn - 1 ? q + 1 : q] / 3];
+                f = x ? chain_moved(F + o, p, nn, rr.y, rm.y, rp.y, m.D) : chain_moved(F + o, p, nn, rr.x, rm.x, rp.x, m.D);
+                if (dbits(f) == 0x7FF8000000000000LL) {
+                    if (atomicExch(&B.ok[0][i], GP_REST) != GP_REST) rest[atomicAdd(&nrest, 1)] = B.sg[i];
+                    continue;
+                }
+            }
+            const long long flip = x ? LLONG_MIN : 0;
+            auto sgn = [&](double v) { return __longlong_as_double(dbits(v) ^ flip); };
+            a = 0;
+            if (p >= 2) {
+                a = B.Q[x][q - 1] - G[q - 1] * f;                      /* term p - 1 */
+                if (p > 2) a = sgn(B.M[0][q - 2]) + a;
+            }
+            if (p < nn - 1) {
+                const double t2 = f * G[q + 1] - B.Q[1 - x][q];        /* term p */
+                a = p == 1 ? t2 : a + t2;
+                for (int k = q + 1; k < o + nn - 1; k++) a = a + sgn(B.T[k]);
+            }
+        }
+        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = B.se[i] * diff_near(dabs(dscale_down<1>(a)), B.absA[i]);
+    }
+    __syncthreads();
+    }
+    /* the rest, a warp per grain */
+    GrainRest &Z = reinterpret_cast<GrainRest *>(smem)[warp];
+    for (int q = warp; q < nrest; q += W) grain_by_warp(m, rest[q], Z.P, Z.R, lane);
+}
+constexpr int GRAIN_SMALL = 32 * 1024;   /* see launch_grain_pass */
 
 /* The step computes every output-only value (extinction times of all
  * boundaries, dA/dt of all grains) when it can export or is asked to
@@ -349,28 +535,13 @@ __global__ void k_vlen_hist(DevMesh m, int *cnt, int *cursor, int *total)
  * threshold is crossed once per run.  Else only what the step can observe
  * is computed.  flags[0] = the decision, taken on the device so that no
  * host round trip separates the step's first half from its second. */
-__global__ void k_full_flag(const int *n_two_three, const int *vbucket, int *flags, unsigned *stamp)
+__global__ void k_full_flag(const int *n_two_three, const int *n_three, int *flags, unsigned *stamp)
 {
-    int mg = flags[2], curr = flags[3], n3 = vbucket[3 * NBUCKET + 3];
+    int mg = flags[2], curr = flags[3], n3 = *n_three;
     long long reach = (long long)curr - n3 - 40LL * *n_two_three - 64;
     flags[0] = flags[1] || (mg > 0 && reach <= mg);
     *stamp += 1;   /* a new step: every value saved by the last step's events is stale */
 }
-__global__ void k_vlen_scatter(DevMesh m, int *cursor, int *perm)
-{
-    __shared__ int h[NBUCKET], base[NBUCKET];
-    if (threadIdx.x < NBUCKET) h[threadIdx.x] = 0;
-    __syncthreads();
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    int b = -1, r = 0;
-    if (g < m.ng && m.gen[g]) { b = min(m.gvlen[g], NBUCKET - 1); r = atomicAdd(&h[b], 1); }
-    __syncthreads();
-    if (threadIdx.x < NBUCKET) base[threadIdx.x] = h[threadIdx.x] ? atomicAdd(&cursor[threadIdx.x], h[threadIdx.x]) : 0;
-    __syncthreads();
-    if (b >= 0) perm[base[b] + r] = g;
-}
-
-
 /* vertex pass: src/calculus.h:19-73 (boundary part) and :143-154;
  * vertex_compute_energy src/geometry.h:472-479.
  *
@@ -435,17 +606,17 @@ __global__ void k_vertex_fd(DevMesh m, double mu)
  * src/geometry.h:779-787 streamed over the list */
 __device__ void dadt_of(const DevMesh &m, int g);
 
-/* every enabled grain when flags[0], else the 3-sided ones (bucket 3 of
- * the side-count order) */
-__global__ void k_grain_dadt(DevMesh m, const int *perm, const int *vbucket, const int *flags)
+/* every enabled grain when flags[0], else the 3-sided ones (listed by the
+ * grain pass) */
+__global__ void k_grain_dadt(DevMesh m, const int *three, const int *n_three, const int *flags)
 {
     int stride = gridDim.x * blockDim.x;
     if (flags[0]) {
         for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < m.ng; g += stride)
             if (m.gen[g]) dadt_of(m, g);
     } else {
-        int n3 = vbucket[3 * NBUCKET + 3], start = vbucket[2 * NBUCKET + 3];
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += stride) dadt_of(m, perm[start + i]);
+        const int n3 = *n_three;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += stride) dadt_of(m, three[i]);
     }
 }
 
@@ -568,7 +739,7 @@ __global__ void k_text_label(DevMesh m, double dt, float Df, float hDf, float in
 /* The step's summary in one buffer; each per-step record it packs (event
  * counts, error bits, polling iterations and convergence, 2x3 pass counts)
  * is zeroed once read, and so are the exactness marks of the grains' dA/dt
- * and the polling iteration total, so the next step starts from zeros
+ * and the polling iteration total and the list of 3-sided grains, so the next step starts from zeros
  * without resets of its own (the reset each step would otherwise begin
  * with: src/main.cu's per-step clears of these values). */
 __global__ void k_pack_summary(DevMesh m, DevScratch x, int ninst, int *out)
@@ -586,7 +757,7 @@ __global__ void k_pack_summary(DevMesh m, DevScratch x, int ninst, int *out)
         else if ((k -= ne) < 4) { v = m.err[k]; m.err[k] = 0; }
         else if ((k -= 4) < np) { v = x.piters[k]; x.piters[k] = 0; m.pdone[k] = 0; }
         else if ((k -= np) < ns) { v = x.segcnt[k]; x.segcnt[k] = 0; }
-        else { v = x.flags[0]; *x.ptot = 0; }
+        else { v = x.flags[0]; *x.ptot = 0; *x.n_three = 0; }
         out[i] = v;
     }
     const size_t nw = (size_t)m.ng / 16;                   /* gexact as 16-byte words (256-byte aligned array) */
@@ -636,7 +807,7 @@ __global__ void k_count_grains(DevMesh m, int *counters)
  * reference's grid (blockIdx.y = instance) so that the floating-point sum
  * order is the same: per-thread strided partial sums over the instance's
  * grain indices, then the shared-memory tree. */
-__global__ void k_nucl_area_blocks(DevMesh m, double *block_out)
+__global__ void k_nucl_area_blocks(DevMesh m, double *block_out, int *counters)
 {
     __shared__ double t[256];
     int inst = blockIdx.y;
@@ -659,17 +830,18 @@ __global__ void k_nucl_area_blocks(DevMesh m, double *block_out)
         __syncthreads();
     }
     if (threadIdx.x == 0) block_out[(size_t)inst * gridDim.x + blockIdx.x] = t[0];
-}
-
-/* host loop of nucleated_fraction_area, src/calculus.h:373-377, one
- * thread per instance */
-__global__ void k_nucl_area_final(const double *block_out, int nblocks, int ninst, double D, int *counters)
-{
-    int inst = blockIdx.x * blockDim.x + threadIdx.x;
-    if (inst >= ninst) return;
-    double s = 0.0;
-    for (int i = 0; i < nblocks; i++) s += block_out[(size_t)inst * nblocks + i];
-    *reinterpret_cast<double *>(counters + (size_t)inst * CTR_COUNT + CTR_NUCL_AREA_SLOT) = 100 * s / (D * D);
+    /* host loop of nucleated_fraction_area, src/calculus.h:373-377: the last
+     * block, one thread per instance */
+    const bool last = last_block(m.lastblk + 1);
+    if (last) {
+        __threadfence();
+        const int nblocks = gridDim.x;
+        for (int i = threadIdx.x; i < m.ninst; i += blockDim.x) {
+            double s = 0.0;
+            for (int b = 0; b < nblocks; b++) s += __ldcg(block_out + (size_t)i * nblocks + b);
+            *reinterpret_cast<double *>(counters + (size_t)i * CTR_COUNT + CTR_NUCL_AREA_SLOT) = 100 * s / (m.D * m.D);
+        }
+    }
 }
 
 } // namespace
@@ -679,25 +851,25 @@ void launch_boundary_geometry(const DevMesh &m, double eps, double scaling, cons
     int t = sh.tpb_boundary;
     COUNT_LAUNCHES(1), k_boundary_geometry<<<(m.nb + t - 1) / t, t, 0, s>>>(m, eps, scaling);
 }
-void launch_grain_sort(const DevMesh &m, const DevScratch &x, cudaStream_t s)
+void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s)
 {
-    COUNT_LAUNCHES(1), k_vlen_hist<<<nblk(m.ng), TPB, 0, s>>>(m, x.vbucket, x.vbucket + NBUCKET, x.n_perm);
-    COUNT_LAUNCHES(1), k_vlen_scatter<<<nblk(m.ng), TPB, 0, s>>>(m, x.vbucket + NBUCKET, x.perm);
-}
-void launch_grain_fd_wide(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s)
-{
-    /* one warp per grain, grid-stride: enough warps that each takes only a
-     * few of the widest grains (their areas are chains of dependent FP64
-     * operations, so warps in flight hide the latency) */
-    COUNT_LAUNCHES(1), k_grain_fd_wide<<<8 * 152, 32 * WIDE_WARPS, 0, s>>>(m, x.perm, x.vbucket, x.n_perm, sh.wide_sides);
-}
-void launch_grain_fd_sorted(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s)
-{
-    int g = (m.ng + 127) / 128;
-    if (sh.grain_occ >= 8) COUNT_LAUNCHES(1), k_grain_fd_sorted<8><<<g, 128, 0, s>>>(m, x.perm, x.vbucket, sh.wide_sides);
-    else if (sh.grain_occ >= 6) COUNT_LAUNCHES(1), k_grain_fd_sorted<6><<<g, 128, 0, s>>>(m, x.perm, x.vbucket, sh.wide_sides);
-    else if (sh.grain_occ == 5) COUNT_LAUNCHES(1), k_grain_fd_sorted<5><<<g, 128, 0, s>>>(m, x.perm, x.vbucket, sh.wide_sides);
-    else COUNT_LAUNCHES(1), k_grain_fd_sorted<4><<<g, 128, 0, s>>>(m, x.perm, x.vbucket, sh.wide_sides);
+    /* coordinates from here on take the general path (adding eps could
+     * reach D): a margin of 1e-7, or of a few ulps of a large D */
+    double lim = m.D - std::max(1e-7, m.D * 0x1p-50);
+    long long dlim;
+    memcpy(&dlim, &lim, sizeof dlim);
+    const int wide = sh.wide_sides >= 12 ? GP_NMAX : sh.wide_sides;
+    auto go = [&](auto kernel, int gpb, int nt) {
+        COUNT_LAUNCHES(1), kernel<<<(m.ng + gpb - 1) / gpb, nt, 0, s>>>(m, x.three, x.n_three, wide, dlim);
+    };
+    /* 32 grains a block at every size (blocks of 64 in two chunks measured
+     * the same at 1M grains and 10% more at 100K; they stay for the
+     * autotuner).  Below GRAIN_SMALL grains an SM holds few blocks, and
+     * eight warps shorten each one's phases: 3-11 us less per step at 2K-20K
+     * grains than four; from 50K on four are as fast. */
+    if (sh.grain_occ < 6) go(k_grain_pass<64, 128>, 64, 128);
+    else if (m.ng < GRAIN_SMALL) go(k_grain_pass<32, 256>, 32, 256);
+    else go(k_grain_pass<32, 128>, 32, 128);
 }
 
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s)
@@ -708,12 +880,12 @@ void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const Launch
 }
 void launch_full_flag(const DevMesh &m, const DevScratch &x, cudaStream_t s)
 {
-    COUNT_LAUNCHES(1), k_full_flag<<<1, 1, 0, s>>>(x.n_b, x.vbucket, x.flags, m.stamp);
+    COUNT_LAUNCHES(1), k_full_flag<<<1, 1, 0, s>>>(x.n_b, x.n_three, x.flags, m.stamp);
 }
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s)
 {
     int g = nblk(m.ng);   /* grid-stride: every grain, or only the 3-sided ones, decided on the device */
-    COUNT_LAUNCHES(1), k_grain_dadt<<<g < 8 * 152 ? g : 8 * 152, TPB, 0, s>>>(m, x.perm, x.vbucket, x.flags);
+    COUNT_LAUNCHES(1), k_grain_dadt<<<g < 8 * 152 ? g : 8 * 152, TPB, 0, s>>>(m, x.three, x.n_three, x.flags);
 }
 void launch_text_label(const DevMesh &m, const DevScratch &x, double dt, const LaunchShape &sh, cudaStream_t s)
 {
@@ -743,7 +915,5 @@ void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, c
     if (gx > 4096) gx = 4096;
     if (gx < 1) gx = 1;
     COUNT_LAUNCHES(1), k_count_grains<<<dim3(gx, p.ninst), TPB, 0, s>>>(m, x.counters);
-    COUNT_LAUNCHES(1), k_nucl_area_blocks<<<dim3(p.n_blocks, p.ninst), p.n_threads, 0, s>>>(m, x.block_area);
-    COUNT_LAUNCHES(1), k_nucl_area_final<<<(p.ninst + 127) / 128, 128, 0, s>>>(x.block_area, p.n_blocks, p.ninst, m.D,
-                                                                              x.counters);
+    COUNT_LAUNCHES(1), k_nucl_area_blocks<<<dim3(p.n_blocks, p.ninst), p.n_threads, 0, s>>>(m, x.block_area, x.counters);
 }

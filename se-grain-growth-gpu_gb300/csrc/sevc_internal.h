@@ -27,10 +27,10 @@ struct DevScratch {
     curandState *rng, *rng_saved;    /* 8192 cuRAND states + pre-attempt copy, per instance */
     int *nucl_buf;                   /* 96 ints per instance: per-block pick, alive count, pick's rank */
     int *nucl_on;                    /* per instance: attempt a nucleation this step */
-    int *vbucket;                    /* 64 ints: side-count histogram + cursors */
+    int *reserved64;                 /* 64 ints no kernel uses: keeps the block's layout (checkpoint files) */
     int *flags;                      /* 4 ints: the step's output decision, see launch_full_flag */
     int *summary;                    /* the step's summary packed for one readback */
-    int *perm, *n_perm;              /* enabled grains ordered by side count */
+    int *three, *n_three;            /* the enabled 3-sided grains, listed by the grain pass (any order) */
     unsigned long long *digest;      /* SEVC_DIGEST_FIELDS sums of sevc_state_digest */
     /* events applied in parallel (removals, flips): reservation keys of
      * every vertex and boundary, the events of the phase (list positions),
@@ -65,8 +65,8 @@ enum {
 struct LaunchShape {
     int tpb_vertex = 128;    /* threads per block of the vertex pass */
     int tpb_boundary = 128;  /* of the per-boundary passes (geometry, t_ext) */
-    int wide_sides = 11;     /* grains of this many sides or more get a warp each */
-    int grain_occ = 6;       /* resident blocks per SM of the thread-per-grain grain pass (4, 5, 6, 8) */
+    int wide_sides = 12;     /* 9..11: grains of this many sides or more get a warp each; 12: of 32 or more */
+    int grain_occ = 6;       /* grains per block of the grain pass: 64 below 6, else 32 (4, 5, 6, 8) */
 };
 
 struct StepParams {
@@ -80,17 +80,10 @@ struct StepParams {
 
 /* geometry (sevc_geometry.cu) */
 void launch_boundary_geometry(const DevMesh &m, double eps, double scaling, const LaunchShape &sh, cudaStream_t s);
-/* grain pass: side-count order (x.perm / x.vbucket), then the warp-per-grain
- * kernel for grains of wide_sides or more and the thread-per-grain kernel
- * for the rest (disjoint grains: the two may run concurrently) */
-void launch_grain_sort(const DevMesh &m, const DevScratch &x, cudaStream_t s);
-void launch_grain_fd_wide(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s);
-void launch_grain_fd_sorted(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s);
+/* grain pass: areas, moved areas, and the list of 3-sided grains */
+void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s);
 /* unit_gamma: every boundary energy is exactly 1 (GB_eps = 0, GB_scaling = 1) */
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s);
-/* side-count histogram layout in DevScratch::vbucket */
-#define VB_START(b) (32 + (b))
-#define VB_COUNT(b) (48 + (b))
 /* x.flags: [0] computed "full" decision, [1] host part of it, [2]
  * min_grains, [3] current grain count (see k_full_flag); also advances
  * the step stamp of the events' save-on-write (m.stamp) */
@@ -105,7 +98,7 @@ void launch_pack_summary(const DevMesh &m, const DevScratch &x, int ninst, int *
 /* topology (sevc_topology.cu) */
 enum CompactKind { CK_CAND = 0, CK_TWO_THREE = 1, CK_GRAIN_CAND = 2, CK_GVLEN3 = 3, CK_MARKED = 4 };
 void launch_compact(const DevMesh &m, const DevScratch &x, CompactKind kind, int *out, int *n_out, cudaStream_t s);
-/* the CK_TWO_THREE list from the 3-sided bucket of this step's grain pass */
+/* the CK_TWO_THREE list from the 3-sided grains of this step's grain pass */
 void launch_two_three_first(const DevMesh &m, const DevScratch &x, int *out, int *n_out, cudaStream_t s);
 /* one polling iteration for every instance not yet converged; leaves the
  * number still running in x.nrun */
@@ -129,8 +122,8 @@ void launch_tt_cond(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStr
 /* the 3-sided labels, bucket or full as x.tt_first says (no 2x3 removal:
  * the bucket) */
 void launch_label_3sided_auto(const DevMesh &m, const DevScratch &x, double dt, cudaStream_t s);
-/* bucket: no grain list changed since this step's side-count order, so
- * only its 3-sided bucket is visited */
+/* bucket: no grain list changed since this step's grain pass, so only the
+ * 3-sided grains it listed are visited */
 void launch_label_3sided(const DevMesh &m, const DevScratch &x, double dt, bool bucket, cudaStream_t s);
 void launch_remove_grains(const DevMesh &m, const DevScratch &x, const int *list, const int *n, cudaStream_t s);
 /* clears the candidate flag of every listed grain (after the removals) */

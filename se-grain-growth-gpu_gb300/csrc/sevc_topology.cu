@@ -533,14 +533,14 @@ __device__ bool two_three_qualifies(const DevMesh &m, int b, int *gic)
 
 /* The step's first 2x3 count: a qualifying boundary lies on two 3-sided
  * grains, so only the boundaries at the vertices of the 3-sided grains
- * (bucket 3 of this step's side-count order) are tested; the ordered
+ * (listed by this step's grain pass) are tested; the ordered
  * compaction of the marks then gives the same ascending list as testing
  * every boundary. */
-__global__ void k_mark_two_three(DevMesh m, const int *perm, const int *vbucket)
+__global__ void k_mark_two_three(DevMesh m, const int *three, const int *n_three)
 {
-    int n3 = vbucket[VB_COUNT(3)], start = vbucket[VB_START(3)];
+    const int n3 = *n_three;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        const int *L = m.glist + (size_t)SEVC_MAXV * perm[start + i];
+        const int *L = m.glist + (size_t)SEVC_MAXV * three[i];
         for (int k = 0; k < 3; k++) {
             int4 s = m.vb[L[k]];
             for (int j = 0; j < 3; j++) {
@@ -655,28 +655,28 @@ __global__ void k_label_3sided(DevMesh m, double dt)
     if (g >= m.ng || !m.gen[g]) return;
     m.gcand[g] = m.gvlen[g] == 3 ? label3_cand(m, g, dt) : 0;
 }
-/* The same when no list changed since this step's side-count order: only
- * the grains of its 3-sided bucket are visited.  Every other enabled grain
+/* The same when no list changed since this step's grain pass: only the
+ * 3-sided grains it listed are visited.  Every other enabled grain
  * already has gcand = 0, because each step clears the flag of every grain
  * it listed as a candidate (k_remove_reserve). */
-__global__ void k_label_3sided_bucket(DevMesh m, double dt, const int *perm, const int *vbucket)
+__global__ void k_label_3sided_bucket(DevMesh m, double dt, const int *three, const int *n_three)
 {
     griddep_wait();
-    int n3 = vbucket[VB_COUNT(3)], start = vbucket[VB_START(3)];
+    const int n3 = *n_three;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        int g = perm[start + i];
+        int g = three[i];
         m.gcand[g] = label3_cand(m, g, dt);
     }
 }
 /* either of the two above, as the step's first 2x3 count says: no 2x3
- * removal (count 0) leaves every list as the side-count order saw it */
-__global__ void k_label_3sided_auto(DevMesh m, double dt, const int *perm, const int *vbucket, const int *tt_first)
+ * removal (count 0) leaves every list as the grain pass saw it */
+__global__ void k_label_3sided_auto(DevMesh m, double dt, const int *three, const int *n_three, const int *tt_first)
 {
     griddep_wait();
     if (*tt_first == 0) {
-        int n3 = vbucket[VB_COUNT(3)], start = vbucket[VB_START(3)];
+        const int n3 = *n_three;
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-            int g = perm[start + i];
+            int g = three[i];
             m.gcand[g] = label3_cand(m, g, dt);
         }
     } else {
@@ -1572,7 +1572,7 @@ void launch_two_three_first(const DevMesh &m, const DevScratch &x, int *out, int
 {
     cudaMemsetAsync(m.bmark, 0, (size_t)m.nb, s);
     int g = (m.ng + TPB - 1) / TPB;
-    COUNT_LAUNCHES(1), k_mark_two_three<<<g < 4 * WL_BLOCKS ? g : 4 * WL_BLOCKS, TPB, 0, s>>>(m, x.perm, x.vbucket);
+    COUNT_LAUNCHES(1), k_mark_two_three<<<g < 4 * WL_BLOCKS ? g : 4 * WL_BLOCKS, TPB, 0, s>>>(m, x.three, x.n_three);
     compact_impl<CK_MARKED>(m, x, m.nb, out, n_out, s);
 }
 
@@ -1629,14 +1629,14 @@ void launch_tt_cond(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStr
 void launch_label_3sided_auto(const DevMesh &m, const DevScratch &x, double dt, cudaStream_t s)
 {
     int g = (m.ng + TPB - 1) / TPB;
-    launch_dep(k_label_3sided_auto, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.perm, x.vbucket, x.tt_first);
+    launch_dep(k_label_3sided_auto, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.three, x.n_three, x.tt_first);
 }
 
 void launch_label_3sided(const DevMesh &m, const DevScratch &x, double dt, bool bucket, cudaStream_t s)
 {
     if (bucket) {
         int g = (m.ng + TPB - 1) / TPB;
-        launch_dep(k_label_3sided_bucket, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.perm, x.vbucket);
+        launch_dep(k_label_3sided_bucket, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.three, x.n_three);
     } else {
         launch_dep(k_label_3sided, (m.ng + TPB - 1) / TPB, TPB, s, m, dt);
     }
