@@ -323,12 +323,11 @@ sevc_status sevc_set_exact_all(sevc_handle *h, int on);
 sevc_status sevc_set_limits(sevc_handle *h, int polling_cap, int worklist_cap);
 
 /* Launch mode.  on = 1 (the default): a step is one CUDA graph, captured
- * on first use and replayed, whose polling and 2x3 loops are conditional
- * nodes driven from the device; on = 2: the step's fixed launch sequences
- * (its first half, one polling iteration, the second half of a step
- * without 2x3 pairs) are graphs and the loops run on the host; on = 0
- * launches every kernel directly.  Results are identical in every mode.
- * Profiling and adjoint replays always launch directly. */
+ * on first use and replayed; on = 2 is accepted and means the same (its
+ * polling and 2x3 loops used to run on the host; they are loops inside a
+ * kernel in every mode now); on = 0 launches every kernel directly.
+ * Results are identical in every mode.  Profiling and the steps an adjoint
+ * replay records inside always launch directly. */
 sevc_status sevc_set_graphs(sevc_handle *h, int on);
 
 /* Launch-shape autotuner (no counterpart in the reference): times `steps`

@@ -29,7 +29,7 @@ CFLAGS = ["-O2", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-fopenmp", "-W
 CU = ["sevc_geometry.cu", "sevc_topology.cu", "sevc_nucleation.cu", "sevc_adjoint.cu", "sevc_check.cu",
       "sevc_engine.cu"]
 C = ["sevc_host.c", "sevc_voronoi.c"]
-HDRS = ["sevc_device.cuh", "sevc_internal.h", "sevc_host.h"]
+HDRS = ["sevc_device.cuh", "sevc_internal.h", "sevc_tail.cuh", "sevc_host.h"]
 
 
 def _stale(out, deps):

@@ -51,7 +51,6 @@ struct DevMesh {
     uint8_t *ven;
     int4 *vb, *vg;
     int4 *vmod;          /* 4 per vertex */
-    int *voted;
     uint8_t *vmodmark;
     /* boundaries */
     int2 *bv;
@@ -61,7 +60,7 @@ struct DevMesh {
     /* grains */
     int *glist, *gvlen;
     double *garea, *gdadt, *gori, *gse, *gq;
-    uint8_t *gen, *gcand, *gfix, *gtype;
+    uint8_t *gen, *gfix, *gtype;
     /* worklists of the grain-list fix-up (src/topological.h:1209); the
      * capacities are the array sizes unless sevc_set_limits lowers them */
     int *fixlist, *nfix;
@@ -99,7 +98,6 @@ struct DevMesh {
     int2 *bv0;
     unsigned *vstamp, *bstamp, *stamp;
     uint8_t *bexact, *gexact;
-    uint8_t *bmark;      /* boundaries marked by a sparse pass, compacted next */
     int *lastblk;        /* arrival counters of last_block, zero between launches */
 };
 

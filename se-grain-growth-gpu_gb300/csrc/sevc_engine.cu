@@ -28,7 +28,6 @@
 #include <vector>
 
 long long sevc_kernel_launches = 0;
-thread_local bool sevc_pdl_off = false;
 thread_local int sevc_pdl_skip = 0;
 
 struct ProfEntry { double ms = 0; int64_t launches = 0; };
@@ -96,15 +95,8 @@ struct sevc_handle {
     int *h_flags = nullptr;/* host part of the step's output decision (x.flags) */
     size_t dbytes = 0;     /* size of the device block */
     Tape tape;
-    /* CUDA graphs of the step's fixed launch sequences: the first half
-     * without / with a nucleation attempt, one polling iteration, and the
-     * second half of a step without 2x3 pairs */
-    StepGraph g_pre[2], g_poll, g_post;
-    /* the whole step as one graph (without / with a nucleation attempt):
-     * the polling and 2x3 loops are conditional WHILE nodes driven by the
-     * device, so a step is one graph launch and one readback */
+    /* a step without / with a nucleation attempt as one CUDA graph */
     StepGraph g_step[2];
-    bool device_loops = true;
     bool use_graphs = true;
     bool force_direct = false;   /* this step launches directly (an adjoint replay records inside it) */
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -120,7 +112,7 @@ struct sevc_handle {
     /* side streams of the step (branches that do not depend on each other
      * run concurrently; captured as graph branches) and the fork / join
      * events between them: 0-5 in the first half, 6-7 in the tail */
-    cudaStream_t side[3] = { nullptr, nullptr, nullptr };   /* [2]: capture of loop bodies */
+    cudaStream_t side[2] = { nullptr, nullptr };
     cudaEvent_t evfork[10] = {};
     bool profiling = false;
     std::map<std::string, ProfEntry> prof;
@@ -201,29 +193,29 @@ bool alloc_device(sevc_handle *h)
         { (void **)&m.contrib, V * 48 }, { (void **)&m.venergy, V * 8 }, { (void **)&m.ven, V },
         { (void **)&m.vspd, V * 4 },
         { (void **)&m.vb, V * 16 }, { (void **)&m.vg, V * 16 }, { (void **)&m.vmod, V * 64 },
-        { (void **)&m.voted, V * 4 }, { (void **)&m.vmodmark, V }, { (void **)&m.modlist, V * 4 },
+        { &x.reserved, V * 4 }, { (void **)&m.vmodmark, V }, { (void **)&m.modlist, V * 4 },
         { (void **)&m.bv, B * 8 }, { (void **)&m.benergy, B * 8 }, { (void **)&m.blen, B * 8 },
         { (void **)&m.btext, B * 8 }, { (void **)&m.ben, B }, { (void **)&m.bcand, B },
         { (void **)&m.bcandbuf, B }, { (void **)&m.bvotes, B * 4 }, { (void **)&m.bconf, B * 4 },
         { (void **)&m.glist, G * SEVC_MAXV * 4 }, { (void **)&m.gvlen, G * 4 }, { (void **)&m.garea, G * 8 },
         { (void **)&m.gdadt, G * 8 }, { (void **)&m.gori, G * 8 }, { (void **)&m.gse, G * 8 },
-        { (void **)&m.gq, G * 8 }, { (void **)&m.gen, G }, { (void **)&m.gcand, G }, { (void **)&m.gfix, G },
+        { (void **)&m.gq, G * 8 }, { (void **)&m.gen, G }, { &x.reserved, G }, { (void **)&m.gfix, G },
         { (void **)&m.gtype, G }, { (void **)&m.fixlist, G * 4 }, { (void **)&m.nfix, 4 }, { (void **)&m.nmod, 4 },
         { (void **)&m.err, 16 }, { (void **)&m.evt, I * EVT_COUNT * 4 },
         { (void **)&x.list_a, maxn * 4 }, { (void **)&x.list_b, maxn * 4 }, { (void **)&x.list_c, maxn * 4 },
-        { (void **)&x.n_a, 4 }, { (void **)&x.n_b, 4 }, { (void **)&x.n_c, 4 }, { (void **)&x.blockcnt, tiles * 4 },
+        { (void **)&x.n_a, 4 }, { (void **)&x.n_b, 4 }, { (void **)&x.n_c, 4 }, { &x.reserved, tiles * 4 },
         { (void **)&x.extra, I * EXTRA_CAP * 4 }, { (void **)&x.threadfail, I * grid * 4 },
         { (void **)&x.block_area, I * h->p.n_blocks * 8 }, { (void **)&x.counters, I * CTR_COUNT * 4 },
         { (void **)&x.rng, nrng * sizeof(curandState) }, { (void **)&x.rng_saved, nrng * sizeof(curandState) },
-        { (void **)&x.nucl_buf, I * 96 * 4 }, { (void **)&x.reserved64, 64 * 4 }, { (void **)&x.three, G * 4 },
+        { (void **)&x.nucl_buf, I * 96 * 4 }, { &x.reserved, 64 * 4 }, { (void **)&x.three, G * 4 },
         { (void **)&x.n_three, 4 }, { (void **)&m.nlist, G * 4 }, { (void **)&m.nnlist, I * 4 }, { (void **)&m.pos0, V * 16 },
         { (void **)&m.vel0, V * 16 }, { (void **)&m.bv0, B * 8 }, { (void **)&m.vstamp, V * 4 },
         { (void **)&m.bstamp, B * 4 }, { (void **)&m.stamp, 4 }, { (void **)&m.bexact, B }, { (void **)&m.gexact, G },
-        { (void **)&m.bmark, B }, { (void **)&m.lastblk, 8 * 4 },
+        { &x.reserved, B }, { (void **)&m.lastblk, 8 * 4 },
         { (void **)&x.digest, SEVC_DIGEST_FIELDS * 8 },
         { (void **)&x.vown, V * 8 }, { (void **)&x.bown, B * 8 }, { (void **)&x.ehits, maxn * 4 },
-        { (void **)&x.n_ehits, 4 }, { (void **)&x.edefer, maxn }, { (void **)&x.ndefer, I * 4 },
-        { (void **)&x.ptot, 4 }, { (void **)&x.tt_first, 4 }, { (void **)&x.tt_pass, 4 },
+        { (void **)&x.n_ehits, 4 }, { &x.reserved, maxn }, { &x.reserved, I * 4 },
+        { &x.reserved, 4 }, { &x.reserved, 4 }, { &x.reserved, 4 },
     };
     size_t total = 0;
     for (auto &q : r) total += align256(q.bytes);
@@ -233,10 +225,7 @@ bool alloc_device(sevc_handle *h)
     h->dblock = base;
     h->dbytes = total;
     for (auto &q : r) { *q.p = base; base += align256(q.bytes); }
-    /* the count of 3-sided grains is zero between steps; the first word of
-     * its 256 bytes held another count in earlier checkpoint files, so it
-     * takes the second */
-    x.n_three += 1;
+    x.n_fail = x.nrun + 1;   /* every piece of the block has at least 256 bytes */
     /* reservation keys start above every key an event writes */
     if (!cuda_ok(cudaMemsetAsync(x.vown, 0xFF, V * 8, h->stream), "memset") ||
         !cuda_ok(cudaMemsetAsync(x.bown, 0xFF, B * 8, h->stream), "memset"))
@@ -270,8 +259,6 @@ bool upload(sevc_handle *h, const sevc_mesh_host &hm)
     {
         std::vector<int4> md(4 * V, make_int4(-1, -1, -1, FIX_NONE));
         if (!put(h->m.vmod, md.data(), 4 * V * 16)) return false;
-        std::vector<int> neg(V, -1);
-        if (!put(h->m.voted, neg.data(), V * 4)) return false;
     }
     std::vector<int2> bv(B);
     for (size_t i = 0; i < B; i++) bv[i] = make_int2(hm.bini[i], hm.bend[i]);
@@ -347,21 +334,16 @@ sevc_status create_from_host(const sevc_options *opt, sevc_hmesh *hm, sevc_handl
     h->iallow.assign(ninst, 0);
     h->iarea.assign(ninst, 0.0);
     h->iinfo.assign(ninst, sevc_step_info{});
-    int max_ng = 0;
-    for (int i = 0; i < ninst; i++) {
-        h->icurr[i] = h->goff[i + 1] - h->goff[i];
-        if (h->icurr[i] > max_ng) max_ng = h->icurr[i];
-    }
+    for (int i = 0; i < ninst; i++) h->icurr[i] = h->goff[i + 1] - h->goff[i];
     h->p.dt = opt->dt; h->p.eps = opt->GB_eps; h->p.scaling = opt->GB_scaling; h->p.MC_k = opt->MC_k;
     h->p.n_blocks = opt->n_blocks; h->p.n_threads = opt->n_threads;
     h->p.ninst = ninst;
-    h->p.max_inst_ng = max_ng;
     h->p.mu = 1.0;
     h->curr_n_grains = h->ng;
     /* readback: counters, events, polling iterations, 2x3 counts per instance */
     h->h_big_ints = (size_t)ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 64;
     bool streams_ok = cuda_ok(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
-    for (int k = 0; streams_ok && k < 3; k++)
+    for (int k = 0; streams_ok && k < 2; k++)
         streams_ok = cuda_ok(cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking), "stream");
     for (int k = 0; streams_ok && k < 10; k++)
         streams_ok = cuda_ok(cudaEventCreateWithFlags(&h->evfork[k], cudaEventDisableTiming), "event");
@@ -445,8 +427,7 @@ void tape_free(sevc_handle *h)
 
 void drop_graphs(sevc_handle *h)
 {
-    StepGraph *gs[] = { &h->g_pre[0], &h->g_pre[1], &h->g_poll, &h->g_post, &h->g_step[0], &h->g_step[1] };
-    for (StepGraph *g : gs) {
+    for (StepGraph *g : { &h->g_step[0], &h->g_step[1] }) {
         if (g->exec) cudaGraphExecDestroy(g->exec);
         *g = StepGraph();
     }
@@ -481,14 +462,13 @@ template <class F> bool run_seq(sevc_handle *h, StepGraph &g, F &&enqueue)
     return cuda_ok(cudaGraphLaunch(g.exec, h->stream), "graph launch");
 }
 
-/* first half of the step, up to the candidate list (src/main.cu:121-216) */
+/* first half of the step, up to the labels (src/main.cu:121-216) */
 void enqueue_pre(sevc_handle *h, bool nucleation)
 {
     cudaStream_t s = h->stream;
     const sevc_options &o = h->opt;
     DevMesh &m = h->m;
     DevScratch &x = h->x;
-    size_t I = h->ninst;
     /* the per-step records (event counts, error bits, 2x3 pass counts,
      * polling state, dA/dt exactness marks) are zero here: the previous
      * step's summary kernel cleared them as it read them (a new handle's
@@ -514,12 +494,10 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
     if (h->profiling) {
         { Prof pr(h, "boundary_geometry"); launch_boundary_geometry(m, o.GB_eps, o.GB_scaling, h->p.shape, s); }
         { Prof pr(h, "grain_fd"); launch_grain_pass(m, x, h->p.shape, s); }
-        { Prof pr(h, "two_three_count"); launch_two_three_first(m, x, x.list_b, x.n_b, s); }
-        launch_full_flag(m, x, s);
+        { Prof pr(h, "two_three_count"); launch_two_three_first(m, x, s); }
         { Prof pr(h, "vertex_fd"); launch_vertex_fd(m, h->p.mu, unit_gamma, h->p.shape, s); }
         { Prof pr(h, "grain_dadt"); launch_grain_dadt(m, x, s); }
-        { Prof pr(h, "text_label"); launch_text_label(m, x, o.dt, h->p.shape, s); }
-        { Prof pr(h, "compact"); launch_compact(m, x, CK_CAND, x.list_a, x.n_a, s); }
+        { Prof pr(h, "text_label"); launch_text_label(m, x, h->p, s); }
     } else {
         cudaStream_t s0 = h->side[0], s1 = h->side[1];
         cudaEvent_t *ev = h->evfork;
@@ -530,8 +508,7 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
         launch_grain_pass(m, x, h->p.shape, s);                                        /* :127,:203 */
         cudaEventRecord(ev[2], s);
         cudaStreamWaitEvent(s1, ev[2], 0);
-        launch_two_three_first(m, x, x.list_b, x.n_b, s1);                             /* :228 */
-        launch_full_flag(m, x, s1);
+        launch_two_three_first(m, x, s1);                                              /* :228 */
         cudaEventRecord(ev[3], s1);
         cudaStreamWaitEvent(s, ev[1], 0);
         launch_vertex_fd(m, h->p.mu, unit_gamma, h->p.shape, s);                       /* :133,:203 */
@@ -541,152 +518,66 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
         launch_grain_dadt(m, x, s0);                                                   /* :206 */
         cudaEventRecord(ev[5], s0);
         sevc_pdl_skip = 1;       /* two predecessors */
-        launch_text_label(m, x, o.dt, h->p.shape, s);                                  /* :212-216 */
+        launch_text_label(m, x, h->p, s);                                              /* :212-216 */
         sevc_pdl_skip = 0;
-        launch_compact(m, x, CK_CAND, x.list_a, x.n_a, s);
         cudaStreamWaitEvent(s, ev[5], 0);
     }
 }
 
-void enqueue_poll(sevc_handle *h)
-{
-    Prof pr(h, "polling");
-    launch_poll_iteration(h->m, h->x, h->x.list_a, h->x.n_a, h->p, h->stream);
-}
-
-/* from the 3-sided labels to the end of the step (src/main.cu:252-325);
- * lists_unchanged: no 2x3 removal edited a list since the side-count order
- * (1), some did (0), the device knows (-1: the step's first 2x3 count
- * recorded by the whole-step graph decides) */
-void enqueue_tail(sevc_handle *h, int lists_unchanged)
-{
-    cudaStream_t s = h->stream;
-    const sevc_options &o = h->opt;
-    DevMesh &m = h->m;
-    DevScratch &x = h->x;
-    if (lists_unchanged < 0) {                                                                    /* :252-255 */
-        sevc_pdl_skip = 1;       /* the first kernel after a conditional node */
-        launch_label_3sided_auto(m, x, o.dt, s);
-        sevc_pdl_skip = 0;
-    } else {
-        Prof pr(h, "label_3sided");
-        launch_label_3sided(m, x, o.dt, lists_unchanged != 0, s);
-    }
-    { Prof pr(h, "compact"); launch_compact(m, x, CK_GRAIN_CAND, x.list_c, x.n_c, s); }
-    { Prof pr(h, "remove_grains"); launch_remove_grains(m, x, x.list_c, x.n_c, s); }              /* :259 */
-    { Prof pr(h, "fix_lists"); launch_fix_lists(m, s); }                                          /* :262 */
-    /* The counts (:317-325) read only grain flags, types and areas, which
-     * are final here (the flips and the list fix-up after them change
-     * none): side0 computes them beside the flips, the fix-up and the
-     * position update, joining before the summary. */
-    if (!h->profiling) {
-        cudaEventRecord(h->evfork[6], s);
-        cudaStreamWaitEvent(h->side[0], h->evfork[6], 0);
-        launch_counts(m, x, h->p, h->side[0]);
-        cudaEventRecord(h->evfork[7], h->side[0]);
-    }
-    { Prof pr(h, "flips"); launch_flips(m, o.GB_eps, x.list_a, x.n_a, x, s); }             /* :282, :289 */
-    if (h->profiling) {
-        { Prof pr(h, "fix_lists"); launch_fix_lists(m, s, false); }                               /* :294 */
-        { Prof pr(h, "update"); launch_update_positions(m, o.dt, s); }                            /* :314 */
-        { Prof pr(h, "counts"); launch_counts(m, x, h->p, s); }
-    } else {
-        /* the position update reads positions and velocities, final once
-         * the flips are applied; the fix-up after them edits only lists
-         * and mods: side1 updates beside it */
-        cudaEventRecord(h->evfork[8], s);
-        cudaStreamWaitEvent(h->side[1], h->evfork[8], 0);
-        sevc_pdl_skip = 1;
-        launch_update_positions(m, o.dt, h->side[1]);                                             /* :314 */
-        sevc_pdl_skip = 0;
-        cudaEventRecord(h->evfork[9], h->side[1]);
-        launch_fix_lists(m, s, false);                                                            /* :294 */
-        cudaStreamWaitEvent(s, h->evfork[9], 0);
-        cudaStreamWaitEvent(s, h->evfork[7], 0);
-    }
-    launch_pack_summary(m, x, h->ninst, x.summary, s);
-}
-
-/* second half of a step without 2x3 pairs: conflicts, then the tail */
-void enqueue_post(sevc_handle *h)
-{
-    { Prof pr(h, "conflicts"); launch_conflicts(h->m, h->x.list_a, h->x.n_a, h->stream); }         /* :222-225 */
-    enqueue_tail(h, 1);
-}
-
-/* Add a WHILE conditional node at the current point of the capture on the
- * handle's stream.  pre(handle) enqueues on that stream what runs just
- * before the node (it may set the condition); body(stream, handle)
- * enqueues the loop body onto the given stream, captured into the node's
- * body graph.  The body's first kernel goes without programmatic
- * serialisation (nothing precedes it in the body); the others keep it. */
-template <class Pre, class Body>
-bool capture_while(sevc_handle *h, unsigned dflt, unsigned flags, Pre &&pre, Body &&body)
-{
-    cudaStream_t s = h->stream;
-    cudaStreamCaptureStatus st;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    const cudaGraphEdgeData *ed = nullptr;
-    size_t nd = 0;
-    if (!cuda_ok(cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, &deps, &ed, &nd), "capture info")) return false;
-    cudaGraphConditionalHandle hnd;
-    if (!cuda_ok(cudaGraphConditionalHandleCreate(&hnd, cg, dflt, flags), "conditional handle")) return false;
-    pre(hnd);
-    if (!cuda_ok(cudaStreamGetCaptureInfo(s, &st, nullptr, &cg, &deps, &ed, &nd), "capture info")) return false;
-    std::vector<cudaGraphNode_t> dv(deps, deps + nd);
-    cudaGraphNodeParams np = { cudaGraphNodeTypeConditional };
-    np.conditional.handle = hnd;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (!cuda_ok(cudaGraphAddNode(&node, cg, dv.data(), nullptr, dv.size(), &np), "conditional node")) return false;
-    cudaGraph_t bodyg = np.conditional.phGraph_out[0];
-    if (!cuda_ok(cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies),
-                 "capture dependencies"))
-        return false;
-    cudaStream_t bs = h->side[2];
-    bool ok = cuda_ok(cudaStreamBeginCaptureToGraph(bs, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
-                      "body capture");
-    if (ok) {
-        sevc_pdl_skip = 1;       /* the body's first kernel has no kernel before it */
-        body(bs, hnd);
-        sevc_pdl_skip = 0;
-        cudaGraph_t out = nullptr;
-        ok = cuda_ok(cudaStreamEndCapture(bs, &out), "body capture");
-    }
-    return ok;
-}
-
-/* The whole step as one launch sequence for a graph (src/main.cu:121-325):
- * the first half, the polling loop and the 2x3 loop as device-driven
- * WHILE nodes with the conflicts in between, then the tail.  Only while
- * capturing. */
-bool enqueue_step_graph(sevc_handle *h, bool nucleation)
+/* from the polling to the end of the step (src/main.cu:219-325) */
+void enqueue_tail(sevc_handle *h)
 {
     cudaStream_t s = h->stream;
     DevMesh &m = h->m;
     DevScratch &x = h->x;
-    enqueue_pre(h, nucleation);
-    bool ok = capture_while(h, 1u, cudaGraphCondAssignDefault, [](cudaGraphConditionalHandle) {},   /* :219 */
-                            [&](cudaStream_t bs, cudaGraphConditionalHandle hnd) {
-                                launch_poll_iteration(m, x, x.list_a, x.n_a, h->p, bs);
-                                launch_poll_cond(m, x, hnd, h->polling_cap, bs);
-                            });
-    if (!ok) return false;
-    sevc_pdl_skip = 1;           /* the first kernel after a conditional node */
-    launch_conflicts(m, x.list_a, x.n_a, s);                                                        /* :222-225 */
+    const StepParams &p = h->p;
+    if (!h->profiling) sevc_pdl_skip = 1;   /* joins the dA/dt branch: two predecessors */
+    if (tail_whole(m)) {
+        Prof pr(h, "tail");
+        launch_tail_whole(m, x, p, h->polling_cap, x.summary, s);
+        sevc_pdl_skip = 0;
+        return;
+    }
+    { Prof pr(h, "removals"); launch_tail_removals(m, x, p, h->polling_cap, s); }                 /* :219-266 */
     sevc_pdl_skip = 0;
-    ok = capture_while(h, 0u, 0u, [&](cudaGraphConditionalHandle hnd) { launch_tt_init(x, hnd, s); },  /* :227-250 */
-                       [&](cudaStream_t bs, cudaGraphConditionalHandle hnd) {
-                           launch_remove_two_three_dev(m, x, x.list_b, x.n_b, bs);
-                           launch_fix_lists(m, bs);
-                           launch_compact(m, x, CK_TWO_THREE, x.list_b, x.n_b, bs);
-                           launch_tt_cond(x, hnd, bs);
-                       });
-    if (!ok) return false;
-    enqueue_tail(h, -1);
-    return true;
+    if (h->profiling) {
+        { Prof pr(h, "flips"); launch_tail_flips(m, x, p, s); }                                   /* :282, :289 */
+        { Prof pr(h, "fix_lists"); launch_tail_fix(m, x, p, s); }                                 /* :294 */
+        { Prof pr(h, "update"); launch_update_positions(m, p.dt, s); }                            /* :314 */
+        { Prof pr(h, "counts"); launch_counts(m, x, p, s); }                                      /* :317-325 */
+    } else {
+        /* The counts read only grain flags, types and areas, which are final
+         * here (the flips and the list fix-up after them change none): side0
+         * computes them beside the flips, the fix-up and the position
+         * update.  The position update reads positions and velocities, final
+         * once the flips are applied; the fix-up after them edits only lists
+         * and mods: side1 updates beside it.  Both join before the summary. */
+        cudaEvent_t *ev = h->evfork;
+        cudaEventRecord(ev[6], s);
+        cudaStreamWaitEvent(h->side[0], ev[6], 0);
+        launch_counts(m, x, p, h->side[0]);
+        cudaEventRecord(ev[7], h->side[0]);
+        launch_tail_flips(m, x, p, s);
+        cudaEventRecord(ev[8], s);
+        cudaStreamWaitEvent(h->side[1], ev[8], 0);
+        sevc_pdl_skip = 1;
+        launch_update_positions(m, p.dt, h->side[1]);
+        sevc_pdl_skip = 0;
+        cudaEventRecord(ev[9], h->side[1]);
+        launch_tail_fix(m, x, p, s);
+        cudaStreamWaitEvent(s, ev[9], 0);
+        cudaStreamWaitEvent(s, ev[7], 0);
+        sevc_pdl_skip = 1;
+    }
+    launch_pack_summary(m, x, x.summary, s);
+    sevc_pdl_skip = 0;
+}
+
+/* the whole step (src/main.cu:121-325) */
+void enqueue_step(sevc_handle *h, bool nucleation)
+{
+    enqueue_pre(h, nucleation);
+    enqueue_tail(h);
 }
 
 sevc_status err_bits_to_status(int bits)
@@ -716,7 +607,7 @@ size_t summary_bytes(const sevc_handle *h)
  * attempted a nucleation) into the run state and `info`; then n++ and
  * t = n dt (src/main.cu:388-391).  loc carries n, t and the attempt flag of
  * the step. */
-sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, bool whole, float ms, int launches,
+sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms, int launches,
                         sevc_step_info loc, sevc_step_info *info)
 {
     const sevc_options &o = h->opt;
@@ -769,16 +660,14 @@ sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, bool who
         loc.n_nucleations += ii.n_nucleations;
         loc.n_conflicts += ii.n_conflicts;
     }
-    if (whole) {        /* the loops' counts, as the host loops report them */
-        loc.polling_iters = 0;
-        for (int i = 0; i < I; i++) loc.polling_iters = std::max(loc.polling_iters, h->iinfo[i].polling_iters);
-        for (int k = 0; k < TWO_THREE_PASSES; k++) {
-            int c = 0;
-            for (int i = 0; i < I; i++) c += hb[o_seg + (size_t)k * I + i];
-            loc.two_three_counts[k] = c;
-            loc.n_two_three_iters = k + 1;
-            if (c == 0) break;
-        }
+    loc.polling_iters = 0;
+    for (int i = 0; i < I; i++) loc.polling_iters = std::max(loc.polling_iters, h->iinfo[i].polling_iters);
+    for (int k = 0; k < TWO_THREE_PASSES; k++) {
+        int c = 0;
+        for (int i = 0; i < I; i++) c += hb[o_seg + (size_t)k * I + i];
+        loc.two_three_counts[k] = c;
+        loc.n_two_three_iters = k + 1;
+        if (c == 0) break;
     }
     h->curr_n_grains = total;
     h->nucleated_area = batch ? area_sum / I : area_sum;
@@ -979,7 +868,6 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     if (!h) return SEVC_ERR_ARG;
     cudaStream_t s = h->stream;
     const sevc_options &o = h->opt;
-    DevMesh &m = h->m;
     DevScratch &x = h->x;
     const int I = h->ninst;
     const bool batch = I > 1;
@@ -1009,52 +897,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     if (!cuda_ok(cudaMemcpyAsync(x.flags + 1, h->h_flags + 1, 3 * sizeof(int), cudaMemcpyHostToDevice, s), "upload"))
         return SEVC_ERR_CUDA;
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
-    const bool whole = graphs_on(h) && h->device_loops;
-    if (whole) {
-        /* one graph: the loops run on the device, their counts come back
-         * with the step summary */
-        bool cap_ok = true;
-        if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { cap_ok = enqueue_step_graph(h, n_on > 0); }) || !cap_ok)
-            return SEVC_ERR_CUDA;
-    } else {
-    if (!run_seq(h, h->g_pre[n_on ? 1 : 0], [&] { enqueue_pre(h, n_on > 0); })) return SEVC_ERR_CUDA;
-
-    /* polling (:219); the first readback also brings the 2x3 count */
-    int running = 1, it = 0, c23 = 0;
-    while (running) {
-        if (it >= h->polling_cap) { sevc_set_error("polling did not converge"); return SEVC_ERR_NONCONVERGED; }
-        it++;
-        if (!run_seq(h, h->g_poll, [&] { enqueue_poll(h); })) return SEVC_ERR_CUDA;
-        if (!cuda_ok(cudaMemcpyAsync(h->h_ctr, x.nrun, 4, cudaMemcpyDeviceToHost, s), "readback") ||
-            (it == 1 && !cuda_ok(cudaMemcpyAsync(h->h_ctr + 1, x.n_b, 4, cudaMemcpyDeviceToHost, s), "readback")) ||
-            !cuda_ok(cudaStreamSynchronize(s), "sync"))
-            return SEVC_ERR_CUDA;
-        running = h->h_ctr[0];
-        if (it == 1) c23 = h->h_ctr[1];
-    }
-    loc.polling_iters = it;
-
-    if (c23 == 0) {                                  /* the usual step: no 2x3 pair */
-        loc.two_three_counts[0] = 0;
-        loc.n_two_three_iters = 1;
-        if (!run_seq(h, h->g_post, [&] { enqueue_post(h); })) return SEVC_ERR_CUDA;
-    } else {
-        { Prof pr(h, "conflicts"); launch_conflicts(m, x.list_a, x.n_a, s); }                     /* :222-225 */
-        for (int k = 0; k < TWO_THREE_PASSES; k++) {                                               /* :227-250 */
-            int c = c23;
-            if (k > 0) {
-                { Prof pr(h, "two_three_count"); launch_compact(m, x, CK_TWO_THREE, x.list_b, x.n_b, s); }
-                if (read_ints(h, x.n_b, 1, &c)) return SEVC_ERR_CUDA;
-            }
-            loc.two_three_counts[k] = c;
-            loc.n_two_three_iters = k + 1;
-            if (c == 0) break;
-            { Prof pr(h, "two_three_remove"); launch_remove_two_three(m, x, x.list_b, x.n_b, k, s); }
-            { Prof pr(h, "fix_lists"); launch_fix_lists(m, s); }
-        }
-        enqueue_tail(h, 0);
-    }
-    }
+    if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
 
     /* one readback: counters, events, error bits, polling iterations and
@@ -1067,7 +910,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     if (h->profiling) prof_collect(h);
     int launches = (int)(sevc_kernel_launches - launches0);
-    return finish_step(h, hb, h->h_on, whole, ms, launches, loc, info);
+    return finish_step(h, hb, h->h_on, ms, launches, loc, info);
 }
 
 sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *done)
@@ -1078,10 +921,10 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
     const int I = h->ninst;
     const bool batch = I > 1;
     const int mg = o.min_grains;
-    /* pipelined: one graph per step, nothing read inside a step, and no
+    /* pipelined: one graph per step and no
      * input of a step that depends on the previous step's counts (a single
      * mesh with a grain-count stop feeds its count to the output decision) */
-    const bool pipe = graphs_on(h) && h->device_loops && !h->profiling && h->tape.every <= 0 && (batch || mg <= 0);
+    const bool pipe = graphs_on(h) && h->tape.every <= 0 && (batch || mg <= 0);
     if (!pipe) {
         for (int k = 0; k < nsteps; k++) {
             sevc_step_info inf;
@@ -1112,7 +955,7 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         float ms = 0;
         cudaEventElapsedTime(&ms, sl.ev0, sl.ev1);
         sevc_step_info inf;
-        sevc_status r = finish_step(h, sl.big, sl.on, true, ms, (int)sl.launches, sl.loc, &inf);
+        sevc_status r = finish_step(h, sl.big, sl.on, ms, (int)sl.launches, sl.loc, &inf);
         if (infos) infos[finished] = inf;
         finished++;
         if (done) *done = finished;
@@ -1154,8 +997,7 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         }
         cudaEventRecord(sl.ev0, s);
         long long k0 = sevc_kernel_launches;
-        bool cap_ok = true;
-        if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { cap_ok = enqueue_step_graph(h, n_on > 0); }) || !cap_ok) {
+        if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); })) {
             st = SEVC_ERR_CUDA;
             break;
         }
@@ -1471,7 +1313,6 @@ sevc_status sevc_set_graphs(sevc_handle *h, int on)
 {
     if (!h || on < 0 || on > 2) return SEVC_ERR_ARG;
     h->use_graphs = on != 0;
-    h->device_loops = on == 1;
     drop_graphs(h);
     return SEVC_OK;
 }
@@ -1714,6 +1555,12 @@ sevc_status sevc_checkpoint_load(sevc_handle *h, const char *path)
     h->p.mu = hd.mu; h->opt.GB_scaling = hd.gb_scaling; h->p.scaling = hd.gb_scaling;
     h->outputs_complete = hd.outputs_complete;
     drop_graphs(h);
+    /* a file may hold the last step's list lengths and polling results here;
+     * between steps they are zero */
+    DevScratch &x = h->x;
+    for (int *p : { x.n_a, x.n_b, x.n_c, x.n_fail, x.n_ehits, x.n_three }) cudaMemsetAsync(p, 0, 4, h->stream);
+    cudaMemsetAsync(x.pblock, 0, I * h->p.n_blocks * 4, h->stream);
+    if (!cuda_ok(cudaStreamSynchronize(h->stream), "sync")) return SEVC_ERR_CUDA;
     h->icurr = icurr; h->iallow = iallow; h->iarea = iarea;
     return SEVC_OK;
 }

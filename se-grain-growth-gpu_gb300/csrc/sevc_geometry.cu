@@ -13,7 +13,7 @@
  * Both passes repeat the reference's arithmetic in the same order, so the
  * results are the ones energy_diff computes.
  */
-#include "sevc_internal.h"
+#include "sevc_tail.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -527,21 +527,6 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
 }
 constexpr int GRAIN_SMALL = 32 * 1024;   /* see launch_grain_pass */
 
-/* The step computes every output-only value (extinction times of all
- * boundaries, dA/dt of all grains) when it can export or is asked to
- * (flags[1], set by the host), or when it could end at the stop threshold
- * (a final export): every removal takes a 3-sided grain, and a pass of the
- * 2x3 loop can make at most two per pair; the bound is generous, as the
- * threshold is crossed once per run.  Else only what the step can observe
- * is computed.  flags[0] = the decision, taken on the device so that no
- * host round trip separates the step's first half from its second. */
-__global__ void k_full_flag(const int *n_two_three, const int *n_three, int *flags, unsigned *stamp)
-{
-    int mg = flags[2], curr = flags[3], n3 = *n_three;
-    long long reach = (long long)curr - n3 - 40LL * *n_two_three - 64;
-    flags[0] = flags[1] || (mg > 0 && reach <= mg);
-    *stamp += 1;   /* a new step: every value saved by the last step's events is stale */
-}
 /* vertex pass: src/calculus.h:19-73 (boundary part) and :143-154;
  * vertex_compute_energy src/geometry.h:472-479.
  *
@@ -637,9 +622,27 @@ __device__ void dadt_of(const DevMesh &m, int g)
  * (finalize_boundary).  The proof that a boundary is not a candidate is the
  * binary32 certificate text_outside_dt.
  */
-__device__ __forceinline__ void text_label_one(const DevMesh &m, int b, uint8_t en, double2 pi, double2 pe,
-                                               double2 vi, double2 ve, double dt, float Df, float hDf, float inv_dt,
-                                               int full)
+/* label_boundaries' result for boundary b.  A candidate joins the list the
+ * polling and the flips work on.  For any other boundary the first polling
+ * iteration's comparison (src/topological.h:466-511) happens here: its flag
+ * is 0 and stays 0, so it mismatches if the buffer (buf, as the last step's
+ * polling left it) holds 1, and the buffer becomes 0.  (A listed boundary is
+ * enabled; a disabled one has its buffer cleared and never mismatches.) */
+__device__ __forceinline__ void set_label(const DevMesh &m, const DevScratch &x, const PollGrid &pg, int b, uint8_t en,
+                                          uint8_t buf, unsigned cand)
+{
+    m.bcand[b] = (uint8_t)cand;
+    m.bconf[b] = -1;
+    if (en && cand) {
+        x.list_a[atomicAdd(x.n_a, 1)] = b;
+    } else if (buf) {
+        m.bcandbuf[b] = 0;
+        if (en) poll_fail(m, x, pg, b);
+    }
+}
+__device__ __forceinline__ void text_label_one(const DevMesh &m, const DevScratch &x, const PollGrid &pg, int b,
+                                               uint8_t en, uint8_t buf, double2 pi, double2 pe, double2 vi, double2 ve,
+                                               double dt, float Df, float hDf, float inv_dt, int full)
 {
     long long tb;
     if (en) {
@@ -649,8 +652,7 @@ __device__ __forceinline__ void text_label_one(const DevMesh &m, int b, uint8_t 
              * which then computes it (finalize_boundary) */
             m.btext[b] = SEVC_MAX_T_EXT_D;
             m.bexact[b] = 0;
-            m.bcand[b] = 0;
-            m.bconf[b] = -1;
+            set_label(m, x, pg, b, en, buf, 0);
             return;
         }
         double text = text_exact_call(pi, pe, vi, ve, m.D);
@@ -673,8 +675,7 @@ __device__ __forceinline__ void text_label_one(const DevMesh &m, int b, uint8_t 
         "or.pred p, p, z;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(cand) : "l"(tb), "l"(dbits(dt)));
-    m.bcand[b] = (uint8_t)cand;
-    m.bconf[b] = -1;
+    set_label(m, x, pg, b, en, buf, cand);
 }
 /* Two boundaries per thread (b and b + blockDim.x of the block's pair of
  * tiles), every load of both issued before either is labelled: the pass
@@ -690,18 +691,20 @@ __device__ __forceinline__ void text_label_one(const DevMesh &m, int b, uint8_t 
  * candidate, and is labelled as the certificate labels one (without
  * reading its ends' positions and velocities).  The others take the
  * certificate and, if undecided, the exact value. */
-__global__ void k_text_label(DevMesh m, double dt, float Df, float hDf, float inv_dt, float dt_up, const int *flags)
+__global__ void k_text_label(DevMesh m, DevScratch x, PollGrid pg, double dt, float Df, float hDf, float inv_dt,
+                             float dt_up)
 {
     griddep_wait();
     int b0 = 2 * blockIdx.x * blockDim.x + threadIdx.x;
-    int full = flags[0];
-    uint8_t en[2];
+    int full = x.flags[0];
+    uint8_t en[2], buf[2];
     int2 e[2];
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         int b = b0 + k * blockDim.x;
         bool in = b < m.nb;
         en[k] = in ? m.ben[b] : 0;
+        buf[k] = in ? m.bcandbuf[b] : 0;
         e[k] = in ? m.bv[b] : make_int2(0, 0);   /* loaded beside the flag: one round trip less */
     }
     bool far[2] = { false, false };
@@ -724,123 +727,39 @@ __global__ void k_text_label(DevMesh m, double dt, float Df, float hDf, float in
         if (far[k]) {
             m.btext[b] = SEVC_MAX_T_EXT_D;       /* as text_label_one's certified skip */
             m.bexact[b] = 0;
-            m.bcand[b] = 0;
-            m.bconf[b] = -1;
+            set_label(m, x, pg, b, en[k], buf[k], 0);
         } else {
-            text_label_one(m, b, en[k], pi[k], pe[k], vi[k], ve[k], dt, Df, hDf, inv_dt, full);
+            text_label_one(m, x, pg, b, en[k], buf[k], pi[k], pe[k], vi[k], ve[k], dt, Df, hDf, inv_dt, full);
         }
     }
 }
 
 
-/* the step's summary in one buffer, for one readback: counters, events,
- * error bits, polling iterations, 2x3 pass counts (all per instance) and
- * the output decision */
-/* The step's summary in one buffer; each per-step record it packs (event
- * counts, error bits, polling iterations and convergence, 2x3 pass counts)
- * is zeroed once read, and so are the exactness marks of the grains' dA/dt
- * and the polling iteration total and the list of 3-sided grains, so the next step starts from zeros
- * without resets of its own (the reset each step would otherwise begin
- * with: src/main.cu's per-step clears of these values). */
-__global__ void k_pack_summary(DevMesh m, DevScratch x, int ninst, int *out)
+__global__ void k_pack_summary(DevMesh m, DevScratch x, int *out)
 {
     griddep_wait();
-    size_t nc = (size_t)ninst * CTR_COUNT, ne = (size_t)ninst * EVT_COUNT, np = ninst,
-           ns = (size_t)ninst * TWO_THREE_PASSES;
-    size_t total = nc + ne + 4 + np + ns + 1;
-    const size_t stride = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = t0; i < total; i += stride) {
-        size_t k = i;
-        int v;
-        if (k < nc) v = x.counters[k];
-        else if ((k -= nc) < ne) { v = m.evt[k]; m.evt[k] = 0; }
-        else if ((k -= ne) < 4) { v = m.err[k]; m.err[k] = 0; }
-        else if ((k -= 4) < np) { v = x.piters[k]; x.piters[k] = 0; m.pdone[k] = 0; }
-        else if ((k -= np) < ns) { v = x.segcnt[k]; x.segcnt[k] = 0; }
-        else { v = x.flags[0]; *x.ptot = 0; *x.n_three = 0; }
-        out[i] = v;
-    }
-    const size_t nw = (size_t)m.ng / 16;                   /* gexact as 16-byte words (256-byte aligned array) */
-    for (size_t i = t0; i < nw; i += stride) reinterpret_cast<uint4 *>(m.gexact)[i] = make_uint4(0, 0, 0, 0);
-    for (size_t i = 16 * nw + t0; i < (size_t)m.ng; i += stride) m.gexact[i] = 0;
+    pack_summary(m, x, out, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 __global__ void k_reset_ngrains(int *counters, int ninst)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ninst) counters[(size_t)i * CTR_COUNT + CTR_NGRAINS] = 0;
 }
-
-/* update_vertices_positions, src/calculus.h:391-404 */
 __global__ void k_update(DevMesh m, double dt)
 {
     griddep_wait();
     int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= m.nv || !m.ven[v]) return;
-    double2 p = m.pos[v], w = m.vel[v];
-    p.x += w.x * dt;
-    p.y += w.y * dt;
-    p.x = dmod(p.x, m.D);
-    p.y = dmod(p.y, m.D);
-    m.pos[v] = p;
+    if (v < m.nv) update_vertex(m, v, dt);
 }
-
-/* current_n_grains (src/calculus.h:264-313): an integer count per
- * instance (blockIdx.y), added into counters[inst * CTR_COUNT + CTR_NGRAINS] */
-__global__ void k_count_grains(DevMesh m, int *counters)
+/* both counts; the last block finishes the nucleated area */
+__global__ void __launch_bounds__(TPB) k_counts(DevMesh m, int *counters, double *block_area, int nblocks, int tpb)
 {
-    int inst = blockIdx.y;
-    int lo = m.goff[inst], hi = m.goff[inst + 1];
-    int c = 0;
-    for (int g = lo + blockIdx.x * blockDim.x + threadIdx.x; g < hi; g += gridDim.x * blockDim.x) c += m.gen[g] ? 1 : 0;
-    __shared__ int part[32];
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += part[w];
-        if (t) atomicAdd(counters + (size_t)inst * CTR_COUNT + CTR_NGRAINS, t);
-    }
-}
-
-/* nucl_area_per_block (src/calculus.h:322-348): launched on the
- * reference's grid (blockIdx.y = instance) so that the floating-point sum
- * order is the same: per-thread strided partial sums over the instance's
- * grain indices, then the shared-memory tree. */
-__global__ void k_nucl_area_blocks(DevMesh m, double *block_out, int *counters)
-{
-    __shared__ double t[256];
-    int inst = blockIdx.y;
-    int go = m.goff[inst];
-    int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    int stride = gridDim.x * blockDim.x;
-    double a = 0.0;
-    /* the thread's stride set in ascending order, restricted to the slots
-     * that can be NUCLEATED (the instance's nlist part is ascending) */
-    int nn = m.nnlist[inst];
-    const int *nl = m.nlist + go;
-    for (int i = 0; i < nn; i++) {
-        int g = nl[i];
-        if ((g - go) % stride == tid && m.gen[g] && m.gtype[g] == GT_NUCLEATED) a += m.garea[g];
-    }
-    t[threadIdx.x] = a;
-    __syncthreads();
-    for (int i = blockDim.x / 2; i != 0; i /= 2) {
-        if ((int)threadIdx.x < i) t[threadIdx.x] += t[threadIdx.x + i];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) block_out[(size_t)inst * gridDim.x + blockIdx.x] = t[0];
-    /* host loop of nucleated_fraction_area, src/calculus.h:373-377: the last
-     * block, one thread per instance */
+    count_grains(m, counters, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    nucl_area_blocks(m, block_area, nblocks, tpb, blockIdx.x, gridDim.x);
     const bool last = last_block(m.lastblk + 1);
     if (last) {
         __threadfence();
-        const int nblocks = gridDim.x;
-        for (int i = threadIdx.x; i < m.ninst; i += blockDim.x) {
-            double s = 0.0;
-            for (int b = 0; b < nblocks; b++) s += __ldcg(block_out + (size_t)i * nblocks + b);
-            *reinterpret_cast<double *>(counters + (size_t)i * CTR_COUNT + CTR_NUCL_AREA_SLOT) = 100 * s / (m.D * m.D);
-        }
+        nucl_area_final(m, block_area, nblocks, counters, threadIdx.x, blockDim.x);
     }
 }
 
@@ -878,18 +797,15 @@ void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const Launch
     if (unit_gamma) COUNT_LAUNCHES(1), k_vertex_fd<true><<<(m.nv + t - 1) / t, t, 0, s>>>(m, mu);
     else COUNT_LAUNCHES(1), k_vertex_fd<false><<<(m.nv + t - 1) / t, t, 0, s>>>(m, mu);
 }
-void launch_full_flag(const DevMesh &m, const DevScratch &x, cudaStream_t s)
-{
-    COUNT_LAUNCHES(1), k_full_flag<<<1, 1, 0, s>>>(x.n_b, x.n_three, x.flags, m.stamp);
-}
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s)
 {
     int g = nblk(m.ng);   /* grid-stride: every grain, or only the 3-sided ones, decided on the device */
     COUNT_LAUNCHES(1), k_grain_dadt<<<g < 8 * 152 ? g : 8 * 152, TPB, 0, s>>>(m, x.three, x.n_three, x.flags);
 }
-void launch_text_label(const DevMesh &m, const DevScratch &x, double dt, const LaunchShape &sh, cudaStream_t s)
+void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
-    int t = sh.tpb_boundary;
+    const double dt = p.dt;
+    int t = p.shape.tpb_boundary;
     /* binary32 copies for the certificate (text_outside_dt): rounded to
      * nearest, within 2^-24 of the binary64 values */
     float Df = (float)m.D, hDf = (float)(m.D / 2.0), inv_dt = (float)(1.0 / dt);
@@ -897,23 +813,20 @@ void launch_text_label(const DevMesh &m, const DevScratch &x, double dt, const L
     float dt_up = std::nextafter((float)(dt * (1.0 + 1e-6)), INFINITY);
     if ((double)dt_up < dt * (1.0 + 1e-6)) dt_up = std::nextafter(dt_up, INFINITY);
     if (m.nb > 0)
-        launch_dep(k_text_label, (m.nb + 2 * t - 1) / (2 * t), t, s, m, dt, Df, hDf, inv_dt, dt_up, x.flags);
+        launch_dep(k_text_label, (m.nb + 2 * t - 1) / (2 * t), t, s, m, x, poll_grid(p), dt, Df, hDf, inv_dt, dt_up);
 }
 void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s) { launch_dep(k_update, nblk(m.nv), TPB, s, m, dt); }
 
-void launch_pack_summary(const DevMesh &m, const DevScratch &x, int ninst, int *out, cudaStream_t s)
+void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s)
 {
-    size_t total = (size_t)ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 5;
+    size_t total = (size_t)m.ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 5;
     int g = (int)((total + TPB - 1) / TPB);
-    launch_dep(k_pack_summary, g < 152 ? g : 152, TPB, s, m, x, ninst, out);
+    launch_dep(k_pack_summary, g < 152 ? g : 152, TPB, s, m, x, out);
 }
 
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
     COUNT_LAUNCHES(1), k_reset_ngrains<<<(p.ninst + 127) / 128, 128, 0, s>>>(x.counters, p.ninst);
-    int gx = nblk(p.max_inst_ng);
-    if (gx > 4096) gx = 4096;
-    if (gx < 1) gx = 1;
-    COUNT_LAUNCHES(1), k_count_grains<<<dim3(gx, p.ninst), TPB, 0, s>>>(m, x.counters);
-    COUNT_LAUNCHES(1), k_nucl_area_blocks<<<dim3(p.n_blocks, p.ninst), p.n_threads, 0, s>>>(m, x.block_area, x.counters);
+    int g = nblk(m.ng);
+    COUNT_LAUNCHES(1), k_counts<<<g < 152 ? g : 152, TPB, 0, s>>>(m, x.counters, x.block_area, p.n_blocks, p.n_threads);
 }

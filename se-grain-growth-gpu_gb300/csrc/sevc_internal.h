@@ -12,36 +12,54 @@
 /* Scratch shared by launches of one handle.  Arrays marked "per instance"
  * hold one block for each instance of a batched handle. */
 struct DevScratch {
-    int *list_a, *list_b, *list_c;   /* ordered index lists (capacity max(nb, ng)) */
-    int *n_a, *n_b, *n_c;            /* their lengths */
-    int *blockcnt;                   /* per-tile counts for ordered compaction */
+    /* index lists (capacity max(nb, ng), any order) and their lengths, zero
+     * between steps: flip candidates; qualifying boundaries of the 2x3 loop;
+     * failed threads of a polling iteration, then 3-sided candidates */
+    int *list_a, *list_b, *list_c;
+    int *n_a, *n_b, *n_c, *n_fail;
     int *extra;                      /* dynamic insertions of the 2x3 pass, EXTRA_CAP per instance */
-    int *threadfail;                 /* polling predicate: one flag per grid thread, per instance */
-    int *pblock;                     /* polling predicate: one result per grid block, per instance */
-    int *pcnt;                       /* per instance: blocks of k_poll_final done (zero between launches) */
+    /* polling predicate, see poll_fail (zero between iterations): one flag
+     * per grid thread, failed threads per grid block, failed blocks, all per
+     * instance */
+    int *threadfail, *pblock, *pcnt;
     int *piters;                     /* polling iterations this step, per instance */
-    int *nrun;                       /* instances whose polling has not converged */
+    int *nrun;                       /* violations counted by check_data */
     int *segcnt;                     /* 2x3 count of each pass (20), per instance */
     double *block_area;              /* nucleated-area partial per block, per instance */
     int *counters;                   /* CTR_COUNT device counters per instance, see CTR_* */
     curandState *rng, *rng_saved;    /* 8192 cuRAND states + pre-attempt copy, per instance */
     int *nucl_buf;                   /* 96 ints per instance: per-block pick, alive count, pick's rank */
     int *nucl_on;                    /* per instance: attempt a nucleation this step */
-    int *reserved64;                 /* 64 ints no kernel uses: keeps the block's layout (checkpoint files) */
-    int *flags;                      /* 4 ints: the step's output decision, see launch_full_flag */
+    void *reserved;                  /* pieces of the block no kernel uses: they keep its layout (checkpoint files) */
+    int *flags;                      /* 4 ints: the step's output decision, see launch_two_three_first */
     int *summary;                    /* the step's summary packed for one readback */
     int *three, *n_three;            /* the enabled 3-sided grains, listed by the grain pass (any order) */
     unsigned long long *digest;      /* SEVC_DIGEST_FIELDS sums of sevc_state_digest */
     /* events applied in parallel (removals, flips): reservation keys of
-     * every vertex and boundary, the events of the phase (list positions),
-     * the deferred ones (flag per list position, count per instance) */
+     * every vertex and boundary, the deferred events (also the grains a 2x3
+     * pass left with three sides) */
     unsigned long long *vown, *bown;
     int *ehits, *n_ehits;
-    uint8_t *edefer;
-    int *ndefer;
-    /* device-driven loops of a whole-step graph: polling iterations taken
-     * (all instances), the first 2x3 count and the 2x3 pass index */
-    int *ptot, *tt_first, *tt_pass;
+};
+/* The reference's launch grid (n_blocks x n_threads), whose partition the
+ * polling predicate shows: thread t of a block enters the block's result
+ * through the shared-memory tree of topological.h:526-537, which halves its
+ * width (rounding down) each round, so for a width that is not a power of
+ * two some threads never do (counts). */
+struct PollGrid {
+    int blocks, tpb;
+    int counting;      /* threads of a block that enter its result */
+    __host__ __device__ int threads() const { return blocks * tpb; }
+    __host__ __device__ static bool counts(int t, int w)
+    {
+        while (w > 1) {
+            int h = w / 2;
+            if (t >= 2 * h) return false;
+            if (t >= h) t -= h;
+            w = h;
+        }
+        return true;
+    }
 };
 constexpr int EXTRA_CAP = 1024;
 constexpr int TWO_THREE_PASSES = 20;  /* src/main.cu:227 */
@@ -73,7 +91,6 @@ struct StepParams {
     double dt, eps, scaling, MC_k;
     int n_blocks, n_threads; /* reference launch grid, drives observable partitions */
     int ninst;               /* instances in the handle */
-    int max_inst_ng;         /* grains of the largest instance */
     double mu;               /* mobility (velocity factor); 1 in the reference */
     LaunchShape shape;
 };
@@ -84,52 +101,30 @@ void launch_boundary_geometry(const DevMesh &m, double eps, double scaling, cons
 void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s);
 /* unit_gamma: every boundary energy is exactly 1 (GB_eps = 0, GB_scaling = 1) */
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s);
-/* x.flags: [0] computed "full" decision, [1] host part of it, [2]
- * min_grains, [3] current grain count (see k_full_flag); also advances
- * the step stamp of the events' save-on-write (m.stamp) */
-void launch_full_flag(const DevMesh &m, const DevScratch &x, cudaStream_t s);
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s);
-void launch_text_label(const DevMesh &m, const DevScratch &x, double dt, const LaunchShape &sh, cudaStream_t s);
+/* also lists the candidates and starts the polling's first comparison */
+void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s);
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 /* counters | events | error bits | polling iterations | 2x3 counts | output decision, into out */
-void launch_pack_summary(const DevMesh &m, const DevScratch &x, int ninst, int *out, cudaStream_t s);
+void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s);
 
 /* topology (sevc_topology.cu) */
-enum CompactKind { CK_CAND = 0, CK_TWO_THREE = 1, CK_GRAIN_CAND = 2, CK_GVLEN3 = 3, CK_MARKED = 4 };
-void launch_compact(const DevMesh &m, const DevScratch &x, CompactKind kind, int *out, int *n_out, cudaStream_t s);
-/* the CK_TWO_THREE list from the 3-sided grains of this step's grain pass */
-void launch_two_three_first(const DevMesh &m, const DevScratch &x, int *out, int *n_out, cudaStream_t s);
-/* one polling iteration for every instance not yet converged; leaves the
- * number still running in x.nrun */
-void launch_poll_iteration(const DevMesh &m, const DevScratch &x, const int *cand, const int *ncand,
-                           const StepParams &p, cudaStream_t s);
-void launch_conflicts(const DevMesh &m, const int *cand, const int *ncand, cudaStream_t s);
-/* pass `pass` of the 2x3 loop (per-instance counts go to x.segcnt) */
-void launch_remove_two_three(const DevMesh &m, const DevScratch &x, const int *list, const int *n, int pass,
-                             cudaStream_t s);
-/* the same with the pass index read from x.tt_pass on the device */
-void launch_remove_two_three_dev(const DevMesh &m, const DevScratch &x, const int *list, const int *n, cudaStream_t s);
-/* Loop control of the whole-step graph (conditional WHILE nodes):
- * poll_cond after each polling iteration: continue while an instance has
- * not converged, up to `cap` iterations (past it: ERRB_NONCONVERGED);
- * tt_init before the 2x3 loop: record the first count, start while it is
- * nonzero; tt_cond after each pass: the next pass runs while the count
- * just compacted is nonzero and fewer than TWO_THREE_PASSES ran. */
-void launch_poll_cond(const DevMesh &m, const DevScratch &x, cudaGraphConditionalHandle hnd, int cap, cudaStream_t s);
-void launch_tt_init(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStream_t s);
-void launch_tt_cond(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStream_t s);
-/* the 3-sided labels, bucket or full as x.tt_first says (no 2x3 removal:
- * the bucket) */
-void launch_label_3sided_auto(const DevMesh &m, const DevScratch &x, double dt, cudaStream_t s);
-/* bucket: no grain list changed since this step's grain pass, so only the
- * 3-sided grains it listed are visited */
-void launch_label_3sided(const DevMesh &m, const DevScratch &x, double dt, bool bucket, cudaStream_t s);
-void launch_remove_grains(const DevMesh &m, const DevScratch &x, const int *list, const int *n, cudaStream_t s);
-/* clears the candidate flag of every listed grain (after the removals) */
-void launch_flips(const DevMesh &m, double eps, const int *cand, const int *ncand, const DevScratch &x,
-                  cudaStream_t s);
-void launch_fix_lists(const DevMesh &m, cudaStream_t s, bool areas = true);
+PollGrid poll_grid(const StepParams &p);
+/* The first 2x3 count (x.list_b, from the 3-sided grains of this step's
+ * grain pass), the decision x.flags[0] ([1] the host's part of it, [2]
+ * min_grains, [3] current grain count), and the next step stamp of the
+ * events' save-on-write (m.stamp). */
+void launch_two_three_first(const DevMesh &m, const DevScratch &x, cudaStream_t s);
+/* The sparse phases (k_tail): all of them, the position update, the counts
+ * and the summary in one launch for meshes that tail_whole accepts; else the
+ * removals, the flips and the flips' list fix-up, beside which the update
+ * and the counts run as kernels over the whole GPU. */
+bool tail_whole(const DevMesh &m);
+void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s);
+void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s);
+void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
+void launch_tail_fix(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s);
 
 /* check_data on the device (sevc_check.cu): violations counted into *out */
@@ -174,12 +169,8 @@ void launch_grain_stats(const DevMesh &m, int lo, int hi, double *out, cudaStrea
 
 /* kernels launched by this process (reported per step) */
 extern long long sevc_kernel_launches;
-/* set while launches must go without the programmatic-serialisation
- * attribute (a whole stretch of capture); sevc_pdl_skip counts the next
- * launches that must (the first kernel of a conditional node's body and
- * the first kernel after a conditional node, whose predecessor is not a
- * kernel) */
-extern thread_local bool sevc_pdl_off;
+/* counts the next launches that must go without the programmatic-
+ * serialisation attribute (a kernel with two predecessors) */
 extern thread_local int sevc_pdl_skip;
 #define COUNT_LAUNCHES(k) (sevc_kernel_launches += (k))
 
@@ -201,7 +192,7 @@ inline void launch_dep(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cfg.attrs = at;
-    bool plain = sevc_pdl_off || sevc_pdl_skip > 0;
+    bool plain = sevc_pdl_skip > 0;
     if (sevc_pdl_skip > 0) sevc_pdl_skip--;
     cfg.numAttrs = plain ? 0 : 1;
     COUNT_LAUNCHES(1);

@@ -230,7 +230,6 @@ __device__ void init_vertex_dev(const DevMesh &m, int v, double2 p) /* init_vert
     m.ven[v] = 1;
     m.vg[v] = make_int4(-1, -1, -1, -1);
     m.vb[v] = make_int4(-1, -1, -1, -1);
-    m.voted[v] = -1;
     for (int j = 0; j < 4; j++) m.vmod[4 * (size_t)v + j] = make_int4(-1, -1, -1, FIX_NONE);
 }
 __device__ void init_boundary_dev(const DevMesh &m, int b, int ini, int end) /* init_boundary :491 */
@@ -377,7 +376,7 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
     int *L = m.glist + (size_t)SEVC_MAXV * g;              /* nucleate_grain :596 */
     for (int i = 0; i < SEVC_MAXV; i++) L[i] = -1;
     m.gvlen[g] = 0; m.garea[g] = 0; m.gse[g] = 0; m.gori[g] = 0;
-    m.gen[g] = 1; m.gcand[g] = 0; m.gfix[g] = 0; m.gtype[g] = GT_NUCLEATED;
+    m.gen[g] = 1; m.gfix[g] = 0; m.gtype[g] = GT_NUCLEATED;
     m.gori[g] = nucl_ori;
     L[0] = A; L[1] = B; L[2] = C;
     m.gvlen[g] = 3;

@@ -1,24 +1,27 @@
 /*
  * Topological transitions of one time step (src/topological.h of the
- * reference): candidate compaction, the polling system, conflict
- * resolution, removal of adjacent 3-sided pairs, 3-sided grain removal,
- * T1 flips and the deferred grain-list edits.
+ * reference): the polling system, conflict resolution, removal of adjacent
+ * 3-sided pairs, 3-sided grain removal, T1 flips and the deferred grain-list
+ * edits.
  *
- * Candidates are gathered by an order-preserving warp-ballot compaction,
- * so every later pass touches only the few boundaries and grains that can
- * change.  Edits whose order is observable run in ascending index order,
- * like the reference's single-thread kernels; the list edits
- * (ADD -> REMOVE -> REPLACE) touch only the grain being edited and run one
- * thread per grain, which gives the reference's serial result.
+ * All of it works on short lists (the candidates the t_ext labels append,
+ * the 3-sided grains the grain pass lists, the grains an event queues), and
+ * it is a chain of about twenty dependent phases.  One thread-block cluster
+ * runs the chain: a phase boundary is the cluster's hardware barrier
+ * instead of a kernel launch, and the polling and 2x3 loops are loops (see
+ * k_tail).  Edits whose order is observable have the result of the
+ * reference's ascending index order; the list edits (ADD -> REMOVE ->
+ * REPLACE) touch only the grain being edited and run one warp per grain,
+ * which gives the reference's serial result.
  */
-#include "sevc_internal.h"
+#include "sevc_tail.cuh"
 
 namespace {
 
 constexpr int TPB = 256;
-constexpr int CT_ITEMS = 16;
-constexpr int CT_TILE = TPB * CT_ITEMS;
 constexpr int WL_BLOCKS = 152;
+/* the cluster of the sparse phases */
+constexpr int TAIL_BLOCKS = 16, TAIL_TPB = 512, TAIL_WARPS = TAIL_TPB / 32;
 
 /* ------------------------------------------------------------------ */
 /* grain-list primitives, src/geometry.h:614-734                       */
@@ -41,38 +44,6 @@ __device__ int glist_consecutive(const DevMesh &m, int g, int A, int B) /* :724 
     }
     return -1;
 }
-__device__ void glist_add_after(const DevMesh &m, int g, int v, int prev) /* :629 */
-{
-    int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g], pos = -1;
-    for (int i = 0; i < n; i++)
-        if (L[i] == prev) { pos = i + 1; break; }
-    if (pos < 0) { raise_err(m, ERRB_TOPOLOGY); return; }
-    if (n >= SEVC_MAXV) { raise_err(m, ERRB_CAPACITY); return; }
-    for (int i = n; i > pos; i--) L[i] = L[i - 1];
-    L[pos] = v;
-    m.gvlen[g] = n + 1;
-}
-__device__ void glist_remove(const DevMesh &m, int g, int v)      /* :653 */
-{
-    int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    for (int i = 0; i < n; i++)
-        if (L[i] == v) {
-            for (int j = i; j < n - 1; j++) L[j] = L[j + 1];
-            m.gvlen[g] = n - 1;
-            L[n - 1] = -1;
-            return;
-        }
-}
-__device__ void glist_replace(const DevMesh &m, int g, int oldv, int newv) /* :686 */
-{
-    int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    for (int i = 0; i < n; i++)
-        if (L[i] == oldv) { L[i] = newv; return; }
-}
-
 /* Set flags[i] (a 0/1 byte) to 1; true for the one caller that changed
  * it.  Events that run concurrently may queue the same grain. */
 __device__ __forceinline__ bool claim_byte(uint8_t *flags, int i)
@@ -107,303 +78,139 @@ __device__ void set_mod(const DevMesh &m, int v, int slot, int fix, int grn, int
 }
 
 /* ------------------------------------------------------------------ */
-/* order-preserving compaction                                         */
+/* the team: one cluster                                               */
 /* ------------------------------------------------------------------ */
-template <int KIND>
-__device__ __forceinline__ bool pred(const DevMesh &m, int i)
-{
-    if (KIND == CK_CAND) return m.ben[i] && m.bcand[i];
-    if (KIND == CK_GRAIN_CAND) return m.gen[i] && m.gcand[i];
-    if (KIND == CK_GVLEN3) return m.gvlen[i] == 3;
-    if (KIND == CK_MARKED) return m.bmark[i] != 0;
-    /* CK_TWO_THREE: enabled boundary whose two common grains both have
-     * three vertices (src/topological.h:31-35, :970-974) */
-    if (!m.ben[i]) return false;
-    int2 e = m.bv[i];
-    int gic[2];
-    if (gintersect(m.vg[e.x], m.vg[e.y], gic) < 2) return false;
-    return m.gvlen[gic[0]] == 3 && m.gvlen[gic[1]] == 3;
-}
+/* Every thread of the cluster's blocks; a phase ends at sync(): what any
+ * thread wrote before it, any thread reads after it (release / acquire at
+ * cluster scope).  The grid is exactly one cluster. */
+struct Team {
+    int tid, n;            /* thread of the team, threads */
+    int warp, nwarps, lane;
+    __device__ Team()
+    {
+        tid = blockIdx.x * blockDim.x + threadIdx.x;
+        n = gridDim.x * blockDim.x;
+        warp = tid >> 5;
+        nwarps = n >> 5;
+        lane = tid & 31;
+    }
+    __device__ __forceinline__ void sync() const
+    {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    }
+};
 
-template <int KIND>
-__global__ void k_compact_count(DevMesh m, int n, int *blockcnt)
+/* ids[0..n) (distinct) in ascending order into out, by rank; the caller
+ * syncs.  Short lists: the reference's serial order of rare events. */
+__device__ void rank_sort(const Team &T, const int *ids, int n, int *out)
 {
-    int base = blockIdx.x * CT_TILE, c = 0;
-    for (int k = 0; k < CT_ITEMS; k++) {
-        int i = base + k * TPB + threadIdx.x;
-        if (i < n && pred<KIND>(m, i)) c++;
+    for (int i = T.tid; i < n; i += T.n) {
+        int v = ids[i], r = 0;
+        for (int j = 0; j < n; j++) r += ids[j] < v;
+        out[r] = v;
     }
-    __shared__ int s[TPB / 32];
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < TPB / 32; w++) t += s[w];
-        blockcnt[blockIdx.x] = t;
-    }
-}
-
-template <int KIND>
-__global__ void k_compact_scatter(DevMesh m, int n, const int *blockcnt, int *out, int *n_out)
-{
-    __shared__ int s[TPB / 32 + 1];
-    __shared__ int base_off;
-    int part = 0;
-    for (int j = threadIdx.x; j < (int)blockIdx.x; j += TPB) part += blockcnt[j];
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < TPB / 32; w++) t += s[w];
-        base_off = t;
-    }
-    __syncthreads();
-    int off = base_off;
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < CT_ITEMS; k++) {
-        int i = blockIdx.x * CT_TILE + k * TPB + threadIdx.x;
-        bool f = i < n && pred<KIND>(m, i);
-        unsigned bal = __ballot_sync(0xffffffffu, f);
-        __syncthreads();
-        if (lane == 0) s[warp] = __popc(bal);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int acc = 0;
-            for (int w = 0; w < TPB / 32; w++) { int t = s[w]; s[w] = acc; acc += t; }
-            s[TPB / 32] = acc;
-        }
-        __syncthreads();
-        if (f) out[off + s[warp] + __popc(bal & ((1u << lane) - 1))] = i;
-        off += s[TPB / 32];
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *n_out = off;
-}
-
-/* The same compaction for the kinds whose predicate is a byte flag (or the
- * AND of two): each thread owns 16 consecutive items, read as one 16-byte
- * word per flag array, so a tile costs one round trip to memory instead of
- * sixteen.  Items keep ascending order (thread order, then bit order).
- * Flag arrays are allocated in 256-byte multiples, so the word of the last
- * partial group stays inside its allocation; items >= n are masked off. */
-template <int KIND>
-__device__ __forceinline__ unsigned flag_mask16(const DevMesh &m, int i0, int n)
-{
-    const uint8_t *a = KIND == CK_CAND ? m.ben : (KIND == CK_GRAIN_CAND ? m.gen : m.bmark);
-    uint4 w = *reinterpret_cast<const uint4 *>(a + i0);
-    if constexpr (KIND == CK_CAND || KIND == CK_GRAIN_CAND) {
-        const uint8_t *b = KIND == CK_CAND ? m.bcand : m.gcand;
-        uint4 v = *reinterpret_cast<const uint4 *>(b + i0);
-        w.x &= v.x; w.y &= v.y; w.z &= v.z; w.w &= v.w;   /* flags are 0 / 1 */
-    }
-    unsigned q[4] = { w.x, w.y, w.z, w.w }, mask = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            mask |= (((q[j] >> (8 * k)) & 0xffu) != 0u ? 1u : 0u) << (4 * j + k);
-    int valid = n - i0;
-    return valid >= 16 ? mask : (mask & ((1u << valid) - 1u));
-}
-template <int KIND>
-__global__ void k_flag_count(DevMesh m, int n, int *blockcnt)
-{
-    griddep_wait();
-    int i0 = (blockIdx.x * TPB + threadIdx.x) * CT_ITEMS;
-    int c = i0 < n ? __popc(flag_mask16<KIND>(m, i0, n)) : 0;
-    __shared__ int s[TPB / 32];
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < TPB / 32; w++) t += s[w];
-        blockcnt[blockIdx.x] = t;
-    }
-}
-template <int KIND>
-__global__ void k_flag_scatter(DevMesh m, int n, const int *blockcnt, int *out, int *n_out)
-{
-    griddep_wait();
-    __shared__ int s[TPB / 32];
-    __shared__ int base_off, tot;
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int part = 0;
-    for (int j = threadIdx.x; j < (int)blockIdx.x; j += TPB) part += blockcnt[j];
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-    if (lane == 0) s[warp] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < TPB / 32; w++) t += s[w];
-        base_off = t;
-    }
-    __syncthreads();
-    int i0 = (blockIdx.x * TPB + threadIdx.x) * CT_ITEMS;
-    unsigned mask = i0 < n ? flag_mask16<KIND>(m, i0, n) : 0u;
-    int c = __popc(mask), incl = c;
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) s[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int w = 0; w < TPB / 32; w++) { int t = s[w]; s[w] = acc; acc += t; }
-        tot = acc;
-    }
-    __syncthreads();
-    int pos = base_off + s[warp] + incl - c;
-    while (mask) {
-        int k = __ffs(mask) - 1;
-        mask &= mask - 1;
-        out[pos++] = i0 + k;
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *n_out = base_off + tot;
 }
 
 /* ------------------------------------------------------------------ */
 /* polling system, src/topological.h:362-578                           */
 /* ------------------------------------------------------------------ */
-/* vertices_vote (:362) for the endpoints of listed boundaries; it also
- * zeroes the iteration's count of unconverged instances (the previous
- * iteration's was read before this kernel starts) */
-__global__ void k_poll_vote(DevMesh m, const int *list, const int *n, int *nrun)
+/* vertices_vote (:362) for one vertex: its boundary with the smallest
+ * extinction time among the candidates (the last such slot) */
+__device__ int vertex_vote(const DevMesh &m, int v)
 {
-    griddep_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nrun = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
-    if (m.pdone[m.binst[list[i]]]) continue;
-    int2 e = m.bv[list[i]];
-    for (int k = 0; k < 2; k++) {
-        int v = k == 0 ? e.x : e.y;
-        if (!m.ven[v]) continue;
-        int4 sb = m.vb[v];
-        double mt = 99999999;
-        int am = 0;
-        for (int j = 0; j < 3; j++) {
-            int b = slot3(sb, j);
-            if (m.btext[b] <= mt && m.bcand[b]) { mt = m.btext[b]; am = j; }
-        }
-        m.voted[v] = slot3(sb, am);
+    if (!m.ven[v]) return -1;
+    int4 sb = m.vb[v];
+    double mt = 99999999;
+    int am = 0;
+    for (int j = 0; j < 3; j++) {
+        int b = slot3(sb, j);
+        if (m.btext[b] <= mt && m.bcand[b]) { mt = m.btext[b]; am = j; }
     }
+    return slot3(sb, am);
+}
+
+/* One polling loop (:549-578) over the candidate list.  An iteration:
+ *   votes    vertices_vote and count_boundaries_votes (:406): whether both
+ *            ends of a candidate vote for it
+ *   unlabel  (:441) a two-vote candidate clears its neighbours.  It is never
+ *            adjacent to another two-vote candidate (their shared vertex
+ *            votes once), so the parallel writes change no decision.
+ *   compare  write_candidate_results (:466-477) and flips_per_block
+ *            (:486-511): a mismatch marks its thread of the reference's grid
+ *            (poll_fail).  Only listed boundaries can mismatch here: the
+ *            t_ext labels compared and wrote every other one, whose flag no
+ *            iteration changes.
+ *   result   compare_candidates (:526-537): an instance with no block whose
+ *            threads all failed has converged and takes no further
+ *            iteration this step
+ * Leaves the marks to the caller (poll_reset). */
+__device__ void poll_reset(const DevMesh &m, const DevScratch &x, const Team &T, const PollGrid &pg, int nfail)
+{
+    for (int i = T.tid; i < nfail; i += T.n) {
+        int b = x.list_c[i], inst = m.binst[b], t = (b - m.boff[inst]) % pg.threads();
+        x.threadfail[(size_t)inst * pg.threads() + t] = 0;
+        x.pblock[(size_t)inst * pg.blocks + t / pg.tpb] = 0;
     }
+    for (int i = T.tid; i < m.ninst; i += T.n) x.pcnt[i] = 0;
+    if (T.tid == 0) *x.n_fail = 0;
 }
-/* count_boundaries_votes (:406) */
-__global__ void k_poll_count(DevMesh m, const int *list, const int *n)
+__device__ int poll_loop(const DevMesh &m, const DevScratch &x, const Team &T, const PollGrid &pg, int cap)
 {
-    griddep_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
-        int b = list[i];
-        if (!(m.ben[b] && m.bcand[b]) || m.pdone[m.binst[b]]) continue;
-        int2 e = m.bv[b];
-        m.bvotes[b] = (m.voted[e.x] == b) + (m.voted[e.y] == b);
-    }
-}
-/* unlabel (:441).  A two-vote candidate is never adjacent to another
- * two-vote candidate (their shared vertex votes once), so the parallel
- * writes cannot change any thread's decision. */
-__global__ void k_poll_unlabel(DevMesh m, const int *list, const int *n)
-{
-    griddep_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
-        int b = list[i];
-        if (!(m.ben[b] && m.bcand[b] && m.bvotes[b] == 2) || m.pdone[m.binst[b]]) continue;
-        int2 e = m.bv[b];
-        int4 si = m.vb[e.x], se = m.vb[e.y];
-        for (int j = 0; j < 3; j++) {
-            int x = slot3(si, j), y = slot3(se, j);
-            if (x != b) m.bcand[x] = 0;
-            if (y != b) m.bcand[y] = 0;
-        }
-    }
-}
-/* flips_per_block (:486-511) part one: a mismatch of boundary b marks
- * grid thread (b mod grid) as failed, b counted within its instance; then
- * write_candidate_results (:466-477) for the same element. */
-__global__ void k_poll_compare_write(DevMesh m, int *threadfail, int grid)
-{
-    griddep_wait();
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= m.nb) return;
-    int inst = m.binst[b];
-    if (m.pdone[inst]) return;
-    uint8_t en = m.ben[b], c = m.bcand[b];
-    if (en && c != m.bcandbuf[b]) threadfail[(size_t)inst * grid + (b - m.boff[inst]) % grid] = 1;
-    m.bcandbuf[b] = en ? c : 0;
-}
-/* The same for a single instance: 16 consecutive boundaries per thread,
- * the three flag arrays read and the buffer written as 16-byte words
- * (allocations are 256-byte multiples; bytes past nb are written back
- * unchanged).  grid >= 16. */
-__global__ void k_poll_compare_write16(DevMesh m, int *threadfail, int grid)
-{
-    griddep_wait();
-    int b0 = (blockIdx.x * blockDim.x + threadIdx.x) * 16;
-    if (b0 >= m.nb || m.pdone[0]) return;
-    uint4 we = *reinterpret_cast<const uint4 *>(m.ben + b0);
-    uint4 wc = *reinterpret_cast<const uint4 *>(m.bcand + b0);
-    uint4 wb = *reinterpret_cast<const uint4 *>(m.bcandbuf + b0);
-    unsigned e4[4] = { we.x, we.y, we.z, we.w }, c4[4] = { wc.x, wc.y, wc.z, wc.w }, b4[4] = { wb.x, wb.y, wb.z, wb.w };
-    int slot = b0 % grid;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        unsigned nb4 = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            int i = 4 * j + k;
-            unsigned e = (e4[j] >> (8 * k)) & 0xffu, c = (c4[j] >> (8 * k)) & 0xffu, o = (b4[j] >> (8 * k)) & 0xffu;
-            unsigned nbyte = o;
-            if (b0 + i < m.nb) {
-                if (e && c != o) {
-                    int t = slot + i;
-                    threadfail[t >= grid ? t - grid : t] = 1;
-                }
-                nbyte = e ? c : 0u;
+    const int *list = x.list_a;
+    const int n = *x.n_a;
+    for (int it = 1;; it++) {
+        if (n > 0) {
+            for (int i = T.tid; i < n; i += T.n) {
+                int b = list[i];
+                if (!(m.ben[b] && m.bcand[b]) || m.pdone[m.binst[b]]) continue;
+                int2 e = m.bv[b];
+                m.bvotes[b] = vertex_vote(m, e.x) == b && vertex_vote(m, e.y) == b ? 2 : 0;
             }
-            nb4 |= nbyte << (8 * k);
+            T.sync();
+            for (int i = T.tid; i < n; i += T.n) {
+                int b = list[i];
+                if (!(m.ben[b] && m.bcand[b] && m.bvotes[b] == 2) || m.pdone[m.binst[b]]) continue;
+                int2 e = m.bv[b];
+                int4 si = m.vb[e.x], se = m.vb[e.y];
+                for (int j = 0; j < 3; j++) {
+                    int u = slot3(si, j), w = slot3(se, j);
+                    if (u != b) m.bcand[u] = 0;
+                    if (w != b) m.bcand[w] = 0;
+                }
+            }
+            T.sync();
+            for (int i = T.tid; i < n; i += T.n) {
+                int b = list[i];
+                if (m.pdone[m.binst[b]]) continue;
+                uint8_t en = m.ben[b], c = m.bcand[b];
+                if (en && c != m.bcandbuf[b]) poll_fail(m, x, pg, b);
+                m.bcandbuf[b] = en ? c : 0;
+            }
+            T.sync();
         }
-        b4[j] = nb4;
+        /* every block forms the result for itself; block 0 records it (the
+         * others see an instance it marks as done either way) */
+        bool run = false;
+        for (int i = threadIdx.x; i < m.ninst; i += blockDim.x) {
+            if (m.pdone[i]) continue;
+            bool again = x.pcnt[i] != 0;
+            run |= again;
+            if (blockIdx.x == 0) {
+                x.piters[i]++;
+                if (!again) m.pdone[i] = 1;
+            }
+        }
+        run = __syncthreads_or(run);
+        const int nfail = *x.n_fail;
+        if (run && it >= cap) {
+            if (T.tid == 0) atomicOr(m.err, ERRB_NONCONVERGED);
+            run = false;
+        }
+        if (!run) return nfail;
+        T.sync();
+        poll_reset(m, x, T, pg, nfail);
+        T.sync();
     }
-    *reinterpret_cast<uint4 *>(m.bcandbuf + b0) = make_uint4(b4[0], b4[1], b4[2], b4[3]);
-}
-/* part two, on the reference's grid (blockIdx.y = instance): per thread
- * AND over its stride set (already folded into threadfail), per block the
- * shared-memory tree whose bool += acts as OR (compare_candidates
- * :526-537); then, in the instance's last block to finish, the host's AND
- * over blocks (:533-535): an instance whose blocks all passed has
- * converged and takes no further iteration this step */
-__global__ void k_poll_final(DevMesh m, int *threadfail, int *pblock, int *pcnt, int *piters, int *nrun)
-{
-    griddep_wait();
-    __shared__ int t[256];
-    __shared__ int last;
-    int inst = blockIdx.y;
-    if (m.pdone[inst]) return;                       /* uniform over the instance's blocks */
-    size_t tid = (size_t)inst * gridDim.x * blockDim.x + blockIdx.x * blockDim.x + threadIdx.x;
-    t[threadIdx.x] = threadfail[tid] ? 0 : 1;
-    threadfail[tid] = 0;
-    __syncthreads();
-    for (int i = blockDim.x / 2; i != 0; i /= 2) {
-        if ((int)threadIdx.x < i) t[threadIdx.x] = (t[threadIdx.x] || t[threadIdx.x + i]) ? 1 : 0;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        pblock[(size_t)inst * gridDim.x + blockIdx.x] = t[0];
-        __threadfence();
-        last = atomicAdd(pcnt + inst, 1) == (int)gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    pcnt[inst] = 0;
-    __threadfence();
-    piters[inst]++;
-    int ok = 1;
-    for (int i = 0; i < (int)gridDim.x; i++) ok &= __ldcg(pblock + (size_t)inst * gridDim.x + i) != 0;
-    if (ok) m.pdone[inst] = 1;
-    else atomicAdd(nrun, 1);
 }
 
 /* ------------------------------------------------------------------ */
@@ -437,11 +244,9 @@ __device__ void conflict_check_one(const DevMesh &m, int b)
  * to a candidate (the only ones it can mark); one thread per candidate and
  * slot of its ends, so the six neighbours' load chains run side by side
  * (every visit of a boundary writes the same winner) */
-__global__ void k_conflict_check(DevMesh m, const int *list, const int *n)
+__device__ void conflict_check(const DevMesh &m, const Team &T, const int *list, int n)
 {
-    griddep_wait();
-    const int total = 6 * *n;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    for (int t = T.tid; t < 6 * n; t += T.n) {
         int i = t / 6, r = t - 6 * i;
         int c = list[i];
         if (!(m.ben[c] && m.bcand[c])) continue;
@@ -450,10 +255,9 @@ __global__ void k_conflict_check(DevMesh m, const int *list, const int *n)
         if (b != c) conflict_check_one(m, b);
     }
 }
-__global__ void k_conflict_unlabel(DevMesh m, const int *list, const int *n)
+__device__ void conflict_unlabel(const DevMesh &m, const Team &T, const int *list, int n)
 {
-    griddep_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < *n; i += gridDim.x * blockDim.x) {
+    for (int i = T.tid; i < n; i += T.n) {
         int b = list[i];
         if (!(m.ben[b] && m.bcand[b])) continue;
         int2 e = m.bv[b];
@@ -531,23 +335,41 @@ __device__ bool two_three_qualifies(const DevMesh &m, int b, int *gic)
     return m.gvlen[gic[0]] == 3 && m.gvlen[gic[1]] == 3;
 }
 
-/* The step's first 2x3 count: a qualifying boundary lies on two 3-sided
- * grains, so only the boundaries at the vertices of the 3-sided grains
- * (listed by this step's grain pass) are tested; the ordered
- * compaction of the marks then gives the same ascending list as testing
- * every boundary. */
-__global__ void k_mark_two_three(DevMesh m, const int *three, const int *n_three)
+/* Qualifying boundaries among those at the vertices of the 3-sided grains
+ * a[0..na) and then b[0..): a qualifying boundary lies on two of them, so testing these
+ * gives every one; each is appended once, by the smaller of its two grains
+ * at its first end.  t: one (grain, vertex, slot). */
+__device__ __forceinline__ void find_two_three(const DevMesh &m, const int *a, int na, const int *b, int t, int *out,
+                                               int *n_out)
 {
-    const int n3 = *n_three;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        const int *L = m.glist + (size_t)SEVC_MAXV * three[i];
-        for (int k = 0; k < 3; k++) {
-            int4 s = m.vb[L[k]];
-            for (int j = 0; j < 3; j++) {
-                int b = slot3(s, j), gic[2];
-                if (two_three_qualifies(m, b, gic)) m.bmark[b] = 1;
-            }
-        }
+    int i = t / 9, r = t - 9 * i, k = r / 3, j = r - 3 * k, g = i < na ? a[i] : b[i - na];
+    if (!m.gen[g] || m.gvlen[g] != 3) return;
+    int v = m.glist[(size_t)SEVC_MAXV * g + k], e = slot3(m.vb[v], j), gic[2];
+    if (m.bv[e].x != v || !two_three_qualifies(m, e, gic)) return;
+    if (g == (gic[0] < gic[1] ? gic[0] : gic[1])) out[atomicAdd(n_out, 1)] = e;
+}
+/* The step's first 2x3 count (topological.h:228), from the 3-sided grains
+ * the grain pass listed.  The last block then decides whether the step
+ * computes every output-only value (extinction times of all boundaries,
+ * dA/dt of all grains): when it can export or is asked to (flags[1], set by
+ * the host), or when it could end at the stop threshold (a final export):
+ * every removal takes a 3-sided grain, and a pass of the 2x3 loop can make
+ * at most two per pair; the bound is generous, as the threshold is crossed
+ * once per run.  Else only what the step can observe is computed.  flags[0]
+ * = the decision, taken on the device so that no host round trip separates
+ * the step's first half from its second. */
+__global__ void k_two_three_first(DevMesh m, DevScratch x)
+{
+    const int n3 = *x.n_three;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 9 * n3; t += gridDim.x * blockDim.x)
+        find_two_three(m, x.three, n3, nullptr, t, x.list_b, x.n_b);
+    const bool last = last_block(m.lastblk + 2);
+    if (last && threadIdx.x == 0) {
+        __threadfence();
+        int mg = x.flags[2], curr = x.flags[3];
+        long long reach = (long long)curr - n3 - 40LL * __ldcg(x.n_b) - 64;
+        x.flags[0] = x.flags[1] || (mg > 0 && reach <= mg);
+        *m.stamp += 1;   /* a new step: every value saved by the last step's events is stale */
     }
 }
 
@@ -564,16 +386,12 @@ __device__ bool sorted_contains(const int *a, int lo, int hi, int x)
 /* remove_two_grains_configurations (:965-985) is one thread scanning every
  * boundary in index order.  Only listed boundaries (those qualifying at the
  * count) and boundaries re-wired during the scan (CE) can qualify, so the
- * scan visits exactly those, in index order, re-testing each on visit. */
-/* One thread per instance, each over its own part of the ascending list. */
-__global__ void k_remove_two_three(DevMesh m, const int *list, const int *n, int *extra, int *segcnt,
-                                   const int *pass_dev)
+ * scan visits exactly those, in index order, re-testing each on visit.
+ * One thread per instance, each over its own part of the ascending list. */
+__device__ void remove_two_three(const DevMesh &m, const int *list, int n, int *extra, int *segcnt, int inst)
 {
-    int inst = blockIdx.x * blockDim.x + threadIdx.x;
-    if (inst >= m.ninst) return;
-    if (pass_dev) segcnt += (size_t)*pass_dev * m.ninst;
-    int i = lower_bound_i(list, *n, m.boff[inst]);
-    int N = lower_bound_i(list, *n, m.boff[inst + 1]);
+    int i = lower_bound_i(list, n, m.boff[inst]);
+    int N = lower_bound_i(list, n, m.boff[inst + 1]);
     segcnt[inst] = N - i;
     extra += (size_t)inst * EXTRA_CAP;
     int *evt = m.evt + EVT_COUNT * inst;
@@ -647,69 +465,6 @@ __device__ uint8_t label3_cand(const DevMesh &m, int g, double dt)
     }
     return cand || ans / 2 == 3;
 }
-/* clear_grains_state + label_3sided_grains for enabled grains */
-__global__ void k_label_3sided(DevMesh m, double dt)
-{
-    griddep_wait();
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= m.ng || !m.gen[g]) return;
-    m.gcand[g] = m.gvlen[g] == 3 ? label3_cand(m, g, dt) : 0;
-}
-/* The same when no list changed since this step's grain pass: only the
- * 3-sided grains it listed are visited.  Every other enabled grain
- * already has gcand = 0, because each step clears the flag of every grain
- * it listed as a candidate (k_remove_reserve). */
-__global__ void k_label_3sided_bucket(DevMesh m, double dt, const int *three, const int *n_three)
-{
-    griddep_wait();
-    const int n3 = *n_three;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        int g = three[i];
-        m.gcand[g] = label3_cand(m, g, dt);
-    }
-}
-/* either of the two above, as the step's first 2x3 count says: no 2x3
- * removal (count 0) leaves every list as the grain pass saw it */
-__global__ void k_label_3sided_auto(DevMesh m, double dt, const int *three, const int *n_three, const int *tt_first)
-{
-    griddep_wait();
-    if (*tt_first == 0) {
-        const int n3 = *n_three;
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-            int g = three[i];
-            m.gcand[g] = label3_cand(m, g, dt);
-        }
-    } else {
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < m.ng; g += gridDim.x * blockDim.x)
-            if (m.gen[g]) m.gcand[g] = m.gvlen[g] == 3 ? label3_cand(m, g, dt) : 0;
-    }
-}
-/* loop control of the whole-step graph (one thread) */
-__global__ void k_poll_cond(cudaGraphConditionalHandle hnd, const int *nrun, int *ptot, int cap, int *err)
-{
-    if (threadIdx.x) return;
-    int it = ++*ptot;
-    bool run = *nrun > 0;
-    if (run && it >= cap) {
-        atomicOr(err, ERRB_NONCONVERGED);
-        run = false;
-    }
-    cudaGraphSetConditional(hnd, run ? 1u : 0u);
-}
-__global__ void k_tt_init(cudaGraphConditionalHandle hnd, const int *n, int *first, int *pass)
-{
-    if (threadIdx.x) return;
-    *first = *n;
-    *pass = 0;
-    cudaGraphSetConditional(hnd, *n > 0 ? 1u : 0u);
-}
-__global__ void k_tt_cond(cudaGraphConditionalHandle hnd, const int *n, int *pass)
-{
-    if (threadIdx.x) return;
-    int p = ++*pass;
-    cudaGraphSetConditional(hnd, (*n > 0 && p < TWO_THREE_PASSES) ? 1u : 0u);
-}
-
 /* remove_grain (:687-822) */
 __device__ void remove_grain_dev(const DevMesh &m, int grn)
 {
@@ -790,7 +545,7 @@ __device__ void remove_grain_dev(const DevMesh &m, int grn)
 /* ------------------------------------------------------------------ */
 /* The reference applies the 3-sided removals one at a time in ascending
  * grain order (remove_grains <<<1,1>>>, :994) and defines no order for the
- * flips; here both phases follow ascending list order.  An event reads and
+ * flips; here both phases follow ascending index order.  An event reads and
  * writes only its footprint (its vertices and the boundaries in their
  * slots) plus grain-level records that commute: queueing a grain for the
  * fix-up (an atomic claim of its flag), its mod slots (per vertex) and the
@@ -798,20 +553,21 @@ __device__ void remove_grain_dev(const DevMesh &m, int grn)
  * of the phase runs).  Two events with disjoint footprints therefore
  * commute, and the serial result is obtained by deterministic reservation:
  *   reserve  every event writes its key into each footprint record
- *            (atomicMin); the key orders events by list position;
+ *            (atomicMin); the key orders events by grain or boundary index,
+ *            the serial order (the lists themselves are in any order);
  *   apply    an event that holds every one of its records shares none
  *            with an earlier event: it runs at once, all such in parallel;
  *            any other is deferred;
- *   deferred the deferred events run one at a time in list order, after
+ *   deferred the deferred events run one at a time in index order, after
  *            the parallel ones; each shares records only with earlier
  *            events, which have all run (in parallel or before it here),
  *            and commutes with every later parallel one.
  * Keys carry a per-phase epoch in their high half that grows every step,
  * so records never need clearing: an earlier step's key is larger and is
  * replaced by the first reservation of a later step. */
-__device__ __forceinline__ unsigned long long resv_key(unsigned epoch, int pos)
+__device__ __forceinline__ unsigned long long resv_key(unsigned epoch, int id)
 {
-    return ((unsigned long long)(0xFFFFFFFFu - epoch) << 32) | (unsigned)pos;
+    return ((unsigned long long)(0xFFFFFFFFu - epoch) << 32) | (unsigned)id;
 }
 __device__ __forceinline__ bool valid_v(const DevMesh &m, int v) { return (unsigned)v < (unsigned)m.nv; }
 __device__ __forceinline__ bool valid_b(const DevMesh &m, int b) { return (unsigned)b < (unsigned)m.nb; }
@@ -903,86 +659,63 @@ __device__ bool holds_vertex(const DevMesh &m, const DevScratch &x, int v, unsig
     return true;
 }
 
-/* 3-sided removals (remove_grains, :994): a listed grain that is enabled
- * and a candidate is removed; a removal disables only its own grain, so
- * the set is known up front.  One warp per listed grain, which also
- * clears the grain's candidate flag (src/main.cu:260; nothing after this
- * test reads it this step). */
-__global__ void k_remove_reserve(DevMesh m, DevScratch x, const int *list, const int *n)
+/* 3-sided removals (remove_grains, :994) of the listed grains: a removal
+ * disables only its own grain, so the set is known up front.  One warp per
+ * grain: first every removal reserves its records, then its records are
+ * brought into L1 and lane 0 applies it (or it defers, when an earlier
+ * removal holds a record). */
+__device__ void remove_reserve(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
 {
-    griddep_wait();
     const unsigned ep = 2u * *m.stamp;
-    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < *n; i += nw) {
+    for (int i = T.warp; i < n; i += T.nwarps) {
         int g = list[i];
-        bool rm = m.gen[g] && m.gcand[g];
-        __syncwarp();
-        if (lane == 0) m.gcand[g] = 0;
-        if (!rm) continue;
         const int *L = m.glist + (size_t)SEVC_MAXV * g;
         int verts[3] = { L[0], L[1], L[2] };
-        reserve_warp(m, x, verts, 3, resv_key(ep, i), lane, true);
-        if (lane == 0) {
-            int p = atomicAdd(x.n_ehits, 1);
-            x.ehits[p] = i;
-        }
+        reserve_warp(m, x, verts, 3, resv_key(ep, g), T.lane, true);
     }
 }
-/* one warp per removal: its records are brought into L1, then lane 0
- * applies it (or defers it when an earlier removal holds a record) */
-__global__ void k_remove_apply(DevMesh m, DevScratch x, const int *list)
+__device__ void remove_apply(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
 {
-    griddep_wait();
     const unsigned ep = 2u * *m.stamp;
-    const int nh = *x.n_ehits;
-    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nh; t += nw) {
-        int i = x.ehits[t], g = list[i];
+    for (int i = T.warp; i < n; i += T.nwarps) {
+        int g = list[i];
         const int *L = m.glist + (size_t)SEVC_MAXV * g;
         int verts[3] = { L[0], L[1], L[2] };
-        unsigned long long key = resv_key(ep, i);
+        unsigned long long key = resv_key(ep, g);
         bool own = true;
-        if (lane == 0)
+        if (T.lane == 0)
             for (int k = 0; k < 3 && own; k++) own = valid_v(m, verts[k]) && holds_vertex(m, x, verts[k], key);
         own = __shfl_sync(0xffffffffu, own, 0);
-        if (own) prefetch_event(m, verts, 3, lane);
+        if (own) prefetch_event(m, verts, 3, T.lane);
         __syncwarp();
-        if (lane == 0) {
+        if (T.lane == 0) {
             if (own) {
                 remove_grain_dev(m, g);
                 atomicAdd(&m.evt[EVT_COUNT * m.ginst[g] + EVT_REMOVALS], 1);
             } else {
-                x.edefer[i] = 1;
-                atomicAdd(&x.ndefer[m.ginst[g]], 1);
+                x.ehits[atomicAdd(x.n_ehits, 1)] = g;
             }
         }
         __syncwarp();
     }
 }
-/* one warp per instance: its deferred removals in list order */
-__global__ void k_remove_deferred(DevMesh m, DevScratch x, const int *list, const int *n)
+/* The deferred events x.ehits[0..nd) in ascending order, one warp per
+ * instance over its own part (off: the instances' first indices). */
+template <class Apply>
+__device__ void run_deferred(const DevMesh &m, const DevScratch &x, const Team &T, int nd, const int *off, Apply apply)
 {
-    griddep_wait();
-    int inst = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (inst == 0 && lane == 0) *x.n_ehits = 0;
-    if (inst >= m.ninst || x.ndefer[inst] == 0) return;
-    int lo = lower_bound_i(list, *n, m.goff[inst]);
-    int hi = lower_bound_i(list, *n, m.goff[inst + 1]);
-    for (int base = lo; base < hi; base += 32) {
-        int i = base + lane;
-        bool f = i < hi && x.edefer[i];
-        unsigned hits = __ballot_sync(0xffffffffu, f);
-        if (lane == 0)
-            while (hits) {
-                int j = __ffs(hits) - 1;
-                hits &= hits - 1;
-                x.edefer[base + j] = 0;
-                remove_grain_dev(m, list[base + j]);
-                m.evt[EVT_COUNT * inst + EVT_REMOVALS]++;
-            }
-        __syncwarp();
+    int *sorted = x.list_b;               /* the 2x3 list, done with */
+    rank_sort(T, x.ehits, nd, sorted);
+    T.sync();
+    if (T.tid == 0) *x.n_ehits = 0;
+    for (int inst = T.warp; inst < m.ninst; inst += T.nwarps) {
+        int lo = 0, hi = nd;
+        if (m.ninst > 1) {
+            lo = lower_bound_i(sorted, nd, off[inst]);
+            hi = lower_bound_i(sorted, nd, off[inst + 1]);
+        }
+        for (int i = lo; i < hi; i++) apply(sorted[i], inst);
     }
-    if (lane == 0) x.ndefer[inst] = 0;
 }
 
 /* unlabel_boundaries_st2 (:588-606) for an enabled candidate b: it stays
@@ -1256,109 +989,53 @@ __device__ void flip_planned(const DevMesh &m, int bnd, double eps, const FlipPl
 
 /* apply_flippings (:1016-1026): the reference flips every remaining
  * candidate in parallel, with unsynchronised writes when two share
- * records; here flips follow ascending list (boundary) order, which is
- * every race-free outcome.  A flip changes no boundary's enabled or
- * candidate flag, so the flips are known up front.  Reservation, parallel
+ * records; here flips follow ascending boundary order, which is every
+ * race-free outcome.  A flip changes no boundary's enabled or candidate
+ * flag, so the flips are known up front.  Reservation, parallel
  * application and the deferred pass as for the removals (epoch 2 * stamp
  * + 1); the footprint is both ends with their slots. */
-__global__ void k_flip_reserve(DevMesh m, DevScratch x, const int *list, const int *n)
+__device__ void flip_reserve(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
 {
-    griddep_wait();
     const unsigned ep = 2u * *m.stamp + 1u;
-    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < *n; i += nw) {
+    for (int i = T.warp; i < n; i += T.nwarps) {
         int b = list[i];
         if (!(m.ben[b] && m.bcand[b])) continue;
         if (!unlabel_st2_keeps(m, b)) continue;
         int2 e = m.bv[b];
         int verts[2] = { e.x, e.y };
-        reserve_warp(m, x, verts, 2, resv_key(ep, i), lane, false);
-        if (lane == 0) {
-            int p = atomicAdd(x.n_ehits, 1);
-            x.ehits[p] = i;
-        }
+        reserve_warp(m, x, verts, 2, resv_key(ep, b), T.lane, false);
     }
 }
-/* one warp per flip: lanes prefetch its neighbourhood and derive the
- * plan, lane 0 applies it */
-__global__ void k_flip_apply(DevMesh m, DevScratch x, double eps, const int *list)
+/* a warp: its lanes prefetch the flip's neighbourhood and derive the plan,
+ * lane 0 applies it */
+__device__ void flip_warp(const DevMesh &m, int b, double eps, int lane)
 {
-    griddep_wait();
+    prefetch_flip(m, b, lane);
+    FlipPlan P;
+    bool planned = flip_plan(m, b, lane, P) && P.AC != P.BE;
+    __syncwarp();
+    if (lane == 0) {
+        if (planned) flip_planned(m, b, eps, P);
+        else flip_dev(m, b, eps);
+        atomicAdd(&m.evt[EVT_COUNT * m.binst[b] + EVT_FLIPS], 1);
+    }
+    __syncwarp();
+}
+__device__ void flip_apply(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n, double eps)
+{
     const unsigned ep = 2u * *m.stamp + 1u;
-    const int nh = *x.n_ehits;
-    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nh; t += nw) {
-        int i = x.ehits[t], b = list[i];
+    for (int i = T.warp; i < n; i += T.nwarps) {
+        int b = list[i];
+        if (!(m.ben[b] && m.bcand[b])) continue;
         int2 e = m.bv[b];
-        unsigned long long key = resv_key(ep, i);
+        unsigned long long key = resv_key(ep, b);
         bool own = false;
-        if (lane == 0)
+        if (T.lane == 0)
             own = valid_v(m, e.x) && valid_v(m, e.y) && holds_vertex(m, x, e.x, key) && holds_vertex(m, x, e.y, key);
         own = __shfl_sync(0xffffffffu, own, 0);
-        if (own) {
-            prefetch_flip(m, b, lane);
-            FlipPlan P;
-            bool planned = flip_plan(m, b, lane, P) && P.AC != P.BE;
-            __syncwarp();
-            if (lane == 0) {
-                if (planned) flip_planned(m, b, eps, P);
-                else flip_dev(m, b, eps);
-                atomicAdd(&m.evt[EVT_COUNT * m.binst[b] + EVT_FLIPS], 1);
-            }
-        } else if (lane == 0) {
-            x.edefer[i] = 1;
-            atomicAdd(&x.ndefer[m.binst[b]], 1);
-        }
-        __syncwarp();
+        if (own) flip_warp(m, b, eps, T.lane);
+        else if (T.lane == 0) x.ehits[atomicAdd(x.n_ehits, 1)] = b;
     }
-}
-/* One block per instance: its deferred flips in list order.  The block
- * tests FLIP_TPB entries at a time and warp 0 applies the deferred ones,
- * its lanes prefetching each flip's records. */
-constexpr int FLIP_TPB = 512;
-__global__ void __launch_bounds__(FLIP_TPB) k_flip_deferred(DevMesh m, DevScratch x, double eps, const int *list,
-                                                            const int *n)
-{
-    griddep_wait();
-    __shared__ unsigned hitmask[FLIP_TPB / 32];
-    int inst = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (inst == 0 && threadIdx.x == 0) *x.n_ehits = 0;
-    if (x.ndefer[inst] == 0) return;
-    int lo = 0, hi = *n;
-    if (m.ninst > 1) {
-        lo = lower_bound_i(list, hi, m.boff[inst]);
-        hi = lower_bound_i(list, hi, m.boff[inst + 1]);
-    }
-    for (int base = lo; base < hi; base += FLIP_TPB) {
-        int i = base + (int)threadIdx.x;
-        bool f = i < hi && x.edefer[i];
-        unsigned w = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) hitmask[warp] = w;
-        if (!__syncthreads_or(f)) continue;           /* the barrier also publishes hitmask */
-        if (warp == 0) {
-            for (int k = 0; k < FLIP_TPB / 32; k++) {
-                unsigned hits = hitmask[k];
-                while (hits) {
-                    int j = __ffs(hits) - 1;
-                    hits &= hits - 1;
-                    int b = list[base + 32 * k + j];
-                    prefetch_flip(m, b, lane);
-                    FlipPlan P;
-                    bool planned = flip_plan(m, b, lane, P) && P.AC != P.BE;
-                    __syncwarp();
-                    if (lane == 0) {
-                        x.edefer[base + 32 * k + j] = 0;
-                        if (planned) flip_planned(m, b, eps, P);
-                        else flip_dev(m, b, eps);
-                        m.evt[EVT_COUNT * inst + EVT_FLIPS]++;
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) x.ndefer[inst] = 0;
 }
 
 /* ------------------------------------------------------------------ */
@@ -1380,7 +1057,6 @@ __global__ void __launch_bounds__(FLIP_TPB) k_flip_deferred(DevMesh m, DevScratc
  * lanes write back every entry the passes touched.  The long chain of
  * dependent global reads of one thread per grain becomes one parallel
  * round and a few L1 hits. */
-constexpr int FIX_TPB = 256, FIX_WARPS = FIX_TPB / 32;
 __device__ __forceinline__ unsigned mod_ops_for(const DevMesh &m, int v, int g)
 {
     if ((unsigned)v >= (unsigned)m.nv) return 0;
@@ -1447,35 +1123,38 @@ __device__ void fix_grain_serial(const DevMesh &m, int g, int *Ls, unsigned char
         }
     }
 }
-__global__ void __launch_bounds__(FIX_TPB) k_fix_edit(DevMesh m)
+struct FixShared {
+    int Ls[TAIL_WARPS][SEVC_MAXV], Ss[TAIL_WARPS][SEVC_MAXV], Nw[TAIL_WARPS][2];
+    unsigned char Fs[TAIL_WARPS][SEVC_MAXV], SFs[TAIL_WARPS][SEVC_MAXV];
+};
+/* three, n_three (may be null): grains the edit leaves with three sides are
+ * listed there */
+__device__ void fix_edit(const DevMesh &m, const Team &T, FixShared &S, int *three, int *n_three)
 {
-    griddep_wait();
-    __shared__ int Ls[FIX_WARPS][SEVC_MAXV], Ss[FIX_WARPS][SEVC_MAXV];
-    __shared__ unsigned char Fs[FIX_WARPS][SEVC_MAXV], SFs[FIX_WARPS][SEVC_MAXV];
-    __shared__ int Nw[FIX_WARPS][2];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int nf = min(*m.nfix, m.fixcap), nw = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nf; w += nw) {
+    const int lane = T.lane, wib = threadIdx.x >> 5;
+    const int nf = min(*m.nfix, m.fixcap);
+    for (int w = T.warp; w < nf; w += T.nwarps) {
         const int g = m.fixlist[w];
         if (!(m.gen[g] && m.gfix[g])) continue;
         int *L = m.glist + (size_t)SEVC_MAXV * g;
         const int n = m.gvlen[g];
         for (int i = lane; i < n; i += 32) {
             int v = L[i];
-            Ls[wib][i] = v;
-            Fs[wib][i] = (unsigned char)mod_ops_for(m, v, g);
+            S.Ls[wib][i] = v;
+            S.Fs[wib][i] = (unsigned char)mod_ops_for(m, v, g);
         }
         __syncwarp();
         if (lane == 0) {
             int nn = n, hi = n;
-            fix_grain_serial(m, g, Ls[wib], Fs[wib], Ss[wib], SFs[wib], nn, hi);
-            Nw[wib][0] = nn;
-            Nw[wib][1] = hi;
+            fix_grain_serial(m, g, S.Ls[wib], S.Fs[wib], S.Ss[wib], S.SFs[wib], nn, hi);
+            S.Nw[wib][0] = nn;
+            S.Nw[wib][1] = hi;
             if (nn != n) m.gvlen[g] = nn;
+            if (n_three && nn == 3 && n != 3) three[atomicAdd(n_three, 1)] = g;
         }
         __syncwarp();
-        const int hi = Nw[wib][1];
-        for (int i = lane; i < hi; i += 32) L[i] = Ls[wib][i];
+        const int hi = S.Nw[wib][1];
+        for (int i = lane; i < hi; i += 32) L[i] = S.Ls[wib][i];
         __syncwarp();
     }
 }
@@ -1491,11 +1170,10 @@ __global__ void __launch_bounds__(FIX_TPB) k_fix_edit(DevMesh m)
  * passes, then the removals) is computed again by each, the last one on
  * the final positions.  The flips' fix-up comes after the counts and needs
  * none (the next step's grain pass computes every area). */
-__global__ void k_fix_clear(DevMesh m, int areas)
+__device__ void fix_clear(const DevMesh &m, const Team &T, bool areas)
 {
-    griddep_wait();
     int nf = min(*m.nfix, m.fixcap), nm = min(*m.nmod, m.modcap);
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nf; w += gridDim.x * blockDim.x) {
+    for (int w = T.tid; w < nf; w += T.n) {
         int g = m.fixlist[w];
         if (m.gen[g]) {
             m.gfix[g] = 0;
@@ -1505,7 +1183,7 @@ __global__ void k_fix_clear(DevMesh m, int areas)
             }
         }
     }
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nm; w += gridDim.x * blockDim.x) {
+    for (int w = T.tid; w < nm; w += T.n) {
         int v = m.modlist[w];
         m.vmodmark[v] = 0;
         int4 sg = m.vg[v];
@@ -1517,10 +1195,129 @@ __global__ void k_fix_clear(DevMesh m, int areas)
         if (listed)
             for (int j = 0; j < 4; j++) m.vmod[4 * (size_t)v + j] = make_int4(-1, -1, -1, FIX_NONE);
     }
-    /* empty both work lists once every block has read their lengths */
-    if (last_block(m.lastblk + 0) && threadIdx.x == 0) {
-        *m.nfix = 0;
-        *m.nmod = 0;
+}
+/* fix_grain_lists (:1209-1227): the edits, then the clearing; both work
+ * lists empty afterwards.  Ends with a sync. */
+__device__ void fix_lists(const DevMesh &m, const Team &T, FixShared &S, bool areas, int *three, int *n_three)
+{
+    if (*m.nfix == 0 && *m.nmod == 0) return;      /* the same in every block: written before the last sync */
+    fix_edit(m, T, S, three, n_three);
+    T.sync();
+    fix_clear(m, T, areas);
+    T.sync();
+    if (T.tid == 0) *m.nfix = *m.nmod = 0;
+    T.sync();
+}
+
+/* ------------------------------------------------------------------ */
+/* the sparse phases                                                   */
+/* ------------------------------------------------------------------ */
+/* the 2x3 loop (src/main.cu:227-250) from its first count, n > 0 */
+__device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team &T, FixShared &S)
+{
+    int *sorted = x.list_c;
+    int n = *x.n_b;
+    for (int pass = 0; n > 0 && pass < TWO_THREE_PASSES; pass++) {
+        rank_sort(T, x.list_b, n, sorted);
+        T.sync();
+        if (T.tid == 0) *x.n_b = 0;
+        for (int i = T.tid; i < m.ninst; i += T.n)
+            remove_two_three(m, sorted, n, x.extra, x.segcnt + (size_t)pass * m.ninst, i);
+        T.sync();
+        fix_lists(m, T, S, true, x.ehits, x.n_ehits);
+        const int n3 = *x.n_three, more = *x.n_ehits;
+        for (int t = T.tid; t < 9 * (n3 + more); t += T.n)
+            find_two_three(m, x.three, n3, x.ehits, t, x.list_b, x.n_b);
+        T.sync();
+        n = *x.n_b;
+    }
+}
+
+/* The part of a step after the t_ext labels (src/main.cu:219-325) as one
+ * launch of one cluster.  PART selects what a launch covers:
+ *   TAIL_REMOVE  polling (:219), conflicts (:222-225), the 2x3 loop
+ *                (:227-250), 3-sided labels (:252-255), removals (:259), list
+ *                fix-up with the areas after it (:262-266)
+ *   TAIL_FLIP    flips (:282-289)
+ *   TAIL_FIX     the flips' list fix-up (:294)
+ *   TAIL_END     position update (:314), counts (:317-325), step summary
+ *
+ * What bounds it: nothing but the chain of its phases, each a handful of
+ * dependent loads.  As ~25 kernels (programmatic dependent launch between
+ * them) and two conditional graph nodes the chain took 100-150 us a step; a
+ * cluster barrier costs well under a microsecond.  16 blocks of 512 are the
+ * largest cluster; with a warp per event that is 256 events at once. */
+constexpr int TAIL_WHOLE_NV = 64 * 1024;
+enum { TAIL_REMOVE = 1, TAIL_FLIP = 2, TAIL_FIX = 4, TAIL_END = 8 };
+template <int PART>
+__global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, PollGrid pg, int cap, double dt, double eps,
+                                                  int *summary)
+{
+    griddep_wait();
+    __shared__ FixShared S;
+    const Team T;
+    const int na = *x.n_a;
+    if (PART & TAIL_END)
+        for (int i = T.tid; i < m.ninst; i += T.n) x.counters[(size_t)i * CTR_COUNT + CTR_NGRAINS] = 0;
+    if (PART & TAIL_REMOVE) {
+        const int nfail = poll_loop(m, x, T, pg, cap);
+        if (na > 0) conflict_check(m, T, x.list_a, na);
+        T.sync();
+        if (na > 0) conflict_unlabel(m, T, x.list_a, na);
+        poll_reset(m, x, T, pg, nfail);
+        T.sync();
+        if (*x.n_b > 0) two_three_loop(m, x, T, S);
+        const int n3 = *x.n_three, more = *x.n_ehits;
+        for (int i = T.tid; i < n3 + more; i += T.n) {
+            int g = i < n3 ? x.three[i] : x.ehits[i - n3];
+            if (m.gen[g] && m.gvlen[g] == 3 && label3_cand(m, g, dt)) x.list_c[atomicAdd(x.n_c, 1)] = g;
+        }
+        T.sync();
+        const int nc = *x.n_c;
+        if (nc > 0) {
+            if (T.tid == 0) *x.n_ehits = 0;
+            remove_reserve(m, x, T, x.list_c, nc);
+            T.sync();
+            remove_apply(m, x, T, x.list_c, nc);
+            T.sync();
+            const int nd = *x.n_ehits;
+            if (nd > 0) {
+                run_deferred(m, x, T, nd, m.goff, [&](int g, int inst) {
+                    if (T.lane == 0) {
+                        remove_grain_dev(m, g);
+                        m.evt[EVT_COUNT * inst + EVT_REMOVALS]++;
+                    }
+                    __syncwarp();
+                });
+                T.sync();
+            }
+            fix_lists(m, T, S, true, nullptr, nullptr);
+        } else if (more > 0) {
+            T.sync();
+            if (T.tid == 0) *x.n_ehits = 0;
+            T.sync();
+        }
+    }
+    if ((PART & TAIL_FLIP) && na > 0) {
+        flip_reserve(m, x, T, x.list_a, na);
+        T.sync();
+        flip_apply(m, x, T, x.list_a, na, eps);
+        T.sync();
+        const int nd = *x.n_ehits;
+        if (nd > 0) {
+            run_deferred(m, x, T, nd, m.boff, [&](int b, int) { flip_warp(m, b, eps, T.lane); });
+            T.sync();
+        }
+    }
+    if (PART & TAIL_FIX) fix_lists(m, T, S, false, nullptr, nullptr);
+    if (PART & TAIL_END) {
+        for (int v = T.tid; v < m.nv; v += T.n) update_vertex(m, v, dt);
+        count_grains(m, x.counters, T.tid, T.n);
+        nucl_area_blocks(m, x.block_area, pg.blocks, pg.tpb, blockIdx.x, gridDim.x);
+        T.sync();
+        nucl_area_final(m, x.block_area, pg.blocks, x.counters, T.tid, T.n);
+        T.sync();
+        pack_summary(m, x, summary, T.tid, T.n);
     }
 }
 
@@ -1534,134 +1331,65 @@ __global__ void k_fill_instance_ids(DevMesh m)
         m.ginst[g] = lower_bound_i(m.goff, m.ninst + 1, g + 1) - 1;
 }
 
-template <int KIND>
-void compact_impl(const DevMesh &m, const DevScratch &x, int n, int *out, int *n_out, cudaStream_t s)
+/* k_tail<PART> as one cluster, after the previous kernel of the stream (or
+ * without programmatic serialisation, see launch_dep) */
+template <int PART>
+void launch_tail_part(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s)
 {
-    int tiles = (n + CT_TILE - 1) / CT_TILE;
-    if (tiles == 0) { cudaMemsetAsync(n_out, 0, sizeof(int), s); return; }
-    /* the 16-byte flag reads need 16-byte aligned arrays (the handle's
-     * allocation gives 256) */
-    uintptr_t al = KIND == CK_CAND ? ((uintptr_t)m.ben | (uintptr_t)m.bcand)
-                 : KIND == CK_GRAIN_CAND ? ((uintptr_t)m.gen | (uintptr_t)m.gcand) : (uintptr_t)m.bmark;
-    bool flags16 = (KIND == CK_CAND || KIND == CK_GRAIN_CAND || KIND == CK_MARKED) && (al & 15u) == 0;
-    if (flags16) {
-        launch_dep(k_flag_count<KIND>, tiles, TPB, s, m, n, x.blockcnt);
-        launch_dep(k_flag_scatter<KIND>, tiles, TPB, s, m, n, x.blockcnt, out, n_out);
-    } else {
-        COUNT_LAUNCHES(1), k_compact_count<KIND><<<tiles, TPB, 0, s>>>(m, n, x.blockcnt);
-        COUNT_LAUNCHES(1), k_compact_scatter<KIND><<<tiles, TPB, 0, s>>>(m, n, x.blockcnt, out, n_out);
-    }
+    auto k = k_tail<PART>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = TAIL_BLOCKS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = TAIL_BLOCKS;
+    cfg.blockDim = TAIL_TPB;
+    cfg.stream = s;
+    cfg.attrs = at;
+    bool plain = sevc_pdl_skip > 0;
+    if (sevc_pdl_skip > 0) sevc_pdl_skip--;
+    cfg.numAttrs = plain ? 1 : 2;
+    COUNT_LAUNCHES(1);
+    cudaLaunchKernelEx(&cfg, k, m, x, poll_grid(p), cap, p.dt, p.eps, summary);
 }
-
-inline int listgrid(int cap) { int g = (cap + TPB - 1) / TPB; return g < 4 * WL_BLOCKS ? g : 4 * WL_BLOCKS; }
 
 } // namespace
 
-void launch_compact(const DevMesh &m, const DevScratch &x, CompactKind kind, int *out, int *n_out, cudaStream_t s)
+PollGrid poll_grid(const StepParams &p)
 {
-    switch (kind) {
-    case CK_CAND: compact_impl<CK_CAND>(m, x, m.nb, out, n_out, s); break;
-    case CK_TWO_THREE: compact_impl<CK_TWO_THREE>(m, x, m.nb, out, n_out, s); break;
-    case CK_GRAIN_CAND: compact_impl<CK_GRAIN_CAND>(m, x, m.ng, out, n_out, s); break;
-    case CK_GVLEN3: compact_impl<CK_GVLEN3>(m, x, m.ng, out, n_out, s); break;
-    case CK_MARKED: compact_impl<CK_MARKED>(m, x, m.nb, out, n_out, s); break;
-    }
+    PollGrid g;
+    g.blocks = p.n_blocks;
+    g.tpb = p.n_threads;
+    g.counting = 0;
+    for (int t = 0; t < g.tpb; t++) g.counting += PollGrid::counts(t, g.tpb);
+    return g;
 }
 
-void launch_two_three_first(const DevMesh &m, const DevScratch &x, int *out, int *n_out, cudaStream_t s)
+void launch_two_three_first(const DevMesh &m, const DevScratch &x, cudaStream_t s)
 {
-    cudaMemsetAsync(m.bmark, 0, (size_t)m.nb, s);
+    /* nine threads per 3-sided grain, of which there are a few percent */
     int g = (m.ng + TPB - 1) / TPB;
-    COUNT_LAUNCHES(1), k_mark_two_three<<<g < 4 * WL_BLOCKS ? g : 4 * WL_BLOCKS, TPB, 0, s>>>(m, x.three, x.n_three);
-    compact_impl<CK_MARKED>(m, x, m.nb, out, n_out, s);
+    COUNT_LAUNCHES(1), k_two_three_first<<<g < 4 * WL_BLOCKS ? g : 4 * WL_BLOCKS, TPB, 0, s>>>(m, x);
 }
-
-void launch_poll_iteration(const DevMesh &m, const DevScratch &x, const int *cand, const int *ncand,
-                           const StepParams &p, cudaStream_t s)
+bool tail_whole(const DevMesh &m) { return m.nv <= TAIL_WHOLE_NV; }
+void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s)
 {
-    int g = listgrid(m.nb);
-    launch_dep(k_poll_vote, g, TPB, s, m, cand, ncand, x.nrun);
-    launch_dep(k_poll_count, g, TPB, s, m, cand, ncand);
-    launch_dep(k_poll_unlabel, g, TPB, s, m, cand, ncand);
-    int grid = p.n_blocks * p.n_threads;
-    bool aligned = (((uintptr_t)m.ben | (uintptr_t)m.bcand | (uintptr_t)m.bcandbuf) & 15u) == 0;
-    if (p.ninst == 1 && grid >= 16 && aligned) {
-        int th = (m.nb + 15) / 16;
-        launch_dep(k_poll_compare_write16, (th + TPB - 1) / TPB, TPB, s, m, x.threadfail, grid);
-    } else {
-        launch_dep(k_poll_compare_write, (m.nb + TPB - 1) / TPB, TPB, s, m, x.threadfail, grid);
-    }
-    launch_dep(k_poll_final, dim3(p.n_blocks, p.ninst), p.n_threads, s, m, x.threadfail, x.pblock, x.pcnt, x.piters,
-               x.nrun);
+    launch_tail_part<TAIL_REMOVE | TAIL_FLIP | TAIL_FIX | TAIL_END>(m, x, p, cap, summary, s);
 }
-
-void launch_conflicts(const DevMesh &m, const int *cand, const int *ncand, cudaStream_t s)
+void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s)
 {
-    int g = listgrid(m.nb);
-    launch_dep(k_conflict_check, g, TPB, s, m, cand, ncand);
-    launch_dep(k_conflict_unlabel, g, TPB, s, m, cand, ncand);
+    launch_tail_part<TAIL_REMOVE>(m, x, p, cap, nullptr, s);
 }
-
-inline int instgrid(const DevMesh &m) { return (m.ninst + 31) / 32; }
-
-void launch_remove_two_three(const DevMesh &m, const DevScratch &x, const int *list, const int *n, int pass,
-                             cudaStream_t s)
+void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
-    COUNT_LAUNCHES(1), k_remove_two_three<<<instgrid(m), 32, 0, s>>>(m, list, n, x.extra,
-                                                                     x.segcnt + (size_t)pass * m.ninst, nullptr);
+    launch_tail_part<TAIL_FLIP>(m, x, p, 0, nullptr, s);
 }
-void launch_remove_two_three_dev(const DevMesh &m, const DevScratch &x, const int *list, const int *n, cudaStream_t s)
+void launch_tail_fix(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
-    COUNT_LAUNCHES(1), k_remove_two_three<<<instgrid(m), 32, 0, s>>>(m, list, n, x.extra, x.segcnt, x.tt_pass);
-}
-void launch_poll_cond(const DevMesh &m, const DevScratch &x, cudaGraphConditionalHandle hnd, int cap, cudaStream_t s)
-{
-    COUNT_LAUNCHES(1), k_poll_cond<<<1, 32, 0, s>>>(hnd, x.nrun, x.ptot, cap, m.err);
-}
-void launch_tt_init(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStream_t s)
-{
-    COUNT_LAUNCHES(1), k_tt_init<<<1, 32, 0, s>>>(hnd, x.n_b, x.tt_first, x.tt_pass);
-}
-void launch_tt_cond(const DevScratch &x, cudaGraphConditionalHandle hnd, cudaStream_t s)
-{
-    COUNT_LAUNCHES(1), k_tt_cond<<<1, 32, 0, s>>>(hnd, x.n_b, x.tt_pass);
-}
-void launch_label_3sided_auto(const DevMesh &m, const DevScratch &x, double dt, cudaStream_t s)
-{
-    int g = (m.ng + TPB - 1) / TPB;
-    launch_dep(k_label_3sided_auto, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.three, x.n_three, x.tt_first);
-}
-
-void launch_label_3sided(const DevMesh &m, const DevScratch &x, double dt, bool bucket, cudaStream_t s)
-{
-    if (bucket) {
-        int g = (m.ng + TPB - 1) / TPB;
-        launch_dep(k_label_3sided_bucket, g < 4 * 152 ? g : 4 * 152, TPB, s, m, dt, x.three, x.n_three);
-    } else {
-        launch_dep(k_label_3sided, (m.ng + TPB - 1) / TPB, TPB, s, m, dt);
-    }
-}
-
-void launch_remove_grains(const DevMesh &m, const DevScratch &x, const int *list, const int *n, cudaStream_t s)
-{
-    launch_dep(k_remove_reserve, 4 * WL_BLOCKS, TPB, s, m, x, list, n);
-    launch_dep(k_remove_apply, 4 * WL_BLOCKS, TPB, s, m, x, list);
-    launch_dep(k_remove_deferred, (m.ninst + 3) / 4, 128, s, m, x, list, n);
-}
-
-
-void launch_flips(const DevMesh &m, double eps, const int *cand, const int *ncand, const DevScratch &x,
-                  cudaStream_t s)
-{
-    launch_dep(k_flip_reserve, 4 * WL_BLOCKS, TPB, s, m, x, cand, ncand);
-    launch_dep(k_flip_apply, 4 * WL_BLOCKS, TPB, s, m, x, eps, cand);
-    launch_dep(k_flip_deferred, m.ninst, FLIP_TPB, s, m, x, eps, cand, ncand);
-}
-
-void launch_fix_lists(const DevMesh &m, cudaStream_t s, bool areas)
-{
-    launch_dep(k_fix_edit, WL_BLOCKS, FIX_TPB, s, m);
-    launch_dep(k_fix_clear, WL_BLOCKS, TPB, s, m, (int)areas);
+    launch_tail_part<TAIL_FIX>(m, x, p, 0, nullptr, s);
 }
 
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s)
