@@ -85,14 +85,14 @@ __device__ void set_mod(const DevMesh &m, int v, int slot, int fix, int grn, int
  * cluster scope).  The grid is exactly one cluster. */
 struct Team {
     int tid, n;            /* thread of the team, threads */
-    int warp, nwarps, lane;
+    int warp, nwarps, lane;/* consecutive warps lie in different blocks: a few events spread over all SMs */
     __device__ Team()
     {
-        tid = blockIdx.x * blockDim.x + threadIdx.x;
+        lane = threadIdx.x & 31;
+        warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        tid = 32 * warp + lane;
         n = gridDim.x * blockDim.x;
-        warp = tid >> 5;
         nwarps = n >> 5;
-        lane = tid & 31;
     }
     __device__ __forceinline__ void sync() const
     {
