@@ -162,7 +162,7 @@ sevc_status sevc_write_snapshot(const sevc_mesh_host *mesh, const sevc_options *
 sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *out);
 sevc_status sevc_mesh_sizes(const sevc_handle *h, int *nv, int *nb, int *ng);
 /* check_data, src/utils.h:85-336: number of violated invariants (>= 0),
- * counted on the device (one thread per boundary, vertex and grain). */
+ * counted on the device. */
 sevc_status sevc_check_data(sevc_handle *h, int *n_bad);
 /* The same count on the host after a download of the mesh. */
 sevc_status sevc_check_data_host(sevc_handle *h, int *n_bad);

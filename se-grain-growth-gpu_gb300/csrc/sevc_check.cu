@@ -1,7 +1,7 @@
 /*
  * Mesh invariants on the device: the checks of check_data
  * (src/utils.h:85-336, the tests that set is_valid = false), one thread
- * per boundary, vertex and grain, counted into one integer.  The host
+ * per boundary and vertex and a warp per grain, counted into one integer.  The host
  * restatement in sevc_host.c (sevc_host_check) counts the same violations
  * in the same way.  An index outside its array counts as one violation and
  * is not followed, so a damaged mesh is reported, never read out of bounds.
@@ -32,9 +32,8 @@ __device__ __forceinline__ bool in_list(const DevMesh &m, int g, int v)
 }
 
 /* src/utils.h:85-158, per enabled boundary */
-__global__ void k_check_boundaries(DevMesh m, int *out)
+__device__ int check_boundary(const DevMesh &m, int b)
 {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
     int bad = 0;
     if (b < m.nb && m.ben[b]) {
         int2 e = m.bv[b];
@@ -59,13 +58,12 @@ __global__ void k_check_boundaries(DevMesh m, int *out)
             bad += k < 2 || gic[0] == gic[1];
         }
     }
-    add_count(out, bad);
+    return bad;
 }
 
 /* src/utils.h:160-280, per enabled vertex */
-__global__ void k_check_vertices(DevMesh m, int *out)
+__device__ int check_vertex(const DevMesh &m, int v)
 {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
     int bad = 0;
     if (v < m.nv && m.ven[v]) {
         int4 s4 = m.vb[v], g4 = m.vg[v];
@@ -85,34 +83,43 @@ __global__ void k_check_vertices(DevMesh m, int *out)
         }
         bad += nb[0] == nb[1] || nb[1] == nb[2] || nb[2] == nb[0];
     }
-    add_count(out, bad);
+    return bad;
 }
 
-/* src/utils.h:282-336, per enabled grain */
-__global__ void k_check_grains(DevMesh m, int *out)
+/* src/utils.h:282-336, per enabled grain, by a warp: its lanes read the
+ * whole list (100 entries, all of them counted) side by side.  The lanes'
+ * results add up to the grain's. */
+__device__ int check_grain(const DevMesh &m, int g, int lane)
 {
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    int bad = 0;
-    if (g < m.ng && m.gen[g]) {
-        const int *L = m.glist + (size_t)SEVC_MAXV * g;
-        int n = m.gvlen[g];
-        if (n < 0 || n > SEVC_MAXV) {
-            bad = 1;
-        } else {
-            bool listed = true;
-            for (int j = 0; j < n; j++) {
-                if (!inr(L[j], m.nv)) { bad++; listed = false; continue; }
-                bad += !m.ven[L[j]];
-            }
-            for (int j = 0; j < n && listed; j++) {
-                int4 s = m.vg[L[j]];
-                if (s.x != g && s.y != g && s.z != g) { bad++; break; }
-            }
-            int cnt = 0;
-            for (int j = 0; j < SEVC_MAXV; j++) cnt += L[j] != -1;
-            bad += cnt != n;
-        }
+    if (g >= m.ng || !m.gen[g]) return 0;
+    const int *L = m.glist + (size_t)SEVC_MAXV * g;
+    const int n = m.gvlen[g];
+    if (n < 0 || n > SEVC_MAXV) return lane == 0;
+    int bad = 0, cnt = 0;
+    bool out = false, stray = false;
+    for (int j = lane; j < SEVC_MAXV; j += 32) {
+        const int v = L[j];
+        cnt += v != -1;
+        if (j >= n) continue;
+        if (!inr(v, m.nv)) { bad++; out = true; continue; }
+        bad += !m.ven[v];
+        int4 s = m.vg[v];
+        stray |= s.x != g && s.y != g && s.z != g;
     }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const bool any_out = __any_sync(0xffffffffu, out), any_stray = __any_sync(0xffffffffu, stray);
+    if (lane == 0) bad += (!any_out && any_stray) + (cnt != n);
+    return bad;
+}
+
+/* all three in one launch: blocks of boundaries, then of vertices, then of
+ * grains (a warp each) */
+__global__ void __launch_bounds__(TPB) k_check(DevMesh m, int bblocks, int vblocks, int *out)
+{
+    int k = blockIdx.x, bad;
+    if (k < bblocks) bad = check_boundary(m, k * TPB + threadIdx.x);
+    else if ((k -= bblocks) < vblocks) bad = check_vertex(m, k * TPB + threadIdx.x);
+    else bad = check_grain(m, (k - vblocks) * (TPB / 32) + (threadIdx.x >> 5), threadIdx.x & 31);
     add_count(out, bad);
 }
 
@@ -310,9 +317,8 @@ extern "C" sevc_status sevc_selftest_arith(long long n, unsigned long long seed,
 void launch_check(const DevMesh &m, int *out, cudaStream_t s)
 {
     cudaMemsetAsync(out, 0, sizeof(int), s);
-    COUNT_LAUNCHES(1), k_check_boundaries<<<(m.nb + TPB - 1) / TPB, TPB, 0, s>>>(m, out);
-    COUNT_LAUNCHES(1), k_check_vertices<<<(m.nv + TPB - 1) / TPB, TPB, 0, s>>>(m, out);
-    COUNT_LAUNCHES(1), k_check_grains<<<(m.ng + TPB - 1) / TPB, TPB, 0, s>>>(m, out);
+    const int bb = (m.nb + TPB - 1) / TPB, vb = (m.nv + TPB - 1) / TPB, gb = (m.ng + TPB / 32 - 1) / (TPB / 32);
+    if (bb + vb + gb > 0) COUNT_LAUNCHES(1), k_check<<<bb + vb + gb, TPB, 0, s>>>(m, bb, vb, out);
 }
 
 void launch_digest(const DevMesh &m, unsigned long long *out, cudaStream_t s)

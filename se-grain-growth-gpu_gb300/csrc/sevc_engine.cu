@@ -94,6 +94,10 @@ struct sevc_handle {
     int *h_on = nullptr;   /* per instance: nucleation attempt this step */
     int *h_flags = nullptr;/* host part of the step's output decision (x.flags) */
     size_t dbytes = 0;     /* size of the device block */
+    /* scratch and result of the statistics calls (device) with a pinned
+     * readback buffer, kept from the first call on */
+    double *stat = nullptr, *h_stat = nullptr;
+    size_t stat_len = 0;
     Tape tape;
     /* a step without / with a nucleation attempt as one CUDA graph */
     StepGraph g_step[2];
@@ -401,6 +405,25 @@ void load_run(sevc_handle *h, const RunState &r)
     h->icurr = r.icurr;
     h->iallow = r.iallow;
     h->iarea = r.iarea;
+}
+/* device scratch for a statistics call with `nout` results (at most 1024):
+ * results in h->stat[0..nout), partial results after them */
+bool stat_scratch(sevc_handle *h, int nout)
+{
+    size_t need = 1024 + stat_doubles(nout);
+    if (!h->h_stat && !cuda_ok(cudaMallocHost(&h->h_stat, 1024 * 8), "pinned")) return false;
+    if (h->stat_len >= need) return true;
+    if (h->stat) cudaFree(h->stat);
+    h->stat = nullptr;
+    h->stat_len = 0;
+    if (!cuda_ok(cudaMalloc(&h->stat, need * 8), "cudaMalloc")) return false;
+    h->stat_len = need;
+    return true;
+}
+bool stat_read(sevc_handle *h, int nout)
+{
+    return cuda_ok(cudaMemcpyAsync(h->h_stat, h->stat, nout * 8, cudaMemcpyDeviceToHost, h->stream), "readback") &&
+           cuda_ok(cudaStreamSynchronize(h->stream), "sync");
 }
 bool tape_checkpoint(sevc_handle *h)
 {
@@ -830,6 +853,8 @@ void sevc_destroy(sevc_handle *h)
     if (!h) return;
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->dblock) cudaFree(h->dblock);
+    if (h->stat) cudaFree(h->stat);
+    if (h->h_stat) cudaFreeHost(h->h_stat);
     if (h->h_ctr) cudaFreeHost(h->h_ctr);
     if (h->h_big) cudaFreeHost(h->h_big);
     if (h->h_on) cudaFreeHost(h->h_on);
@@ -1348,15 +1373,12 @@ sevc_status sevc_tape_stop(sevc_handle *h)
 sevc_status sevc_area_histogram(sevc_handle *h, int nbins, double amax, double *hist)
 {
     if (!h || nbins < 1 || nbins > 1024 || !(amax > 0) || !hist) return SEVC_ERR_ARG;
-    int nb = histogram_blocks(h->m);
-    double *d = nullptr;
-    if (!cuda_ok(cudaMalloc(&d, ((size_t)nb + 1) * nbins * 8), "cudaMalloc")) return SEVC_ERR_CUDA;
+    if (!stat_scratch(h, nbins)) return SEVC_ERR_CUDA;
     double nnorm = h->curr_n_grains, sc = nnorm / (h->ninst * h->opt.domain_bound * h->opt.domain_bound);
-    launch_histogram(h->m, nbins, amax, sc, nnorm, d + nbins, d, h->stream);
-    bool ok = cuda_ok(cudaMemcpyAsync(hist, d, nbins * 8, cudaMemcpyDeviceToHost, h->stream), "readback") &&
-              cuda_ok(cudaStreamSynchronize(h->stream), "sync");
-    cudaFree(d);
-    return ok ? SEVC_OK : SEVC_ERR_CUDA;
+    launch_histogram(h->m, nbins, amax, sc, nnorm, h->stat + 1024, h->stat, h->stream);
+    if (!stat_read(h, nbins)) return SEVC_ERR_CUDA;
+    memcpy(hist, h->h_stat, nbins * 8);
+    return SEVC_OK;
 }
 
 sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const double *dloss_dhist,
@@ -1365,6 +1387,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
     if (!h || nbins < 1 || nbins > 1024 || !(amax > 0) || !dloss_dhist) return SEVC_ERR_ARG;
     Tape &tp = h->tape;
     if (tp.every <= 0) { sevc_set_error("no tape: call sevc_tape_start before the steps"); return SEVC_ERR_ARG; }
+    if (!stat_scratch(h, 1)) return SEVC_ERR_CUDA;
     cudaStream_t s = h->stream;
     size_t V = h->nv, B = h->nb, G = h->ng;
     /* adjoint buffers */
@@ -1411,7 +1434,9 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
     cudaMemsetAsync(a.gmu, 0, V * 8, s);
     cudaMemsetAsync(a.ggam, 0, V * 8, s);
     double nnorm = h->curr_n_grains, sc = nnorm / (h->ninst * h->opt.domain_bound * h->opt.domain_bound);
-    launch_hist_seed(h->m, nbins, amax, sc, nnorm, d_dldh, a.dlda, a.lam, s);
+    double zero_sum = 0;
+    for (int k = 0; k < nbins; k++) zero_sum += 0.0 * dloss_dhist[k];
+    launch_hist_seed(h->m, nbins, amax, sc, nnorm, d_dldh, zero_sum, a.dlda, a.lam, s);
 
     void *fin = nullptr;
     if (!cuda_ok(cudaMalloc(&fin, h->dbytes), "cudaMalloc") || !d2d(fin, h->dblock, h->dbytes)) return SEVC_ERR_CUDA;
@@ -1474,8 +1499,8 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
     h->force_direct = false;
     if (!d2d(h->dblock, fin, h->dbytes)) st = SEVC_ERR_CUDA;
     load_run(h, rfin);
-    launch_sum_ordered(a.gmu, (int)V, a.scalars, s);
-    launch_sum_ordered(a.ggam, (int)V, a.scalars + 1, s);
+    launch_sum_ordered(h->m, a.gmu, (int)V, h->stat + 1024, a.scalars, s);
+    launch_sum_ordered(h->m, a.ggam, (int)V, h->stat + 1024, a.scalars + 1, s);
     double sc2[2] = { 0, 0 };
     if (!st && grad_se && !cuda_ok(cudaMemcpyAsync(grad_se, a.gse, G * 8, cudaMemcpyDeviceToHost, s), "readback"))
         st = SEVC_ERR_CUDA;
@@ -1569,14 +1594,10 @@ sevc_status sevc_grain_stats(sevc_handle *h, int inst, sevc_grain_stats_t *out)
 {
     if (!h || !out || inst < -1 || inst >= h->ninst) return SEVC_ERR_ARG;
     int lo = inst < 0 ? 0 : h->goff[inst], hi = inst < 0 ? h->ng : h->goff[inst + 1];
-    double *d = nullptr;
-    if (!cuda_ok(cudaMalloc(&d, 8 * 8), "cudaMalloc")) return SEVC_ERR_CUDA;
-    launch_grain_stats(h->m, lo, hi, d, h->stream);
-    double r[8];
-    bool ok = cuda_ok(cudaMemcpyAsync(r, d, sizeof r, cudaMemcpyDeviceToHost, h->stream), "readback") &&
-              cuda_ok(cudaStreamSynchronize(h->stream), "sync");
-    cudaFree(d);
-    if (!ok) return SEVC_ERR_CUDA;
+    if (!stat_scratch(h, 8)) return SEVC_ERR_CUDA;
+    launch_grain_stats(h->m, lo, hi, h->stat + 1024, h->stat, h->stream);
+    if (!stat_read(h, 8)) return SEVC_ERR_CUDA;
+    const double *r = h->h_stat;
     double n = r[0];
     out->n_grains = (int)n;
     out->mean_area = n > 0 ? r[1] / n : 0;

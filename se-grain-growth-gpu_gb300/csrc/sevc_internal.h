@@ -149,21 +149,25 @@ struct AdjointBuffers {
     double *dlda;    /* dL/dA per grain of the statistic */
     double *scalars; /* reduced dL/dmu, dL/dGB_scaling */
 };
-/* soft histogram of a_g = |A_g| sc over nbins bins of [0, amax), divided by nnorm */
-void launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *blockbins,
-                      double *hist, cudaStream_t s);
-int histogram_blocks(const DevMesh &m);
-/* lam = d(sum_k dldh_k h_k)/dx at the current state */
+/* soft histogram of a_g = |A_g| sc over nbins bins of [0, amax), divided by
+ * nnorm; part: stat_doubles(nbins) doubles of scratch */
+size_t stat_doubles(int nbins);
+void launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *part, double *hist,
+                      cudaStream_t s);
+/* lam = d(sum_k dldh_k h_k)/dx at the current state; zero_sum: see
+ * k_hist_grad_area */
 void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, double nnorm, const double *dldh,
-                      double *dlda, double2 *lam, cudaStream_t s);
+                      double zero_sum, double *dlda, double2 *lam, cudaStream_t s);
 /* one step backward: `rec` views the mesh as recorded at the step's start,
  * log / ven1 / vel1 its events and the enabled flags and velocities after it */
 void launch_adjoint_step(const DevMesh &rec, const AdjointBuffers &a, double dt, double mu, double eps, double s_gb,
                          const EventRec *log, const int *nlog, const uint8_t *ven1, const double2 *vel1,
                          cudaStream_t s);
-void launch_sum_ordered(const double *a, int n, double *out, cudaStream_t s);
-/* out[0..6] = count, sum |A|, sum A^2, sum vlen, 3-sided count, min |A|, max |A| over grains [lo, hi) */
-void launch_grain_stats(const DevMesh &m, int lo, int hi, double *out, cudaStream_t s);
+/* *out = the sum of a[0..n); part: stat_doubles(1) doubles of scratch */
+void launch_sum_ordered(const DevMesh &m, const double *a, int n, double *part, double *out, cudaStream_t s);
+/* out[0..6] = count, sum |A|, sum A^2, sum vlen, 3-sided count, min |A|, max
+ * |A| over grains [lo, hi); part: stat_doubles(1) doubles of scratch */
+void launch_grain_stats(const DevMesh &m, int lo, int hi, double *part, double *out, cudaStream_t s);
 
 #define SEVC_CUDA_OK(expr) ((expr) == cudaSuccess)
 
