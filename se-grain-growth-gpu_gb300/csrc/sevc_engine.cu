@@ -69,6 +69,7 @@ struct Tape {
 struct sevc_handle {
     sevc_options opt;
     int nv = 0, nb = 0, ng = 0;
+    int device = 0;
     cudaStream_t stream = nullptr;
     void *dblock = nullptr;
     DevMesh m{};
@@ -320,6 +321,7 @@ sevc_status create_from_host(const sevc_options *opt, sevc_hmesh *hm, sevc_handl
     *out = nullptr;
     if (require_device()) return SEVC_ERR_CUDA;
     sevc_handle *h = new sevc_handle();
+    cudaGetDevice(&h->device);
     h->opt = *opt;
     h->nv = hm->m.nv; h->nb = hm->m.nb; h->ng = hm->m.ng;
     h->ninst = ninst;
@@ -1067,39 +1069,41 @@ sevc_status sevc_mesh_sizes(const sevc_handle *h, int *nv, int *nb, int *ng)
 sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *o)
 {
     if (!h || !o) return SEVC_ERR_ARG;
-    size_t V = h->nv, B = h->nb, G = h->ng;
     cudaStream_t s = h->stream;
-    std::vector<double2> d2(V);
-    std::vector<DevMesh::FdTerms> d4(V);
-    std::vector<int4> i4(V);
-    std::vector<int2> i2(B);
-    auto get = [&](void *dst, const void *src, size_t bytes) {
-        return cuda_ok(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "download");
-    };
-    bool ok = get(d2.data(), h->m.pos, V * 16) && cuda_ok(cudaStreamSynchronize(s), "sync");
-    if (!ok) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < V; i++) { o->px[i] = d2[i].x; o->py[i] = d2[i].y; }
-    if (!get(d2.data(), h->m.vel, V * 16) || !cuda_ok(cudaStreamSynchronize(s), "sync")) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < V; i++) { o->vx[i] = d2[i].x; o->vy[i] = d2[i].y; }
-    if (!get(d4.data(), h->m.terms, V * 32) || !cuda_ok(cudaStreamSynchronize(s), "sync")) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < V; i++) {            /* src/calculus.h:63-69: -term / grad_eps */
-        o->vel_bnd_x[i] = -d4[i].bx / SEVC_GRAD_EPS;
-        o->vel_grn_x[i] = -d4[i].gx / SEVC_GRAD_EPS;
-        o->vel_bnd_y[i] = -d4[i].by / SEVC_GRAD_EPS;
-        o->vel_grn_y[i] = -d4[i].gy / SEVC_GRAD_EPS;
+    sevc_mesh_host d = *o;
+    d.nv = h->nv; d.nb = h->nb; d.ng = h->ng;
+    void *ptr[SEVC_HOST_FIELDS];
+    size_t bytes[SEVC_HOST_FIELDS];
+    sevc_host_fields(&d, ptr, bytes);
+    int direct = 0;   /* the device can store to the caller's (pageable) memory */
+    cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccess, h->device);
+    if (direct && sevc_host_aligned(&d)) {
+        /* the device writes the caller's arrays, the grains' (60% of the
+         * bytes) while the host maps the pages of the others */
+        const int n = SEVC_HOST_FIELDS, ngf = SEVC_HOST_GRAIN_FIELDS;
+        if (bytes[0] < (size_t)16 << 20) {
+            sevc_host_touch(n, ptr, bytes);
+            launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s);
+        } else {
+            sevc_host_touch(ngf, ptr, bytes);
+            launch_export(h->m, d, EXPORT_GRAINS, s);
+            sevc_host_touch(n - ngf, ptr + ngf, bytes + ngf);
+            launch_export(h->m, d, EXPORT_REST, s);
+        }
+        return cuda_ok(cudaGetLastError(), "export") && cuda_ok(cudaStreamSynchronize(s), "sync") ? SEVC_OK : SEVC_ERR_CUDA;
     }
-    if (!get(i4.data(), h->m.vb, V * 16) || !cuda_ok(cudaStreamSynchronize(s), "sync")) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < V; i++) { o->vb[3 * i] = i4[i].x; o->vb[3 * i + 1] = i4[i].y; o->vb[3 * i + 2] = i4[i].z; }
-    if (!get(i4.data(), h->m.vg, V * 16) || !cuda_ok(cudaStreamSynchronize(s), "sync")) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < V; i++) { o->vg[3 * i] = i4[i].x; o->vg[3 * i + 1] = i4[i].y; o->vg[3 * i + 2] = i4[i].z; }
-    if (!get(i2.data(), h->m.bv, B * 8) || !cuda_ok(cudaStreamSynchronize(s), "sync")) return SEVC_ERR_CUDA;
-    for (size_t i = 0; i < B; i++) { o->bini[i] = i2[i].x; o->bend[i] = i2[i].y; }
-    ok = get(o->venergy, h->m.venergy, V * 8) && get(o->ven, h->m.ven, V) && get(o->benergy, h->m.benergy, B * 8) &&
-         get(o->blen, h->m.blen, B * 8) && get(o->btext, h->m.btext, B * 8) && get(o->ben, h->m.ben, B) &&
-         get(o->bcand, h->m.bcand, B) && get(o->glist, h->m.glist, G * SEVC_MAXV * 4) &&
-         get(o->gvlen, h->m.gvlen, G * 4) && get(o->garea, h->m.garea, G * 8) && get(o->gdadt, h->m.gdadt, G * 8) &&
-         get(o->gori, h->m.gori, G * 8) && get(o->gse, h->m.gse, G * 8) && get(o->gen, h->m.gen, G) &&
-         get(o->gtype, h->m.gtype, G) && cuda_ok(cudaStreamSynchronize(s), "sync");
+    /* else through device memory in the same layout */
+    size_t off[SEVC_HOST_FIELDS], total = 0;
+    for (int f = 0; f < SEVC_HOST_FIELDS; f++) { off[f] = total; total += align256(bytes[f]); }
+    char *dev = nullptr;
+    if (!cuda_ok(cudaMalloc(&dev, total), "cudaMalloc")) return SEVC_ERR_CUDA;
+    sevc_host_relocate(&d, dev, off);
+    launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s);
+    bool ok = cuda_ok(cudaGetLastError(), "export");
+    for (int f = 0; f < SEVC_HOST_FIELDS && ok; f++)
+        ok = cuda_ok(cudaMemcpyAsync(ptr[f], dev + off[f], bytes[f], cudaMemcpyDeviceToHost, s), "download");
+    ok = cuda_ok(cudaStreamSynchronize(s), "sync") && ok;
+    cudaFree(dev);
     return ok ? SEVC_OK : SEVC_ERR_CUDA;
 }
 

@@ -16,6 +16,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
 #ifndef M_PI
 #define M_PI 3.14159265358979323846
@@ -126,6 +127,53 @@ sevc_status sevc_load_ini(const char *path, sevc_options *o)
 /* ---------------------------------------------------------------- */
 /* host mesh storage                                                 */
 /* ---------------------------------------------------------------- */
+/* X(field, type, elements) in the order of SEVC_HOST_FIELDS */
+#define HOST_FIELDS(X) \
+    X(glist, int32_t, SEVC_MAX_VRT_PER_GRN * G) X(gvlen, int32_t, G) X(garea, double, G) X(gdadt, double, G) \
+    X(gori, double, G) X(gse, double, G) X(gen, uint8_t, G) X(gtype, uint8_t, G) \
+    X(px, double, V) X(py, double, V) X(vx, double, V) X(vy, double, V) X(venergy, double, V) \
+    X(vel_bnd_x, double, V) X(vel_grn_x, double, V) X(vel_bnd_y, double, V) X(vel_grn_y, double, V) \
+    X(ven, uint8_t, V) X(vb, int32_t, 3 * V) X(vg, int32_t, 3 * V) \
+    X(bini, int32_t, B) X(bend, int32_t, B) X(benergy, double, B) X(blen, double, B) X(btext, double, B) \
+    X(ben, uint8_t, B) X(bcand, uint8_t, B)
+
+void sevc_host_fields(const sevc_mesh_host *m, void **ptr, size_t *bytes)
+{
+    const size_t V = m->nv, B = m->nb, G = m->ng;
+    int n = 0;
+#define X(f, t, c) ptr[n] = (void *)m->f; bytes[n++] = (c) * sizeof(t);
+    HOST_FIELDS(X)
+#undef X
+}
+int sevc_host_aligned(const sevc_mesh_host *m)
+{
+    uintptr_t bad = 0;
+#define X(f, t, c) bad |= (uintptr_t)m->f % sizeof(t);
+    HOST_FIELDS(X)
+#undef X
+    return bad == 0;
+}
+void sevc_host_relocate(sevc_mesh_host *m, char *base, const size_t *off)
+{
+    int n = 0;
+#define X(f, t, c) m->f = (t *)(base + off[n++]);
+    HOST_FIELDS(X)
+#undef X
+}
+
+void sevc_host_touch(int n, void *const *ptr, const size_t *bytes)
+{
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    for (int f = 0; f < n; f++) {
+        volatile char *p = (volatile char *)ptr[f];
+        if (bytes[f] == 0) continue;
+        const long steps = (long)((bytes[f] - 1) / page);
+#pragma omp parallel for schedule(static) if (steps >= 32)
+        for (long k = 0; k <= steps; k++) p[(size_t)k * page] = 0;
+        p[bytes[f] - 1] = 0;
+    }
+}
+
 int sevc_hmesh_alloc(sevc_hmesh *hm, int nv, int nb, int ng)
 {
     memset(hm, 0, sizeof(*hm));

@@ -39,6 +39,20 @@ int sevc_host_check(const sevc_mesh_host *m);
 
 void sevc_set_error(const char *fmt, ...);
 
+/* Fields of a host mesh as pointers and sizes (SEVC_HOST_FIELDS of them);
+ * the grains' fields are the first SEVC_HOST_GRAIN_FIELDS. */
+#define SEVC_HOST_FIELDS 27
+#define SEVC_HOST_GRAIN_FIELDS 8
+void sevc_host_fields(const sevc_mesh_host *m, void **ptr, size_t *bytes);
+/* whether every field lies at a multiple of its element size */
+int sevc_host_aligned(const sevc_mesh_host *m);
+/* the same fields at base + off[f] */
+void sevc_host_relocate(sevc_mesh_host *m, char *base, const size_t *off);
+/* Write one byte in every page of n buffers (by all host threads when they
+ * are large), so that a device storing to them meets no absent page: host
+ * threads map 700 MB in 4 ms, the device's own faults take 130 ms. */
+void sevc_host_touch(int n, void *const *ptr, const size_t *bytes);
+
 #ifdef __cplusplus
 }
 #endif

@@ -6,6 +6,7 @@
 #ifndef SEVC_INTERNAL_H
 #define SEVC_INTERNAL_H
 
+#include "sevc.h"
 #include "sevc_device.cuh"
 #include <curand_kernel.h>
 
@@ -126,6 +127,11 @@ void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParam
 void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 void launch_tail_fix(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s);
+
+/* The mesh in the layout of sevc_mesh_host, written by the device through
+ * pointers it can store to.  part: EXPORT_GRAINS, EXPORT_REST or both. */
+enum { EXPORT_GRAINS = 1, EXPORT_REST = 2 };
+void launch_export(const DevMesh &m, const sevc_mesh_host &o, int part, cudaStream_t s);
 
 /* check_data on the device (sevc_check.cu): violations counted into *out */
 void launch_check(const DevMesh &m, int *out, cudaStream_t s);
