@@ -56,8 +56,7 @@ __device__ __forceinline__ double bspline2_d(double s)
 /* signed area of grain g (src/geometry.h:757 order) */
 __device__ __forceinline__ double grain_area(const DevMesh &m, int g)
 {
-    double2 none = make_double2(0, 0);
-    return area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, -1, none, m.D);
+    return area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, m.D);
 }
 
 /* position of vertex v in grain g's list, its list neighbours */

@@ -534,26 +534,46 @@ __device__ __forceinline__ double add_closing_term(double acc, double x, double 
     return acc;
 }
 
-/* compute_area (src/geometry.h:757-765, with adjust_origin_for_points
- * :908-931) streamed over a grain list: point 0 becomes the origin,
- * later points accumulate wrapped deltas, shoelace terms add in list
- * order.  Slot `ps` (if >= 0) is replaced by position `pp`. */
-__device__ __forceinline__ double area_stream(const int *__restrict__ L, int n, const double2 *__restrict__ pos,
-                                              int ps, double2 pp, double D)
+/* Entries base .. base + 7 of a grain list row (100 entries, 16-byte
+ * aligned), those at n and beyond replaced by the row's first */
+__device__ __forceinline__ void list_batch(const int *L, int n, int base, int (&v)[8])
 {
-    double area = 0;
-    if (n > 0) {
-        double2 r0 = (ps == 0) ? pp : pos[L[0]];
-        double ax = 0, ay = 0, rx = r0.x, ry = r0.y;
-        for (int k = 1; k < n; k++) {
-            double2 r = (k == ps) ? pp : pos[L[k]];
-            double nx = ax + wrapd(r.x, rx, D);
-            double ny = ay + wrapd(r.y, ry, D);
-            if (k > 1) area += ax * ny - ay * nx;   /* term k-1; term 0 leaves +0 */
-            ax = nx; ay = ny; rx = r.x; ry = r.y;
+    const int4 a = *reinterpret_cast<const int4 *>(L + base);
+    const int4 b = base + 4 < SEVC_MAXV ? *reinterpret_cast<const int4 *>(L + base + 4) : a;
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    const int v0 = base == 0 ? a.x : L[0];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = base + j < n ? v[j] : v0;
+}
+/* compute_area (src/geometry.h:757-765, with adjust_origin_for_points
+ * :908-931) over a grain list row: point 0 becomes the origin, later points
+ * accumulate wrapped deltas, shoelace terms add in list order.  Eight
+ * positions are loaded at once (one after another, each vertex would wait
+ * for the last one's); the sum is a rolled loop over them, because where it
+ * runs once per launch the fetch of an unrolled one costs more. */
+__device__ __forceinline__ double area_stream(const int *L, int n, const double2 *pos, double D)
+{
+    double area = 0, ax = 0, ay = 0, rx = 0, ry = 0;
+    for (int base = 0; base < n; base += 8) {
+        int v[8];
+        double2 r[8];
+        list_batch(L, n, base, v);
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = pos[v[j]];
+        const int end = n - base < 8 ? n - base : 8;
+#pragma unroll 1
+        for (int j = 0; j < end; j++) {
+            if (base + j > 0) {
+                double nx = ax + wrapd(r[j].x, rx, D);
+                double ny = ay + wrapd(r[j].y, ry, D);
+                if (base + j > 1) area += ax * ny - ay * nx;   /* term k-1; term 0 leaves +0 */
+                ax = nx; ay = ny;
+            }
+            rx = r[j].x; ry = r[j].y;
         }
-        area = add_closing_term(area, ax, ay);
     }
+    if (n > 0) area = add_closing_term(area, ax, ay);
     return dscale_down<1>(area);
 }
 
@@ -711,25 +731,34 @@ __device__ __forceinline__ bool text_outside_dt(double2 pi, double2 pe, double2 
 }
 
 /* compute_dAdt (src/geometry.h:779-787) of grain g over its list; get(v,
- * r, w) gives vertex v's position and velocity */
+ * r, w) gives vertex v's position and velocity, eight vertices at a time
+ * (see area_stream) */
 template <class Get> __device__ __forceinline__ double dadt_over(const DevMesh &m, int g, Get get)
 {
     const int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    double d = 0;
-    if (n > 0) {
-        double2 r0, v0;
-        get(L[0], r0, v0);
-        double ax = 0, ay = 0, rx = r0.x, ry = r0.y, vxk = v0.x, vyk = v0.y;
-        for (int k = 1; k < n; k++) {
-            double2 r, w;
-            get(L[k], r, w);
-            double nx = ax + wrapd(r.x, rx, m.D);
-            double ny = ay + wrapd(r.y, ry, m.D);
-            d += (vxk * ny + ax * w.y);
-            d -= (vyk * nx + ay * w.x);
-            ax = nx; ay = ny; rx = r.x; ry = r.y; vxk = w.x; vyk = w.y;
+    const int n = m.gvlen[g];
+    double d = 0, ax = 0, ay = 0, rx = 0, ry = 0, vxk = 0, vyk = 0;
+    double2 v0 = make_double2(0, 0);
+    for (int base = 0; base < n; base += 8) {
+        int v[8];
+        double2 r[8], w[8];
+        list_batch(L, n, base, v);
+        get(v, r, w);
+        if (base == 0) v0 = w[0];
+        const int end = n - base < 8 ? n - base : 8;
+#pragma unroll 1
+        for (int j = 0; j < end; j++) {
+            if (base + j > 0) {
+                double nx = ax + wrapd(r[j].x, rx, m.D);
+                double ny = ay + wrapd(r[j].y, ry, m.D);
+                d += (vxk * ny + ax * w[j].y);
+                d -= (vyk * nx + ay * w[j].x);
+                ax = nx; ay = ny;
+            }
+            rx = r[j].x; ry = r[j].y; vxk = w[j].x; vyk = w[j].y;
         }
+    }
+    if (n > 0) {
         d += (vxk * 0.0 + ax * v0.y);
         d -= (vyk * 0.0 + ay * v0.x);
     }
@@ -737,7 +766,10 @@ template <class Get> __device__ __forceinline__ double dadt_over(const DevMesh &
 }
 __device__ __forceinline__ double dadt_from(const DevMesh &m, int g, const double2 *pos, const double2 *vel)
 {
-    return dadt_over(m, g, [&](int v, double2 &r, double2 &w) { r = pos[v]; w = vel[v]; });
+    return dadt_over(m, g, [&](const int (&v)[8], double2 (&r)[8], double2 (&w)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) { r[j] = pos[v[j]]; w[j] = vel[v[j]]; }
+    });
 }
 
 /* an event is about to overwrite vertex v's position or velocity: keep
@@ -787,7 +819,14 @@ __device__ __forceinline__ void finalize_grain(const DevMesh &m, int g)
 {
     if (m.gexact[g]) return;
     unsigned st = *m.stamp;
-    m.gdadt[g] = dadt_over(m, g, [&](int v, double2 &r, double2 &w) { start_state(m, v, st, r, w); });
+    m.gdadt[g] = dadt_over(m, g, [&](const int (&v)[8], double2 (&r)[8], double2 (&w)[8]) {
+        bool saved[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) { r[j] = m.pos[v[j]]; w[j] = m.vel[v[j]]; saved[j] = m.vstamp[v[j]] == st; }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (saved[j]) { r[j] = m.pos0[v[j]]; w[j] = m.vel0[v[j]]; }
+    });
     m.gexact[g] = 1;
 }
 

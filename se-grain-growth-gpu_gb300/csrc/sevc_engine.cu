@@ -506,7 +506,7 @@ void enqueue_pre(sevc_handle *h, bool nucleation)
      * streams, graph branches when captured):
      *   main   grain pass (:127,:203), vertex pass, t_ext labels
      *   side0  boundary arclengths and energies (:124-130 / :171-181), which
-     *          the vertex pass reads; then dA/dt of the 3-sided grains beside
+     *          the vertex pass reads; then dA/dt, on steps that compute it, beside
      *          the t_ext labels
      *   side1  beside the vertex pass: the first 2x3 count (:228), which
      *          depends only on the topology that nothing changes before that

@@ -591,18 +591,14 @@ __global__ void k_vertex_fd(DevMesh m, double mu)
  * src/geometry.h:779-787 streamed over the list */
 __device__ void dadt_of(const DevMesh &m, int g);
 
-/* every enabled grain when flags[0], else the 3-sided ones (listed by the
- * grain pass) */
-__global__ void k_grain_dadt(DevMesh m, const int *three, const int *n_three, const int *flags)
+/* every enabled grain, on a step that computes every output-only value
+ * (flags[0]); on the others the events settle the grains they change */
+__global__ void k_grain_dadt(DevMesh m, const int *flags)
 {
+    if (!flags[0]) return;
     int stride = gridDim.x * blockDim.x;
-    if (flags[0]) {
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < m.ng; g += stride)
-            if (m.gen[g]) dadt_of(m, g);
-    } else {
-        const int n3 = *n_three;
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += stride) dadt_of(m, three[i]);
-    }
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < m.ng; g += stride)
+        if (m.gen[g]) dadt_of(m, g);
 }
 
 __device__ void dadt_of(const DevMesh &m, int g)
@@ -799,8 +795,8 @@ void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const Launch
 }
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s)
 {
-    int g = nblk(m.ng);   /* grid-stride: every grain, or only the 3-sided ones, decided on the device */
-    COUNT_LAUNCHES(1), k_grain_dadt<<<g < 8 * 152 ? g : 8 * 152, TPB, 0, s>>>(m, x.three, x.n_three, x.flags);
+    int g = nblk(m.ng);
+    COUNT_LAUNCHES(1), k_grain_dadt<<<g < 8 * 152 ? g : 8 * 152, TPB, 0, s>>>(m, x.flags);
 }
 void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {

@@ -28,10 +28,16 @@ constexpr int TAIL_BLOCKS = 16, TAIL_TPB = 512, TAIL_WARPS = TAIL_TPB / 32;
 /* ------------------------------------------------------------------ */
 __device__ int glist_find(const DevMesh &m, int g, int v)          /* grain_contains_vertex :703 */
 {
-    const int *L = m.glist + (size_t)SEVC_MAXV * g;
+    /* rows are 400 bytes in a 256-byte aligned array: four entries a load */
+    const int4 *L = reinterpret_cast<const int4 *>(m.glist + (size_t)SEVC_MAXV * g);
     int n = m.gvlen[g];
-    for (int i = 0; i < n; i++)
-        if (L[i] == v) return i;
+    for (int i = 0; i < n; i += 4) {
+        int4 q = L[i / 4];
+        if (q.x == v) return i;
+        if (i + 1 < n && q.y == v) return i + 1;
+        if (i + 2 < n && q.z == v) return i + 2;
+        if (i + 3 < n && q.w == v) return i + 3;
+    }
     return -1;
 }
 __device__ int glist_consecutive(const DevMesh &m, int g, int A, int B) /* :724 */
@@ -52,11 +58,9 @@ __device__ __forceinline__ bool claim_byte(uint8_t *flags, int i)
     unsigned bit = 1u << (8 * (unsigned)(a & 3));
     return !(atomicOr((unsigned *)(a & ~(uintptr_t)3), bit) & bit);
 }
-/* queue a grain for the fix-up pass (grain.fix = true); its list is
- * about to change, so its dA/dt for this step is settled first */
+/* queue a grain for the fix-up pass (grain.fix = true) */
 __device__ void mark_fix(const DevMesh &m, int g)
 {
-    finalize_grain(m, g);
     if (!claim_byte(m.gfix, g)) return;
     int i = atomicAdd(m.nfix, 1);
     if (i < m.fixcap) m.fixlist[i] = g; else raise_err(m, ERRB_WORKLIST);
@@ -279,7 +283,7 @@ __device__ void conflict_unlabel(const DevMesh &m, const Team &T, const int *lis
 /* removal of two adjacent 3-sided grains, src/topological.h:840-985   */
 /* ------------------------------------------------------------------ */
 /* remove_two_grains (:840-955); returns the rewired boundary CE or -1 */
-__device__ int remove_two_grains_dev(const DevMesh &m, int bnd, const int *gnic)
+__device__ __noinline__ int remove_two_grains_dev(const DevMesh &m, int bnd, const int *gnic)
 {
     int2 eb = m.bv[bnd];
     int A = eb.x, B = eb.y;
@@ -314,13 +318,9 @@ __device__ int remove_two_grains_dev(const DevMesh &m, int bnd, const int *gnic)
     set_mod(m, B, 2, FIX_REMOVE, G4, D, -2);
     sa = m.vb[A]; sbv = m.vb[B];
     for (int i = 0; i < 3; i++) {
-        finalize_boundary(m, slot3(sa, i));
-        finalize_boundary(m, slot3(sbv, i));
         m.ben[slot3(sa, i)] = 0;
         m.ben[slot3(sbv, i)] = 0;
     }
-    finalize_boundary(m, DF);
-    finalize_boundary(m, bnd);
     m.ben[DF] = 0;
     m.ben[bnd] = 0;
     m.ven[A] = 0; m.ven[D] = 0; m.ven[C] = 0; m.ven[B] = 0;
@@ -387,8 +387,10 @@ __device__ bool sorted_contains(const int *a, int lo, int hi, int x)
  * boundary in index order.  Only listed boundaries (those qualifying at the
  * count) and boundaries re-wired during the scan (CE) can qualify, so the
  * scan visits exactly those, in index order, re-testing each on visit.
- * One thread per instance, each over its own part of the ascending list. */
-__device__ void remove_two_three(const DevMesh &m, const int *list, int n, int *extra, int *segcnt, int inst)
+ * One thread per instance, each over its own part of the ascending list;
+ * the grains it removes are appended to gone. */
+__device__ void remove_two_three(const DevMesh &m, const int *list, int n, int *extra, int *segcnt, int *gone,
+                                 int *n_gone, int inst)
 {
     int i = lower_bound_i(list, n, m.boff[inst]);
     int N = lower_bound_i(list, n, m.boff[inst + 1]);
@@ -413,6 +415,9 @@ __device__ void remove_two_three(const DevMesh &m, const int *list, int n, int *
         int CE = remove_two_grains_dev(m, b, gnic);
         m.gen[gic[0]] = 0;
         m.gen[gic[1]] = 0;
+        int o = atomicAdd(n_gone, 2);
+        gone[o] = gic[0];
+        gone[o + 1] = gic[1];
         evt[EVT_TWO_THREE]++;
         if (CE > b && !sorted_contains(list, i, N, CE)) {
             int g2[2];
@@ -433,40 +438,46 @@ __device__ void remove_two_three(const DevMesh &m, const int *list, int n, int *
 /* ------------------------------------------------------------------ */
 /* 3-sided grain removal, src/topological.h:614-822, :994-1004         */
 /* ------------------------------------------------------------------ */
-/* label_3sided_grains (:994-1004) for one 3-sided grain */
-__device__ uint8_t label3_cand(const DevMesh &m, int g, double dt)
+/* label_3sided_grains (:994-1004) for the 3-sided grain g: -1, or, if g is
+ * to be removed, its lowest enabled boundary with 0 <= t_ext <= dt (there is
+ * one: a flip candidate is such a boundary, and so are all three in the
+ * reference's other case).  L, bs: its vertices and their boundaries. */
+__device__ int label3_first(const DevMesh &m, int g, double dt, int (&L)[3], int (&bs)[9])
 {
     /* The reference breaks out of a vertex's boundary loop once a flip
      * candidate inside the grain is found; that sets the result to 1 for
      * good, so testing every boundary gives the same answer and lets all
      * nine records load at once. */
-    const int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int l0 = L[0], l1 = L[1], l2 = L[2];
-    int4 s[3] = { m.vb[l0], m.vb[l1], m.vb[l2] };
-    int bs[9];
+    const int *row = m.glist + (size_t)SEVC_MAXV * g;
+    L[0] = row[0]; L[1] = row[1]; L[2] = row[2];
+    int4 s[3] = { m.vb[L[0]], m.vb[L[1]], m.vb[L[2]] };
     int2 e[9];
 #pragma unroll
     for (int j = 0; j < 9; j++) bs[j] = slot3(s[j / 3], j % 3);
 #pragma unroll
     for (int j = 0; j < 9; j++) e[j] = m.bv[bs[j]];
     bool cand = false;
-    int ans = 0;
+    int ans = 0, low = INT_MAX;
 #pragma unroll
     for (int j = 0; j < 9; j++) {
-        bool ii = e[j].x == l0 || e[j].x == l1 || e[j].x == l2;
-        bool ee = e[j].y == l0 || e[j].y == l1 || e[j].y == l2;
+        bool ii = e[j].x == L[0] || e[j].x == L[1] || e[j].x == L[2];
+        bool ee = e[j].y == L[0] || e[j].y == L[1] || e[j].y == L[2];
         if (ii && ee) {
             int b = bs[j];
             uint8_t en = m.ben[b], ca = m.bcand[b];
             double t = m.btext[b];
             cand |= ca && en;
-            ans += (t >= 0 && t <= dt) && en;
+            if (t >= 0 && t <= dt && en) {
+                ans++;
+                low = b < low ? b : low;
+            }
         }
     }
-    return cand || ans / 2 == 3;
+    return cand || ans / 2 == 3 ? low : -1;
 }
+
 /* remove_grain (:687-822) */
-__device__ void remove_grain_dev(const DevMesh &m, int grn)
+__device__ __noinline__ void remove_grain_dev(const DevMesh &m, int grn)
 {
     const int *L = m.glist + (size_t)SEVC_MAXV * grn;
     int A = L[0], B = L[1], C = L[2];
@@ -497,7 +508,7 @@ __device__ void remove_grain_dev(const DevMesh &m, int grn)
     for (int i = 0; i < 3; i++) {
         int x = slot3(sc, i);
         int2 e = m.bv[x];
-        if ((e.x == B && e.y == C) || (e.y == B && e.x == C)) { finalize_boundary(m, x); m.ben[x] = 0; break; }
+        if ((e.x == B && e.y == C) || (e.y == B && e.x == C)) { m.ben[x] = 0; break; }
     }
     int BE = -1, CF = -1;
     for (int i = 0; i < 3; i++) {
@@ -520,12 +531,12 @@ __device__ void remove_grain_dev(const DevMesh &m, int grn)
     for (int i = 0; i < 3; i++) {
         int x = slot3(sa, i);
         int2 f = m.bv[x];
-        if (f.x == B || f.y == B) { finalize_boundary(m, x); m.ben[x] = 0; set_slot3(sa, i, BE); break; }
+        if (f.x == B || f.y == B) { m.ben[x] = 0; set_slot3(sa, i, BE); break; }
     }
     for (int i = 0; i < 3; i++) {
         int x = slot3(sa, i);
         int2 f = m.bv[x];
-        if (f.x == C || f.y == C) { finalize_boundary(m, x); m.ben[x] = 0; set_slot3(sa, i, CF); break; }
+        if (f.x == C || f.y == C) { m.ben[x] = 0; set_slot3(sa, i, CF); break; }
     }
     m.vb[A] = sa;
     m.ven[B] = 0;
@@ -548,9 +559,7 @@ __device__ void remove_grain_dev(const DevMesh &m, int grn)
  * flips; here both phases follow ascending index order.  An event reads and
  * writes only its footprint (its vertices and the boundaries in their
  * slots) plus grain-level records that commute: queueing a grain for the
- * fix-up (an atomic claim of its flag), its mod slots (per vertex) and the
- * dA/dt settled from the step's starting values (settled before any event
- * of the phase runs).  Two events with disjoint footprints therefore
+ * fix-up (an atomic claim of its flag) and its mod slots (per vertex).  Two events with disjoint footprints therefore
  * commute, and the serial result is obtained by deterministic reservation:
  *   reserve  every event writes its key into each footprint record
  *            (atomicMin); the key orders events by grain or boundary index,
@@ -575,59 +584,16 @@ __device__ __forceinline__ bool valid_g(const DevMesh &m, int g) { return (unsig
 
 /* bring a record into this SM's L1 (no register result, no wait) */
 __device__ __forceinline__ void l1_touch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-/* An event's warp reserves its vertices and the boundaries in their slots
- * (lane 3j + k: vertex j, slot k) and settles the dA/dt of every grain
- * around them, one grain per lane (a grain an earlier lane also sees is
- * left to that lane), so the settling runs side by side instead of one
- * grain after another.  With `internal`, the extinction times of the
- * boundaries joining two of the event's vertices (the ones a 3-sided
- * removal disables) are settled too, each by the lane at its first end.
- * Settling reads only the step's starting values, which nothing changes
- * before the events apply, and is idempotent (an event that defers and
- * then finds other boundaries settles those itself).  Warp-uniform
- * arguments; every lane calls it. */
-__device__ void reserve_warp(const DevMesh &m, const DevScratch &x, const int *verts, int nverts,
-                             unsigned long long key, int lane, bool internal)
+/* one thread reserves a vertex and the boundaries in its slots */
+__device__ __forceinline__ void reserve_vertex(const DevMesh &m, const DevScratch &x, int v, int4 slots,
+                                               unsigned long long key)
 {
-    int j = lane / 3, k = lane - 3 * j, h = -1;
-    if (lane < 3 * nverts) {
-        int v = verts[j];
-        if (valid_v(m, v)) {
-            if (k == 0) atomicMin(x.vown + v, key);
-            int b = slot3(m.vb[v], k);
-            if (valid_b(m, b)) {
-                atomicMin(x.bown + b, key);
-                if (internal) {
-                    int2 e = m.bv[b];
-                    bool in = false;
-                    for (int q = 0; q < nverts; q++) in |= verts[q] != v && (verts[q] == e.x || verts[q] == e.y);
-                    if (in && e.x == v) finalize_boundary(m, b);
-                }
-            }
-            h = slot3(m.vg[v], k);
-            if (!valid_g(m, h)) h = -1;
-        }
+    atomicMin(x.vown + v, key);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        int b = slot3(slots, k);
+        if (valid_b(m, b)) atomicMin(x.bown + b, key);
     }
-    bool first = h >= 0;
-    for (int q = 0; q < 9; q++) {
-        int hq = __shfl_sync(0xffffffffu, h, q);
-        if (q < lane && hq == h) first = false;
-    }
-    /* settling walks the grain's list with three dependent loads per
-     * vertex: the lanes first bring their grains' lists and vertex records
-     * into L1, every load of a list issued at once */
-    if (first && !m.gexact[h]) {
-        const int *L = m.glist + (size_t)SEVC_MAXV * h;
-        int n = m.gvlen[h];
-        n = n < SEVC_MAXV ? n : SEVC_MAXV;
-#pragma unroll 4
-        for (int k = 0; k < n; k++) {
-            int v = L[k];
-            if (valid_v(m, v)) { l1_touch(m.pos + v); l1_touch(m.vel + v); l1_touch(m.vstamp + v); }
-        }
-    }
-    __syncwarp();
-    if (first) finalize_grain(m, h);
 }
 /* the records an event's single-thread code reads, brought into L1 by
  * the warp in two parallel rounds: the vertices' own records, then the
@@ -646,33 +612,176 @@ __device__ void prefetch_event(const DevMesh &m, const int *verts, int nverts, i
     if (valid_b(m, b)) { l1_touch(m.bv + b); l1_touch(m.bstamp + b); l1_touch(m.bexact + b); l1_touch(m.ben + b); }
     if (valid_g(m, h)) { l1_touch(m.gfix + h); l1_touch(m.gexact + h); l1_touch(m.gvlen + h); }
 }
-/* whether v and every boundary in its slots hold key; nothing but the
- * event holding v writes its slots, so they are the reserved ones */
-__device__ bool holds_vertex(const DevMesh &m, const DevScratch &x, int v, unsigned long long key)
+/* whether every vertex of an event and every boundary in their slots hold
+ * its key (lane 3j + k: vertex j, slot k); nothing but the event holding a
+ * vertex writes its slots, so they are the reserved ones */
+__device__ bool warp_holds(const DevMesh &m, const DevScratch &x, const int *verts, int nverts, unsigned long long key,
+                           int lane)
 {
-    if (x.vown[v] != key) return false;
-    int4 s = m.vb[v];
-    for (int j = 0; j < 3; j++) {
-        int b = slot3(s, j);
-        if (!valid_b(m, b) || x.bown[b] != key) return false;
+    bool ok = true;
+    if (lane < 3 * nverts) {
+        int j = lane / 3, v = verts[j];
+        ok = valid_v(m, v);
+        if (ok) {
+            int b = slot3(m.vb[v], lane - 3 * j);
+            ok = x.vown[v] == key && valid_b(m, b) && x.bown[b] == key;
+        }
     }
+    return __all_sync(0xffffffffu, ok);
+}
+
+/* remove_grain_dev for the usual case: the same writes with the same
+ * values, but every record it reads is loaded up front, in two rounds,
+ * instead of behind the writes that precede it, and the work-list appends
+ * take one atomic each (the fix-up edits each queued grain on its own, so
+ * the order of the entries does not matter).  False, with nothing
+ * written, when a boundary or grain the removal needs is not found or an
+ * outer boundary also joins A: remove_grain_dev then does it step by step.
+ * nAB, nBC, nCA: the triangle's sides. */
+__device__ bool remove_planned(const DevMesh &m, int grn, double nAB, double nBC, double nCA)
+{
+    const int *row = m.glist + (size_t)SEVC_MAXV * grn;
+    const int A = row[0], B = row[1], C = row[2];
+    const double D = m.D;
+    double2 pa = m.pos[A], pb = m.pos[B], pc = m.pos[C], va = m.vel[A];
+    int4 sa = m.vb[A], sb = m.vb[B], sc = m.vb[C], ga = m.vg[A], gb = m.vg[B], gc = m.vg[C];
+    int4 mB0 = m.vmod[4 * (size_t)B], mC0 = m.vmod[4 * (size_t)C], mB1 = m.vmod[4 * (size_t)B + 1];
+    uint8_t mkB = m.vmodmark[B], mkC = m.vmodmark[C];
+    unsigned st = *m.stamp, stA = m.vstamp[A];
+    int2 ea[3], eb[3], ec[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) { ea[i] = m.bv[slot3(sa, i)]; eb[i] = m.bv[slot3(sb, i)]; ec[i] = m.bv[slot3(sc, i)]; }
+    int BC = -1, BE = -1, CF = -1, AB = -1, CA = -1, iAB = 0, iCA = 0;
+    int2 eBE = make_int2(0, 0), eCF = make_int2(0, 0);
+#pragma unroll
+    for (int i = 2; i >= 0; i--) {                  /* the first match of each search */
+        if ((ec[i].x == B && ec[i].y == C) || (ec[i].y == B && ec[i].x == C)) BC = slot3(sc, i);
+        if (!(eb[i].x == A || eb[i].y == A) && !(eb[i].x == C || eb[i].y == C)) { BE = slot3(sb, i); eBE = eb[i]; }
+        if (!(ec[i].x == A || ec[i].y == A) && !(ec[i].x == B || ec[i].y == B)) { CF = slot3(sc, i); eCF = ec[i]; }
+        if (ea[i].x == B || ea[i].y == B) { AB = slot3(sa, i); iAB = i; }
+    }
+#pragma unroll
+    for (int i = 2; i >= 0; i--)
+        if (!(AB >= 0 && i == iAB) && (ea[i].x == C || ea[i].y == C)) { CA = slot3(sa, i); iCA = i; }
+    int gbc[2], gab[2], gac[2];
+    gintersect(gb, gc, gbc);
+    gintersect(ga, gb, gab);
+    gintersect(ga, gc, gac);
+    const int G3 = gbc[0] == grn ? gbc[1] : gbc[0], G2 = gab[0] == grn ? gab[1] : gab[0];
+    const int G1 = gac[0] == grn ? gac[1] : gac[0];
+    if (BC < 0 || BE < 0 || CF < 0 || AB < 0 || CA < 0 || G1 < 0 || G2 < 0 || G3 < 0 || BE == CF) return false;
+    if (sa.x == BE || sa.y == BE || sa.z == BE || sa.x == CF || sa.y == CF || sa.z == CF) return false;
+    unsigned sBE = m.bstamp[BE], sCF = m.bstamp[CF];
+    log_event(m, EV_REMOVE, A, B, C, pa, pb, pc);
+    /* mark_fix of the three grains: claims and appends */
+    const int G[3] = { G2, G1, G3 };
+    bool nf[3];
+    int nfix = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        nf[k] = claim_byte(m.gfix, G[k]);
+        nfix += nf[k];
+    }
+    const int nm = (mkB ? 0 : 1) + (mkC ? 0 : 1);
+    int f0 = nfix ? atomicAdd(m.nfix, nfix) : 0, m0 = nm ? atomicAdd(m.nmod, nm) : 0;
+    double denom = nAB + nBC + nCA;
+    double x0 = 0, y0 = 0;                                      /* adjust_origin_for_points, 3 points */
+    double x1 = x0 + wrapd(pb.x, pa.x, D), y1 = y0 + wrapd(pb.y, pa.y, D);
+    double x2 = x1 + wrapd(pc.x, pb.x, D), y2 = y1 + wrapd(pc.y, pb.y, D);
+    double2 q = pa;
+    q.x += (nBC * x0 + nCA * x1 + nAB * x2) / denom;
+    q.y += (nBC * y0 + nCA * y1 + nAB * y2) / denom;
+    q.x = dmod(q.x, D);
+    q.y = dmod(q.y, D);
+    if (stA != st) { m.pos0[A] = pa; m.vel0[A] = va; m.vstamp[A] = st; }     /* save_vertex */
+    m.pos[A] = q;
+    m.vel[A] = make_double2(0.0, 0.0);
+    m.ben[BC] = 0;
+    m.ben[AB] = 0;
+    m.ben[CA] = 0;
+    if (sBE != st) { m.bv0[BE] = eBE; m.bstamp[BE] = st; }                   /* save_ends */
+    if (sCF != st) { m.bv0[CF] = eCF; m.bstamp[CF] = st; }
+    if (eBE.x == B) eBE.x = A; else eBE.y = A;
+    if (eCF.x == C) eCF.x = A; else eCF.y = A;
+    m.bv[BE] = eBE;
+    m.bv[CF] = eCF;
+    set_slot3(sa, iAB, BE);
+    set_slot3(sa, iCA, CF);
+    m.vb[A] = sa;
+    m.ven[B] = 0;
+    m.ven[C] = 0;
+    m.gen[grn] = 0;
+    /* set_mod(B, 0, REMOVE, G2, B), (C, 0, REMOVE, G1, C), (B, 1, REMOVE, G3,
+     * B), (C, 1, REPLACE, G3, A, C) */
+    mB0.x = G2; mB0.y = B; mB0.w = FIX_REMOVE;
+    mC0.x = G1; mC0.y = C; mC0.w = FIX_REMOVE;
+    mB1.x = G3; mB1.y = B; mB1.w = FIX_REMOVE;
+    m.vmod[4 * (size_t)B] = mB0;
+    m.vmod[4 * (size_t)C] = mC0;
+    m.vmod[4 * (size_t)B + 1] = mB1;
+    m.vmod[4 * (size_t)C + 1] = make_int4(G3, A, C, FIX_REPLACE);
+    if (!mkB) {
+        m.vmodmark[B] = 1;
+        if (m0 < m.modcap) m.modlist[m0] = B; else raise_err(m, ERRB_WORKLIST);
+        m0++;
+    }
+    if (!mkC) {
+        m.vmodmark[C] = 1;
+        if (m0 < m.modcap) m.modlist[m0] = C; else raise_err(m, ERRB_WORKLIST);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        if (nf[k]) {
+            if (f0 < m.fixcap) m.fixlist[f0] = G[k]; else raise_err(m, ERRB_WORKLIST);
+            f0++;
+        }
+    for (int i = 0; i < 3; i++) if (slot3(ga, i) == grn) set_slot3(ga, i, G3);
+    m.vg[A] = ga;
     return true;
 }
 
-/* 3-sided removals (remove_grains, :994) of the listed grains: a removal
- * disables only its own grain, so the set is known up front.  One warp per
- * grain: first every removal reserves its records, then its records are
- * brought into L1 and lane 0 applies it (or it defers, when an earlier
- * removal holds a record). */
-__device__ void remove_reserve(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
+/* clear_grains_state and label_3sided_grains (src/main.cu:252-255), then the
+ * removals' reservations (remove_grains, :994): a removal disables only its
+ * own grain, so the set is known up front.  A removable grain has an
+ * enabled boundary with 0 <= t_ext <= dt, so it lies beside a boundary of
+ * the candidate list: one thread per listed boundary and grain at its first
+ * end; the grain is listed by its lowest such boundary. */
+__device__ void label3_reserve(const DevMesh &m, const DevScratch &x, const Team &T, int na, double dt)
 {
     const unsigned ep = 2u * *m.stamp;
-    for (int i = T.warp; i < n; i += T.nwarps) {
-        int g = list[i];
-        const int *L = m.glist + (size_t)SEVC_MAXV * g;
-        int verts[3] = { L[0], L[1], L[2] };
-        reserve_warp(m, x, verts, 3, resv_key(ep, g), T.lane, true);
+    for (int t = T.tid; t < 3 * na; t += T.n) {
+        int i = t / 3, j = t - 3 * i, b = x.list_a[i];
+        if (!m.ben[b]) continue;
+        int2 e = m.bv[b];
+        int4 ga = m.vg[e.x], gb = m.vg[e.y];
+        int g = slot3(ga, j);
+        if (!valid_g(m, g) || (j > 0 && g == ga.x) || (j > 1 && g == ga.y)) continue;
+        if (g != gb.x && g != gb.y && g != gb.z) continue;
+        if (!m.gen[g] || m.gvlen[g] != 3) continue;
+        int L[3], bs[9];
+        if (label3_first(m, g, dt, L, bs) != b) continue;
+        x.list_c[atomicAdd(x.n_c, 1)] = g;
+        const unsigned long long key = resv_key(ep, g);
+#pragma unroll
+        for (int k = 0; k < 3; k++) reserve_vertex(m, x, L[k], make_int4(bs[3 * k], bs[3 * k + 1], bs[3 * k + 2], -1), key);
     }
+}
+/* One warp per removal: its lanes check that it holds its records and bring
+ * them into L1, lane 0 applies it (or it defers, when an earlier removal
+ * holds a record). */
+__device__ void remove_warp(const DevMesh &m, int g, int inst, int lane)
+{
+    /* lane k < 3: the side from list vertex k to the next */
+    const int *L = m.glist + (size_t)SEVC_MAXV * g;
+    double side = 0;
+    if (lane < 3) side = arclen(m.pos[L[lane]], m.pos[L[lane < 2 ? lane + 1 : 0]], m.D);
+    const double s0 = __shfl_sync(0xffffffffu, side, 0), s1 = __shfl_sync(0xffffffffu, side, 1),
+                 s2 = __shfl_sync(0xffffffffu, side, 2);
+    if (lane == 0) {
+        if (!remove_planned(m, g, s0, s1, s2)) remove_grain_dev(m, g);
+        atomicAdd(&m.evt[EVT_COUNT * inst + EVT_REMOVALS], 1);
+    }
+    __syncwarp();
 }
 __device__ void remove_apply(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
 {
@@ -681,22 +790,10 @@ __device__ void remove_apply(const DevMesh &m, const DevScratch &x, const Team &
         int g = list[i];
         const int *L = m.glist + (size_t)SEVC_MAXV * g;
         int verts[3] = { L[0], L[1], L[2] };
-        unsigned long long key = resv_key(ep, g);
-        bool own = true;
-        if (T.lane == 0)
-            for (int k = 0; k < 3 && own; k++) own = valid_v(m, verts[k]) && holds_vertex(m, x, verts[k], key);
-        own = __shfl_sync(0xffffffffu, own, 0);
-        if (own) prefetch_event(m, verts, 3, T.lane);
-        __syncwarp();
-        if (T.lane == 0) {
-            if (own) {
-                remove_grain_dev(m, g);
-                atomicAdd(&m.evt[EVT_COUNT * m.ginst[g] + EVT_REMOVALS], 1);
-            } else {
-                x.ehits[atomicAdd(x.n_ehits, 1)] = g;
-            }
-        }
-        __syncwarp();
+        prefetch_event(m, verts, 3, T.lane);
+        bool own = warp_holds(m, x, verts, 3, resv_key(ep, g), T.lane);
+        if (own) remove_warp(m, g, m.ginst[g], T.lane);
+        else if (T.lane == 0) x.ehits[atomicAdd(x.n_ehits, 1)] = g;
     }
 }
 /* The deferred events x.ehits[0..nd) in ascending order, one warp per
@@ -718,28 +815,10 @@ __device__ void run_deferred(const DevMesh &m, const DevScratch &x, const Team &
     }
 }
 
-/* unlabel_boundaries_st2 (:588-606) for an enabled candidate b: it stays
- * a candidate unless a grain on either side has 3 sides.  It reads and
- * writes only b's own flags, so it runs inside the flip reservation (one
- * warp per candidate, warp-uniform result). */
-__device__ bool unlabel_st2_keeps(const DevMesh &m, int b)
-{
-    int2 e = m.bv[b];
-    int gic[2];
-    if (gintersect(m.vg[e.x], m.vg[e.y], gic) < 2) {       /* the step fails */
-        if ((threadIdx.x & 31) == 0) raise_err(m, ERRB_TOPOLOGY);
-        return false;
-    }
-    bool keep = !(m.gvlen[gic[0]] == 3 || m.gvlen[gic[1]] == 3);
-    __syncwarp();
-    if (!keep && (threadIdx.x & 31) == 0) m.bcand[b] = 0;
-    return keep;
-}
-
 /* ------------------------------------------------------------------ */
 /* T1 flip, src/topological.h:174-291                                  */
 /* ------------------------------------------------------------------ */
-__device__ void flip_dev(const DevMesh &m, int bnd, double eps)
+__device__ __noinline__ void flip_dev(const DevMesh &m, int bnd, double eps)
 {
     int2 eb = m.bv[bnd];
     int A = eb.x, B = eb.y;
@@ -801,44 +880,6 @@ __device__ void flip_dev(const DevMesh &m, int bnd, double eps)
     m.vel[B] = make_double2(0, 0);
 }
 
-/* Before lane 0 applies a flip (one long chain of dependent loads), the
- * warp brings the flip's neighbourhood into the SM's L1 in a few parallel
- * rounds: the two vertices' slots, positions and velocities; the boundary
- * ends and grain records around them; the lists of those grains; and the
- * positions, velocities and save stamps of the listed vertices (read by
- * finalize_grain).  Loads only, every index checked against its array. */
-__device__ __forceinline__ void touch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-__device__ void prefetch_flip(const DevMesh &m, int bnd, int lane)
-{
-    int2 e = m.bv[bnd];
-    if (e.x < 0 || e.x >= m.nv || e.y < 0 || e.y >= m.nv) return;
-    int4 gA = m.vg[e.x], gB = m.vg[e.y], bA = m.vb[e.x], bB = m.vb[e.y];
-    int gs[6] = { gA.x, gA.y, gA.z, gB.x, gB.y, gB.z }, bs[6] = { bA.x, bA.y, bA.z, bB.x, bB.y, bB.z };
-    if (lane < 6) {
-        int g = gs[lane];
-        if (g >= 0 && g < m.ng) { touch(m.gvlen + g); touch(m.gexact + g); touch(m.gfix + g); }
-        int b = bs[lane];
-        if (b >= 0 && b < m.nb) touch(m.bv + b);
-    } else if (lane < 8) {
-        int v = lane == 6 ? e.x : e.y;
-        touch(m.pos + v); touch(m.vel + v); touch(m.vstamp + v); touch(m.vmod + 4 * (size_t)v);
-    }
-    /* lists of the grains: lane 5k + j reads entries j, j + 5, ... of grain k */
-    int k = lane / 5, j = lane % 5;
-    if (k < 6) {
-        int g = gs[k];
-        if (g >= 0 && g < m.ng) {
-            int n = m.gvlen[g];
-            n = n < SEVC_MAXV ? n : SEVC_MAXV;
-            const int *L = m.glist + (size_t)SEVC_MAXV * g;
-            for (int i = j; i < n; i += 5) {
-                int v = L[i];
-                if (v >= 0 && v < m.nv) { touch(m.pos + v); touch(m.vel + v); touch(m.vstamp + v); }
-            }
-        }
-    }
-}
-
 /* What flip_dev derives before it writes anything: the two ends, their
  * other boundaries AC and BE (the successors of bnd in their slot
  * orders, at slots i and j), the grains on both sides (gic) and at the
@@ -850,15 +891,11 @@ struct FlipPlan {
     int4 sa, sb, ga, gb;
 };
 
-/* Every lane of the warp derives the flip's plan; lanes 0-7 scan the four
- * grain lists at once (a flip edits no list, so the answers are the ones
- * flip_dev's own scans give).  The four grains the flip queues for the
- * fix-up pass (mark_fix) then have their dA/dt settled, each by its own
- * lane: finalize_grain reads only the grain's list and its vertices'
- * positions and velocities at the start of the step, which nothing in a
- * flip changes before those calls, so the values are the ones the flip
- * would compute.  Returns false (nothing settled) on any inconsistency;
- * the flip then runs its own checks and reports it. */
+/* Every lane of the warp derives the flip's plan; eight lanes scan each of
+ * the four grain lists (a flip edits no list, so the answers are the ones
+ * flip_dev's own scans give: glist_consecutive(g, P, Q) is 1 when the first
+ * place where P and Q are neighbours has P first).  Returns false on any
+ * inconsistency; the flip then runs its own checks and reports it. */
 __device__ bool flip_plan(const DevMesh &m, int bnd, int lane, FlipPlan &P)
 {
     int2 eb = m.bv[bnd];
@@ -872,23 +909,30 @@ __device__ bool flip_plan(const DevMesh &m, int bnd, int lane, FlipPlan &P)
     for (int k = 0; k < 3; k++) if (slot3(P.sa, k) == bnd) { P.i = (k + 1) % 3; P.AC = slot3(P.sa, P.i); break; }
     for (int k = 0; k < 3; k++) if (slot3(P.sb, k) == bnd) { P.j = (k + 1) % 3; P.BE = slot3(P.sb, P.j); break; }
     if (P.AC < 0 || P.BE < 0 || P.gnic[0] < 0 || P.gnic[1] < 0) return false;
-    bool hit = false;
-    if (lane < 4) hit = glist_consecutive(m, P.gic[lane & 1], lane < 2 ? A : B, lane < 2 ? B : A) == 1;
-    else if (lane < 8) hit = glist_find(m, P.gnic[lane & 1], lane < 6 ? A : B) >= 0;
-    unsigned h = __ballot_sync(0xffffffffu, hit);
-    P.g2 = (h & 1) ? 0 : (h & 2) ? 1 : 2;
-    P.g4 = (h & 4) ? 0 : (h & 8) ? 1 : 2;
-    P.g3 = (h & 16) ? 0 : (h & 32) ? 1 : 2;
-    P.g1 = (h & 64) ? 0 : (h & 128) ? 1 : 2;
-    if (P.g1 == 2 || P.g2 == 2 || P.g3 == 2 || P.g4 == 2) return false;
-    int G[4] = { P.gic[P.g2], P.gic[P.g4], P.gnic[P.g3], P.gnic[P.g1] };
-    if (lane < 4) {
-        int g = G[lane];
-        bool dup = false;
-        for (int k = 0; k < lane; k++) dup |= G[k] == g;
-        if (!dup) finalize_grain(m, g);
+    const int q = lane >> 3, g = q < 2 ? P.gic[q] : P.gnic[q - 2];
+    const int *L = m.glist + (size_t)SEVC_MAXV * g;
+    const int n = m.gvlen[g];
+    int ab = SEVC_MAXV, ba = SEVC_MAXV;             /* first i with (A, B), (B, A) at i, i + 1 */
+    bool hasA = false, hasB = false;
+    for (int i = lane & 7; i < n; i += 8) {
+        int u = L[i], w = L[i + 1 < n ? i + 1 : 0];
+        if (u == A && w == B && ab == SEVC_MAXV) ab = i;
+        if (u == B && w == A && ba == SEVC_MAXV) ba = i;
+        hasA |= u == A;
+        hasB |= u == B;
     }
-    return true;
+    for (int o = 4; o > 0; o >>= 1) {
+        ab = min(ab, __shfl_xor_sync(0xffffffffu, ab, o));
+        ba = min(ba, __shfl_xor_sync(0xffffffffu, ba, o));
+    }
+    const unsigned f = __ballot_sync(0xffffffffu, ab < SEVC_MAXV && ab <= ba);
+    const unsigned r = __ballot_sync(0xffffffffu, ba < SEVC_MAXV && ba < ab);
+    const unsigned hA = __ballot_sync(0xffffffffu, hasA), hB = __ballot_sync(0xffffffffu, hasB);
+    P.g2 = (f & 0xffu) ? 0 : (f & 0xff00u) ? 1 : 2;
+    P.g4 = (r & 0xffu) ? 0 : (r & 0xff00u) ? 1 : 2;
+    P.g3 = (hA & 0xff0000u) ? 0 : (hA & 0xff000000u) ? 1 : 2;
+    P.g1 = (hB & 0xff0000u) ? 0 : (hB & 0xff000000u) ? 1 : 2;
+    return !(P.g1 == 2 || P.g2 == 2 || P.g3 == 2 || P.g4 == 2);
 }
 
 /* flip_dev from a plan, for the usual case AC != BE: the same writes with
@@ -942,8 +986,8 @@ __device__ void flip_planned(const DevMesh &m, int bnd, double eps, const FlipPl
             if (i0 < m.modcap) m.modlist[i0] = B; else raise_err(m, ERRB_WORKLIST);
         }
     }
-    /* mark_fix of the four grains (their dA/dt is settled); flips running
-     * at the same time may queue the same grain, the claim decides */
+    /* mark_fix of the four grains; flips running at the same time may queue
+     * the same grain, the claim decides */
     bool nf[4];
     int nfix = 0;
 #pragma unroll
@@ -994,23 +1038,34 @@ __device__ void flip_planned(const DevMesh &m, int bnd, double eps, const FlipPl
  * flag, so the flips are known up front.  Reservation, parallel
  * application and the deferred pass as for the removals (epoch 2 * stamp
  * + 1); the footprint is both ends with their slots. */
+/* unlabel_boundaries_st2 (:588-606) for an enabled candidate, then its
+ * reservation: it stays a candidate unless a grain on either side has 3
+ * sides.  One thread per listed boundary. */
 __device__ void flip_reserve(const DevMesh &m, const DevScratch &x, const Team &T, const int *list, int n)
 {
     const unsigned ep = 2u * *m.stamp + 1u;
-    for (int i = T.warp; i < n; i += T.nwarps) {
+    for (int i = T.tid; i < n; i += T.n) {
         int b = list[i];
         if (!(m.ben[b] && m.bcand[b])) continue;
-        if (!unlabel_st2_keeps(m, b)) continue;
         int2 e = m.bv[b];
-        int verts[2] = { e.x, e.y };
-        reserve_warp(m, x, verts, 2, resv_key(ep, b), T.lane, false);
+        int4 sa = m.vb[e.x], sb = m.vb[e.y];
+        int gic[2];
+        if (gintersect(m.vg[e.x], m.vg[e.y], gic) < 2) {       /* the step fails */
+            raise_err(m, ERRB_TOPOLOGY);
+            continue;
+        }
+        if (m.gvlen[gic[0]] == 3 || m.gvlen[gic[1]] == 3) {
+            m.bcand[b] = 0;
+            continue;
+        }
+        const unsigned long long key = resv_key(ep, b);
+        reserve_vertex(m, x, e.x, sa, key);
+        reserve_vertex(m, x, e.y, sb, key);
     }
 }
-/* a warp: its lanes prefetch the flip's neighbourhood and derive the plan,
- * lane 0 applies it */
+/* a warp: its lanes derive the plan, lane 0 applies it */
 __device__ void flip_warp(const DevMesh &m, int b, double eps, int lane)
 {
-    prefetch_flip(m, b, lane);
     FlipPlan P;
     bool planned = flip_plan(m, b, lane, P) && P.AC != P.BE;
     __syncwarp();
@@ -1028,11 +1083,9 @@ __device__ void flip_apply(const DevMesh &m, const DevScratch &x, const Team &T,
         int b = list[i];
         if (!(m.ben[b] && m.bcand[b])) continue;
         int2 e = m.bv[b];
-        unsigned long long key = resv_key(ep, b);
-        bool own = false;
-        if (T.lane == 0)
-            own = valid_v(m, e.x) && valid_v(m, e.y) && holds_vertex(m, x, e.x, key) && holds_vertex(m, x, e.y, key);
-        own = __shfl_sync(0xffffffffu, own, 0);
+        int verts[2] = { e.x, e.y };
+        prefetch_event(m, verts, 2, T.lane);
+        bool own = warp_holds(m, x, verts, 2, resv_key(ep, b), T.lane);
         if (own) flip_warp(m, b, eps, T.lane);
         else if (T.lane == 0) x.ehits[atomicAdd(x.n_ehits, 1)] = b;
     }
@@ -1177,23 +1230,59 @@ __device__ void fix_clear(const DevMesh &m, const Team &T, bool areas)
         int g = m.fixlist[w];
         if (m.gen[g]) {
             m.gfix[g] = 0;
-            if (areas) {
-                double2 none = make_double2(0, 0);
-                m.garea[g] = area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, -1, none, m.D);
-            }
+            if (areas) m.garea[g] = area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, m.D);
         }
     }
-    for (int w = T.tid; w < nm; w += T.n) {
-        int v = m.modlist[w];
-        m.vmodmark[v] = 0;
-        int4 sg = m.vg[v];
-        bool listed = false;
-        for (int j = 0; j < 3 && !listed; j++) {
-            int g = slot3(sg, j);
-            if (g >= 0 && m.gen[g] && glist_find(m, g, v) >= 0) listed = true;
+    /* a thread per marked vertex and grain around it, from the other end of
+     * the team; each that finds the vertex listed writes the same */
+    for (int t = T.n - 1 - T.tid; t < 3 * nm; t += T.n) {
+        int w = t / 3, j = t - 3 * w, v = m.modlist[w];
+        if (j == 0) m.vmodmark[v] = 0;
+        int g = slot3(m.vg[v], j);
+        if (g >= 0 && m.gen[g] && glist_find(m, g, v) >= 0)
+            for (int k = 0; k < 4; k++) m.vmod[4 * (size_t)v + k] = make_int4(-1, -1, -1, FIX_NONE);
+    }
+}
+__device__ __noinline__ void settle_boundary(const DevMesh &m, int b) { finalize_boundary(m, b); }
+/* Output-only values that the events make final (see DevMesh): the dA/dt of
+ * the queued grains, whose lists the fix-up is about to change, and of the
+ * removed ones (gone[0..ngone)), one grain per thread; and the extinction
+ * times of the boundaries at the removed grains' vertices that are now
+ * disabled.  All from the step's starting state, which the events saved.
+ * A boundary costs some 400 FP64 operations (atan2, cos, sin), so its
+ * threads are the k-th (k < 3) such boundary of each removed grain, not its
+ * nine slots with mostly idle lanes; the third takes any beyond. */
+__device__ void settle(const DevMesh &m, const Team &T, const int *gone, int ngone)
+{
+    const int nf = min(*m.nfix, m.fixcap);
+    for (int t = T.tid; t < nf + ngone; t += T.n) finalize_grain(m, t < nf ? m.fixlist[t] : gone[t - nf]);
+    /* the boundaries from the other end of the team, beside the grains */
+    for (int t = T.n - 1 - T.tid; t < 3 * ngone; t += T.n) {
+        const int i = t / 3, k = t - 3 * i;
+        const int *L = m.glist + (size_t)SEVC_MAXV * gone[i];
+        int b[9];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            int4 s = m.vb[L[j]];
+            b[3 * j] = s.x; b[3 * j + 1] = s.y; b[3 * j + 2] = s.z;
         }
-        if (listed)
-            for (int j = 0; j < 4; j++) m.vmod[4 * (size_t)v + j] = make_int4(-1, -1, -1, FIX_NONE);
+        unsigned due = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            bool off = valid_b(m, b[j]) && !m.ben[b[j]] && !m.bexact[b[j]];
+#pragma unroll
+            for (int q = 0; q < j; q++) off = off && b[q] != b[j];
+            due |= off ? 1u << j : 0u;
+        }
+        for (int c = 0; due; c++, due &= due - 1) {
+            if (c < k) continue;
+            const int j = __ffs(due) - 1;
+            int x = b[0];
+#pragma unroll
+            for (int q = 1; q < 9; q++) x = q == j ? b[q] : x;
+            settle_boundary(m, x);
+            if (k < 2) break;
+        }
     }
 }
 /* fix_grain_lists (:1209-1227): the edits, then the clearing; both work
@@ -1221,8 +1310,13 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
         rank_sort(T, x.list_b, n, sorted);
         T.sync();
         if (T.tid == 0) *x.n_b = 0;
+        T.sync();
         for (int i = T.tid; i < m.ninst; i += T.n)
-            remove_two_three(m, sorted, n, x.extra, x.segcnt + (size_t)pass * m.ninst, i);
+            remove_two_three(m, sorted, n, x.extra, x.segcnt + (size_t)pass * m.ninst, x.list_b, x.n_b, i);
+        T.sync();
+        settle(m, T, x.list_b, *x.n_b);       /* the removed grains, listed by the removals */
+        T.sync();
+        if (T.tid == 0) *x.n_b = 0;
         T.sync();
         fix_lists(m, T, S, true, x.ehits, x.n_ehits);
         const int n3 = *x.n_three, more = *x.n_ehits;
@@ -1267,35 +1361,21 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
         poll_reset(m, x, T, pg, nfail);
         T.sync();
         if (*x.n_b > 0) two_three_loop(m, x, T, S);
-        const int n3 = *x.n_three, more = *x.n_ehits;
-        for (int i = T.tid; i < n3 + more; i += T.n) {
-            int g = i < n3 ? x.three[i] : x.ehits[i - n3];
-            if (m.gen[g] && m.gvlen[g] == 3 && label3_cand(m, g, dt)) x.list_c[atomicAdd(x.n_c, 1)] = g;
-        }
+        if (na > 0) label3_reserve(m, x, T, na, dt);
+        if (T.tid == 0) *x.n_ehits = 0;              /* the grains a 2x3 pass left with three sides */
         T.sync();
         const int nc = *x.n_c;
         if (nc > 0) {
-            if (T.tid == 0) *x.n_ehits = 0;
-            remove_reserve(m, x, T, x.list_c, nc);
-            T.sync();
             remove_apply(m, x, T, x.list_c, nc);
             T.sync();
             const int nd = *x.n_ehits;
             if (nd > 0) {
-                run_deferred(m, x, T, nd, m.goff, [&](int g, int inst) {
-                    if (T.lane == 0) {
-                        remove_grain_dev(m, g);
-                        m.evt[EVT_COUNT * inst + EVT_REMOVALS]++;
-                    }
-                    __syncwarp();
-                });
+                run_deferred(m, x, T, nd, m.goff, [&](int g, int inst) { remove_warp(m, g, inst, T.lane); });
                 T.sync();
             }
+            settle(m, T, x.list_c, nc);
+            T.sync();
             fix_lists(m, T, S, true, nullptr, nullptr);
-        } else if (more > 0) {
-            T.sync();
-            if (T.tid == 0) *x.n_ehits = 0;
-            T.sync();
         }
     }
     if ((PART & TAIL_FLIP) && na > 0) {
@@ -1306,6 +1386,10 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
         const int nd = *x.n_ehits;
         if (nd > 0) {
             run_deferred(m, x, T, nd, m.boff, [&](int b, int) { flip_warp(m, b, eps, T.lane); });
+            T.sync();
+        }
+        if (*m.nfix > 0) {
+            settle(m, T, nullptr, 0);
             T.sync();
         }
     }
