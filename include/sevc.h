@@ -136,7 +136,7 @@ sevc_status sevc_run_steps(sevc_handle *h, int nsteps, int *done, sevc_step_info
  * `done` = steps run.  It does not stop at the reference's stop criterion
  * (src/main.cu:120, :391): the caller reads keep_going and the
  * counts from `infos`.  With one graph per step (sevc_set_graphs(h, 1), the
- * default), no profiling or tape, and no grain-count stop (min_grains <= 0,
+ * default), no profiling, and no grain-count stop (min_grains <= 0,
  * or a batch), the steps are pipelined: each step is launched while the one
  * before it runs and its summary is read back afterwards, so the GPU does
  * not wait on the host between steps (an attempt step waits for the step

@@ -35,6 +35,7 @@
 namespace {
 
 constexpr int TPB = 256;
+constexpr int ADJ_BLOCK = 64;   /* of the backward pass's long threads: small meshes spread over the SMs */
 inline int nblk(int n) { return (n + TPB - 1) / TPB; }
 
 /* quadratic B-spline (partition of unity over unit-spaced bins) and its derivative */
@@ -59,18 +60,24 @@ __device__ __forceinline__ double grain_area(const DevMesh &m, int g)
     return area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, m.D);
 }
 
-/* position of vertex v in grain g's list, its list neighbours */
-__device__ __forceinline__ int list_pos(const DevMesh &m, int g, int v, int *prev, int *next)
+/* list neighbours of vertex v in grain g (false: not listed); eight entries
+ * of the list a load */
+__device__ __forceinline__ bool list_neighbours(const DevMesh &m, int g, int v, int &prev, int &next)
 {
     const int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    for (int p = 0; p < n; p++)
-        if (L[p] == v) {
-            *prev = L[p == 0 ? n - 1 : p - 1];
-            *next = L[p == n - 1 ? 0 : p + 1];
-            return p;
+    const int n = m.gvlen[g];
+    for (int base = 0; base < n; base += 8) {
+        int e[8], at = -1;
+        list_batch(L, n, base, e);
+#pragma unroll
+        for (int j = 7; j >= 0; j--) at = base + j < n && e[j] == v ? base + j : at;
+        if (at >= 0) {
+            prev = L[at == 0 ? n - 1 : at - 1];
+            next = L[at == n - 1 ? 0 : at + 1];
+            return true;
         }
-    return -1;
+    }
+    return false;
 }
 
 /* ---------------- histogram of normalised grain areas ---------------- */
@@ -162,7 +169,7 @@ __global__ void k_area_grad_to_vertices(DevMesh m, const double *dlda, double2 *
             int g = slot3(sg, j);
             if (g < 0 || !m.gen[g]) continue;
             int pv, nx;
-            if (list_pos(m, g, v, &pv, &nx) < 0) continue;
+            if (!list_neighbours(m, g, v, pv, nx)) continue;
             double2 a = m.pos[pv], b = m.pos[nx];
             /* unwrapped neighbour coordinates relative to v */
             double xp = wrapd(a.x, p.x, m.D), yp = wrapd(a.y, p.y, m.D);
@@ -175,30 +182,18 @@ __global__ void k_area_grad_to_vertices(DevMesh m, const double *dlda, double2 *
 }
 
 /* ---------------- adjoint of one step ---------------- */
-/* vertices moved by an event this step (their velocity was zeroed) */
-__global__ void k_adj_mark_events(uint8_t *mark, const EventRec *log, const int *nlog)
-{
-    int n = *nlog;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        EventRec r = log[i];
-        if (r.type != EV_FLIP && r.type != EV_REMOVE) continue;
-        mark[r.a] = 1;
-        mark[r.b] = 1;
-        if (r.type == EV_REMOVE) mark[r.c] = 1;
-    }
-}
-
 /* translation x_{n+1} = x' + dt v': lambda_x' = lambda (vertices alive
- * after the step), lambda_v = dt lambda (alive, not moved by an event);
- * d/dmu of the step: dt * lambda . v' / mu */
+ * after the step), lambda_v = dt lambda (k_adj_events zeroes it for the
+ * vertices an event moved); d/dmu of the step: dt * lambda . v' / mu */
 __global__ void k_adj_translate(int nv, double dt, double mu, const double2 *lam, const uint8_t *ven1,
-                                const double2 *vel1, const uint8_t *mark, double2 *lx, double2 *lv, double *gmu)
+                                const double2 *vel1, double2 *lx, double2 *lv, double *gmu)
 {
+    griddep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nv) return;
     double2 l = ven1[i] ? lam[i] : make_double2(0, 0);
     lx[i] = l;
-    lv[i] = (ven1[i] && !mark[i]) ? make_double2(dt * l.x, dt * l.y) : make_double2(0, 0);
+    lv[i] = make_double2(dt * l.x, dt * l.y);
     double2 w = vel1[i];
     gmu[i] += dt * (l.x * w.x + l.y * w.y) / mu;
 }
@@ -271,13 +266,21 @@ __device__ __forceinline__ bool in_instance(const int *voff, int ninst, int inst
     return ninst <= 1 || (v >= voff[inst] && v < voff[inst + 1]);
 }
 
-/* the step's flips and 3-sided removals in reverse order, per instance */
+/* the step's flips and 3-sided removals in reverse order, per instance; the
+ * vertices they moved have no velocity (it was zeroed) */
 __global__ void __launch_bounds__(ADJ_TPB) k_adj_events(double D, const EventRec *log, const int *nlog, double2 *lx,
-                                                        const int *voff, int ninst)
+                                                        double2 *lv, const int *voff, int ninst)
 {
-    const int inst = blockIdx.x;
+    griddep_wait();
+    const int inst = blockIdx.x, n = *nlog;
+    for (int i = threadIdx.x; i < n; i += ADJ_TPB) {
+        const EventRec r = log[i];
+        if ((r.type != EV_FLIP && r.type != EV_REMOVE) || !in_instance(voff, ninst, inst, r.a)) continue;
+        lv[r.a] = lv[r.b] = make_double2(0, 0);
+        if (r.type == EV_REMOVE) lv[r.c] = make_double2(0, 0);
+    }
     walk_log_reverse(
-        log, *nlog,
+        log, n,
         [&](int e) {
             EventRec r = log[e];
             return (r.type == EV_FLIP || r.type == EV_REMOVE) && in_instance(voff, ninst, inst, r.a);
@@ -336,6 +339,7 @@ __device__ void adj_nucleation_one(double D, const EventRec &r, const EventRec &
 __global__ void __launch_bounds__(ADJ_TPB) k_adj_nucleation(double D, const EventRec *log, const int *nlog,
                                                             double2 *lam, const int *voff, int ninst)
 {
+    griddep_wait();
     const int inst = blockIdx.x, n = *nlog;
     walk_log_reverse(
         log, n,
@@ -347,28 +351,50 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_nucleation(double D, const Even
         [&](int e) { adj_nucleation_one(D, log[e], log[e + 1], lam); });
 }
 
-/* per grain: sign of the area at the step's start, and
+/* per grain: sign of the area at the step's start (area_stream's sum), and
  * dL/dSE_g += sum_p lambda_v(p) . (-mu sign(A) dA/dx_p) (not for a
- * nucleated grain, whose stored energy is 0, not a parameter) */
-__global__ void k_adj_grains(DevMesh m, double mu, const double2 *lv, double *sgn, double *gse)
+ * nucleated grain, whose stored energy is 0, not a parameter).  One walk of
+ * the list for both, eight vertices' positions and lambdas loaded at once;
+ * the delta to a vertex's predecessor is minus the predecessor's to it. */
+__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_grains(DevMesh m, double mu, const double2 *lv, double *sgn, double *gse)
 {
+    griddep_wait();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= m.ng) return;
     if (!m.gen[g]) { sgn[g] = 0.0; return; }
     const int *L = m.glist + (size_t)SEVC_MAXV * g;
-    int n = m.gvlen[g];
-    double A = grain_area(m, g);
-    double s = A > 0 ? 1.0 : (A < 0 ? -1.0 : 0.0);
-    sgn[g] = s;
-    double acc = 0.0;
-    for (int p = 0; p < n; p++) {
-        int v = L[p], pv = L[p == 0 ? n - 1 : p - 1], nx = L[p == n - 1 ? 0 : p + 1];
-        double2 q = m.pos[v], a = m.pos[pv], b = m.pos[nx];
-        double xp = wrapd(a.x, q.x, m.D), yp = wrapd(a.y, q.y, m.D);
-        double xn = wrapd(b.x, q.x, m.D), yn = wrapd(b.y, q.y, m.D);
-        double2 l = lv[v];
-        acc += l.x * (0.5 * (yn - yp)) + l.y * (0.5 * (xp - xn));
+    const int n = m.gvlen[g];
+    double acc = 0.0, area = 0.0, ax = 0, ay = 0, px = 0, py = 0;   /* px, py: predecessor to vertex */
+    double2 first = make_double2(0, 0);
+    for (int base = 0; base < n; base += 8) {
+        int v[8];
+        double2 q[9], l[8];
+        list_batch(L, n, base, v);
+#pragma unroll
+        for (int j = 0; j < 8; j++) { q[j] = m.pos[v[j]]; l[j] = lv[v[j]]; }
+        q[8] = base + 8 < n ? m.pos[L[base + 8]] : make_double2(0, 0);
+        if (base == 0) {
+            first = q[0];
+            const double2 last = m.pos[L[n - 1]];
+            px = wrapd(first.x, last.x, m.D);
+            py = wrapd(first.y, last.y, m.D);
+        }
+        const int end = n - base < 8 ? n - base : 8;
+#pragma unroll 1
+        for (int j = 0; j < end; j++) {
+            const double2 c = q[j], b = base + j == n - 1 ? first : q[j + 1];
+            if (base + j > 0) {
+                double nx = ax + px, ny = ay + py;
+                if (base + j > 1) area += ax * ny - ay * nx;
+                ax = nx; ay = ny;
+            }
+            const double xn = wrapd(b.x, c.x, m.D), yn = wrapd(b.y, c.y, m.D);
+            acc += l[j].x * (0.5 * (yn + py)) + l[j].y * (0.5 * (-px - xn));
+            px = xn; py = yn;
+        }
     }
+    const double s = area > 0 ? 1.0 : (area < 0 ? -1.0 : 0.0);
+    sgn[g] = s;
     if (m.gtype[g] != GT_NUCLEATED) gse[g] += -mu * s * acc;
 }
 
@@ -436,61 +462,116 @@ __device__ __forceinline__ void edge_fd_grad(double dx, double dy, double L2, do
 }
 
 /* per vertex k (gather): lambda_n[k] = lambda_x[k] + (J_v^T lambda_v)[k];
- * d/ds of k's own velocity into ggam[k] */
-__global__ void k_adj_vertices(DevMesh m, double mu, double eps, double s_gb, const double2 *lx, const double2 *lv,
-                               const double *sgn, double2 *lam_out, double *ggam)
+ * d/ds of k's own velocity into ggam[k].  Three lanes per vertex, ten
+ * vertices a warp: lane j takes boundary j and grain j, so the three edges'
+ * chains of dependent FP64 operations and the three list searches run side
+ * by side; the first lane adds the parts in order. */
+constexpr int ADJ_VPB = 10 * (ADJ_BLOCK / 32);     /* vertices per block */
+__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_vertices(DevMesh m, double mu, double eps, double s_gb,
+                                                            const double2 *lx, const double2 *lv, const double *sgn,
+                                                            double2 *lam_out, double *ggam)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= m.nv) return;
-    if (!m.ven[k]) { lam_out[k] = make_double2(0, 0); return; }
+    griddep_wait();
+    const int lane = threadIdx.x & 31, q3 = lane / 3, j = lane - 3 * q3;
+    const int k = blockIdx.x * ADJ_VPB + (threadIdx.x >> 5) * 10 + q3;
+    const bool in = lane < 30 && k < m.nv, live = in && m.ven[k];
     const double E = SEVC_GRAD_EPS_D;
-    double2 out = lx[k];
-    double2 p = m.pos[k];
-    double2 lk = lv[k];
-    int4 sb = m.vb[k];
+    double2 out = make_double2(0, 0);
     double dgam = 0.0;
-    for (int j = 0; j < 3; j++) {
-        int b = slot3(sb, j);
-        if (b < 0) continue;
-        int q = other_end(m.bv[b], k);
-        double f = gb_weight(m, b, eps), gam = s_gb * f;
-        double2 pq = m.pos[q];
-        double dx = wrapd(p.x, pq.x, m.D), dy = wrapd(p.y, pq.y, m.D);
-        double L2 = dx * dx + dy * dy;
-        double invL = L2 > 0 ? rsqrt_newton(L2) : 0.0, L = L2 * invL;
-        /* k moved along x / y (d -> d + eps e_c) and q moved (-d -> -d + eps e_c) */
-        double2 gkx, gky, gqx, gqy;
-        double skx, sky;
-        edge_fd_grad(dx, dy, L2, L, invL, E, 0, &gkx, &skx);
-        edge_fd_grad(dx, dy, L2, L, invL, E, 1, &gky, &sky);
-        double sqx, sqy;
-        edge_fd_grad(-dx, -dy, L2, L, invL, E, 0, &gqx, &sqx);
-        edge_fd_grad(-dx, -dy, L2, L, invL, E, 1, &gqy, &sqy);
-        double cg = -mu * gam;
-        out.x += cg * (lk.x * gkx.x + lk.y * gky.x);
-        out.y += cg * (lk.x * gkx.y + lk.y * gky.y);
-        dgam += -mu * f * (lk.x * skx + lk.y * sky);
-        /* q's velocity: d/dx_k of -(gam/eps) (L(x_q + eps e_c) - L(x)) is
-         * minus the gradient with respect to the moved end */
-        double2 lq = lv[q];
-        double cq = mu * gam;
-        out.x += cq * (lq.x * gqx.x + lq.y * gqy.x);
-        out.y += cq * (lq.x * gqx.y + lq.y * gqy.y);
-    }
-    int4 sg = m.vg[k];
-    for (int j = 0; j < 3; j++) {
-        int g = slot3(sg, j);
-        if (g < 0 || !m.gen[g]) continue;
+    if (live) {
+        const double2 p = m.pos[k], lk = lv[k];
+        const int b = slot3(m.vb[k], j), g = slot3(m.vg[k], j);
+        if (b >= 0) {
+            int q = other_end(m.bv[b], k);
+            double f = gb_weight(m, b, eps), gam = s_gb * f;
+            double2 pq = m.pos[q], lq = lv[q];
+            double dx = wrapd(p.x, pq.x, m.D), dy = wrapd(p.y, pq.y, m.D);
+            double L2 = dx * dx + dy * dy;
+            double invL = L2 > 0 ? rsqrt_newton(L2) : 0.0, L = L2 * invL;
+            /* k moved along x / y (d -> d + eps e_c) and q moved (-d -> -d + eps e_c) */
+            double2 gkx, gky, gqx, gqy;
+            double skx, sky, sqx, sqy;
+            edge_fd_grad(dx, dy, L2, L, invL, E, 0, &gkx, &skx);
+            edge_fd_grad(dx, dy, L2, L, invL, E, 1, &gky, &sky);
+            edge_fd_grad(-dx, -dy, L2, L, invL, E, 0, &gqx, &sqx);
+            edge_fd_grad(-dx, -dy, L2, L, invL, E, 1, &gqy, &sqy);
+            double cg = -mu * gam;
+            out.x += cg * (lk.x * gkx.x + lk.y * gky.x);
+            out.y += cg * (lk.x * gkx.y + lk.y * gky.y);
+            dgam = -mu * f * (lk.x * skx + lk.y * sky);
+            /* q's velocity: d/dx_k of -(gam/eps) (L(x_q + eps e_c) - L(x)) is
+             * minus the gradient with respect to the moved end */
+            double cq = mu * gam;
+            out.x += cq * (lq.x * gqx.x + lq.y * gqy.x);
+            out.y += cq * (lq.x * gqx.y + lq.y * gqy.y);
+        }
         int pv, nx;
-        if (list_pos(m, g, k, &pv, &nx) < 0) continue;
-        double se = m.gtype[g] == GT_NUCLEATED ? 0.0 : m.gse[g];
-        double c = 0.5 * mu * se * sgn[g];
-        double2 a = lv[pv], b = lv[nx];
-        out.x += c * (a.y - b.y);
-        out.y += c * (b.x - a.x);
+        if (g >= 0 && m.gen[g] && list_neighbours(m, g, k, pv, nx)) {
+            double se = m.gtype[g] == GT_NUCLEATED ? 0.0 : m.gse[g];
+            double c = 0.5 * mu * se * sgn[g];
+            double2 a = lv[pv], d = lv[nx];
+            out.x += c * (a.y - d.y);
+            out.y += c * (d.x - a.x);
+        }
     }
-    lam_out[k] = out;
-    ggam[k] += dgam;
+    double2 sum = live && j == 0 ? lx[k] : make_double2(0, 0);
+    double gsum = 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const int src = 3 * q3 + q < 32 ? 3 * q3 + q : 31;
+        sum.x += __shfl_sync(0xffffffffu, out.x, src);
+        sum.y += __shfl_sync(0xffffffffu, out.y, src);
+        gsum += __shfl_sync(0xffffffffu, dgam, src);
+    }
+    if (j == 0 && in) {
+        lam_out[k] = live ? sum : make_double2(0, 0);
+        if (live) ggam[k] += gsum;
+    }
+}
+
+/* ---- tape records (sevc_adjoint_histogram's replay) ---- */
+/* What the adjoint of a step reads, in one launch instead of a copy per
+ * array: the mesh the velocities are computed on, of the grain lists only the
+ * used entries (24 of 400 bytes per grain on average).  start: the record
+ * is the step's first (the event log is emptied and switched on). */
+__device__ __forceinline__ void copy_words(const void *src, void *dst, size_t bytes, size_t t, size_t n)
+{
+    /* 16-byte words; the arrays are padded to 256 bytes on both sides */
+    const uint4 *a = static_cast<const uint4 *>(src);
+    uint4 *b = static_cast<uint4 *>(dst);
+    for (size_t i = t; i < (bytes + 15) / 16; i += n) b[i] = a[i];
+}
+__global__ void __launch_bounds__(TPB) k_tape_record(DevMesh m, TapeRecord r, EventLog log, int start)
+{
+    griddep_wait();
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = (size_t)gridDim.x * blockDim.x;
+    const size_t V = m.nv, B = m.nb, G = m.ng;
+    copy_words(m.pos, r.pos, V * 16, t, n);
+    copy_words(m.vb, r.vb, V * 16, t, n);
+    copy_words(m.vg, r.vg, V * 16, t, n);
+    copy_words(m.ven, r.ven, V, t, n);
+    copy_words(m.bv, r.bv, B * 8, t, n);
+    copy_words(m.ben, r.ben, B, t, n);
+    copy_words(m.gvlen, r.gvlen, G * 4, t, n);
+    copy_words(m.gen, r.gen, G, t, n);
+    copy_words(m.gtype, r.gtype, G, t, n);
+    for (size_t i = t; i < G * (SEVC_MAXV / 4); i += n) {
+        const size_t g = i / (SEVC_MAXV / 4), j = i - g * (SEVC_MAXV / 4);
+        if (4 * (int)j < m.gvlen[g]) reinterpret_cast<int4 *>(r.glist)[i] = reinterpret_cast<const int4 *>(m.glist)[i];
+    }
+    if (start && t == 0) {
+        *log.n = 0;
+        *m.elog = log;
+    }
+}
+/* enabled flags and velocities after the step; the log is switched off */
+__global__ void __launch_bounds__(TPB) k_tape_after(DevMesh m, TapeRecord r)
+{
+    griddep_wait();
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = (size_t)gridDim.x * blockDim.x;
+    copy_words(m.vel, r.vel1, (size_t)m.nv * 16, t, n);
+    copy_words(m.ven, r.ven1, m.nv, t, n);
+    if (t == 0) *m.elog = EventLog{ nullptr, nullptr, 0 };
 }
 
 /* Grain statistics over grains [lo, hi): count, sum |A|, sum A^2, sum of
@@ -597,17 +678,24 @@ void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, doubl
 
 void launch_adjoint_step(const DevMesh &rec, const AdjointBuffers &a, double dt, double mu, double eps, double s_gb,
                          const EventRec *log, const int *nlog, const uint8_t *ven1, const double2 *vel1,
-                         cudaStream_t s)
+                         bool nucleation, cudaStream_t s)
 {
-    cudaMemsetAsync(a.mark, 0, rec.nv, s);
-    COUNT_LAUNCHES(1), k_adj_mark_events<<<4, TPB, 0, s>>>(a.mark, log, nlog);
-    COUNT_LAUNCHES(1), k_adj_translate<<<nblk(rec.nv), TPB, 0, s>>>(rec.nv, dt, mu, a.lam, ven1, vel1, a.mark, a.lx,
-                                                                    a.lv, a.gmu);
-    COUNT_LAUNCHES(1), k_adj_events<<<rec.ninst, ADJ_TPB, 0, s>>>(rec.D, log, nlog, a.lx, rec.voff, rec.ninst);
-    COUNT_LAUNCHES(1), k_adj_grains<<<nblk(rec.ng), TPB, 0, s>>>(rec, mu, a.lv, a.sgn, a.gse);
-    COUNT_LAUNCHES(1), k_adj_vertices<<<nblk(rec.nv), TPB, 0, s>>>(rec, mu, eps, s_gb, a.lx, a.lv, a.sgn, a.lam,
-                                                                   a.ggam);
-    COUNT_LAUNCHES(1), k_adj_nucleation<<<rec.ninst, ADJ_TPB, 0, s>>>(rec.D, log, nlog, a.lam, rec.voff, rec.ninst);
+    launch_dep(k_adj_translate, nblk(rec.nv), TPB, s, rec.nv, dt, mu, a.lam, ven1, vel1, a.lx, a.lv, a.gmu);
+    launch_dep(k_adj_events, rec.ninst, ADJ_TPB, s, rec.D, log, nlog, a.lx, a.lv, rec.voff, rec.ninst);
+    launch_dep(k_adj_grains, (rec.ng + ADJ_BLOCK - 1) / ADJ_BLOCK, ADJ_BLOCK, s, rec, mu, a.lv, a.sgn, a.gse);
+    launch_dep(k_adj_vertices, (rec.nv + ADJ_VPB - 1) / ADJ_VPB, ADJ_BLOCK, s, rec, mu, eps,
+               s_gb, a.lx, a.lv, a.sgn, a.lam, a.ggam);
+    if (nucleation) launch_dep(k_adj_nucleation, rec.ninst, ADJ_TPB, s, rec.D, log, nlog, a.lam, rec.voff, rec.ninst);
+}
+
+static int copy_blocks(const DevMesh &m) { int b = nblk(m.nv); return b < 4 * 152 ? b : 4 * 152; }
+void launch_tape_record(const DevMesh &m, const TapeRecord &r, const EventLog &log, bool start, cudaStream_t s)
+{
+    launch_dep(k_tape_record, copy_blocks(m), TPB, s, m, r, log, (int)start);
+}
+void launch_tape_after(const DevMesh &m, const TapeRecord &r, cudaStream_t s)
+{
+    launch_dep(k_tape_after, copy_blocks(m), TPB, s, m, r);
 }
 
 void launch_grain_stats(const DevMesh &m, int lo, int hi, double *part, double *out, cudaStream_t s)

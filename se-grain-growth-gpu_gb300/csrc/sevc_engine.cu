@@ -112,6 +112,7 @@ struct sevc_handle {
         cudaEvent_t ev0 = nullptr, ev1 = nullptr, done = nullptr;
         sevc_step_info loc;
         long long launches = 0;
+        void *ckpt = nullptr;      /* a tape checkpoint taken after the step */
     } rslot[2];
     bool rslot_ready = false;
     /* side streams of the step (branches that do not depend on each other
@@ -427,14 +428,21 @@ bool stat_read(sevc_handle *h, int nout)
     return cuda_ok(cudaMemcpyAsync(h->h_stat, h->stat, nout * 8, cudaMemcpyDeviceToHost, h->stream), "readback") &&
            cuda_ok(cudaStreamSynchronize(h->stream), "sync");
 }
-bool tape_checkpoint(sevc_handle *h)
+/* a device copy of the whole block as it is at this point of the stream */
+void *tape_copy(sevc_handle *h)
 {
     void *ck = nullptr;
-    if (!cuda_ok(cudaMalloc(&ck, h->dbytes), "cudaMalloc checkpoint")) return false;
+    if (!cuda_ok(cudaMalloc(&ck, h->dbytes), "cudaMalloc checkpoint")) return nullptr;
     if (!cuda_ok(cudaMemcpyAsync(ck, h->dblock, h->dbytes, cudaMemcpyDeviceToDevice, h->stream), "checkpoint")) {
         cudaFree(ck);
-        return false;
+        return nullptr;
     }
+    return ck;
+}
+/* ck (or, if null, a copy taken now) becomes the tape's next checkpoint */
+bool tape_checkpoint(sevc_handle *h, void *ck = nullptr)
+{
+    if (!ck && !(ck = tape_copy(h))) return false;
     h->tape.ckpt.push_back(ck);
     h->tape.runs.push_back(save_run(h));
     return true;
@@ -631,9 +639,9 @@ size_t summary_bytes(const sevc_handle *h)
  * iterations and 2x3 counts of every instance; h_on: the instances that
  * attempted a nucleation) into the run state and `info`; then n++ and
  * t = n dt (src/main.cu:388-391).  loc carries n, t and the attempt flag of
- * the step. */
+ * the step; ckpt a tape checkpoint already copied after it. */
 sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms, int launches,
-                        sevc_step_info loc, sevc_step_info *info)
+                        sevc_step_info loc, sevc_step_info *info, void *ckpt = nullptr)
 {
     const sevc_options &o = h->opt;
     const int I = h->ninst;
@@ -713,12 +721,19 @@ sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms
     sevc_status st = err_bits_to_status(hb[o_err]);
     if (!st && h->tape.every > 0 && !h->tape.replaying) {
         h->tape.nsteps++;
-        if (h->tape.nsteps % h->tape.every == 0 && !tape_checkpoint(h)) return SEVC_ERR_CUDA;
+        if (h->tape.nsteps % h->tape.every == 0 && !tape_checkpoint(h, ckpt)) return SEVC_ERR_CUDA;
     }
     return st;
 }
 
 } // namespace
+
+/* run_steps_core's work around each step, enqueued on the handle's stream
+ * just before and just after it */
+struct StepHooks {
+    std::function<void(int)> before, after;
+};
+sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, int *done, StepHooks *hooks);
 
 extern "C" {
 
@@ -940,7 +955,9 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     return finish_step(h, hb, h->h_on, ms, launches, loc, info);
 }
 
-sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *done)
+} // extern "C"
+
+sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, int *done, StepHooks *hooks)
 {
     if (!h || nsteps < 0) return SEVC_ERR_ARG;
     if (done) *done = 0;
@@ -951,11 +968,13 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
     /* pipelined: one graph per step and no
      * input of a step that depends on the previous step's counts (a single
      * mesh with a grain-count stop feeds its count to the output decision) */
-    const bool pipe = graphs_on(h) && h->tape.every <= 0 && (batch || mg <= 0);
+    const bool pipe = graphs_on(h) && (batch || mg <= 0);
     if (!pipe) {
         for (int k = 0; k < nsteps; k++) {
             sevc_step_info inf;
+            if (hooks) hooks->before(k);
             sevc_status st = sevc_step(h, &inf);
+            if (hooks) hooks->after(k);
             if (infos) infos[k] = inf;
             if (done) *done = k + 1;
             if (st) return st;
@@ -982,7 +1001,8 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         float ms = 0;
         cudaEventElapsedTime(&ms, sl.ev0, sl.ev1);
         sevc_step_info inf;
-        sevc_status r = finish_step(h, sl.big, sl.on, ms, (int)sl.launches, sl.loc, &inf);
+        sevc_status r = finish_step(h, sl.big, sl.on, ms, (int)sl.launches, sl.loc, &inf, sl.ckpt);
+        sl.ckpt = nullptr;
         if (infos) infos[finished] = inf;
         finished++;
         if (done) *done = finished;
@@ -1017,6 +1037,7 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         sl.flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && nk % o.snap_gap == 0);
         sl.flags[2] = batch ? 0 : mg;
         sl.flags[3] = h->curr_n_grains;   /* read only when min_grains > 0: not here */
+        if (hooks) hooks->before(launched);
         if ((n_on && !cuda_ok(cudaMemcpyAsync(x.nucl_on, sl.on, I * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) ||
             !cuda_ok(cudaMemcpyAsync(x.flags + 1, sl.flags + 1, 3 * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) {
             st = SEVC_ERR_CUDA;
@@ -1024,12 +1045,24 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         }
         cudaEventRecord(sl.ev0, s);
         long long k0 = sevc_kernel_launches;
-        if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); })) {
+        h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
+        bool ran = run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); });
+        h->force_direct = false;
+        if (!ran) {
             st = SEVC_ERR_CUDA;
             break;
         }
         sl.launches = sevc_kernel_launches - k0;
         cudaEventRecord(sl.ev1, s);
+        if (hooks) hooks->after(launched);
+        /* a checkpoint of the tape due after this step is copied here, before
+         * the next step goes in; finish_step adds it to the tape */
+        sl.ckpt = nullptr;
+        if (h->tape.every > 0 && !h->tape.replaying && (h->tape.nsteps + (launched - finished) + 1) % h->tape.every == 0 &&
+            !(sl.ckpt = tape_copy(h))) {
+            st = SEVC_ERR_CUDA;
+            break;
+        }
         if (!cuda_ok(cudaMemcpyAsync(sl.big, x.summary, summary_bytes(h), cudaMemcpyDeviceToHost, s), "readback") ||
             !cuda_ok(cudaEventRecord(sl.done, s), "event")) {
             st = SEVC_ERR_CUDA;
@@ -1038,7 +1071,16 @@ sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *don
         launched++;
     }
     if (launched > finished) cudaStreamSynchronize(s);   /* after a failure: let the step in flight end */
+    for (auto &sl : h->rslot)
+        if (sl.ckpt) { cudaFree(sl.ckpt); sl.ckpt = nullptr; }
     return st;
+}
+
+extern "C" {
+
+sevc_status sevc_run(sevc_handle *h, int nsteps, sevc_step_info *infos, int *done)
+{
+    return run_steps_core(h, nsteps, infos, done, nullptr);
 }
 
 sevc_status sevc_run_steps(sevc_handle *h, int nsteps, int *done, sevc_step_info *last)
@@ -1400,7 +1442,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
     {
         struct Req { void **p; size_t bytes; };
         std::vector<Req> r = { { (void **)&a.lam, V * 16 }, { (void **)&a.lx, V * 16 }, { (void **)&a.lv, V * 16 },
-                               { (void **)&a.mark, V }, { (void **)&a.sgn, G * 8 }, { (void **)&a.gse, G * 8 },
+                               { (void **)&a.sgn, G * 8 }, { (void **)&a.gse, G * 8 },
                                { (void **)&a.gmu, V * 8 }, { (void **)&a.ggam, V * 8 }, { (void **)&a.dlda, G * 8 },
                                { (void **)&a.scalars, 16 }, { (void **)&d_dldh, 1024 * 8 } };
         size_t total = 0;
@@ -1428,6 +1470,23 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
         tp.rec_steps = tp.every;
     }
     auto rec = [&](int k, size_t off) { return (char *)tp.rec + (size_t)k * step_bytes + off; };
+    auto record_at = [&](int k) {
+        TapeRecord r;
+        r.pos = (double2 *)rec(k, off_pos);
+        r.vel1 = (double2 *)rec(k, off_vel1);
+        r.vb = (int4 *)rec(k, off_vb);
+        r.vg = (int4 *)rec(k, off_vg);
+        r.bv = (int2 *)rec(k, off_bv);
+        r.glist = (int *)rec(k, off_gl);
+        r.gvlen = (int *)rec(k, off_gvl);
+        r.ven = (uint8_t *)rec(k, off_ven);
+        r.ven1 = (uint8_t *)rec(k, off_ven1);
+        r.ben = (uint8_t *)rec(k, off_ben);
+        r.gen = (uint8_t *)rec(k, off_gen);
+        r.gtype = (uint8_t *)rec(k, off_gty);
+        return r;
+    };
+    auto log_at = [&](int k) { return EventLog{ (EventRec *)rec(k, off_log), (int *)rec(k, off_nlog), tp.log_cap }; };
     auto d2d = [&](void *dst, const void *src, size_t n) {
         return cuda_ok(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToDevice, s), "tape copy");
     };
@@ -1452,50 +1511,35 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
         if (!d2d(h->dblock, tp.ckpt[seg], h->dbytes)) { st = SEVC_ERR_CUDA; break; }
         load_run(h, tp.runs[seg]);
         int K = (int)std::min<long long>(tp.every, tp.nsteps - seg * tp.every);
-        for (int k = 0; k < K && !st; k++) {
-            DevMesh &m = h->m;
-            /* the mesh the step's velocities are computed on: at its start,
-             * or after its nucleation (recorded again from inside the step) */
-            auto record = [&, k](cudaStream_t rs) {
-                auto cp = [&](size_t off, const void *src, size_t n) {
-                    return cudaMemcpyAsync(rec(k, off), src, n, cudaMemcpyDeviceToDevice, rs) == cudaSuccess;
-                };
-                return cp(off_pos, m.pos, V * 16) && cp(off_vb, m.vb, V * 16) && cp(off_vg, m.vg, V * 16) &&
-                       cp(off_ven, m.ven, V) && cp(off_bv, m.bv, B * 8) && cp(off_ben, m.ben, B) &&
-                       cp(off_gl, m.glist, G * SEVC_MAXV * 4) && cp(off_gvl, m.gvlen, G * 4) &&
-                       cp(off_gen, m.gen, G) && cp(off_gty, m.gtype, G);
-            };
-            bool ok = record(s) && cuda_ok(cudaMemsetAsync(rec(k, off_nlog), 0, 4, s), "memset");
-            if (!ok) { st = SEVC_ERR_CUDA; break; }
-            tp.after_nucleation = [&, record](cudaStream_t rs) { if (!record(rs)) sevc_set_error("tape copy"); };
-            EventLog on = { (EventRec *)rec(k, off_log), (int *)rec(k, off_nlog), tp.log_cap }, off = { nullptr, nullptr, 0 };
-            if (!cuda_ok(cudaMemcpyAsync(m.elog, &on, sizeof on, cudaMemcpyHostToDevice, s), "upload")) {
-                st = SEVC_ERR_CUDA;
-                break;
-            }
-            st = sevc_step(h, nullptr);
+        /* replay the segment; around each step, the mesh its velocities are
+         * computed on (at its start or, recorded again from inside the step,
+         * after its nucleation) and the state after it */
+        StepHooks hooks;
+        hooks.before = [&](int k) {
+            launch_tape_record(h->m, record_at(k), log_at(k), true, s);
+            tp.after_nucleation = [&, k](cudaStream_t rs) { launch_tape_record(h->m, record_at(k), log_at(k), false, rs); };
+        };
+        hooks.after = [&](int k) {
             tp.after_nucleation = nullptr;
-            h->force_direct = false;
-            if (!cuda_ok(cudaMemcpyAsync(m.elog, &off, sizeof off, cudaMemcpyHostToDevice, s), "upload"))
-                st = SEVC_ERR_CUDA;
-            if (!st && !(d2d(rec(k, off_vel1), m.vel, V * 16) && d2d(rec(k, off_ven1), m.ven, V))) st = SEVC_ERR_CUDA;
-        }
+            launch_tape_after(h->m, record_at(k), s);
+        };
+        st = run_steps_core(h, K, nullptr, nullptr, &hooks);
         for (int k = K - 1; k >= 0 && !st; k--) {
+            const TapeRecord r = record_at(k);
             DevMesh view = h->m;
-            view.pos = (double2 *)rec(k, off_pos);
-            view.vb = (int4 *)rec(k, off_vb);
-            view.vg = (int4 *)rec(k, off_vg);
-            view.ven = (uint8_t *)rec(k, off_ven);
-            view.bv = (int2 *)rec(k, off_bv);
-            view.ben = (uint8_t *)rec(k, off_ben);
-            view.glist = (int *)rec(k, off_gl);
-            view.gvlen = (int *)rec(k, off_gvl);
-            view.gen = (uint8_t *)rec(k, off_gen);
-            view.gtype = (uint8_t *)rec(k, off_gty);
+            view.pos = r.pos;
+            view.vb = r.vb;
+            view.vg = r.vg;
+            view.ven = r.ven;
+            view.bv = r.bv;
+            view.ben = r.ben;
+            view.glist = r.glist;
+            view.gvlen = r.gvlen;
+            view.gen = r.gen;
+            view.gtype = r.gtype;
             view.gse = tp.separam;           /* a nucleated grain's 0 is applied by its type */
-            launch_adjoint_step(view, a, h->opt.dt, h->p.mu, h->opt.GB_eps, h->opt.GB_scaling,
-                                (const EventRec *)rec(k, off_log), (const int *)rec(k, off_nlog),
-                                (const uint8_t *)rec(k, off_ven1), (const double2 *)rec(k, off_vel1), s);
+            launch_adjoint_step(view, a, h->opt.dt, h->p.mu, h->opt.GB_eps, h->opt.GB_scaling, log_at(k).buf, log_at(k).n,
+                                r.ven1, r.vel1, h->opt.do_nucleation != 0, s);
         }
     }
     tp.replaying = false;

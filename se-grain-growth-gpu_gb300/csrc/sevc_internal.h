@@ -147,7 +147,6 @@ int rng_record(int nstreams, int ndraws, double *host_out);
 struct AdjointBuffers {
     double2 *lam;    /* adjoint of the positions (current step boundary) */
     double2 *lx, *lv;/* adjoint of the post-event positions / of the velocities */
-    uint8_t *mark;   /* vertices moved by an event in the step */
     double *sgn;     /* sign of each grain's area at the step's start */
     double *gse;     /* dL/dSE per grain (accumulated) */
     double *gmu;     /* dL/dmu per vertex (accumulated) */
@@ -155,6 +154,17 @@ struct AdjointBuffers {
     double *dlda;    /* dL/dA per grain of the statistic */
     double *scalars; /* reduced dL/dmu, dL/dGB_scaling */
 };
+/* one step's record on the tape (pieces of one allocation, each padded to
+ * 256 bytes) */
+struct TapeRecord {
+    double2 *pos, *vel1;
+    int4 *vb, *vg;
+    int2 *bv;
+    int *glist, *gvlen;
+    uint8_t *ven, *ven1, *ben, *gen, *gtype;
+};
+void launch_tape_record(const DevMesh &m, const TapeRecord &r, const EventLog &log, bool start, cudaStream_t s);
+void launch_tape_after(const DevMesh &m, const TapeRecord &r, cudaStream_t s);
 /* soft histogram of a_g = |A_g| sc over nbins bins of [0, amax), divided by
  * nnorm; part: stat_doubles(nbins) doubles of scratch */
 size_t stat_doubles(int nbins);
@@ -165,10 +175,11 @@ void launch_histogram(const DevMesh &m, int nbins, double amax, double sc, doubl
 void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, double nnorm, const double *dldh,
                       double zero_sum, double *dlda, double2 *lam, cudaStream_t s);
 /* one step backward: `rec` views the mesh as recorded at the step's start,
- * log / ven1 / vel1 its events and the enabled flags and velocities after it */
+ * log / ven1 / vel1 its events and the enabled flags and velocities after
+ * it; nucleation: the log may hold nucleations */
 void launch_adjoint_step(const DevMesh &rec, const AdjointBuffers &a, double dt, double mu, double eps, double s_gb,
                          const EventRec *log, const int *nlog, const uint8_t *ven1, const double2 *vel1,
-                         cudaStream_t s);
+                         bool nucleation, cudaStream_t s);
 /* *out = the sum of a[0..n); part: stat_doubles(1) doubles of scratch */
 void launch_sum_ordered(const DevMesh &m, const double *a, int n, double *part, double *out, cudaStream_t s);
 /* out[0..6] = count, sum |A|, sum A^2, sum vlen, 3-sided count, min |A|, max
