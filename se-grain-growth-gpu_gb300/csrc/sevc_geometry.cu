@@ -261,23 +261,6 @@ __device__ __forceinline__ int certify_axis(const double *r, int n, double D, lo
     return mh - ml <= (ml >> 1) + (ml >> 2) ? GP_CERT : GP_CHAIN;
 }
 
-/* One axis of an uncertified grain: the unwrapped chain a of its raw
- * coordinates r, and the chain u with vertex 0 moved, each addition as the
- * reference makes it */
-__device__ __noinline__ void chain_axis(const double *r, double *a, double *u, int n, double D)
-{
-    double r0 = r[0], m0 = dmod(r0 + SEVC_GRAD_EPS_D, D), x = 0, y = 0, prev = r0;
-    a[0] = 0;
-    u[0] = 0;
-    for (int k = 1; k < n; k++) {
-        double rk = r[k], d = wrapd(rk, prev, D);
-        x = k == 1 ? zero_plus(d) : x + d;
-        y = k == 1 ? zero_plus(wrapd(rk, m0, D)) : y + d;
-        a[k] = x;
-        u[k] = y;
-        prev = rk;
-    }
-}
 /* The unwrapped coordinate of the moved vertex p > 0 of an uncertified
  * grain (raw coordinates: its own r, the neighbours' rm and rp; a the
  * unwrapped chain).  NaN (no certified value is one) when the chain does
@@ -300,7 +283,7 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
     __shared__ unsigned char sides[GPB];
     __shared__ int cnt[GP_NMAX], start[GP_NMAX];
     __shared__ int first[GP_NMAX];             /* first[j]: first entry of B.moved (and B.inner) with s + 2 = j */
-    __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved;
+    __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved, chains;
     __shared__ long long ntab[GP_E1 - GP_E0 + 1];
     __shared__ double dtab[GP_E1 - GP_E0 + 1];
     constexpr int W = NT / 32;
@@ -410,13 +393,15 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
     }
     __syncthreads();
     /* per grain and axis: certificate */
+    if (tid == 0) chains = 0;
     for (int t = tid; t < 2 * total; t += NT) {
         const int x = t >= total, i = x ? t - total : t;
         B.ok[x][i] = certify_axis(B.R[x] + B.off[i], B.n[i], m.D, dlim, B.c[x][i]);
     }
     __syncthreads();
     /* per slot and axis: coordinate relative to vertex 0, and to vertex 0
-     * moved; the first slot of an uncertified grain walks its chains */
+     * moved; of an uncertified grain the wrapped deltas that its chains add
+     * up, each as the reference forms it */
     for (int t = tid; t < 2 * slots; t += NT) {
         const int x = t >= slots, q = x ? t - slots : t, i = B.owner[q], o = B.off[i], st = B.state(i);
         if (B.dest[q] < 0) B.ok[0][i] = GP_REST;
@@ -428,11 +413,25 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
             if (u != e) atomicOr(&B.c[x][i].up, 1u << (q - o));
             B.A[x][q] = sub_exact(b, b0, e + GP_E0);
             B.M[x][q] = sub_exact(b, b0 + ntab[(int)(b0 >> 52) - GP_E0], e + GP_E0);
-        } else if (st == GP_CHAIN && q == o) {
-            chain_axis(B.R[x] + o, B.A[x] + o, B.M[x] + o, B.n[i], m.D);
+        } else if (st == GP_CHAIN) {
+            chains = 1;
+            const double rk = B.R[x][q];
+            const double d = q == o ? 0.0 : wrapd(rk, B.R[x][q - 1], m.D);
+            B.A[x][q] = d;
+            B.M[x][q] = q == o + 1 ? zero_plus(wrapd(rk, dmod(B.R[x][o] + SEVC_GRAD_EPS_D, m.D), m.D)) : d;
         }
     }
     __syncthreads();
+    if (chains) {                              /* the block has uncertified grains: their running sums */
+        for (int t = tid; t < 4 * total; t += NT) {
+            const int c = t / total, i = t - c * total, o = B.off[i], nn = B.n[i];
+            if (B.state(i) != GP_CHAIN) continue;
+            double *Z = (c < 2 ? B.A[c] : B.M[c - 2]) + o, a = c < 2 ? zero_plus(Z[1]) : Z[1];
+            Z[1] = a;
+            for (int k = 2; k < nn; k++) Z[k] = a = a + Z[k];
+        }
+        __syncthreads();
+    }
     /* per slot 0 < k < n - 1 (by falling k, those of one k a prefix of the
      * order) and polygon (unmoved, vertex 0 moved along x, along y): the
      * shoelace products and their difference.  Along y the difference has

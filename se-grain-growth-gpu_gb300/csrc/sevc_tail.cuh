@@ -59,17 +59,14 @@ __device__ __forceinline__ void count_grains(const DevMesh &m, int *counters, in
  * sums over the instance's grain indices, then the shared-memory tree.
  * CUDA block `rank` of `nranks` (at least tpb threads each) takes the
  * reference's blocks rank, rank + nranks, ...; those of an instance that
- * never held a nucleated grain sum to 0. */
+ * never held a nucleated grain are left out (their sums are 0). */
 __device__ __forceinline__ void nucl_area_blocks(const DevMesh &m, double *block_out, int nblocks, int tpb, int rank,
                                                  int nranks)
 {
     __shared__ double t[256];
     for (int u = rank; u < nblocks * m.ninst; u += nranks) {
         const int inst = u / nblocks, go = m.goff[inst], nn = m.nnlist[inst];
-        if (nn == 0) {
-            if (threadIdx.x == 0) block_out[u] = 0.0;
-            continue;
-        }
+        if (nn == 0) continue;
         const int tid = (u - inst * nblocks) * tpb + threadIdx.x, stride = nblocks * tpb;
         const int *nl = m.nlist + go;
         if ((int)threadIdx.x < tpb) {
@@ -99,7 +96,8 @@ __device__ __forceinline__ void nucl_area_final(const DevMesh &m, const double *
 {
     for (int i = tid; i < m.ninst; i += n) {
         double s = 0.0;
-        for (int b = 0; b < nblocks; b++) s += __ldcg(block_out + (size_t)i * nblocks + b);
+        if (m.nnlist[i] > 0)
+            for (int b = 0; b < nblocks; b++) s += __ldcg(block_out + (size_t)i * nblocks + b);
         *reinterpret_cast<double *>(counters + (size_t)i * CTR_COUNT + CTR_NUCL_AREA_SLOT) = 100 * s / (m.D * m.D);
     }
 }

@@ -1355,16 +1355,20 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
         for (int i = T.tid; i < m.ninst; i += T.n) x.counters[(size_t)i * CTR_COUNT + CTR_NGRAINS] = 0;
     if (PART & TAIL_REMOVE) {
         const int nfail = poll_loop(m, x, T, pg, cap);
-        if (na > 0) conflict_check(m, T, x.list_a, na);
-        T.sync();
-        if (na > 0) conflict_unlabel(m, T, x.list_a, na);
-        poll_reset(m, x, T, pg, nfail);
-        T.sync();
+        if (na > 0 || nfail > 0) {
+            if (na > 0) conflict_check(m, T, x.list_a, na);
+            T.sync();
+            if (na > 0) conflict_unlabel(m, T, x.list_a, na);
+            poll_reset(m, x, T, pg, nfail);
+            T.sync();
+        }
         if (*x.n_b > 0) two_three_loop(m, x, T, S);
-        if (na > 0) label3_reserve(m, x, T, na, dt);
-        if (T.tid == 0) *x.n_ehits = 0;              /* the grains a 2x3 pass left with three sides */
-        T.sync();
-        const int nc = *x.n_c;
+        if (na > 0) {
+            label3_reserve(m, x, T, na, dt);
+            if (T.tid == 0) *x.n_ehits = 0;          /* the grains a 2x3 pass left with three sides */
+            T.sync();
+        }
+        const int nc = na > 0 ? *x.n_c : 0;
         if (nc > 0) {
             remove_apply(m, x, T, x.list_c, nc);
             T.sync();
@@ -1395,10 +1399,15 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
     }
     if (PART & TAIL_FIX) fix_lists(m, T, S, false, nullptr, nullptr);
     if (PART & TAIL_END) {
+        /* the counts were zeroed before the last sync unless no candidate
+         * made one necessary */
+        if (na == 0) T.sync();
         for (int v = T.tid; v < m.nv; v += T.n) update_vertex(m, v, dt);
         count_grains(m, x.counters, T.tid, T.n);
         nucl_area_blocks(m, x.block_area, pg.blocks, pg.tpb, blockIdx.x, gridDim.x);
-        T.sync();
+        /* without nucleated grains (a plain handle) there is nothing to wait for */
+        const bool nucleated = m.ninst > 1 || m.nnlist[0] > 0;
+        if (nucleated) T.sync();
         nucl_area_final(m, x.block_area, pg.blocks, x.counters, T.tid, T.n);
         T.sync();
         pack_summary(m, x, summary, T.tid, T.n);
