@@ -71,9 +71,12 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  * across the wrap); they are walked vertex by vertex as written.
  *
  * What bounds it: the FP64 pipe (2 thread-operations per clock and SM, of
- * which independent chains reach 84%).  The certificate leaves 136 FP64
- * operations per grain (234 when the chains are recomputed), and the
- * integer pipe, otherwise idle, forms the exact differences.
+ * which independent chains reach 84%) together with the latency of the
+ * phases below.  The certificate leaves 111 FP64 operations per grain (234
+ * when the chains are recomputed): the integer pipe forms the exact
+ * differences, and the product of the stored energy with an area difference
+ * (mul_diff).  Forming the shoelace products on the integer pipe as well
+ * gained nothing (389 us with all of them, 378 with half).
  *
  * Layout.  A block takes GPB consecutive grains, orders them by falling
  * side count in shared memory (no order over the whole mesh is needed), and
@@ -93,9 +96,9 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  * `wide` or more sides or of fewer than 3, and the few whose moved chain
  * does not rejoin.
  *
- * Measured (GB300): 1M grains 0.446 ms, FP64 pipe active 68-73% of the
- * cycles, 23.5 of 32 lanes per FP64 instruction (slots of different s or p in
- * one warp); 2,000 grains 25 us.  The form before it (a grain per thread,
+ * Measured (GB300): 1M grains 0.385 ms, FP64 pipe active 69% of the
+ * cycles, 21 of 32 lanes per FP64 instruction (slots of different s or p in
+ * one warp); 2,000 grains 20 us.  The form before it (a grain per thread,
  * polygon in registers, one unrolled body per side count, side-count order
  * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
  * took 0.50 ms and 95 us: on a small mesh each unrolled body runs once and
@@ -124,21 +127,39 @@ __device__ __forceinline__ double div_sides(double x, int n)
     return ddiv_slow(x, (double)n);
 }
 
-/* x - y for x, y >= 0, on the integer pipe when both lie in one binade and
- * differ by less than 2^31 ulps (the difference is then exact: an integer
- * below 2^31 times the ulp) */
-__device__ __forceinline__ double diff_near(double x, double y)
+static __device__ __noinline__ double mul_diff_slow(double se, double x, double y) { return se * (x - y); }
+/* se * (x - y) for x, y >= 0 (src/calculus.h:60), each operation rounded, on
+ * the integer pipe when x and y lie in one binade and differ by less than
+ * 2^31 ulps: the difference is then k ulps exactly, and the product of k
+ * and se's significand, a 96-bit integer, is rounded to nearest even. */
+__device__ __forceinline__ double mul_diff(double se, double x, double y)
 {
-    long long bx = dbits(x), by = dbits(y), k = bx - by;
-    int E = (int)(by >> 52);
-    if ((int)(bx >> 52) != E || k != (long long)(int)k || E <= 64 || E >= 2047 || (int)k == INT_MIN)
-        return dsub_slow(x, y);
-    unsigned a = (unsigned)((int)k < 0 ? -(int)k : (int)k);
-    if (a == 0) return 0.0;
-    int lz = __clz((int)a);
-    unsigned mt = (a << lz) << 1;                      /* the bits below the leading one, left-aligned */
-    unsigned hi = ((unsigned)k & 0x80000000u) | ((unsigned)(E - 52 + 31 - lz) << 20) | (mt >> 12);
-    return __hiloint2double((int)hi, (int)(mt << 20));
+    const long long bx = dbits(x), by = dbits(y), k = bx - by, bs = dbits(se);
+    const int E = (int)(by >> 52), es = (int)((bs >> 52) & 0x7ff);
+    const unsigned a = (unsigned)((int)k < 0 ? -(int)k : (int)k);
+    const int lz = __clz((int)a);
+    int eb = 32 - lz + E + es - 1075;
+    const unsigned hi_sign = ((unsigned)k ^ (unsigned)((unsigned long long)bs >> 32)) & 0x80000000u;
+    /* one binade, k in 32 bits and not 0 or INT_MIN, se and the result well
+     * inside the normal range */
+    if ((int)(bx >> 52) != E || k != (long long)(int)k || a == 0 || a >> 31 || es == 0 || es == 0x7ff || E == 0 ||
+        eb < 2 || eb > 2045)
+        return mul_diff_slow(se, x, y);
+    const unsigned ka = a << lz;
+    const unsigned long long M = (((unsigned long long)bs & 0x000FFFFFFFFFFFFFULL) | (1ULL << 52)) << 11;
+    const unsigned long long p0 = (unsigned long long)ka * (unsigned)M, p1 = (unsigned long long)ka * (unsigned)(M >> 32);
+    unsigned long long h = p1 + (p0 >> 32);            /* bits 32 .. 95 of the product, its leading one at 95 or 94 */
+    unsigned l = (unsigned)p0;
+    if (!(h >> 63)) {
+        h = (h << 1) | (l >> 31);
+        l <<= 1;
+        eb--;
+    }
+    unsigned long long q = h >> 11;
+    const unsigned r = (unsigned)h & 0x7ffu;
+    q += r > 0x400u || (r == 0x400u && (l != 0 || (q & 1)));
+    const unsigned long long bits = ((unsigned long long)(eb - 1) << 52) + q;     /* a carry out of q raises the exponent */
+    return __longlong_as_double((long long)(bits | ((unsigned long long)hi_sign << 32)));
 }
 
 /* area_stream over a polygon staged in shared memory (raw positions P[k]
@@ -201,9 +222,8 @@ __device__ __noinline__ void grain_by_warp(const DevMesh &m, int g, double2 *P, 
 struct AxisCert { int e; unsigned up; };
 enum { GP_REST = 0, GP_CERT = 1, GP_CHAIN = 2 };
 
-constexpr int GP_CHUNK = 32, GP_SLOTS = 9 * GP_CHUNK;
-struct GrainChunk {
-    static constexpr int SLOTS = GP_SLOTS;
+constexpr int GP_CHUNK = 32;
+template <int SLOTS> struct GrainChunk {
     double R[2][SLOTS];                        /* raw coordinates; then the terms k of the polygons with vertex 0 moved */
     double A[2][SLOTS];                        /* unwrapped coordinates */
     double M[2][SLOTS];                        /* the same with vertex 0 moved along the axis; then M[0]: sum of T up to k */
@@ -224,21 +244,33 @@ struct GrainChunk {
     }
 };
 struct GrainRest { double2 P[SEVC_MAXV]; double R[2 * SEVC_MAXV + 1]; };   /* one per warp */
-#define GRAIN_SMEM(NT) (sizeof(GrainChunk) > sizeof(GrainRest) * ((NT) / 32) ? sizeof(GrainChunk) : sizeof(GrainRest) * ((NT) / 32))
-/* a - b for positive binary64 patterns whose exponents are e or e + 1 and
- * whose difference is a multiple of 2^(e - 1075) below 2^53 of them (hence
- * exact), on the integer pipe */
-__device__ __forceinline__ double sub_exact(long long a, long long b, int e)
+template <int NT, int SLOTS> struct GrainSmem {
+    static constexpr size_t rest = sizeof(GrainRest) * (NT / 32), chunk = sizeof(GrainChunk<SLOTS>);
+    static constexpr size_t bytes = chunk > rest ? chunk : rest;
+};
+/* d 2^(e - 1075) for |d| < 2^53: exact, on the integer pipe */
+__device__ __forceinline__ double grid_value(long long d, int e)
 {
-    const long long M = 0x000FFFFFFFFFFFFFLL, H = 1LL << 52;
-    long long ma = (a & M) | H, mb = (b & M) | H;
-    ma <<= (int)(a >> 52) - e;
-    mb <<= (int)(b >> 52) - e;
-    const long long d = ma - mb;
     const unsigned long long u = (unsigned long long)(d < 0 ? -d : d);
     const int sh = __clzll((long long)u) - 11;
     const unsigned long long r = ((unsigned long long)(e - 1 - sh) << 52) + (u << sh);
     return d == 0 ? 0.0 : __longlong_as_double((long long)(r | ((unsigned long long)d & 0x8000000000000000ULL)));
+}
+/* a - b for positive binary64 patterns whose exponents are e or e + 1 and
+ * whose difference is below 2^53 times 2^(e - 1075) */
+__device__ __forceinline__ double sub_exact(long long a, long long b, int e)
+{
+    const long long M = 0x000FFFFFFFFFFFFFLL, H = 1LL << 52;
+    const long long ma = ((a & M) | H) << ((int)(a >> 52) - e), mb = ((b & M) | H) << ((int)(b >> 52) - e);
+    return grid_value(ma - mb, e);
+}
+/* a + n 2^(e - 1075) for a multiple a of 2^(e - 1075), |a| < 2^53 times it */
+__device__ __forceinline__ double add_exact(double a, long long n, int e)
+{
+    const long long b = dbits(a);
+    const int ea = (int)((b >> 52) & 0x7ff);
+    long long m = ((b & 0x000FFFFFFFFFFFFFLL) | (1LL << 52)) >> (ea ? e - ea : 63);
+    return grid_value((b < 0 ? -m : m) + n, e);
 }
 
 /* certificate of one axis over the raw coordinates r[0..n); that no
@@ -274,18 +306,17 @@ __device__ __noinline__ double chain_moved(const double *a, int p, int n, double
     return x;
 }
 
-template <int GPB, int NT>
-__global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n_three, int wide, long long dlim)
+template <int GPB, int NT, int SLOTS>
+__global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m, int *three, int *n_three, int wide, long long dlim)
 {
-    __shared__ __align__(16) unsigned char smem[GRAIN_SMEM(NT)];
-    GrainChunk &B = *reinterpret_cast<GrainChunk *>(smem);
+    __shared__ __align__(16) unsigned char smem[GrainSmem<NT, SLOTS>::bytes];
+    GrainChunk<SLOTS> &B = *reinterpret_cast<GrainChunk<SLOTS> *>(smem);
     __shared__ int order[GPB];                 /* the block's grains by falling side count */
     __shared__ unsigned char sides[GPB];
     __shared__ int cnt[GP_NMAX], start[GP_NMAX];
     __shared__ int first[GP_NMAX];             /* first[j]: first entry of B.moved (and B.inner) with s + 2 = j */
     __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved, chains;
     __shared__ long long ntab[GP_E1 - GP_E0 + 1];
-    __shared__ double dtab[GP_E1 - GP_E0 + 1];
     constexpr int W = NT / 32;
     static_assert(GPB <= NT, "a thread per grain orders them");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -300,13 +331,9 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
     if (tid < GP_NMAX) cnt[tid] = 0;
     if (tid == 0) nrest = 0;
     for (int t = tid; t <= GP_E1 - GP_E0; t += NT) {
-        /* RN(eps / ulp) for coordinates of this exponent, and that multiple
-         * of the ulp as a double (below 2^46 ulps: exact) */
-        int d = t + GP_E0 - GP_EPS_E;
-        long long nk = (GP_EPS_M + (1LL << (d - 1))) >> d;
-        int lz = __clzll(nk) - 11;
-        ntab[t] = nk;
-        dtab[t] = __longlong_as_double(((long long)(t + GP_E0 - 1 - lz) << 52) + (nk << lz));
+        /* RN(eps / ulp) for coordinates of this exponent */
+        const int d = t + GP_E0 - GP_EPS_E;
+        ntab[t] = (GP_EPS_M + (1LL << (d - 1))) >> d;
     }
     __syncthreads();
     /* the block's grains by falling side count */
@@ -337,7 +364,7 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
         sides[start[n] + r] = (unsigned char)n;
     }
     __syncthreads();
-    /* chunks of up to 32 grains (and GP_SLOTS slots) of the order */
+    /* chunks of up to 32 grains (and SLOTS list slots) of the order */
     for (int c0 = 0; c0 < listed; c0 += chunk) {
     if (warp == 0) {
         const int i = c0 + lane, k = i < listed ? sides[i] : 0;
@@ -347,7 +374,7 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
             int y = __shfl_up_sync(0xffffffffu, o, d);
             if (lane >= d) o += y;
         }
-        const bool in = k > 0 && o <= GP_SLOTS;
+        const bool in = k > 0 && o <= SLOTS;
         const int c = __popc(__ballot_sync(0xffffffffu, in));
         o -= k;
         if (in) {
@@ -482,8 +509,11 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
      * F the moved axis and G the other one, the terms p - 1 and p are
      * F[p-1] G[p] - G[p-1] f and f G[p+1] - G[p] F[p+1] for x, minus those
      * for y; along y the whole sum is formed with the opposite sign. */
-    for (int t = tid; t < 2 * nmoved; t += NT) {
-        const int x = t >= nmoved, q = B.moved[x ? t - nmoved : t], i = B.owner[q], o = B.off[i], p = q - o, nn = B.n[i];
+    const int per_axis = (nmoved + 31) & ~31;         /* no warp works on both axes */
+    for (int t = tid; t < 2 * per_axis; t += NT) {
+        const int x = t >= per_axis, w = x ? t - per_axis : t;
+        if (w >= nmoved) continue;
+        const int q = B.moved[w], i = B.owner[q], o = B.off[i], p = q - o, nn = B.n[i];
         const int st = B.state(i);
         if (st == GP_REST) continue;
         double a;         /* twice the moved area */
@@ -493,7 +523,8 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
             const double *F = B.A[x], *G = B.A[1 - x];
             double f;
             if (st == GP_CERT) {
-                f = F[q] + dtab[B.c[x][i].e + ((B.c[x][i].up >> p) & 1)];
+                const int e = B.c[x][i].e, up = (int)((B.c[x][i].up >> p) & 1u);
+                f = add_exact(F[q], ntab[e + up] << up, e + GP_E0);
             } else {
                 const double2 rr = m.pos[B.dest[q] / 3], rm = m.pos[B.dest[q - 1] / 3];
                 const double2 rp = m.pos[B.dest[p < nn - 1 ? q + 1 : q] / 3];
@@ -516,7 +547,7 @@ __global__ void __launch_bounds__(NT) k_grain_pass(DevMesh m, int *three, int *n
                 for (int k = q + 1; k < o + nn - 1; k++) a = a + sgn(B.T[k]);
             }
         }
-        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = B.se[i] * diff_near(dabs(dscale_down<1>(a)), B.absA[i]);
+        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), B.absA[i]);
     }
     __syncthreads();
     }
@@ -776,14 +807,16 @@ void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape 
     auto go = [&](auto kernel, int gpb, int nt) {
         COUNT_LAUNCHES(1), kernel<<<(m.ng + gpb - 1) / gpb, nt, 0, s>>>(m, x.three, x.n_three, wide, dlim);
     };
-    /* 32 grains a block at every size (blocks of 64 in two chunks measured
-     * the same at 1M grains and 10% more at 100K; they stay for the
-     * autotuner).  Below GRAIN_SMALL grains an SM holds few blocks, and
-     * eight warps shorten each one's phases: 3-11 us less per step at 2K-20K
-     * grains than four; from 50K on four are as fast. */
-    if (sh.grain_occ < 6) go(k_grain_pass<64, 128>, 64, 128);
-    else if (m.ng < GRAIN_SMALL) go(k_grain_pass<32, 256>, 32, 256);
-    else go(k_grain_pass<32, 128>, 32, 128);
+    /* 32 grains a block at every size (blocks of 64 in two chunks: 414
+     * against 385 us at 1M grains, 67 against 62 at 100K; they stay for the
+     * autotuner).  Large meshes want blocks on the SM: 208 slots (6.5 per
+     * grain; 3% of the blocks need a second chunk) and 40 registers let
+     * eleven in, 385 us against 397 with ten.  Below GRAIN_SMALL grains an SM
+     * holds few blocks and the longest one is the time: eight warps and
+     * 288 slots, 20 us against 25 at 2,000 grains. */
+    if (sh.grain_occ < 6) go(k_grain_pass<64, 128, 208>, 64, 128);
+    else if (m.ng < GRAIN_SMALL) go(k_grain_pass<32, 256, 288>, 32, 256);
+    else go(k_grain_pass<32, 128, 208>, 32, 128);
 }
 
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s)
