@@ -797,25 +797,6 @@ __device__ __forceinline__ void finalize_boundary(const DevMesh &m, int b)
     m.btext[b] = text_exact(pi, pe, vi, ve, m.D);
     m.bexact[b] = 1;
 }
-/* an event is about to edit grain g's list (or disable it): its dA/dt as
- * the step computed it before any event.  The list itself is still the
- * step's: lists change only in the fix-up pass, after mark_fix has
- * settled every grain it edits. */
-__device__ __forceinline__ void finalize_grain(const DevMesh &m, int g)
-{
-    if (m.gexact[g]) return;
-    unsigned st = *m.stamp;
-    m.gdadt[g] = dadt_over(m, g, [&](const int (&v)[8], double2 (&r)[8], double2 (&w)[8]) {
-        bool saved[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) { r[j] = m.pos[v[j]]; w[j] = m.vel[v[j]]; saved[j] = m.vstamp[v[j]] == st; }
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-            if (saved[j]) { r[j] = m.pos0[v[j]]; w[j] = m.vel0[v[j]]; }
-    });
-    m.gexact[g] = 1;
-}
-
 /* first position of an ascending list whose value is >= x */
 __device__ __forceinline__ int lower_bound_i(const int *a, int n, int x)
 {

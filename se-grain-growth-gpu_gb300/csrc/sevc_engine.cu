@@ -119,7 +119,7 @@ struct sevc_handle {
      * run concurrently; captured as graph branches) and the fork / join
      * events between them: 0-5 in the first half, 6-7 in the tail */
     cudaStream_t side[2] = { nullptr, nullptr };
-    cudaEvent_t evfork[10] = {};
+    cudaEvent_t evfork[8] = {};
     bool profiling = false;
     std::map<std::string, ProfEntry> prof;
     std::vector<std::pair<std::string, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
@@ -352,7 +352,7 @@ sevc_status create_from_host(const sevc_options *opt, sevc_hmesh *hm, sevc_handl
     bool streams_ok = cuda_ok(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
     for (int k = 0; streams_ok && k < 2; k++)
         streams_ok = cuda_ok(cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking), "stream");
-    for (int k = 0; streams_ok && k < 10; k++)
+    for (int k = 0; streams_ok && k < 8; k++)
         streams_ok = cuda_ok(cudaEventCreateWithFlags(&h->evfork[k], cudaEventDisableTiming), "event");
     if (!streams_ok || !cuda_ok(cudaMallocHost(&h->h_ctr, 256), "pinned") ||
         !cuda_ok(cudaMallocHost(&h->h_big, h->h_big_ints * sizeof(int)), "pinned") ||
@@ -575,30 +575,20 @@ void enqueue_tail(sevc_handle *h)
     sevc_pdl_skip = 0;
     if (h->profiling) {
         { Prof pr(h, "flips"); launch_tail_flips(m, x, p, s); }                                   /* :282, :289 */
-        { Prof pr(h, "fix_lists"); launch_tail_fix(m, x, p, s); }                                 /* :294 */
         { Prof pr(h, "update"); launch_update_positions(m, p.dt, s); }                            /* :314 */
         { Prof pr(h, "counts"); launch_counts(m, x, p, s); }                                      /* :317-325 */
     } else {
         /* The counts read only grain flags, types and areas, which are final
          * here (the flips and the list fix-up after them change none): side0
-         * computes them beside the flips, the fix-up and the position
-         * update.  The position update reads positions and velocities, final
-         * once the flips are applied; the fix-up after them edits only lists
-         * and mods: side1 updates beside it.  Both join before the summary. */
+         * computes them beside the flips and the position update.  Both join
+         * before the summary. */
         cudaEvent_t *ev = h->evfork;
         cudaEventRecord(ev[6], s);
         cudaStreamWaitEvent(h->side[0], ev[6], 0);
         launch_counts(m, x, p, h->side[0]);
         cudaEventRecord(ev[7], h->side[0]);
         launch_tail_flips(m, x, p, s);
-        cudaEventRecord(ev[8], s);
-        cudaStreamWaitEvent(h->side[1], ev[8], 0);
-        sevc_pdl_skip = 1;
-        launch_update_positions(m, p.dt, h->side[1]);
-        sevc_pdl_skip = 0;
-        cudaEventRecord(ev[9], h->side[1]);
-        launch_tail_fix(m, x, p, s);
-        cudaStreamWaitEvent(s, ev[9], 0);
+        launch_update_positions(m, p.dt, s);
         cudaStreamWaitEvent(s, ev[7], 0);
         sevc_pdl_skip = 1;
     }

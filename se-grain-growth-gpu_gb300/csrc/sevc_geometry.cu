@@ -771,12 +771,6 @@ __global__ void k_reset_ngrains(int *counters, int ninst)
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ninst) counters[(size_t)i * CTR_COUNT + CTR_NGRAINS] = 0;
 }
-__global__ void k_update(DevMesh m, double dt)
-{
-    griddep_wait();
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < m.nv) update_vertex(m, v, dt);
-}
 /* both counts; the last block finishes the nucleated area */
 __global__ void __launch_bounds__(TPB) k_counts(DevMesh m, int *counters, double *block_area, int nblocks, int tpb)
 {
@@ -843,8 +837,6 @@ void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &
     if (m.nb > 0)
         launch_dep(k_text_label, (m.nb + 2 * t - 1) / (2 * t), t, s, m, x, poll_grid(p), dt, Df, hDf, inv_dt, dt_up);
 }
-void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s) { launch_dep(k_update, nblk(m.nv), TPB, s, m, dt); }
-
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s)
 {
     size_t total = (size_t)m.ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 5;

@@ -105,7 +105,6 @@ void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const Launch
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s);
 /* also lists the candidates and starts the polling's first comparison */
 void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
-void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s);
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 /* counters | events | error bits | polling iterations | 2x3 counts | output decision, into out */
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s);
@@ -119,13 +118,13 @@ PollGrid poll_grid(const StepParams &p);
 void launch_two_three_first(const DevMesh &m, const DevScratch &x, cudaStream_t s);
 /* The sparse phases (k_tail): all of them, the position update, the counts
  * and the summary in one launch for meshes that tail_whole accepts; else the
- * removals, the flips and the flips' list fix-up, beside which the update
- * and the counts run as kernels over the whole GPU. */
+ * removals and the flips, each with the edits of its list fix-up, and the
+ * position update with the rest of the flips' fix-up. */
 bool tail_whole(const DevMesh &m);
 void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s);
 void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s);
 void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
-void launch_tail_fix(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
+void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s);
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s);
 
 /* The mesh in the layout of sevc_mesh_host, written by the device through

@@ -122,7 +122,7 @@ __device__ __forceinline__ void pack_summary(const DevMesh &m, const DevScratch 
         else if ((k -= ne) < 4) { v = m.err[k]; m.err[k] = 0; }
         else if ((k -= 4) < I) { v = x.piters[k]; x.piters[k] = 0; m.pdone[k] = 0; }
         else if ((k -= I) < ns) { v = x.segcnt[k]; x.segcnt[k] = 0; }
-        else { v = x.flags[0]; *x.n_a = *x.n_b = *x.n_c = *x.n_ehits = *x.n_three = 0; }
+        else { v = x.flags[0]; *x.n_a = *x.n_b = *x.n_c = *x.n_ehits = *x.n_three = *m.nfix = *m.nmod = 0; }
         out[i] = v;
     }
     const size_t nw = (size_t)m.ng / 16;                   /* gexact as 16-byte words (256-byte aligned array) */

@@ -82,11 +82,11 @@ __device__ void set_mod(const DevMesh &m, int v, int slot, int fix, int grn, int
 }
 
 /* ------------------------------------------------------------------ */
-/* the team: one cluster                                               */
+/* the team                                                            */
 /* ------------------------------------------------------------------ */
-/* Every thread of the cluster's blocks; a phase ends at sync(): what any
- * thread wrote before it, any thread reads after it (release / acquire at
- * cluster scope).  The grid is exactly one cluster. */
+/* Every thread of the grid.  In k_tail the grid is exactly one cluster and a
+ * phase ends at sync(): what any thread wrote before it, any thread reads
+ * after it (release / acquire at cluster scope). */
 struct Team {
     int tid, n;            /* thread of the team, threads */
     int warp, nwarps, lane;/* consecutive warps lie in different blocks: a few events spread over all SMs */
@@ -336,9 +336,9 @@ __device__ bool two_three_qualifies(const DevMesh &m, int b, int *gic)
 }
 
 /* Qualifying boundaries among those at the vertices of the 3-sided grains
- * a[0..na) and then b[0..): a qualifying boundary lies on two of them, so testing these
- * gives every one; each is appended once, by the smaller of its two grains
- * at its first end.  t: one (grain, vertex, slot). */
+ * a[0..na) and then b[0..): a qualifying boundary lies on two of them, so
+ * testing these gives every one; each is appended once, by the smaller of its
+ * two grains at its first end.  t: one (grain, vertex, slot). */
 __device__ __forceinline__ void find_two_three(const DevMesh &m, const int *a, int na, const int *b, int t, int *out,
                                                int *n_out)
 {
@@ -1176,86 +1176,143 @@ __device__ void fix_grain_serial(const DevMesh &m, int g, int *Ls, unsigned char
         }
     }
 }
-struct FixShared {
-    int Ls[TAIL_WARPS][SEVC_MAXV], Ss[TAIL_WARPS][SEVC_MAXV], Nw[TAIL_WARPS][2];
-    unsigned char Fs[TAIL_WARPS][SEVC_MAXV], SFs[TAIL_WARPS][SEVC_MAXV];
+/* compute_area (RATE false: area_stream) or compute_dAdt (RATE true:
+ * dadt_over, from the step's starting state) over the list L of n entries by
+ * one warp, the same operations in the same order: each lane forms its
+ * vertex's wrapped delta and its terms, and the additions whose order counts,
+ * the running coordinates and the sum, go through the lanes in list order. */
+template <bool RATE> __device__ __forceinline__ double warp_sum(const DevMesh &m, const int *L, int n, int lane, unsigned st)
+{
+    const unsigned all = 0xffffffffu;
+    double acc = 0, X = 0, Y = 0, vx = 0, vy = 0;    /* the sum; the last vertex's coordinates and velocity */
+    double2 pr = make_double2(0, 0), w0 = pr;        /* its position; the first vertex's velocity */
+    for (int base = 0; base < n; base += 32) {
+        const int k = base + lane, len = min(n - base, 32);
+        double2 r = make_double2(0, 0), w = r;
+        if (k < n) {
+            const int v = L[k];
+            r = m.pos[v];
+            if (RATE) {
+                w = m.vel[v];
+                if (m.vstamp[v] == st) { r = m.pos0[v]; w = m.vel0[v]; }
+            }
+        }
+        double2 q = make_double2(__shfl_up_sync(all, r.x, 1), __shfl_up_sync(all, r.y, 1));
+        if (lane == 0) q = pr;
+        double dx = 0, dy = 0, mx = 0, my = 0, px = X, py = Y;
+        if (k > 0 && k < n) { dx = wrapd(r.x, q.x, m.D); dy = wrapd(r.y, q.y, m.D); }
+#pragma unroll 1
+        for (int j = 0; j < len; j++) {
+            if (j == lane) { px = X; py = Y; }
+            X += __shfl_sync(all, dx, j);
+            Y += __shfl_sync(all, dy, j);
+            if (j == lane) { mx = X; my = Y; }
+        }
+        double t, u = 0;
+        if (RATE) {
+            double2 z = make_double2(__shfl_up_sync(all, w.x, 1), __shfl_up_sync(all, w.y, 1));
+            if (lane == 0) z = make_double2(vx, vy);
+            t = z.x * my + px * w.y;
+            u = z.y * mx + py * w.x;
+            if (base == 0) w0 = make_double2(__shfl_sync(all, w.x, 0), __shfl_sync(all, w.y, 0));
+            vx = __shfl_sync(all, w.x, len - 1);
+            vy = __shfl_sync(all, w.y, len - 1);
+        } else {
+            t = px * my - py * mx;
+        }
+        pr = make_double2(__shfl_sync(all, r.x, len - 1), __shfl_sync(all, r.y, len - 1));
+#pragma unroll 1
+        for (int j = base ? 0 : (RATE ? 1 : 2); j < len; j++) {
+            acc += __shfl_sync(all, t, j);
+            if (RATE) acc -= __shfl_sync(all, u, j);
+        }
+    }
+    if (RATE) {
+        if (n > 0) {
+            acc += (vx * 0.0 + X * w0.y);
+            acc -= (vy * 0.0 + Y * w0.x);
+        }
+        return acc;
+    }
+    if (n > 0) acc = add_closing_term(acc, X, Y);
+    return dscale_down<1>(acc);
+}
+template <int WARPS> struct EditShared {
+    int Ls[WARPS][SEVC_MAXV], Ss[WARPS][SEVC_MAXV], Nw[WARPS][2];
+    unsigned char Fs[WARPS][SEVC_MAXV], SFs[WARPS][SEVC_MAXV];
 };
-/* three, n_three (may be null): grains the edit leaves with three sides are
- * listed there */
-__device__ void fix_edit(const DevMesh &m, const Team &T, FixShared &S, int *three, int *n_three)
+__device__ __noinline__ void settle_boundary(const DevMesh &m, int b) { finalize_boundary(m, b); }
+/* fix_grain_lists (:1209-1227), the edits, with what belongs to a grain
+ * before and after its own: one warp per queued grain and per removed one
+ * (gone[0..ngone)), in this order
+ *   settle   the output-only dA/dt (see DevMesh) over the list as it still
+ *            is, from the step's starting state, which the events saved
+ *   edit     the list (queued and enabled grains)
+ *   area     compute_grain_areas after the removals (src/main.cu:266), if
+ *            areas is set.  Only a grain whose list changed since the grain
+ *            pass can have a new area (the vertex a 3-sided removal moves
+ *            belongs only to grains that removal queues), and its list and
+ *            vertices are final for the step here; a grain edited by several
+ *            fix-ups (2x3 passes, then the removals) is computed again by
+ *            each, the last one on the final positions.  The flips' fix-up
+ *            comes after the counts and needs none (the next step's grain
+ *            pass computes every area).
+ * No warp reads another's grain, so nothing separates the three.  three,
+ * n_three (may be null): grains the edit leaves with three sides are listed
+ * there.
+ *
+ * Beside them, the extinction times of the boundaries at the removed grains'
+ * vertices that are now disabled.  One costs some 400 FP64 operations
+ * (atan2, cos, sin), so its threads are the k-th (k < 3) such boundary of each
+ * removed grain, not its nine slots with mostly idle lanes; the third takes
+ * any beyond. */
+template <int WARPS>
+__device__ void edit_grains(const DevMesh &m, const Team &T, EditShared<WARPS> &S, const int *gone, int ngone, bool areas,
+                            int *three, int *n_three)
 {
     const int lane = T.lane, wib = threadIdx.x >> 5;
     const int nf = min(*m.nfix, m.fixcap);
-    for (int w = T.warp; w < nf; w += T.nwarps) {
-        const int g = m.fixlist[w];
-        if (!(m.gen[g] && m.gfix[g])) continue;
+    const unsigned st = *m.stamp;
+    for (int w = T.warp; w < nf + ngone; w += T.nwarps) {
+        const int g = w < nf ? m.fixlist[w] : gone[w - nf];
         int *L = m.glist + (size_t)SEVC_MAXV * g;
-        const int n = m.gvlen[g];
-        for (int i = lane; i < n; i += 32) {
-            int v = L[i];
-            S.Ls[wib][i] = v;
-            S.Fs[wib][i] = (unsigned char)mod_ops_for(m, v, g);
+        int n = m.gvlen[g];
+        const bool due = !m.gexact[g], queued = w < nf && m.gen[g], edit = queued && m.gfix[g];
+        if (edit) {
+            for (int i = lane; i < n; i += 32) {
+                int v = L[i];
+                S.Ls[wib][i] = v;
+                S.Fs[wib][i] = (unsigned char)mod_ops_for(m, v, g);
+            }
+        }
+        if (due) {
+            const double d = warp_sum<true>(m, L, n, lane, st);
+            if (lane == 0) { m.gdadt[g] = d; m.gexact[g] = 1; }
+        }
+        if (edit) {
+            __syncwarp();
+            if (lane == 0) {
+                int nn = n, hi = n;
+                fix_grain_serial(m, g, S.Ls[wib], S.Fs[wib], S.Ss[wib], S.SFs[wib], nn, hi);
+                S.Nw[wib][0] = nn;
+                S.Nw[wib][1] = hi;
+                if (nn != n) m.gvlen[g] = nn;
+                if (n_three && nn == 3 && n != 3) three[atomicAdd(n_three, 1)] = g;
+            }
+            __syncwarp();
+            n = S.Nw[wib][0];
+            const int hi = S.Nw[wib][1];
+            for (int i = lane; i < hi; i += 32) L[i] = S.Ls[wib][i];
+        }
+        if (queued) {
+            if (areas) {
+                const double a = warp_sum<false>(m, edit ? S.Ls[wib] : L, n, lane, 0);
+                if (lane == 0) m.garea[g] = a;
+            }
+            if (lane == 0) m.gfix[g] = 0;            /* clear_grains_fix_state (:1150-1163) */
         }
         __syncwarp();
-        if (lane == 0) {
-            int nn = n, hi = n;
-            fix_grain_serial(m, g, S.Ls[wib], S.Fs[wib], S.Ss[wib], S.SFs[wib], nn, hi);
-            S.Nw[wib][0] = nn;
-            S.Nw[wib][1] = hi;
-            if (nn != n) m.gvlen[g] = nn;
-            if (n_three && nn == 3 && n != 3) three[atomicAdd(n_three, 1)] = g;
-        }
-        __syncwarp();
-        const int hi = S.Nw[wib][1];
-        for (int i = lane; i < hi; i += 32) L[i] = S.Ls[wib][i];
-        __syncwarp();
     }
-}
-/* clear_grains_fix_state (:1150-1163): fix = false for enabled grains and
- * reset the mods of every vertex listed by an enabled grain.  Only queued
- * grains can have fix set and only marked vertices can hold mods.
- *
- * areas: compute_grain_areas after the removals (src/main.cu:266) for the
- * grains this fix-up edited.  Only a grain whose list changed since the
- * grain pass can have a new area (the vertex a 3-sided removal moves
- * belongs only to grains that removal queues), and its list and vertices
- * are final for the step here; a grain edited by several fix-ups (2x3
- * passes, then the removals) is computed again by each, the last one on
- * the final positions.  The flips' fix-up comes after the counts and needs
- * none (the next step's grain pass computes every area). */
-__device__ void fix_clear(const DevMesh &m, const Team &T, bool areas)
-{
-    int nf = min(*m.nfix, m.fixcap), nm = min(*m.nmod, m.modcap);
-    for (int w = T.tid; w < nf; w += T.n) {
-        int g = m.fixlist[w];
-        if (m.gen[g]) {
-            m.gfix[g] = 0;
-            if (areas) m.garea[g] = area_stream(m.glist + (size_t)SEVC_MAXV * g, m.gvlen[g], m.pos, m.D);
-        }
-    }
-    /* a thread per marked vertex and grain around it, from the other end of
-     * the team; each that finds the vertex listed writes the same */
-    for (int t = T.n - 1 - T.tid; t < 3 * nm; t += T.n) {
-        int w = t / 3, j = t - 3 * w, v = m.modlist[w];
-        if (j == 0) m.vmodmark[v] = 0;
-        int g = slot3(m.vg[v], j);
-        if (g >= 0 && m.gen[g] && glist_find(m, g, v) >= 0)
-            for (int k = 0; k < 4; k++) m.vmod[4 * (size_t)v + k] = make_int4(-1, -1, -1, FIX_NONE);
-    }
-}
-__device__ __noinline__ void settle_boundary(const DevMesh &m, int b) { finalize_boundary(m, b); }
-/* Output-only values that the events make final (see DevMesh): the dA/dt of
- * the queued grains, whose lists the fix-up is about to change, and of the
- * removed ones (gone[0..ngone)), one grain per thread; and the extinction
- * times of the boundaries at the removed grains' vertices that are now
- * disabled.  All from the step's starting state, which the events saved.
- * A boundary costs some 400 FP64 operations (atan2, cos, sin), so its
- * threads are the k-th (k < 3) such boundary of each removed grain, not its
- * nine slots with mostly idle lanes; the third takes any beyond. */
-__device__ void settle(const DevMesh &m, const Team &T, const int *gone, int ngone)
-{
-    const int nf = min(*m.nfix, m.fixcap);
-    for (int t = T.tid; t < nf + ngone; t += T.n) finalize_grain(m, t < nf ? m.fixlist[t] : gone[t - nf]);
     /* the boundaries from the other end of the team, beside the grains */
     for (int t = T.n - 1 - T.tid; t < 3 * ngone; t += T.n) {
         const int i = t / 3, k = t - 3 * i;
@@ -1269,13 +1326,16 @@ __device__ void settle(const DevMesh &m, const Team &T, const int *gone, int ngo
         unsigned due = 0;
 #pragma unroll
         for (int j = 0; j < 9; j++) {
-            bool off = valid_b(m, b[j]) && !m.ben[b[j]] && !m.bexact[b[j]];
+            /* not by bexact, which the grain's other threads and those of the
+             * grains around it set meanwhile: all must count alike */
+            bool off = valid_b(m, b[j]) && !m.ben[b[j]];
 #pragma unroll
             for (int q = 0; q < j; q++) off = off && b[q] != b[j];
             due |= off ? 1u << j : 0u;
         }
-        for (int c = 0; due; c++, due &= due - 1) {
-            if (c < k) continue;
+        for (int c = 0; c < k; c++) due &= due - 1;
+        /* the first call is every thread's at once */
+        for (; due; due &= due - 1) {
             const int j = __ffs(due) - 1;
             int x = b[0];
 #pragma unroll
@@ -1285,14 +1345,31 @@ __device__ void settle(const DevMesh &m, const Team &T, const int *gone, int ngo
         }
     }
 }
-/* fix_grain_lists (:1209-1227): the edits, then the clearing; both work
- * lists empty afterwards.  Ends with a sync. */
-__device__ void fix_lists(const DevMesh &m, const Team &T, FixShared &S, bool areas, int *three, int *n_three)
+/* clear_grains_fix_state (:1150-1163), the rest: reset the mods of every
+ * vertex listed by an enabled grain.  Only marked vertices can hold mods.
+ * Thread tid of n: one marked vertex and grain around it; each that finds
+ * the vertex listed writes the same. */
+__device__ __forceinline__ void clear_mods(const DevMesh &m, int tid, int n)
 {
-    if (*m.nfix == 0 && *m.nmod == 0) return;      /* the same in every block: written before the last sync */
-    fix_edit(m, T, S, three, n_three);
+    const int nm = min(*m.nmod, m.modcap);
+    for (int t = tid; t < 3 * nm; t += n) {
+        int w = t / 3, j = t - 3 * w, v = m.modlist[w];
+        if (j == 0) m.vmodmark[v] = 0;
+        int g = slot3(m.vg[v], j);
+        if (g >= 0 && m.gen[g] && glist_find(m, g, v) >= 0)
+            for (int k = 0; k < 4; k++) m.vmod[4 * (size_t)v + k] = make_int4(-1, -1, -1, FIX_NONE);
+    }
+}
+typedef EditShared<TAIL_WARPS> FixShared;
+/* the edits, then the clearing; both work lists empty afterwards.  Ends with
+ * a sync. */
+__device__ void fix_lists(const DevMesh &m, const Team &T, FixShared &S, const int *gone, int ngone, bool areas,
+                          int *three, int *n_three)
+{
+    if (*m.nfix == 0 && *m.nmod == 0 && ngone == 0) return; /* the same in every block: written before the last sync */
+    edit_grains(m, T, S, gone, ngone, areas, three, n_three);
     T.sync();
-    fix_clear(m, T, areas);
+    clear_mods(m, T.tid, T.n);
     T.sync();
     if (T.tid == 0) *m.nfix = *m.nmod = 0;
     T.sync();
@@ -1314,11 +1391,10 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
         for (int i = T.tid; i < m.ninst; i += T.n)
             remove_two_three(m, sorted, n, x.extra, x.segcnt + (size_t)pass * m.ninst, x.list_b, x.n_b, i);
         T.sync();
-        settle(m, T, x.list_b, *x.n_b);       /* the removed grains, listed by the removals */
-        T.sync();
+        /* with the removed grains, listed by the removals */
+        fix_lists(m, T, S, x.list_b, *x.n_b, true, x.ehits, x.n_ehits);
         if (T.tid == 0) *x.n_b = 0;
         T.sync();
-        fix_lists(m, T, S, true, x.ehits, x.n_ehits);
         const int n3 = *x.n_three, more = *x.n_ehits;
         for (int t = T.tid; t < 9 * (n3 + more); t += T.n)
             find_two_three(m, x.three, n3, x.ehits, t, x.list_b, x.n_b);
@@ -1330,11 +1406,12 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
 /* The part of a step after the t_ext labels (src/main.cu:219-325) as one
  * launch of one cluster.  PART selects what a launch covers:
  *   TAIL_REMOVE  polling (:219), conflicts (:222-225), the 2x3 loop
- *                (:227-250), 3-sided labels (:252-255), removals (:259), list
- *                fix-up with the areas after it (:262-266)
+ *                (:227-250), 3-sided labels (:252-255), removals (:259)
  *   TAIL_FLIP    flips (:282-289)
- *   TAIL_FIX     the flips' list fix-up (:294)
- *   TAIL_END     position update (:314), counts (:317-325), step summary
+ *   TAIL_END     the list fix-ups (:262-266, :294), position update (:314),
+ *                counts (:317-325), step summary
+ * On a large mesh TAIL_REMOVE and TAIL_FLIP are launches of their own and
+ * the fix-ups run on the whole GPU behind each (k_edit).
  *
  * What bounds it: nothing but the chain of its phases, each a handful of
  * dependent loads.  As ~25 kernels (programmatic dependent launch between
@@ -1342,7 +1419,7 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
  * cluster barrier costs well under a microsecond.  16 blocks of 512 are the
  * largest cluster; with a warp per event that is 256 events at once. */
 constexpr int TAIL_WHOLE_NV = 64 * 1024;
-enum { TAIL_REMOVE = 1, TAIL_FLIP = 2, TAIL_FIX = 4, TAIL_END = 8 };
+enum { TAIL_REMOVE = 1, TAIL_FLIP = 2, TAIL_END = 4 };
 template <int PART>
 __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, PollGrid pg, int cap, double dt, double eps,
                                                   int *summary)
@@ -1377,9 +1454,17 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
                 run_deferred(m, x, T, nd, m.goff, [&](int g, int inst) { remove_warp(m, g, inst, T.lane); });
                 T.sync();
             }
-            settle(m, T, x.list_c, nc);
+            if (PART & TAIL_END) fix_lists(m, T, S, x.list_c, nc, true, nullptr, nullptr);
+        }
+    }
+    if ((PART & TAIL_FLIP) && !(PART & TAIL_END)) {
+        /* the rest of the removals' fix-up, after k_edit */
+        const bool queued = *m.nfix > 0 || *m.nmod > 0;
+        if (queued) {
+            clear_mods(m, T.tid, T.n);
             T.sync();
-            fix_lists(m, T, S, true, nullptr, nullptr);
+            if (T.tid == 0) *m.nfix = *m.nmod = 0;
+            T.sync();
         }
     }
     if ((PART & TAIL_FLIP) && na > 0) {
@@ -1392,13 +1477,9 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
             run_deferred(m, x, T, nd, m.boff, [&](int b, int) { flip_warp(m, b, eps, T.lane); });
             T.sync();
         }
-        if (*m.nfix > 0) {
-            settle(m, T, nullptr, 0);
-            T.sync();
-        }
     }
-    if (PART & TAIL_FIX) fix_lists(m, T, S, false, nullptr, nullptr);
     if (PART & TAIL_END) {
+        fix_lists(m, T, S, nullptr, 0, false, nullptr, nullptr);
         /* the counts were zeroed before the last sync unless no candidate
          * made one necessary */
         if (na == 0) T.sync();
@@ -1412,6 +1493,31 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
         T.sync();
         pack_summary(m, x, summary, T.tid, T.n);
     }
+}
+
+/* edit_grains over the whole GPU, after the removals (REMOVED) or the
+ * flips; the clearing of the mods is left to the next kernel, TAIL_FLIP or
+ * k_update.  With 70 removals and 50 flips a step (100K grains) some 300
+ * grains are edited after each, with 200 and 350 (400K grains) some 1,000,
+ * and the cluster's sixteen SMs took 60 and 93 thousand cycles over the
+ * first, 60 and 110 over the second, bound by their FP64 pipes and by the
+ * rounds of 256 warps; a launch costs some 3. */
+constexpr int EDIT_TPB = 256;
+template <bool REMOVED>
+__global__ void __launch_bounds__(EDIT_TPB) k_edit(DevMesh m, DevScratch x)
+{
+    griddep_wait();
+    __shared__ EditShared<EDIT_TPB / 32> S;
+    const Team T;
+    edit_grains(m, T, S, x.list_c, REMOVED ? *x.n_c : 0, REMOVED, nullptr, nullptr);
+}
+/* the position update and the rest of the flips' fix-up */
+__global__ void __launch_bounds__(TPB) k_update(DevMesh m, double dt)
+{
+    griddep_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < m.nv) update_vertex(m, t, dt);
+    clear_mods(m, t, gridDim.x * blockDim.x);
 }
 
 /* instance of every boundary and grain from the offset tables */
@@ -1470,19 +1576,21 @@ void launch_two_three_first(const DevMesh &m, const DevScratch &x, cudaStream_t 
 bool tail_whole(const DevMesh &m) { return m.nv <= TAIL_WHOLE_NV; }
 void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s)
 {
-    launch_tail_part<TAIL_REMOVE | TAIL_FLIP | TAIL_FIX | TAIL_END>(m, x, p, cap, summary, s);
+    launch_tail_part<TAIL_REMOVE | TAIL_FLIP | TAIL_END>(m, x, p, cap, summary, s);
 }
 void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s)
 {
     launch_tail_part<TAIL_REMOVE>(m, x, p, cap, nullptr, s);
+    launch_dep(k_edit<true>, WL_BLOCKS, EDIT_TPB, s, m, x);
 }
 void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
     launch_tail_part<TAIL_FLIP>(m, x, p, 0, nullptr, s);
+    launch_dep(k_edit<false>, WL_BLOCKS, EDIT_TPB, s, m, x);
 }
-void launch_tail_fix(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
+void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s)
 {
-    launch_tail_part<TAIL_FIX>(m, x, p, 0, nullptr, s);
+    launch_dep(k_update, (m.nv + TPB - 1) / TPB, TPB, s, m, dt);
 }
 
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s)
