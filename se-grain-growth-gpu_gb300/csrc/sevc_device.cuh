@@ -583,14 +583,20 @@ __device__ __forceinline__ int gintersect(int4 a, int4 b, int *out)
  * transcendental (1 + 0.5 * 0 * (1 - cos^3) is exactly 1 for every finite
  * cosine).  False (energy unset) when the ends share fewer than two
  * grains. */
-__device__ __forceinline__ bool boundary_gamma(const DevMesh &m, int b, double eps, double scaling, double &gamma)
+template <class Energy>
+__device__ __forceinline__ bool boundary_gamma(const DevMesh &m, int b, double eps, double scaling, double &gamma,
+                                               Energy energy)
 {
     if (eps == 0.0) { gamma = 1.0 * scaling; return true; }
     int2 e = m.bv[b];
     int gic[2];
     if (gintersect(m.vg[e.x], m.vg[e.y], gic) < 2) return false;
-    gamma = gb_energy(m.gori[gic[0]] - m.gori[gic[1]], eps) * scaling;
+    gamma = energy(m.gori[gic[0]] - m.gori[gic[1]], eps) * scaling;
     return true;
+}
+__device__ __forceinline__ bool boundary_gamma(const DevMesh &m, int b, double eps, double scaling, double &gamma)
+{
+    return boundary_gamma(m, b, eps, scaling, gamma, gb_energy);
 }
 /* grains_union + grains_symdiff, src/geometry.h:863-898 */
 __device__ __forceinline__ void gsymdiff(int4 a, int4 b, int *out)

@@ -44,37 +44,54 @@ __global__ void k_rng_draw(curandState *st, int n, int ndraws, double *out)
     st[tid] = s;
 }
 
+/* the enabled ones of vertices v, v + GRID, ... v + 7 GRID below n, one bit
+ * each (eight loads in flight) */
+__device__ __forceinline__ unsigned alive8(const DevMesh &m, int vo, int v, int n)
+{
+    unsigned f = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        if (v + j * GRID < n) f |= m.ven[vo + v + j * GRID] ? 1u << j : 0u;
+    return f;
+}
 /* compute_nucleation_factor's draws + get_vertex_id_per_block
  * (src/nucleation2.cu:239-363), on the reference's 32x256 grid; blockIdx.y
- * is the instance, whose own 8192 streams walk its own vertex indices */
+ * is the instance, whose own 8192 streams walk its own vertex indices.
+ * The selection (:342-358) as one thread's loop of 256 intervals took up to
+ * 80,000 cycles, more than all the rest. */
 __global__ void __launch_bounds__(NTHR) k_nucl_blocks(DevMesh m, curandState *rng, curandState *saved, int *buf,
                                                      const int *nucl_on)
 {
-    __shared__ int alive[NTHR], pick[NTHR], nst[NTHR], stot;
-    __shared__ double share[NTHR];
+    __shared__ int pick[NTHR], nst[NTHR], stot, first;
+    __shared__ double share[NTHR], before[NTHR], draw;
     int inst = blockIdx.y;
     if (!nucl_on[inst]) return;
     int vo = m.voff[inst], nvi = m.voff[inst + 1] - vo;
     rng += (size_t)inst * GRID;
     saved += (size_t)inst * GRID;
     buf += NUCL_BUF * inst;
-    if (threadIdx.x == 0) stot = 0;
+    if (threadIdx.x == 0) { stot = 0; first = NTHR; }
     int tid = blockIdx.x * NTHR + threadIdx.x;
     curandState s = rng[tid];
     saved[tid] = s;
     int n_alive = 0;
-    for (int v = tid; v < nvi; v += GRID) n_alive += m.ven[vo + v] ? 1 : 0;
+    for (int v = tid; v < nvi; v += 8 * GRID) {
+        const unsigned f = alive8(m, vo, v, nvi);
+        n_alive += __popc(f);
+    }
     for (int k = 0; k < 2 * n_alive; k++) (void)curand_uniform_double(&s);
-    alive[threadIdx.x] = n_alive;
     int rid = -1, rid_k = -1;   /* the pick and its rank among the stream's enabled vertices */
     if (n_alive > 0) {
         int n_steps = (int)(curand_uniform_double(&s) * (n_alive - 1));
         int k = 0;
-        for (int v = tid; v < nvi; v += GRID)
-            if (m.ven[vo + v]) {
-                if (k == n_steps) { rid = vo + v; rid_k = k; break; }
-                k++;
-            }
+        for (int v = tid; v < nvi; v += 8 * GRID) {
+            unsigned f = alive8(m, vo, v, nvi);
+            const int c = __popc(f);
+            if (k + c <= n_steps) { k += c; continue; }
+            for (; k < n_steps; k++) f &= f - 1;
+            if (f) { rid = vo + v + GRID * (__ffs((int)f) - 1); rid_k = n_steps; }
+            break;
+        }
     }
     pick[threadIdx.x] = rid;
     nst[threadIdx.x] = rid_k;
@@ -82,41 +99,48 @@ __global__ void __launch_bounds__(NTHR) k_nucl_blocks(DevMesh m, curandState *rn
     atomicAdd(&stot, n_alive);                   /* integers: the same sum in any order */
     __syncthreads();
     const int tot = stot;
-    /* each thread's share alive[i] / tot, the quotient the selection below
-     * compares against (computed once per thread instead of one after
-     * another by thread 0) */
-    share[threadIdx.x] = tot > 0 ? alive[threadIdx.x] / (double)tot : 0.0;
+    /* each thread's share alive[i] / tot, and the running sum before it; the
+     * pick is the first thread whose interval holds the draw.  Only the sum
+     * has an order: thread 0 adds, every thread tests its own interval. */
+    share[threadIdx.x] = tot > 0 ? n_alive / (double)tot : 0.0;
+    __syncthreads();
+    if (threadIdx.x == 0 && tot > 0) {
+        draw = curand_uniform_double(&s);
+        double pc = 0.0;
+#pragma unroll 16
+        for (int i = 0; i < NTHR; i++) {
+            before[i] = pc;
+            pc += share[i];
+        }
+    }
+    __syncthreads();
+    if (tot > 0) {
+        const double pc = before[threadIdx.x], p = draw;
+        if (rid != -1 && pc <= p && p < (pc + share[threadIdx.x])) atomicMin(&first, (int)threadIdx.x);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (tot > 0) {
-            double p = curand_uniform_double(&s);
-            double pc = 0.0;
-            int kk = nst[0];
-            for (int i = 0; i < NTHR; i++) {
-                if (pick[i] != -1 && pc <= p && p < (pc + share[i])) {
-                    pick[0] = pick[i];
-                    kk = nst[i];
-                    break;
-                }
-                pc += share[i];
-            }
-            buf[blockIdx.x] = pick[0];
-            buf[NBLK + blockIdx.x] = tot;
-            buf[2 * NBLK + blockIdx.x] = kk;
-        } else {
-            buf[blockIdx.x] = -1;
-            buf[NBLK + blockIdx.x] = 0;
-            buf[2 * NBLK + blockIdx.x] = -1;
-        }
+        const int i = first < NTHR ? first : 0;
+        buf[blockIdx.x] = tot > 0 ? pick[i] : -1;
+        buf[NBLK + blockIdx.x] = tot;
+        buf[2 * NBLK + blockIdx.x] = tot > 0 ? nst[i] : -1;
     }
     rng[tid] = s;
 }
 
 struct NuclGeo {
-    double2 Apos, Bpos, Cpos;
+    double2 out;                 /* this lane's corner */
     int D, E, F, AD, AE, AF, g1, g2, g3;
     double DeltaE;
 };
+/* gb_energy as a call: where it runs once per launch, fetching its code
+ * (pow, cos) is most of its time.  Isotropic: exactly 1 (see
+ * boundary_gamma). */
+__device__ __noinline__ double energy_call(double d_alpha, double eps)
+{
+    if (eps == 0.0 && isfinite(d_alpha)) return 1.0;
+    return gb_energy(d_alpha, eps);
+}
 
 /* 3-point compute_area (src/geometry.h:757) */
 __device__ double area3(double2 a, double2 b, double2 c, double D)
@@ -132,21 +156,30 @@ __device__ double area3(double2 a, double2 b, double2 c, double D)
     return area;
 }
 
-/* generate_grain_for_nucleation, src/nucleation2.cu:116-212 */
+/* generate_grain_for_nucleation, src/nucleation2.cu:116-212, by one warp:
+ * lane 3 s + k has corner k (A, B, C), the side and the area from corner
+ * k - 1 to it, and the energy against grain k, without (s = 0) and with
+ * (s = 1) the scaling; gam is the energy of A's k-th boundary.  Sums are
+ * formed in the reference's order.  One thread ran this three times over, each
+ * time through newly fetched code: 105,000 cycles an attempt (187,000 with
+ * anisotropic energies) for what takes the six lanes 20,000-40,000. */
 __device__ int gen_triangle(const DevMesh &m, int A, double nucl_r, double nucl_ori, double eps, double scaling,
-                            bool do_scale, const double *gam3, NuclGeo &o)
+                            double gam, int lane, NuclGeo &o)
 {
-    double D = m.D;
-    int4 sa = m.vb[A];
+    const unsigned all = 0xffffffffu;
+    const double D = m.D;
+    const int k = lane % 3, base = lane - k;
+    const bool scale = (lane / 3) & 1;
+    const int4 sa = m.vb[A], ga = m.vg[A];
     o.AD = sa.x; o.AE = sa.y; o.AF = sa.z;
-    o.D = other_end(m.bv[o.AD], A);
-    o.E = other_end(m.bv[o.AE], A);
-    o.F = other_end(m.bv[o.AF], A);
-    int gAD[2], gAE[2], gAF[2];
-    int4 ga = m.vg[A];
-    gintersect(ga, m.vg[o.D], gAD);
-    gintersect(ga, m.vg[o.E], gAE);
-    gintersect(ga, m.vg[o.F], gAF);
+    const int far = other_end(m.bv[slot3(sa, k)], A);
+    o.D = __shfl_sync(all, far, 0);
+    o.E = __shfl_sync(all, far, 1);
+    o.F = __shfl_sync(all, far, 2);
+    int gk[2];
+    gintersect(ga, m.vg[far], gk);
+    const int gAD[2] = { __shfl_sync(all, gk[0], 0), __shfl_sync(all, gk[1], 0) };
+    const int gAE[2] = { __shfl_sync(all, gk[0], 1), __shfl_sync(all, gk[1], 1) };
     if (gAD[0] == gAE[0] || gAD[0] == gAE[1]) { o.g2 = gAD[0]; o.g1 = gAD[1]; }
     else if (gAD[1] == gAE[0] || gAD[1] == gAE[1]) { o.g2 = gAD[1]; o.g1 = gAD[0]; }
     else return -1;
@@ -154,34 +187,24 @@ __device__ int gen_triangle(const DevMesh &m, int A, double nucl_r, double nucl_
     else if (gAE[1] == o.g2) o.g3 = gAE[0];
     else return -1;
     if (o.g1 < 0 || o.g2 < 0 || o.g3 < 0) return -1;
-    double2 pa = m.pos[A];
-    int far[3] = { o.D, o.E, o.F };
-    double2 out[3];
-    for (int k = 0; k < 3; k++) {
-        double2 q = m.pos[far[k]];
-        double tx = wrapd(q.x, pa.x, D), ty = wrapd(q.y, pa.y, D);
-        double w = nucl_r / vmag(tx, ty);
-        if (do_scale) w *= 0.99;
-        double2 r = make_double2(w * tx + pa.x, w * ty + pa.y);
-        r.x = dmod(r.x, D);
-        r.y = dmod(r.y, D);
-        out[k] = r;
-    }
-    o.Apos = out[0]; o.Bpos = out[1]; o.Cpos = out[2];
-    double LAB = arclen(o.Apos, o.Bpos, D), LBC = arclen(o.Bpos, o.Cpos, D), LCA = arclen(o.Cpos, o.Apos, D);
-    double A1 = area3(pa, o.Cpos, o.Apos, D);
-    double A2 = area3(pa, o.Apos, o.Bpos, D);
-    double A3 = area3(pa, o.Bpos, o.Cpos, D);
-    double E0 = 0.0, E1 = 0.0;
-    for (int i = 0; i < 3; i++) {
-        double gam = gam3[i];   /* the energy of A's i-th boundary this step */
-        if (do_scale) E0 += 0.99 * nucl_r * gam;
-        else E0 += nucl_r * gam;
-    }
-    E0 += A1 * m.gse[o.g1] + A2 * m.gse[o.g2] + A3 * m.gse[o.g3];
-    E1 = gb_energy(nucl_ori - m.gori[o.g1], eps) * scaling * LCA;
-    E1 += gb_energy(nucl_ori - m.gori[o.g2], eps) * scaling * LAB;
-    E1 += gb_energy(nucl_ori - m.gori[o.g3], eps) * scaling * LBC;
+    const double2 pa = m.pos[A], q = m.pos[far];
+    const double tx = wrapd(q.x, pa.x, D), ty = wrapd(q.y, pa.y, D);
+    double w = nucl_r / vmag(tx, ty);
+    if (scale) w *= 0.99;
+    o.out = make_double2(dmod(w * tx + pa.x, D), dmod(w * ty + pa.y, D));
+    const int prev = base + (k + 2) % 3;
+    const double2 r = make_double2(__shfl_sync(all, o.out.x, prev), __shfl_sync(all, o.out.y, prev));
+    const double side = arclen(r, o.out, D), area = area3(pa, r, o.out, D);
+    const int g = k == 0 ? o.g1 : k == 1 ? o.g2 : o.g3;
+    const double e = energy_call(nucl_ori - m.gori[g], eps) * scaling * side;
+    const double l = scale ? 0.99 * nucl_r * gam : nucl_r * gam, a = area * m.gse[g];
+    double E0 = 0.0, E1;
+#pragma unroll
+    for (int i = 0; i < 3; i++) E0 += __shfl_sync(all, l, base + i);
+    E0 += __shfl_sync(all, a, base) + __shfl_sync(all, a, base + 1) + __shfl_sync(all, a, base + 2);
+    E1 = __shfl_sync(all, e, base);
+    E1 += __shfl_sync(all, e, base + 1);
+    E1 += __shfl_sync(all, e, base + 2);
     o.DeltaE = E1 - E0;
     return 0;
 }
@@ -245,14 +268,28 @@ __device__ void init_boundary_dev(const DevMesh &m, int b, int ini, int end) /* 
     m.bconf[b] = -1;
 }
 
+/* the lowest `want` (at most 3) indices of flags[lo..hi) that are 0, by one
+ * warp; -1 for those missing */
+__device__ __forceinline__ void lowest_free(const uint8_t *flags, int lo, int hi, int want, int lane, int *out)
+{
+    int n = 0;
+    for (int base = lo; base < hi && n < want; base += 32) {
+        unsigned f = __ballot_sync(0xffffffffu, base + lane < hi && !flags[base + lane]);
+        for (; f && n < want; f &= f - 1) out[n++] = base + __ffs((int)f) - 1;
+    }
+    for (; n < want; n++) out[n] = -1;
+}
+
 /* get_vertex_id2 (:375-443), the chosen vertex's factor
  * (compute_nucleation_factor for that vertex), get_nucleation_ids (:33-72)
- * and nucleate (:474-676); one thread per instance */
-__global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *saved, const int *buf, int *ctr,
-                              const int *nucl_on, double eps, double scaling, double MC_k)
+ * and nucleate (:474-676); one warp per instance, every lane following the
+ * choices, lane 0 writing */
+__global__ void __launch_bounds__(32) k_nucl_finish(DevMesh m, curandState *rng, const curandState *saved, const int *buf,
+                                                    int *ctr, const int *nucl_on, double eps, double scaling, double MC_k)
 {
-    int inst = blockIdx.x * blockDim.x + threadIdx.x;
-    if (inst >= m.ninst || !nucl_on[inst]) return;
+    const unsigned all = 0xffffffffu;
+    const int inst = blockIdx.x, lane = threadIdx.x;
+    if (!nucl_on[inst]) return;
     int vo = m.voff[inst], v_end = m.voff[inst + 1];
     int bo = m.boff[inst], b_end = m.boff[inst + 1];
     int go = m.goff[inst], g_end = m.goff[inst + 1];
@@ -261,23 +298,36 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
     buf += NUCL_BUF * inst;
     ctr += (size_t)inst * CTR_COUNT;
     int *nlist = m.nlist + go, *nnlist = m.nnlist + inst;
-    int tot = 0;
-    for (int i = 0; i < NBLK; i++) tot += buf[NBLK + i];
+    /* lane i: the reference's block i */
+    static_assert(NBLK == 32, "a lane per block");
+    const int bpick = buf[lane], balive = buf[NBLK + lane], brank = buf[2 * NBLK + lane];
+    const int tot = __reduce_add_sync(all, balive);
     curandState s0 = rng[0];
-    double p = curand_uniform_double(&s0);
-    double pc = 0.0, pn = 0.0;
     int cand = ctr[CTR_CANDIDATE], kpick = -1;
+    __syncwarp();                                  /* the state and the candidate are read before lane 0 writes them */
+    double p = curand_uniform_double(&s0);
+    const double pn = ((double)balive) / tot;
+    double pc = 0.0, mine = 0.0;
     for (int i = 0; i < NBLK; i++) {
-        pn = ((double)buf[NBLK + i]) / tot;
-        if (buf[i] != -1 && pc < p && p <= (pc + pn)) { cand = buf[i]; kpick = buf[2 * NBLK + i]; break; }
-        pc += pn;
+        if (i == lane) mine = pc;
+        pc += __shfl_sync(all, pn, i);
+    }
+    const unsigned hit = __ballot_sync(all, bpick != -1 && mine < p && p <= (mine + pn));
+    if (hit) {
+        cand = __shfl_sync(all, bpick, __ffs((int)hit) - 1);
+        kpick = __shfl_sync(all, brank, __ffs((int)hit) - 1);
     }
     int v = cand;
+    auto fail = [&](int err) {
+        if (lane == 0) {
+            raise_err(m, err);
+            ctr[CTR_CANDIDATE] = -1;
+            rng[0] = s0;
+        }
+    };
     if (v < vo || v >= v_end || !m.ven[v]) {
         /* the reference would read a stale or out-of-range vertex here */
-        raise_err(m, ERRB_RNG);
-        ctr[CTR_CANDIDATE] = -1;
-        rng[0] = s0;
+        fail(ERRB_RNG);
         return;
     }
     /* the two draws compute_nucleation_factor made for v: v is the k-th
@@ -287,7 +337,8 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
     int t = (v - vo) % GRID, k = kpick;
     if (k < 0) {
         k = 0;
-        for (int u = vo + t; u < v; u += GRID) k += m.ven[u] ? 1 : 0;
+        for (long long u = (long long)vo + t + (long long)GRID * lane; u < v; u += 32 * GRID) k += m.ven[u] ? 1 : 0;
+        k = __reduce_add_sync(all, k);
     }
     curandState s = saved[t];
     for (int j = 0; j < 2 * k; j++) (void)curand_uniform_double(&s);
@@ -297,34 +348,31 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
      * (compute_boundaries_lengths / _energies, src/main.cu:124-130, run on
      * every boundary before the attempt in the reference; only v's three
      * are read, so they are computed here, with the same arithmetic as
-     * the step's boundary pass that follows) */
-    int4 sb = m.vb[v];
-    double AL[3], gam3[3];
-    for (int i = 0; i < 3; i++) {
-        int b = slot3(sb, i);
-        int2 e = m.bv[b];
-        AL[i] = arclen(m.pos[e.x], m.pos[e.y], m.D);
-        if (!boundary_gamma(m, b, eps, scaling, gam3[i])) {
-            raise_err(m, ERRB_TOPOLOGY);
-            ctr[CTR_CANDIDATE] = -1;
-            rng[0] = s0;
-            return;
-        }
-    }
-    double mn = AL[0];
-    int imin = 0;
-    for (int i = 0; i < 3; i++) if (mn > AL[i]) { mn = AL[i]; imin = i; }   /* min(), src/geometry.h:116 */
-    double nucl_r = 0.8 * mn * u1 + 0.1;
-    double nucl_ori = 2 * M_PI * u2;
-    NuclGeo o0, o1;
-    if (gen_triangle(m, v, nucl_r, nucl_ori, eps, scaling, false, gam3, o0) ||
-        gen_triangle(m, v, nucl_r, nucl_ori, eps, scaling, true, gam3, o1)) {
-        raise_err(m, ERRB_TOPOLOGY);
-        ctr[CTR_CANDIDATE] = -1;
-        rng[0] = s0;
+     * the step's boundary pass that follows): lane 3 j + i has the i-th */
+    const int4 sb = m.vb[v];
+    const int vbnd = slot3(sb, lane % 3);
+    const int2 vends = m.bv[vbnd];
+    const double len = arclen(m.pos[vends.x], m.pos[vends.y], m.D);
+    double gam = 0.0;
+    const bool joined = boundary_gamma(m, vbnd, eps, scaling, gam, energy_call);
+    if (!__all_sync(all, joined)) {
+        fail(ERRB_TOPOLOGY);
         return;
     }
-    double DeltaE = o0.DeltaE, factor = o0.DeltaE - o1.DeltaE;
+    double mn = __shfl_sync(all, len, 0);
+    int imin = 0;
+    for (int i = 0; i < 3; i++) {                                         /* min(), src/geometry.h:116 */
+        const double x = __shfl_sync(all, len, i);
+        if (mn > x) { mn = x; imin = i; }
+    }
+    double nucl_r = 0.8 * mn * u1 + 0.1;
+    double nucl_ori = 2 * M_PI * u2;
+    NuclGeo o;
+    if (gen_triangle(m, v, nucl_r, nucl_ori, eps, scaling, gam, lane, o)) {
+        fail(ERRB_TOPOLOGY);
+        return;
+    }
+    const double DeltaE = __shfl_sync(all, o.DeltaE, 0), factor = DeltaE - __shfl_sync(all, o.DeltaE, 3);
     bool nucl = false;
     if (DeltaE < 0) nucl = true;
     else if (factor < 0) {
@@ -332,26 +380,30 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
         double thr = exp(-MC_k * DeltaE);
         if (q < thr) nucl = true; else cand = -1;
     } else cand = -1;
-    ctr[CTR_CANDIDATE] = cand;
-    rng[0] = s0;
+    if (lane == 0) {
+        ctr[CTR_CANDIDATE] = cand;
+        rng[0] = s0;
+    }
     if (cand < 0 || !nucl) return;
 
     /* get_nucleation_ids: lowest free slots */
-    int gfree = -1, bfree[3] = { -1, -1, -1 }, vfree[2] = { -1, -1 };
-    for (int i = go; i < g_end; i++) if (!m.gen[i]) { gfree = i; break; }
-    for (int i = bo, f = 0; i < b_end && f < 3; i++) if (!m.ben[i]) bfree[f++] = i;
-    for (int i = vo, f = 0; i < v_end && f < 2; i++) if (!m.ven[i]) vfree[f++] = i;
+    int gfree[1], bfree[3], vfree[2];
+    lowest_free(m.gen, go, g_end, 1, lane, gfree);
+    lowest_free(m.ben, bo, b_end, 3, lane, bfree);
+    lowest_free(m.ven, vo, v_end, 2, lane, vfree);
+    /* nucleate's triangle is the scaled one (the reference passes it (scaling,
+     * eps) swapped, which changes only the unused energy) */
+    const double2 Apos = make_double2(__shfl_sync(all, o.out.x, 3), __shfl_sync(all, o.out.y, 3));
+    const double2 Bpos = make_double2(__shfl_sync(all, o.out.x, 4), __shfl_sync(all, o.out.y, 4));
+    const double2 Cpos = make_double2(__shfl_sync(all, o.out.x, 5), __shfl_sync(all, o.out.y, 5));
+    if (lane != 0) return;
     bool diff_vrt = vfree[0] != vfree[1];
     bool diff_bnd = bfree[0] != bfree[1] && bfree[1] != bfree[2] && bfree[2] != bfree[0];
-    if (!diff_bnd || !diff_vrt || gfree == -1) return;      /* :496-499 */
+    if (!diff_bnd || !diff_vrt || gfree[0] == -1) return;      /* :496-499 */
     if (vfree[1] < 0 || bfree[2] < 0) { raise_err(m, ERRB_CAPACITY); return; }
 
     int A = v, B = vfree[0], C = vfree[1];
-    int AB = bfree[0], BC = bfree[1], CA = bfree[2], g = gfree;
-    /* the reference passes (scaling, eps) swapped here; only the unused
-     * energy changes */
-    NuclGeo o;
-    if (gen_triangle(m, A, nucl_r, nucl_ori, scaling, eps, true, gam3, o)) { raise_err(m, ERRB_TOPOLOGY); return; }
+    int AB = bfree[0], BC = bfree[1], CA = bfree[2], g = gfree[0];
     {   /* the triangle's position map, for an adjoint replay */
         EventRec r0, r1;
         r0.type = EV_NUCL; r0.a = A; r0.b = B; r0.c = C;
@@ -360,9 +412,9 @@ __global__ void k_nucl_finish(DevMesh m, curandState *rng, const curandState *sa
         r1.pa = m.pos[o.F]; r1.pb = make_double2(0.8 * u1, nucl_r); r1.pc = make_double2(imin, 0.0);
         log_event_pair(m, r0, r1);
     }
-    init_vertex_dev(m, B, o.Bpos);
-    init_vertex_dev(m, C, o.Cpos);
-    m.pos[A] = o.Apos;
+    init_vertex_dev(m, B, Bpos);
+    init_vertex_dev(m, C, Cpos);
+    m.pos[A] = Apos;
     m.vb[A] = make_int4(-1, -1, -1, -1);
     init_boundary_dev(m, AB, A, B);
     init_boundary_dev(m, BC, B, C);
@@ -417,7 +469,7 @@ void launch_rng_init(curandState *st, int n, cudaStream_t s)
 void launch_nucleation(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {
     COUNT_LAUNCHES(1), k_nucl_blocks<<<dim3(NBLK, p.ninst), NTHR, 0, s>>>(m, x.rng, x.rng_saved, x.nucl_buf, x.nucl_on);
-    COUNT_LAUNCHES(1), k_nucl_finish<<<(p.ninst + 31) / 32, 32, 0, s>>>(m, x.rng, x.rng_saved, x.nucl_buf, x.counters,
+    COUNT_LAUNCHES(1), k_nucl_finish<<<p.ninst, 32, 0, s>>>(m, x.rng, x.rng_saved, x.nucl_buf, x.counters,
                                                                       x.nucl_on, p.eps, p.scaling, p.MC_k);
 }
 
