@@ -118,19 +118,96 @@ __device__ void rank_sort(const Team &T, const int *ids, int n, int *out)
 /* ------------------------------------------------------------------ */
 /* polling system, src/topological.h:362-578                           */
 /* ------------------------------------------------------------------ */
-/* vertices_vote (:362) for one vertex: its boundary with the smallest
- * extinction time among the candidates (the last such slot) */
-__device__ int vertex_vote(const DevMesh &m, int v)
+/* What the phases up to the removals read of a listed boundary's
+ * surroundings.  Polling and conflicts change flags, never the mesh, so each
+ * thread loads this for its first item when the kernel starts, the three kinds
+ * in different warps so that their chains of dependent loads (some 1,000
+ * cycles each) run side by side, and a phase is left with the loads of the
+ * flags it tests: 49,000 -> 25,000 cycles for polling and conflicts at 150
+ * candidates.  Items beyond the team's size load theirs as they come. */
+/* a flag of boundary b, 0 for an empty slot (phases read the slots' flags
+ * before they know whether they need them) */
+__device__ __forceinline__ uint8_t flag_at(const uint8_t *flags, int nb, int b)
 {
-    if (!m.ven[v]) return -1;
-    int4 sb = m.vb[v];
-    double mt = 99999999;
-    int am = 0;
-    for (int j = 0; j < 3; j++) {
-        int b = slot3(sb, j);
-        if (m.btext[b] <= mt && m.bcand[b]) { mt = m.btext[b]; am = j; }
+    return (unsigned)b < (unsigned)nb ? flags[b] : 0;
+}
+struct PollItem { int b, inst, en, buf; bool vi, ve; int4 si, se; };   /* a candidate, its ends' slots */
+struct ConfItem { int c, b; int4 si, se; };                    /* a candidate, a boundary beside it, its ends' slots */
+struct LabelItem { int b, g; };                                /* a candidate, a 3-sided grain on it (-1: none) */
+__device__ __forceinline__ PollItem poll_item(const DevMesh &m, const int *list, int i, int n)
+{
+    PollItem p;
+    p.b = i < n ? list[i] : -1;
+    p.inst = p.en = p.buf = 0;
+    p.vi = p.ve = false;
+    p.si = p.se = make_int4(-1, -1, -1, -1);
+    if (p.b >= 0) {
+        const int2 e = m.bv[p.b];
+        p.inst = m.binst[p.b];
+        p.en = m.ben[p.b];
+        p.buf = m.bcandbuf[p.b];
+        p.si = m.vb[e.x]; p.se = m.vb[e.y];
+        p.vi = m.ven[e.x]; p.ve = m.ven[e.y];
     }
-    return slot3(sb, am);
+    return p;
+}
+__device__ __forceinline__ ConfItem conf_item(const DevMesh &m, const int *list, int t, int n)
+{
+    ConfItem f;
+    f.c = f.b = -1;
+    f.si = f.se = make_int4(-1, -1, -1, -1);
+    if (t < 6 * n) {
+        const int i = t / 6, r = t - 6 * i, c = list[i];
+        const int2 e = m.bv[c];
+        const int b = slot3(m.vb[r < 3 ? e.x : e.y], r < 3 ? r : r - 3);
+        if (b != c && (unsigned)b < (unsigned)m.nb) {
+            const int2 w = m.bv[b];
+            f.c = c;
+            f.b = b;
+            if ((unsigned)w.x < (unsigned)m.nv) f.si = m.vb[w.x];
+            if ((unsigned)w.y < (unsigned)m.nv) f.se = m.vb[w.y];
+        }
+    }
+    return f;
+}
+__device__ __forceinline__ LabelItem label_item(const DevMesh &m, const int *list, int t, int n)
+{
+    LabelItem l;
+    l.b = l.g = -1;
+    if (t < 3 * n) {
+        const int i = t / 3, j = t - 3 * i, b = list[i];
+        const int2 e = m.bv[b];
+        const int4 ga = m.vg[e.x], gb = m.vg[e.y];
+        const int g = slot3(ga, j);
+        const bool first = !(j > 0 && g == ga.x) && !(j > 1 && g == ga.y);
+        if ((unsigned)g < (unsigned)m.ng && first && (g == gb.x || g == gb.y || g == gb.z)) {
+            const int len = m.gvlen[g];
+            if (m.ben[b] && m.gen[g] && len == 3) { l.b = b; l.g = g; }
+        }
+    }
+    return l;
+}
+
+/* vertices_vote (:362) for one vertex (its slots sb; on: enabled): its
+ * boundary with the smallest extinction time among the candidates (the last
+ * such slot) */
+__device__ __forceinline__ int vertex_vote(const DevMesh &m, int4 sb, bool on)
+{
+    if (!on) return -1;
+    double t[3];
+    uint8_t c[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int b = slot3(sb, j);
+        c[j] = flag_at(m.bcand, m.nb, b);
+        t[j] = (unsigned)b < (unsigned)m.nb ? m.btext[b] : 0.0;
+    }
+    double mt = 99999999;
+    int am = sb.x;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+        if (t[j] <= mt && c[j]) { mt = t[j]; am = slot3(sb, j); }
+    return am;
 }
 
 /* One polling loop (:549-578) over the candidate list.  An iteration:
@@ -158,37 +235,43 @@ __device__ void poll_reset(const DevMesh &m, const DevScratch &x, const Team &T,
     for (int i = T.tid; i < m.ninst; i += T.n) x.pcnt[i] = 0;
     if (T.tid == 0) *x.n_fail = 0;
 }
-__device__ int poll_loop(const DevMesh &m, const DevScratch &x, const Team &T, const PollGrid &pg, int cap)
+__device__ int poll_loop(const DevMesh &m, const DevScratch &x, const Team &T, const PollGrid &pg, int cap, PollItem &first)
 {
     const int *list = x.list_a;
     const int n = *x.n_a;
+    auto item = [&](int i) { return i == T.tid ? first : poll_item(m, list, i, n); };
     for (int it = 1;; it++) {
         if (n > 0) {
+            bool two = false, done = false;          /* the first item's */
             for (int i = T.tid; i < n; i += T.n) {
-                int b = list[i];
-                if (!(m.ben[b] && m.bcand[b]) || m.pdone[m.binst[b]]) continue;
-                int2 e = m.bv[b];
-                m.bvotes[b] = vertex_vote(m, e.x) == b && vertex_vote(m, e.y) == b ? 2 : 0;
+                const PollItem p = item(i);
+                const uint8_t over = m.pdone[p.inst], c = m.bcand[p.b];
+                const int vi = vertex_vote(m, p.si, p.vi), ve = vertex_vote(m, p.se, p.ve);
+                if (i == T.tid) done = over;
+                if (!(p.en && c) || over) continue;
+                const bool v = vi == p.b && ve == p.b;
+                m.bvotes[p.b] = v ? 2 : 0;
+                if (i == T.tid) two = v;
             }
             T.sync();
             for (int i = T.tid; i < n; i += T.n) {
-                int b = list[i];
-                if (!(m.ben[b] && m.bcand[b] && m.bvotes[b] == 2) || m.pdone[m.binst[b]]) continue;
-                int2 e = m.bv[b];
-                int4 si = m.vb[e.x], se = m.vb[e.y];
+                const PollItem p = item(i);
+                if (i == T.tid ? !two : !(p.en && m.bcand[p.b] && m.bvotes[p.b] == 2) || m.pdone[p.inst]) continue;
+#pragma unroll
                 for (int j = 0; j < 3; j++) {
-                    int u = slot3(si, j), w = slot3(se, j);
-                    if (u != b) m.bcand[u] = 0;
-                    if (w != b) m.bcand[w] = 0;
+                    int u = slot3(p.si, j), w = slot3(p.se, j);
+                    if (u != p.b) m.bcand[u] = 0;
+                    if (w != p.b) m.bcand[w] = 0;
                 }
             }
             T.sync();
             for (int i = T.tid; i < n; i += T.n) {
-                int b = list[i];
-                if (m.pdone[m.binst[b]]) continue;
-                uint8_t en = m.ben[b], c = m.bcand[b];
-                if (en && c != m.bcandbuf[b]) poll_fail(m, x, pg, b);
-                m.bcandbuf[b] = en ? c : 0;
+                PollItem p = item(i);
+                if (i == T.tid ? done : m.pdone[p.inst] != 0) continue;
+                const uint8_t c = m.bcand[p.b];
+                if (p.en && c != p.buf) poll_fail(m, x, pg, p.b);
+                m.bcandbuf[p.b] = p.en ? c : 0;
+                if (i == T.tid) first.buf = p.en ? c : 0;
             }
             T.sync();
         }
@@ -196,16 +279,17 @@ __device__ int poll_loop(const DevMesh &m, const DevScratch &x, const Team &T, c
          * others see an instance it marks as done either way) */
         bool run = false;
         for (int i = threadIdx.x; i < m.ninst; i += blockDim.x) {
-            if (m.pdone[i]) continue;
-            bool again = x.pcnt[i] != 0;
+            const uint8_t over = m.pdone[i];
+            const bool again = x.pcnt[i] != 0;
+            if (over) continue;
             run |= again;
             if (blockIdx.x == 0) {
                 x.piters[i]++;
                 if (!again) m.pdone[i] = 1;
             }
         }
-        run = __syncthreads_or(run);
         const int nfail = *x.n_fail;
+        run = __syncthreads_or(run);
         if (run && it >= cap) {
             if (T.tid == 0) atomicOr(m.err, ERRB_NONCONVERGED);
             run = false;
@@ -220,62 +304,56 @@ __device__ int poll_loop(const DevMesh &m, const DevScratch &x, const Team &T, c
 /* ------------------------------------------------------------------ */
 /* conflicts, src/topological.h:83-155                                 */
 /* ------------------------------------------------------------------ */
-__device__ void conflict_check_one(const DevMesh &m, int b)
-{
-    if (!(m.ben[b] && !m.bcand[b])) return;
-    int2 e = m.bv[b];
-    int4 si = m.vb[e.x], se = m.vb[e.y];
-    int bi = -1, be = -1;
-    for (int j = 0; j < 3; j++) {
-        int x = slot3(si, j);
-        if (x != b && m.bcand[x]) { bi = x; break; }
-    }
-    for (int j = 0; j < 3; j++) {
-        int x = slot3(se, j);
-        if (x != b && m.bcand[x]) { be = x; break; }
-    }
-    if (bi >= 0 && be >= 0) {
-        double ti = m.btext[bi], te = m.btext[be];
-        int w;
-        if (ti == te) w = bi < be ? bi : be;
-        else w = ti < te ? bi : be;
-        /* b is reached from each candidate next to it and every visit writes
-         * the same w; the first writer (bconf was -1) counts the mark */
-        if (atomicExch(&m.bconf[b], w) == -1) atomicAdd(&m.evt[EVT_COUNT * m.binst[b] + EVT_CONFLICTS], 1);
-    }
-}
 /* check_conflictive_boundaries for every non-candidate boundary adjacent
  * to a candidate (the only ones it can mark); one thread per candidate and
  * slot of its ends, so the six neighbours' load chains run side by side
  * (every visit of a boundary writes the same winner) */
-__device__ void conflict_check(const DevMesh &m, const Team &T, const int *list, int n)
+__device__ void conflict_check(const DevMesh &m, const Team &T, const int *list, int n, const ConfItem &first)
 {
-    for (int t = T.tid; t < 6 * n; t += T.n) {
-        int i = t / 6, r = t - 6 * i;
-        int c = list[i];
-        if (!(m.ben[c] && m.bcand[c])) continue;
-        int2 e = m.bv[c];
-        int b = slot3(m.vb[r < 3 ? e.x : e.y], r < 3 ? r : r - 3);
-        if (b != c) conflict_check_one(m, b);
+    const int t0 = T.n - 1 - T.tid;
+    for (int t = t0; t < 6 * n; t += T.n) {
+        const ConfItem f = t == t0 ? first : conf_item(m, list, t, n);
+        if (f.b < 0) continue;
+        const uint8_t en = m.ben[f.b], cb = m.bcand[f.b], ec = m.ben[f.c], cc = m.bcand[f.c];
+        uint8_t ci[3], ce[3];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            ci[j] = flag_at(m.bcand, m.nb, slot3(f.si, j));
+            ce[j] = flag_at(m.bcand, m.nb, slot3(f.se, j));
+        }
+        if (!(ec && cc) || !(en && !cb)) continue;
+        int bi = -1, be = -1;
+#pragma unroll
+        for (int j = 2; j >= 0; j--) {                     /* the first of each end */
+            const int x = slot3(f.si, j), y = slot3(f.se, j);
+            if (x != f.b && ci[j]) bi = x;
+            if (y != f.b && ce[j]) be = y;
+        }
+        if (bi >= 0 && be >= 0) {
+            double ti = m.btext[bi], te = m.btext[be];
+            int w;
+            if (ti == te) w = bi < be ? bi : be;
+            else w = ti < te ? bi : be;
+            /* b is reached from each candidate next to it and every visit
+             * writes the same w; the first writer (bconf was -1) counts the
+             * mark */
+            if (atomicExch(&m.bconf[f.b], w) == -1) atomicAdd(&m.evt[EVT_COUNT * m.binst[f.b] + EVT_CONFLICTS], 1);
+        }
     }
 }
-__device__ void conflict_unlabel(const DevMesh &m, const Team &T, const int *list, int n)
+__device__ void conflict_unlabel(const DevMesh &m, const Team &T, const int *list, int n, const PollItem &first)
 {
     for (int i = T.tid; i < n; i += T.n) {
-        int b = list[i];
-        if (!(m.ben[b] && m.bcand[b])) continue;
-        int2 e = m.bv[b];
-        int4 si = m.vb[e.x], se = m.vb[e.y];
+        const PollItem p = i == T.tid ? first : poll_item(m, list, i, n);
+        const uint8_t c = m.bcand[p.b];
         bool drop = false;
+#pragma unroll
         for (int j = 0; j < 3; j++) {
-            int x = slot3(si, j);
-            if (b != x && m.bconf[x] != -1) { if (m.bconf[x] != b) { drop = true; break; } }
+            const int u = slot3(p.si, j), w = slot3(p.se, j);
+            const int fu = (unsigned)u < (unsigned)m.nb ? m.bconf[u] : -1, fw = (unsigned)w < (unsigned)m.nb ? m.bconf[w] : -1;
+            drop |= (u != p.b && fu != -1 && fu != p.b) || (w != p.b && fw != -1 && fw != p.b);
         }
-        for (int j = 0; j < 3; j++) {
-            int x = slot3(se, j);
-            if (b != x && m.bconf[x] != -1) { if (m.bconf[x] != b) { drop = true; break; } }
-        }
-        if (drop) m.bcand[b] = 0;
+        if (p.en && c && drop) m.bcand[p.b] = 0;
     }
 }
 
@@ -785,23 +863,21 @@ __device__ bool remove_planned(const DevMesh &m, int grn, double nAB, double nBC
  * own grain, so the set is known up front.  A removable grain has an
  * enabled boundary with 0 <= t_ext <= dt, so it lies beside a boundary of
  * the candidate list: one thread per listed boundary and grain at its first
- * end; the grain is listed by its lowest such boundary. */
-__device__ void label3_reserve(const DevMesh &m, const DevScratch &x, const Team &T, int na, double dt)
+ * end; the grain is listed by its lowest such boundary.  first: this thread's
+ * first item, null if the mesh has changed since it was loaded. */
+__device__ __forceinline__ int label_start(const Team &T) { return T.tid < T.n / 2 ? T.tid + T.n / 2 : T.tid - T.n / 2; }
+__device__ void label3_reserve(const DevMesh &m, const DevScratch &x, const Team &T, int na, double dt,
+                               const LabelItem *first)
 {
     const unsigned ep = 2u * *m.stamp;
-    for (int t = T.tid; t < 3 * na; t += T.n) {
-        int i = t / 3, j = t - 3 * i, b = x.list_a[i];
-        if (!m.ben[b]) continue;
-        int2 e = m.bv[b];
-        int4 ga = m.vg[e.x], gb = m.vg[e.y];
-        int g = slot3(ga, j);
-        if (!valid_g(m, g) || (j > 0 && g == ga.x) || (j > 1 && g == ga.y)) continue;
-        if (g != gb.x && g != gb.y && g != gb.z) continue;
-        if (!m.gen[g] || m.gvlen[g] != 3) continue;
+    const int t0 = label_start(T);
+    for (int t = t0; t < 3 * na; t += T.n) {
+        const LabelItem l = t == t0 && first ? *first : label_item(m, x.list_a, t, na);
+        if (l.g < 0) continue;
         int L[3], bs[9];
-        if (label3_first(m, g, dt, L, bs) != b) continue;
-        x.list_c[atomicAdd(x.n_c, 1)] = g;
-        const unsigned long long key = resv_key(ep, g);
+        if (label3_first(m, l.g, dt, L, bs) != l.b) continue;
+        x.list_c[atomicAdd(x.n_c, 1)] = l.g;
+        const unsigned long long key = resv_key(ep, l.g);
 #pragma unroll
         for (int k = 0; k < 3; k++) reserve_vertex(m, x, L[k], make_int4(bs[3 * k], bs[3 * k + 1], bs[3 * k + 2], -1), key);
     }
@@ -1480,17 +1556,21 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
     if (PART & TAIL_END)
         for (int i = T.tid; i < m.ninst; i += T.n) x.counters[(size_t)i * CTR_COUNT + CTR_NGRAINS] = 0;
     if (PART & TAIL_REMOVE) {
-        const int nfail = poll_loop(m, x, T, pg, cap);
+        PollItem pi = poll_item(m, x.list_a, T.tid, na);
+        const ConfItem ci = conf_item(m, x.list_a, T.n - 1 - T.tid, na);
+        const LabelItem li = label_item(m, x.list_a, label_start(T), na);
+        const int nfail = poll_loop(m, x, T, pg, cap, pi);
         if (na > 0 || nfail > 0) {
-            if (na > 0) conflict_check(m, T, x.list_a, na);
+            if (na > 0) conflict_check(m, T, x.list_a, na, ci);
             T.sync();
-            if (na > 0) conflict_unlabel(m, T, x.list_a, na);
+            if (na > 0) conflict_unlabel(m, T, x.list_a, na, pi);
             poll_reset(m, x, T, pg, nfail);
             T.sync();
         }
-        if (*x.n_b > 0) two_three_loop(m, x, T, S);
+        const bool pairs = *x.n_b > 0;
+        if (pairs) two_three_loop(m, x, T, S);
         if (na > 0) {
-            label3_reserve(m, x, T, na, dt);
+            label3_reserve(m, x, T, na, dt, pairs ? nullptr : &li);
             if (T.tid == 0) *x.n_ehits = 0;          /* the grains a 2x3 pass left with three sides */
             T.sync();
         }
