@@ -68,7 +68,8 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  * the shoelace terms and their running sum round, and those are formed in
  * the reference's order.  On 1M grains (domain 1000) about 0.4% of the
  * grains fail the certificate (next to an axis, where ulps are finer, or
- * across the wrap); they are walked vertex by vertex as written.
+ * across the wrap); their chains are formed as written, the slots of a block's together
+ * (moved_uncertified).
  *
  * What bounds it: the FP64 pipe (2 thread-operations per clock and SM, of
  * which independent chains reach 84%) together with the latency of the
@@ -93,12 +94,12 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  *                       one s are a prefix of the order), so that the lanes
  *                       of a warp run the same operations.
  * Afterwards a warp per grain takes the rest, vertex by vertex: grains of
- * `wide` or more sides or of fewer than 3, and the few whose moved chain
- * does not rejoin.
+ * `wide` or more sides or of fewer than 3, and those with a coordinate
+ * outside the domain or + eps in the next binade.
  *
  * Measured (GB300): 1M grains 0.385 ms, FP64 pipe active 69% of the
  * cycles, 21 of 32 lanes per FP64 instruction (slots of different s or p in
- * one warp); 2,000 grains 20 us.  The form before it (a grain per thread,
+ * one warp); 2,000 grains 18 us.  The form before it (a grain per thread,
  * polygon in registers, one unrolled body per side count, side-count order
  * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
  * took 0.50 ms and 95 us: on a small mesh each unrolled body runs once and
@@ -293,17 +294,62 @@ __device__ __forceinline__ int certify_axis(const double *r, int n, double D, lo
     return mh - ml <= (ml >> 1) + (ml >> 2) ? GP_CERT : GP_CHAIN;
 }
 
-/* The unwrapped coordinate of the moved vertex p > 0 of an uncertified
- * grain (raw coordinates: its own r, the neighbours' rm and rp; a the
- * unwrapped chain).  NaN (no certified value is one) when the chain does
- * not come back to the unmoved value at p + 1, bit for bit: the grain is
- * then walked vertex by vertex. */
-__device__ __noinline__ double chain_moved(const double *a, int p, int n, double r, double rm, double rp, double D)
+/* Twice the area with the vertex of slot q (not the grain's first) of an
+ * uncertified grain moved along axis x, up to its sign (see the moved areas
+ * of certified grains below): the chain is formed as the reference does from
+ * the moved vertex on, and when it does not come back to the unmoved value at
+ * the next vertex, bit for bit, it is walked to its end.  Some 10% of the
+ * grains of a 2,000-grain mesh are uncertified (next to the axes and across
+ * the wrap) and most of them have such a slot; a warp that walked all
+ * 2 n + 1 polygons of each, and chains formed among the certified slots, where
+ * a warp waits for one lane, made the pass of 64 meshes of that size (176,000
+ * grains) 171 us; their slots packed into whole warps make it 129 us. */
+template <int SLOTS>
+__device__ __forceinline__ double moved_uncertified(const DevMesh &m, const GrainChunk<SLOTS> &B, int q, int x)
 {
-    double mv = dmod(r + SEVC_GRAD_EPS_D, D), w = wrapd(mv, rm, D);
-    double x = p == 1 ? zero_plus(w) : a[p - 1] + w;
-    if (p < n - 1 && dbits(x + wrapd(rp, mv, D)) != dbits(a[p + 1])) return __longlong_as_double(0x7FF8000000000000LL);
-    return x;
+    const int i = B.owner[q], o = B.off[i], p = q - o, nn = B.n[i];
+    const double *F = B.A[x], *G = B.A[1 - x];
+    auto raw = [&](int k) { return reinterpret_cast<const double *>(m.pos + B.dest[k] / 3)[x]; };
+    const long long flip = x ? LLONG_MIN : 0;
+    auto sgn = [&](double v) { return __longlong_as_double(dbits(v) ^ flip); };
+    const double D = m.D, rm = raw(q - 1), mv = dmod(raw(q) + SEVC_GRAD_EPS_D, D), w = wrapd(mv, rm, D);
+    double r = raw(p < nn - 1 ? q + 1 : q);
+    const double f = p == 1 ? zero_plus(w) : F[q - 1] + w;
+    double a = 0;
+    if (p >= 2) {
+        a = B.Q[x][q - 1] - G[q - 1] * f;                      /* term p - 1 */
+        if (p > 2) a = sgn(B.M[0][q - 2]) + a;
+    }
+    if (p < nn - 1) {
+        double g = f + wrapd(r, mv, D);                        /* the next vertex's coordinate */
+        const bool joins = dbits(g) == dbits(F[q + 1]);
+        const double t2 = f * G[q + 1] - G[q] * g;             /* term p */
+        a = p == 1 ? t2 : a + t2;
+        for (int k = q + 1; k < o + nn - 1; k++) {
+            if (joins) {
+                a = a + sgn(B.T[k]);
+            } else {
+                const double s = raw(k + 1), h = g + wrapd(s, r, D);
+                a = a + (g * G[k + 1] - G[k] * h);
+                g = h;
+                r = s;
+            }
+        }
+    }
+    return a;
+}
+
+/* the listed slots (2 slot + axis); a call, so that its registers do not
+ * spill the certified slots' */
+template <int NT, int SLOTS>
+__device__ __noinline__ void moved_uncertified_all(const DevMesh &m, const GrainChunk<SLOTS> &B, const unsigned short *odd,
+                                                   int nodd)
+{
+    for (int t = threadIdx.x; t < nodd; t += NT) {
+        const int x = odd[t] & 1, q = odd[t] >> 1, i = B.owner[q];
+        const double a = moved_uncertified(m, B, q, x);
+        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), B.absA[i]);
+    }
 }
 
 template <int GPB, int NT, int SLOTS>
@@ -315,7 +361,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
     __shared__ unsigned char sides[GPB];
     __shared__ int cnt[GP_NMAX], start[GP_NMAX];
     __shared__ int first[GP_NMAX];             /* first[j]: first entry of B.moved (and B.inner) with s + 2 = j */
-    __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved, chains;
+    __shared__ int rest[GPB], nrest, listed, chunk, slots, nmoved, chains, nodd;
     __shared__ long long ntab[GP_E1 - GP_E0 + 1];
     constexpr int W = NT / 32;
     static_assert(GPB <= NT, "a thread per grain orders them");
@@ -420,7 +466,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
     }
     __syncthreads();
     /* per grain and axis: certificate */
-    if (tid == 0) chains = 0;
+    if (tid == 0) chains = nodd = 0;
     for (int t = tid; t < 2 * total; t += NT) {
         const int x = t >= total, i = x ? t - total : t;
         B.ok[x][i] = certify_axis(B.R[x] + B.off[i], B.n[i], m.D, dlim, B.c[x][i]);
@@ -510,6 +556,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
      * F[p-1] G[p] - G[p-1] f and f G[p+1] - G[p] F[p+1] for x, minus those
      * for y; along y the whole sum is formed with the opposite sign. */
     const int per_axis = (nmoved + 31) & ~31;         /* no warp works on both axes */
+    unsigned short *odd = reinterpret_cast<unsigned short *>(B.R[0]);   /* done with; 2 slot + axis */
     for (int t = tid; t < 2 * per_axis; t += NT) {
         const int x = t >= per_axis, w = x ? t - per_axis : t;
         if (w >= nmoved) continue;
@@ -519,21 +566,13 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
         double a;         /* twice the moved area */
         if (p == 0) {
             a = B.sum0[x][i];
+        } else if (st == GP_CHAIN) {
+            odd[atomicAdd(&nodd, 1)] = (unsigned short)(2 * q + x);
+            continue;
         } else {
             const double *F = B.A[x], *G = B.A[1 - x];
-            double f;
-            if (st == GP_CERT) {
-                const int e = B.c[x][i].e, up = (int)((B.c[x][i].up >> p) & 1u);
-                f = add_exact(F[q], ntab[e + up] << up, e + GP_E0);
-            } else {
-                const double2 rr = m.pos[B.dest[q] / 3], rm = m.pos[B.dest[q - 1] / 3];
-                const double2 rp = m.pos[B.dest[p < nn - 1 ? q + 1 : q] / 3];
-                f = x ? chain_moved(F + o, p, nn, rr.y, rm.y, rp.y, m.D) : chain_moved(F + o, p, nn, rr.x, rm.x, rp.x, m.D);
-                if (dbits(f) == 0x7FF8000000000000LL) {
-                    if (atomicExch(&B.ok[0][i], GP_REST) != GP_REST) rest[atomicAdd(&nrest, 1)] = B.sg[i];
-                    continue;
-                }
-            }
+            const int e = B.c[x][i].e, up = (int)((B.c[x][i].up >> p) & 1u);
+            const double f = add_exact(F[q], ntab[e + up] << up, e + GP_E0);
             const long long flip = x ? LLONG_MIN : 0;
             auto sgn = [&](double v) { return __longlong_as_double(dbits(v) ^ flip); };
             a = 0;
@@ -548,6 +587,10 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
             }
         }
         reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), B.absA[i]);
+    }
+    if (chains) {                              /* the uncertified grains' slots */
+        __syncthreads();
+        moved_uncertified_all<NT>(m, B, odd, nodd);
     }
     __syncthreads();
     }
@@ -807,7 +850,8 @@ void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape 
      * grain; 3% of the blocks need a second chunk) and 40 registers let
      * eleven in, 385 us against 397 with ten.  Below GRAIN_SMALL grains an SM
      * holds few blocks and the longest one is the time: eight warps and
-     * 288 slots, 20 us against 25 at 2,000 grains. */
+     * 288 slots, 20 us against 25 at 2,000 grains (before the uncertified grains'
+     * slots were packed). */
     if (sh.grain_occ < 6) go(k_grain_pass<64, 128, 208>, 64, 128);
     else if (m.ng < GRAIN_SMALL) go(k_grain_pass<32, 256, 288>, 32, 256);
     else go(k_grain_pass<32, 128, 208>, 32, 128);
