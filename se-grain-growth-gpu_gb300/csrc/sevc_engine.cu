@@ -926,8 +926,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     h->h_flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && h->n % o.snap_gap == 0);
     h->h_flags[2] = batch ? 0 : mg;   /* a batch does not stop at min_grains */
     h->h_flags[3] = h->curr_n_grains;
-    if (!cuda_ok(cudaMemcpyAsync(x.flags + 1, h->h_flags + 1, 3 * sizeof(int), cudaMemcpyHostToDevice, s), "upload"))
-        return SEVC_ERR_CUDA;
+    launch_set_flags(x, h->h_flags, s);
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
     if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
@@ -935,8 +934,8 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     /* one readback: counters, events, error bits, polling iterations and
      * 2x3 counts of every instance */
     int *hb = h->h_big;
-    if (!cuda_ok(cudaMemcpyAsync(hb, x.summary, summary_bytes(h), cudaMemcpyDeviceToHost, s), "readback") ||
-        !cuda_ok(cudaStreamSynchronize(s), "readback sync"))
+    launch_read_out(x.summary, hb, (int)(summary_bytes(h) / sizeof(int)), s);
+    if (!cuda_ok(cudaGetLastError(), "readback") || !cuda_ok(cudaStreamSynchronize(s), "readback sync"))
         return SEVC_ERR_CUDA;
     float ms = 0;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
@@ -1028,11 +1027,11 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         sl.flags[2] = batch ? 0 : mg;
         sl.flags[3] = h->curr_n_grains;   /* read only when min_grains > 0: not here */
         if (hooks) hooks->before(launched);
-        if ((n_on && !cuda_ok(cudaMemcpyAsync(x.nucl_on, sl.on, I * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) ||
-            !cuda_ok(cudaMemcpyAsync(x.flags + 1, sl.flags + 1, 3 * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) {
+        if (n_on && !cuda_ok(cudaMemcpyAsync(x.nucl_on, sl.on, I * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) {
             st = SEVC_ERR_CUDA;
             break;
         }
+        launch_set_flags(x, sl.flags, s);
         cudaEventRecord(sl.ev0, s);
         long long k0 = sevc_kernel_launches;
         h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
@@ -1053,7 +1052,8 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
             st = SEVC_ERR_CUDA;
             break;
         }
-        if (!cuda_ok(cudaMemcpyAsync(sl.big, x.summary, summary_bytes(h), cudaMemcpyDeviceToHost, s), "readback") ||
+        launch_read_out(x.summary, sl.big, (int)(summary_bytes(h) / sizeof(int)), s);
+        if (!cuda_ok(cudaGetLastError(), "readback") ||
             !cuda_ok(cudaEventRecord(sl.done, s), "event")) {
             st = SEVC_ERR_CUDA;
             break;

@@ -106,6 +106,10 @@ void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s);
 /* also lists the candidates and starts the polling's first comparison */
 void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
+/* the host's part of the output decision, flags[1..3], into x.flags; and n
+ * ints into pinned host memory, both in stream order */
+void launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s);
+void launch_read_out(const int *from, int *host, int n, cudaStream_t s);
 /* counters | events | error bits | polling iterations | 2x3 counts | output decision, into out */
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s);
 
