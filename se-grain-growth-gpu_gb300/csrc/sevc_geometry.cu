@@ -895,8 +895,11 @@ void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &
 }
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s)
 {
-    size_t total = (size_t)m.ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 5;
-    int g = (int)((total + TPB - 1) / TPB);
+    /* the exactness marks it zeroes, 16 at a time, outnumber the words it
+     * packs: with blocks for the words alone (one, on a single mesh) it took
+     * 17 us at 1M grains, with blocks for both 3 us */
+    size_t words = (size_t)m.ninst * (CTR_COUNT + EVT_COUNT + 1 + TWO_THREE_PASSES) + 5, marks = (size_t)m.ng / 16 + 1;
+    int g = (int)(((words > marks ? words : marks) + TPB - 1) / TPB);
     launch_dep(k_pack_summary, g < 152 ? g : 152, TPB, s, m, x, out);
 }
 
