@@ -396,18 +396,18 @@ KERNEL_BYTES = {
 }
 
 # DRAM bytes (read + write) per unit measured by ncu for each kernel phase on
-# the 200K-grain mesh (the ncu summaries of k_grain_fd_sorted and
+# the 200K-grain mesh (the ncu summaries of k_grain_pass and
 # k_vertex_fd under profiles/); traffic grows with the units processed, so
 # a full launch is scaled by its units.
 NCU_TRAFFIC_PER_UNIT = {
-    "grain_fd": (52.807e6 + 11.475e6) / 200000,
-    "vertex_fd": (50.061e6 + 0.945e6) / 400000,
+    "grain_fd": (45.263e6 + 1.599e6) / 200000,
+    "vertex_fd": (50.058e6 + 1.700e6) / 400000,
 }
 # FP64 pipe activity of the same captures (of elapsed cycles)
-NCU_FP64_ACTIVE = {"grain_fd": 0.557, "vertex_fd": 0.650}
+NCU_FP64_ACTIVE = {"grain_fd": 0.555, "vertex_fd": 0.684}
 # DADD + DMUL + DFMA thread instructions per unit, ncu counters on the
 # 200K-grain mesh (the FP64 instruction summary kept with the profiles)
-NCU_FP64_INST_PER_UNIT = {"grain_fd": (46.032e6 + 0.702e6) / 200000, "vertex_fd": 24.405e6 / 400000}
+NCU_FP64_INST_PER_UNIT = {"grain_fd": 22.010e6 / 200000, "vertex_fd": 24.405e6 / 400000}
 
 
 def run_engine(args):
@@ -552,8 +552,8 @@ def run_engine(args):
                    "launch_shapes": {"tpb_vertex": shapes[0], "tpb_boundary": shapes[1], "wide_sides": shapes[2],
                                      "grain_blocks_per_sm": shapes[3],
                                      "picked_by": "sevc_autotune, 10 steps per candidate"},
-                   "launch_mode": {"graph": "one CUDA graph per step (device-driven loops)",
-                                   "hostloops": "CUDA graphs of the step's fixed sequences, loops on the host",
+                   "launch_mode": {"graph": "one CUDA graph per step (loops inside its kernels)",
+                                   "hostloops": "as graph (kept for callers that select it)",
                                    "direct": "direct launches"}[args.launch]},
         "e2e": {"value": vs / e_wall, "unit": UNIT, "h2d_bytes_per_step": host_bytes / k,
                 "d2h_bytes_per_step": step_info_bytes + state_bytes / k,

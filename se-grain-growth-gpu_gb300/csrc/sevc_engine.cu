@@ -920,8 +920,8 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
         if (!cuda_ok(cudaMemcpyAsync(x.nucl_on, h->h_on, I * sizeof(int), cudaMemcpyHostToDevice, s), "upload"))
             return SEVC_ERR_CUDA;
     }
-    /* host part of the output decision (k_full_flag): steps that can export,
-     * long steps, exact_all, and every step of a batch */
+    /* host part of the output decision (k_two_three_first): steps that can
+     * export, long steps and exact_all */
     int mg = o.min_grains;
     h->h_flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && h->n % o.snap_gap == 0);
     h->h_flags[2] = batch ? 0 : mg;   /* a batch does not stop at min_grains */
