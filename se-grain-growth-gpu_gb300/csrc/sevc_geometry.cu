@@ -99,7 +99,7 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  *
  * Measured (GB300): 1M grains 0.385 ms, FP64 pipe active 69% of the
  * cycles, 21 of 32 lanes per FP64 instruction (slots of different s or p in
- * one warp); 2,000 grains 18 us.  The form before it (a grain per thread,
+ * one warp); 2,000 grains 16 us.  The form before it (a grain per thread,
  * polygon in registers, one unrolled body per side count, side-count order
  * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
  * took 0.50 ms and 95 us: on a small mesh each unrolled body runs once and
@@ -353,7 +353,7 @@ __device__ __noinline__ void moved_uncertified_all(const DevMesh &m, const Grain
 }
 
 template <int GPB, int NT, int SLOTS>
-__global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m, int *three, int *n_three, int wide, long long dlim)
+__global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMesh m, int *three, int *n_three, int wide, long long dlim)
 {
     __shared__ __align__(16) unsigned char smem[GrainSmem<NT, SLOTS>::bytes];
     GrainChunk<SLOTS> &B = *reinterpret_cast<GrainChunk<SLOTS> *>(smem);
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 11 : 1) k_grain_pass(DevMesh m
     GrainRest &Z = reinterpret_cast<GrainRest *>(smem)[warp];
     for (int q = warp; q < nrest; q += W) grain_by_warp(m, rest[q], Z.P, Z.R, lane);
 }
-constexpr int GRAIN_SMALL = 32 * 1024;   /* see launch_grain_pass */
+constexpr int GRAIN_TINY = 6 * 1024, GRAIN_SMALL = 32 * 1024;   /* see launch_grain_pass */
 
 /* vertex pass: src/calculus.h:19-73 (boundary part) and :143-154;
  * vertex_compute_energy src/geometry.h:472-479.
@@ -856,16 +856,18 @@ void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape 
     auto go = [&](auto kernel, int gpb, int nt) {
         COUNT_LAUNCHES(1), kernel<<<(m.ng + gpb - 1) / gpb, nt, 0, s>>>(m, x.three, x.n_three, wide, dlim);
     };
-    /* 32 grains a block at every size (blocks of 64 in two chunks: 414
-     * against 385 us at 1M grains, 67 against 62 at 100K; they stay for the
-     * autotuner).  Large meshes want blocks on the SM: 208 slots (6.5 per
+    /* Large meshes want blocks on the SM: 32 grains, 208 slots (6.5 per
      * grain; 3% of the blocks need a second chunk) and 40 registers let
-     * eleven in, 385 us against 397 with ten.  Below GRAIN_SMALL grains an SM
-     * holds few blocks and the longest one is the time: eight warps and
-     * 288 slots, 20 us against 25 at 2,000 grains (before the uncertified grains'
-     * slots were packed). */
+     * eleven in, 385 us at 1M grains against 397 with ten (blocks of 64 in two
+     * chunks: 414, and 67 against 62 at 100K; they stay for the autotuner).
+     * Below, an SM holds few blocks and the longest one is the time: 16
+     * grains from GRAIN_SMALL down (31 us against 35 at 32,000 grains; above
+     * it 41 against 39 at 50,000 and 68 against 56 at 100,000), 8 from
+     * GRAIN_TINY down (16 us against 18 at 2,000, 17 against 18 at 6,000;
+     * above it 23 against 19 at 10,000). */
     if (sh.grain_occ < 6) go(k_grain_pass<64, 128, 208>, 64, 128);
-    else if (m.ng < GRAIN_SMALL) go(k_grain_pass<32, 256, 288>, 32, 256);
+    else if (m.ng <= GRAIN_TINY) go(k_grain_pass<8, 128, 80>, 8, 128);
+    else if (m.ng <= GRAIN_SMALL) go(k_grain_pass<16, 128, 144>, 16, 128);
     else go(k_grain_pass<32, 128, 208>, 32, 128);
 }
 
