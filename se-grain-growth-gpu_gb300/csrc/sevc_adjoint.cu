@@ -351,20 +351,36 @@ __global__ void __launch_bounds__(ADJ_TPB) k_adj_nucleation(double D, const Even
         [&](int e) { adj_nucleation_one(D, log[e], log[e + 1], lam); });
 }
 
-/* per grain: sign of the area at the step's start (area_stream's sum), and
- * dL/dSE_g += sum_p lambda_v(p) . (-mu sign(A) dA/dx_p) (not for a
- * nucleated grain, whose stored energy is 0, not a parameter).  One walk of
- * the list for both, eight vertices' positions and lambdas loaded at once;
- * the delta to a vertex's predecessor is minus the predecessor's to it. */
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_grains(DevMesh m, double mu, const double2 *lv, double *sgn, double *gse)
+/* Sign of every grain's area at the start of each recorded step (area_stream's
+ * sum), for a whole segment at once: blockIdx.y is the step, `bytes` the
+ * distance of the records. */
+__global__ void __launch_bounds__(TPB) k_adj_signs(TapeRecord r, size_t bytes, int ng, double D)
 {
     griddep_wait();
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= m.ng) return;
-    if (!m.gen[g]) { sgn[g] = 0.0; return; }
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ng) return;
+    const size_t o = blockIdx.y * bytes;
+    auto at = [&](const void *p) { return static_cast<const char *>(p) + o; };
+    int sign = 0;
+    if (*reinterpret_cast<const uint8_t *>(at(r.gen + g))) {
+        const double a = area_stream(reinterpret_cast<const int *>(at(r.glist + (size_t)SEVC_MAXV * g)),
+                                     *reinterpret_cast<const int *>(at(r.gvlen + g)),
+                                     reinterpret_cast<const double2 *>(at(r.pos)), D);
+        sign = a > 0 ? 1 : (a < 0 ? -1 : 0);
+    }
+    r.sgn[o + g] = (signed char)sign;
+}
+/* per grain: dL/dSE_g += sum_p lambda_v(p) . (-mu sign(A) dA/dx_p) (not for a
+ * nucleated grain, whose stored energy is 0, not a parameter).  Eight
+ * vertices' positions and lambdas are loaded at once; the delta to a vertex's
+ * predecessor is minus the predecessor's to it. */
+__device__ __forceinline__ void adj_grain(const DevMesh &m, int g, double mu, const double2 *lv, const signed char *sgn,
+                                          double *gse)
+{
+    if (g >= m.ng || !m.gen[g] || m.gtype[g] == GT_NUCLEATED) return;
     const int *L = m.glist + (size_t)SEVC_MAXV * g;
     const int n = m.gvlen[g];
-    double acc = 0.0, area = 0.0, ax = 0, ay = 0, px = 0, py = 0;   /* px, py: predecessor to vertex */
+    double acc = 0.0, px = 0, py = 0;                /* px, py: predecessor to vertex */
     double2 first = make_double2(0, 0);
     for (int base = 0; base < n; base += 8) {
         int v[8];
@@ -383,19 +399,12 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_grains(DevMesh m, double mu, 
 #pragma unroll 1
         for (int j = 0; j < end; j++) {
             const double2 c = q[j], b = base + j == n - 1 ? first : q[j + 1];
-            if (base + j > 0) {
-                double nx = ax + px, ny = ay + py;
-                if (base + j > 1) area += ax * ny - ay * nx;
-                ax = nx; ay = ny;
-            }
             const double xn = wrapd(b.x, c.x, m.D), yn = wrapd(b.y, c.y, m.D);
             acc += l[j].x * (0.5 * (yn + py)) + l[j].y * (0.5 * (-px - xn));
             px = xn; py = yn;
         }
     }
-    const double s = area > 0 ? 1.0 : (area < 0 ? -1.0 : 0.0);
-    sgn[g] = s;
-    if (m.gtype[g] != GT_NUCLEATED) gse[g] += -mu * s * acc;
+    gse[g] += -mu * (double)sgn[g] * acc;
 }
 
 /* For the edge vector d (length L) and its end moved by eps along axis c,
@@ -467,11 +476,9 @@ __device__ __forceinline__ void edge_fd_grad(double dx, double dy, double L2, do
  * chains of dependent FP64 operations and the three list searches run side
  * by side; the first lane adds the parts in order. */
 constexpr int ADJ_VPB = 10 * (ADJ_BLOCK / 32);     /* vertices per block */
-__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_vertices(DevMesh m, double mu, double eps, double s_gb,
-                                                            const double2 *lx, const double2 *lv, const double *sgn,
-                                                            double2 *lam_out, double *ggam)
+__device__ __forceinline__ void adj_vertex(const DevMesh &m, double mu, double eps, double s_gb, const double2 *lx,
+                                           const double2 *lv, const signed char *sgn, double2 *lam_out, double *ggam)
 {
-    griddep_wait();
     const int lane = threadIdx.x & 31, q3 = lane / 3, j = lane - 3 * q3;
     const int k = blockIdx.x * ADJ_VPB + (threadIdx.x >> 5) * 10 + q3;
     const bool in = lane < 30 && k < m.nv, live = in && m.ven[k];
@@ -508,7 +515,7 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_vertices(DevMesh m, double mu
         int pv, nx;
         if (g >= 0 && m.gen[g] && list_neighbours(m, g, k, pv, nx)) {
             double se = m.gtype[g] == GT_NUCLEATED ? 0.0 : m.gse[g];
-            double c = 0.5 * mu * se * sgn[g];
+            double c = 0.5 * mu * se * (double)sgn[g];
             double2 a = lv[pv], d = lv[nx];
             out.x += c * (a.y - d.y);
             out.y += c * (d.x - a.x);
@@ -529,10 +536,24 @@ __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_vertices(DevMesh m, double mu
     }
 }
 
+/* both gathers of a step: the first vb blocks take the vertices, the others
+ * the grains.  Neither fills the GPU at 10,000 grains; one after the other
+ * they took 14 + 20 us, with the area signs in the first; this takes 22. */
+__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_gather(DevMesh m, double mu, double eps, double s_gb, const double2 *lx,
+                                                          const double2 *lv, const signed char *sgn, double2 *lam_out,
+                                                          double *ggam, double *gse, int vb)
+{
+    griddep_wait();
+    if ((int)blockIdx.x < vb) adj_vertex(m, mu, eps, s_gb, lx, lv, sgn, lam_out, ggam);
+    else adj_grain(m, (blockIdx.x - vb) * blockDim.x + threadIdx.x, mu, lv, sgn, gse);
+}
+
 /* ---- tape records (sevc_adjoint_histogram's replay) ---- */
 /* What the adjoint of a step reads, in one launch instead of a copy per
  * array: the mesh the velocities are computed on, of the grain lists only the
- * used entries (24 of 400 bytes per grain on average).  start: the record
+ * used entries (24 of 400 bytes per grain on average).  blockIdx.y is the array:
+ * one thread copying a piece of each waits for them in turn (10 us a step at
+ * 10,000 grains, 7.5 so).  start: the record
  * is the step's first (the event log is emptied and switched on). */
 __device__ __forceinline__ void copy_words(const void *src, void *dst, size_t bytes, size_t t, size_t n)
 {
@@ -546,20 +567,27 @@ __global__ void __launch_bounds__(TPB) k_tape_record(DevMesh m, TapeRecord r, Ev
     griddep_wait();
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = (size_t)gridDim.x * blockDim.x;
     const size_t V = m.nv, B = m.nb, G = m.ng;
-    copy_words(m.pos, r.pos, V * 16, t, n);
-    copy_words(m.vb, r.vb, V * 16, t, n);
-    copy_words(m.vg, r.vg, V * 16, t, n);
-    copy_words(m.ven, r.ven, V, t, n);
-    copy_words(m.bv, r.bv, B * 8, t, n);
-    copy_words(m.ben, r.ben, B, t, n);
-    copy_words(m.gvlen, r.gvlen, G * 4, t, n);
-    copy_words(m.gen, r.gen, G, t, n);
-    copy_words(m.gtype, r.gtype, G, t, n);
-    for (size_t i = t; i < G * (SEVC_MAXV / 4); i += n) {
-        const size_t g = i / (SEVC_MAXV / 4), j = i - g * (SEVC_MAXV / 4);
-        if (4 * (int)j < m.gvlen[g]) reinterpret_cast<int4 *>(r.glist)[i] = reinterpret_cast<const int4 *>(m.glist)[i];
+    switch (blockIdx.y) {
+    case 0: copy_words(m.pos, r.pos, V * 16, t, n); break;
+    case 1: copy_words(m.vb, r.vb, V * 16, t, n); break;
+    case 2: copy_words(m.vg, r.vg, V * 16, t, n); break;
+    case 3: copy_words(m.bv, r.bv, B * 8, t, n); break;
+    case 4:
+        copy_words(m.ven, r.ven, V, t, n);
+        copy_words(m.ben, r.ben, B, t, n);
+        break;
+    case 5:
+        copy_words(m.gvlen, r.gvlen, G * 4, t, n);
+        copy_words(m.gen, r.gen, G, t, n);
+        copy_words(m.gtype, r.gtype, G, t, n);
+        break;
+    default:
+        for (size_t i = t; i < G * (SEVC_MAXV / 4); i += n) {
+            const size_t g = i / (SEVC_MAXV / 4), j = i - g * (SEVC_MAXV / 4);
+            if (4 * (int)j < m.gvlen[g]) reinterpret_cast<int4 *>(r.glist)[i] = reinterpret_cast<const int4 *>(m.glist)[i];
+        }
     }
-    if (start && t == 0) {
+    if (start && t == 0 && blockIdx.y == 0) {
         *log.n = 0;
         *m.elog = log;
     }
@@ -678,20 +706,29 @@ void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, doubl
 
 void launch_adjoint_step(const DevMesh &rec, const AdjointBuffers &a, double dt, double mu, double eps, double s_gb,
                          const EventRec *log, const int *nlog, const uint8_t *ven1, const double2 *vel1,
-                         bool nucleation, cudaStream_t s)
+                         const signed char *sgn, bool nucleation, cudaStream_t s)
 {
     launch_dep(k_adj_translate, nblk(rec.nv), TPB, s, rec.nv, dt, mu, a.lam, ven1, vel1, a.lx, a.lv, a.gmu);
     launch_dep(k_adj_events, rec.ninst, ADJ_TPB, s, rec.D, log, nlog, a.lx, a.lv, rec.voff, rec.ninst);
-    launch_dep(k_adj_grains, (rec.ng + ADJ_BLOCK - 1) / ADJ_BLOCK, ADJ_BLOCK, s, rec, mu, a.lv, a.sgn, a.gse);
-    launch_dep(k_adj_vertices, (rec.nv + ADJ_VPB - 1) / ADJ_VPB, ADJ_BLOCK, s, rec, mu, eps,
-               s_gb, a.lx, a.lv, a.sgn, a.lam, a.ggam);
+    const int vb = (rec.nv + ADJ_VPB - 1) / ADJ_VPB, gb = (rec.ng + ADJ_BLOCK - 1) / ADJ_BLOCK;
+    launch_dep(k_adj_gather, vb + gb, ADJ_BLOCK, s, rec, mu, eps, s_gb, a.lx, a.lv, sgn, a.lam, a.ggam, a.gse, vb);
     if (nucleation) launch_dep(k_adj_nucleation, rec.ninst, ADJ_TPB, s, rec.D, log, nlog, a.lam, rec.voff, rec.ninst);
 }
 
 static int copy_blocks(const DevMesh &m) { int b = nblk(m.nv); return b < 4 * 152 ? b : 4 * 152; }
 void launch_tape_record(const DevMesh &m, const TapeRecord &r, const EventLog &log, bool start, cudaStream_t s)
 {
-    launch_dep(k_tape_record, copy_blocks(m), TPB, s, m, r, log, (int)start);
+    const int b = copy_blocks(m);
+    launch_dep(k_tape_record, dim3(b < 152 ? b : 152, 7), TPB, s, m, r, log, (int)start);
+}
+void launch_adjoint_signs(const DevMesh &m, const TapeRecord &first, size_t bytes, int steps, cudaStream_t s)
+{
+    for (int k = 0; k < steps; k += 65535) {
+        TapeRecord r = first;
+        auto shift = [&](auto *&p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((char *)p + k * bytes); };
+        shift(r.pos); shift(r.glist); shift(r.gvlen); shift(r.gen); shift(r.sgn);
+        launch_dep(k_adj_signs, dim3(nblk(m.ng), steps - k < 65535 ? steps - k : 65535), TPB, s, r, bytes, m.ng, m.D);
+    }
 }
 void launch_tape_after(const DevMesh &m, const TapeRecord &r, cudaStream_t s)
 {

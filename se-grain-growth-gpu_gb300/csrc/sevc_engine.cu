@@ -1432,7 +1432,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
     {
         struct Req { void **p; size_t bytes; };
         std::vector<Req> r = { { (void **)&a.lam, V * 16 }, { (void **)&a.lx, V * 16 }, { (void **)&a.lv, V * 16 },
-                               { (void **)&a.sgn, G * 8 }, { (void **)&a.gse, G * 8 },
+                               { (void **)&a.gse, G * 8 },
                                { (void **)&a.gmu, V * 8 }, { (void **)&a.ggam, V * 8 }, { (void **)&a.dlda, G * 8 },
                                { (void **)&a.scalars, 16 }, { (void **)&d_dldh, 1024 * 8 } };
         size_t total = 0;
@@ -1450,7 +1450,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
            off_vel1 = off_vg + align256(V * 16), off_ven = off_vel1 + align256(V * 16), off_ven1 = off_ven + align256(V),
            off_bv = off_ven1 + align256(V), off_ben = off_bv + align256(B * 8), off_gl = off_ben + align256(B),
            off_gvl = off_gl + align256(G * SEVC_MAXV * 4), off_gen = off_gvl + align256(G * 4),
-           off_gty = off_gen + align256(G), off_log = off_gty + align256(G),
+           off_gty = off_gen + align256(G), off_sgn = off_gty + align256(G), off_log = off_sgn + align256(G),
            off_nlog = off_log + align256((size_t)tp.log_cap * sizeof(EventRec)), step_bytes = off_nlog + 256;
     if (!tp.rec || tp.rec_step_bytes != step_bytes || tp.rec_steps < tp.every) {
         if (tp.rec) cudaFree(tp.rec);
@@ -1474,6 +1474,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
         r.ben = (uint8_t *)rec(k, off_ben);
         r.gen = (uint8_t *)rec(k, off_gen);
         r.gtype = (uint8_t *)rec(k, off_gty);
+        r.sgn = (signed char *)rec(k, off_sgn);
         return r;
     };
     auto log_at = [&](int k) { return EventLog{ (EventRec *)rec(k, off_log), (int *)rec(k, off_nlog), tp.log_cap }; };
@@ -1514,6 +1515,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
             launch_tape_after(h->m, record_at(k), s);
         };
         st = run_steps_core(h, K, nullptr, nullptr, &hooks);
+        if (!st) launch_adjoint_signs(h->m, record_at(0), step_bytes, K, s);
         for (int k = K - 1; k >= 0 && !st; k--) {
             const TapeRecord r = record_at(k);
             DevMesh view = h->m;
@@ -1529,7 +1531,7 @@ sevc_status sevc_adjoint_histogram(sevc_handle *h, int nbins, double amax, const
             view.gtype = r.gtype;
             view.gse = tp.separam;           /* a nucleated grain's 0 is applied by its type */
             launch_adjoint_step(view, a, h->opt.dt, h->p.mu, h->opt.GB_eps, h->opt.GB_scaling, log_at(k).buf, log_at(k).n,
-                                r.ven1, r.vel1, h->opt.do_nucleation != 0, s);
+                                r.ven1, r.vel1, r.sgn, h->opt.do_nucleation != 0, s);
         }
     }
     tp.replaying = false;

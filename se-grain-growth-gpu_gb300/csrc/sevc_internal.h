@@ -150,7 +150,6 @@ int rng_record(int nstreams, int ndraws, double *host_out);
 struct AdjointBuffers {
     double2 *lam;    /* adjoint of the positions (current step boundary) */
     double2 *lx, *lv;/* adjoint of the post-event positions / of the velocities */
-    double *sgn;     /* sign of each grain's area at the step's start */
     double *gse;     /* dL/dSE per grain (accumulated) */
     double *gmu;     /* dL/dmu per vertex (accumulated) */
     double *ggam;    /* dL/dGB_scaling per vertex (accumulated) */
@@ -165,9 +164,12 @@ struct TapeRecord {
     int2 *bv;
     int *glist, *gvlen;
     uint8_t *ven, *ven1, *ben, *gen, *gtype;
+    signed char *sgn;   /* signs of the grains' areas, by launch_adjoint_signs */
 };
 void launch_tape_record(const DevMesh &m, const TapeRecord &r, const EventLog &log, bool start, cudaStream_t s);
 void launch_tape_after(const DevMesh &m, const TapeRecord &r, cudaStream_t s);
+/* the signs of `steps` records, `bytes` apart */
+void launch_adjoint_signs(const DevMesh &m, const TapeRecord &first, size_t bytes, int steps, cudaStream_t s);
 /* soft histogram of a_g = |A_g| sc over nbins bins of [0, amax), divided by
  * nnorm; part: stat_doubles(nbins) doubles of scratch */
 size_t stat_doubles(int nbins);
@@ -182,7 +184,7 @@ void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, doubl
  * it; nucleation: the log may hold nucleations */
 void launch_adjoint_step(const DevMesh &rec, const AdjointBuffers &a, double dt, double mu, double eps, double s_gb,
                          const EventRec *log, const int *nlog, const uint8_t *ven1, const double2 *vel1,
-                         bool nucleation, cudaStream_t s);
+                         const signed char *sgn, bool nucleation, cudaStream_t s);
 /* *out = the sum of a[0..n); part: stat_doubles(1) doubles of scratch */
 void launch_sum_ordered(const DevMesh &m, const double *a, int n, double *part, double *out, cudaStream_t s);
 /* out[0..6] = count, sum |A|, sum A^2, sum vlen, 3-sided count, min |A|, max
