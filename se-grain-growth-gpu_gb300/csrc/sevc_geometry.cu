@@ -97,9 +97,9 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  * `wide` or more sides or of fewer than 3, and those with a coordinate
  * outside the domain or + eps in the next binade.
  *
- * Measured (GB300): 1M grains 0.385 ms, FP64 pipe active 69% of the
+ * Measured (GB300): 1M grains 0.368 ms, FP64 pipe active 69% of the
  * cycles, 21 of 32 lanes per FP64 instruction (slots of different s or p in
- * one warp); 2,000 grains 16 us.  The form before it (a grain per thread,
+ * one warp); 2,000 grains 15 us.  The form before it (a grain per thread,
  * polygon in registers, one unrolled body per side count, side-count order
  * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
  * took 0.50 ms and 95 us: on a small mesh each unrolled body runs once and
@@ -232,7 +232,7 @@ template <int SLOTS> struct GrainChunk {
     int dest[SLOTS];                           /* 3 v + grain slot */
     unsigned short moved[SLOTS], inner[SLOTS]; /* the slots in the order they are worked on */
     unsigned char owner[SLOTS];
-    double se[GP_CHUNK], absA[GP_CHUNK], sum0[2][GP_CHUNK];   /* sum0: twice the areas with vertex 0 moved */
+    double se[GP_CHUNK], area[GP_CHUNK], sum0[2][GP_CHUNK];   /* sum0: twice the areas with vertex 0 moved */
     int sg[GP_CHUNK];
     unsigned short off[GP_CHUNK];              /* first slot */
     unsigned char n[GP_CHUNK];
@@ -303,7 +303,7 @@ __device__ __forceinline__ int certify_axis(const double *r, int n, double D, lo
  * the wrap) and most of them have such a slot; a warp that walked all
  * 2 n + 1 polygons of each, and chains formed among the certified slots, where
  * a warp waits for one lane, made the pass of 64 meshes of that size (176,000
- * grains) 171 us; their slots packed into whole warps make it 129 us. */
+ * grains) 171 us; with their slots packed into whole warps it took 129 us. */
 template <int SLOTS>
 __device__ __forceinline__ double moved_uncertified(const DevMesh &m, const GrainChunk<SLOTS> &B, int q, int x)
 {
@@ -348,7 +348,7 @@ __device__ __noinline__ void moved_uncertified_all(const DevMesh &m, const Grain
     for (int t = threadIdx.x; t < nodd; t += NT) {
         const int x = odd[t] & 1, q = odd[t] >> 1, i = B.owner[q];
         const double a = moved_uncertified(m, B, q, x);
-        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), B.absA[i]);
+        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), dabs(B.area[i]));
     }
 }
 
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
     __syncthreads();
     if (chains) {                              /* the block has uncertified grains: their running sums */
         for (int t = tid; t < 4 * total; t += NT) {
-            const int c = t / total, i = t - c * total, o = B.off[i], nn = B.n[i];
+            const int i = t >> 2, c = t & 3, o = B.off[i], nn = B.n[i];
             if (B.state(i) != GP_CHAIN) continue;
             double *Z = (c < 2 ? B.A[c] : B.M[c - 2]) + o, a = c < 2 ? zero_plus(Z[1]) : Z[1];
             Z[1] = a;
@@ -526,9 +526,11 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
     /* per grain and polygon: the running sum; of the unmoved one, the area.
      * (Sums that only a magnitude is taken of leave out the reference's
      * 0.0 + first term and its closing +-0: those change the sign of a zero
-     * at most.) */
+     * at most.)  A grain's three sums lie side by side, so a warp's grains have
+     * like numbers of sides: with a polygon per warp each waited for the
+     * chunk's longest list (380 against 368 us at 1M grains). */
     for (int t = tid; t < 3 * total; t += NT) {
-        const int c = t >= 2 * total ? 2 : (t >= total ? 1 : 0), i = t - c * total, o = B.off[i], nn = B.n[i];
+        const int i = t / 3, c = t - 3 * i, o = B.off[i], nn = B.n[i];
         if (B.state(i) == GP_REST) {
             if (c == 0) rest[atomicAdd(&nrest, 1)] = B.sg[i];
             continue;
@@ -543,9 +545,8 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
         if (c == 0) {
             acc = add_closing_term(acc, B.A[0][o + nn - 1], B.A[1][o + nn - 1]);
             const double A = dscale_down<1>(acc);
-            B.absA[i] = dabs(A);
+            B.area[i] = A;
             m.garea[B.sg[i]] = A;
-            m.gq[B.sg[i]] = div_sides(B.se[i] * A, nn);
         } else {
             B.sum0[c - 1][i] = acc;
         }
@@ -566,6 +567,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
         double a;         /* twice the moved area */
         if (p == 0) {
             a = B.sum0[x][i];
+            if (x == 0) m.gq[B.sg[i]] = div_sides(B.se[i] * B.area[i], nn);
         } else if (st == GP_CHAIN) {
             odd[atomicAdd(&nodd, 1)] = (unsigned short)(2 * q + x);
             continue;
@@ -586,7 +588,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
                 for (int k = q + 1; k < o + nn - 1; k++) a = a + sgn(B.T[k]);
             }
         }
-        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), B.absA[i]);
+        reinterpret_cast<double *>(m.contrib + B.dest[q])[x] = mul_diff(B.se[i], dabs(dscale_down<1>(a)), dabs(B.area[i]));
     }
     if (chains) {                              /* the uncertified grains' slots */
         __syncthreads();
