@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
     }
     __syncthreads();
     /* chunks of up to 32 grains (and SLOTS list slots) of the order */
-    for (int c0 = 0; c0 < listed; c0 += chunk) {
+    for (int c0 = 0; c0 < listed;) {
     if (warp == 0) {
         const int i = c0 + lane, k = i < listed ? sides[i] : 0;
         int o = k;
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
         if (c0 + lane < listed) B.se[lane] = m.gse[order[c0 + lane]];
     }
     __syncthreads();
-    const int total = chunk;
+    const int total = chunk;                   /* read here: warp 0 sets the next chunk's behind the last barrier */
     /* per slot: position, where the vertex keeps this grain's terms, places
      * in the work orders */
 #pragma unroll 2
@@ -595,6 +595,7 @@ __global__ void __launch_bounds__(NT, SLOTS == 208 ? 11 : 1) k_grain_pass(DevMes
         moved_uncertified_all<NT>(m, B, odd, nodd);
     }
     __syncthreads();
+    c0 += total;
     }
     /* the rest, a warp per grain */
     GrainRest &Z = reinterpret_cast<GrainRest *>(smem)[warp];
