@@ -66,6 +66,14 @@ struct Tape {
     std::function<void(cudaStream_t)> after_nucleation;
 };
 
+/* A step is launched in its dense form (launch_tail_removals) when the last
+ * finished one had more events than this.  A step of some 1,000 events takes
+ * 330 us in the sparse form and 284 in the dense one on 100,003 grains, 488
+ * and 455 on 400,001; of 75 events 181 and 187 (the four launches more), of
+ * 300 (400,001 grains) 414 and 411.  The line lies at the upper end because a
+ * run that passes it captures a second graph (0.1 ms). */
+constexpr int DENSE_EVENTS = 1024;
+
 struct sevc_handle {
     sevc_options opt;
     int nv = 0, nb = 0, ng = 0;
@@ -100,8 +108,10 @@ struct sevc_handle {
     double *stat = nullptr, *h_stat = nullptr;
     size_t stat_len = 0;
     Tape tape;
-    /* a step without / with a nucleation attempt as one CUDA graph */
-    StepGraph g_step[2];
+    /* a step without / with a nucleation attempt as one CUDA graph, in its
+     * sparse and its dense form */
+    StepGraph g_step[2][2];
+    bool dense = false;          /* the last finished step had many events: see DENSE_EVENTS */
     bool use_graphs = true;
     bool force_direct = false;   /* this step launches directly (an adjoint replay records inside it) */
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -460,10 +470,11 @@ void tape_free(sevc_handle *h)
 
 void drop_graphs(sevc_handle *h)
 {
-    for (StepGraph *g : { &h->g_step[0], &h->g_step[1] }) {
-        if (g->exec) cudaGraphExecDestroy(g->exec);
-        *g = StepGraph();
-    }
+    for (auto &of : h->g_step)
+        for (StepGraph &g : of) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = StepGraph();
+        }
 }
 
 /* Graphs replay launches with their captured arguments: not while
@@ -571,10 +582,10 @@ void enqueue_tail(sevc_handle *h)
         sevc_pdl_skip = 0;
         return;
     }
-    { Prof pr(h, "removals"); launch_tail_removals(m, x, p, h->polling_cap, s); }                 /* :219-266 */
+    { Prof pr(h, "removals"); launch_tail_removals(m, x, p, h->polling_cap, h->dense, s); }                 /* :219-266 */
     sevc_pdl_skip = 0;
     if (h->profiling) {
-        { Prof pr(h, "flips"); launch_tail_flips(m, x, p, s); }                                   /* :282, :289 */
+        { Prof pr(h, "flips"); launch_tail_flips(m, x, p, h->dense, s); }                                   /* :282, :289 */
         { Prof pr(h, "update"); launch_update_positions(m, p.dt, s); }                            /* :314 */
         { Prof pr(h, "counts"); launch_counts(m, x, p, s); }                                      /* :317-325 */
     } else {
@@ -587,7 +598,7 @@ void enqueue_tail(sevc_handle *h)
         cudaStreamWaitEvent(h->side[0], ev[6], 0);
         launch_counts(m, x, p, h->side[0]);
         cudaEventRecord(ev[7], h->side[0]);
-        launch_tail_flips(m, x, p, s);
+        launch_tail_flips(m, x, p, h->dense, s);
         launch_update_positions(m, p.dt, s);
         cudaStreamWaitEvent(s, ev[7], 0);
         sevc_pdl_skip = 1;
@@ -692,6 +703,7 @@ sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms
         loc.n_two_three_iters = k + 1;
         if (c == 0) break;
     }
+    h->dense = !tail_whole(h->m) && loc.n_removals + loc.n_flips > DENSE_EVENTS;
     h->curr_n_grains = total;
     h->nucleated_area = batch ? area_sum / I : area_sum;
     loc.curr_n_grains = total;
@@ -928,7 +940,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     h->h_flags[3] = h->curr_n_grains;
     launch_set_flags(x, h->h_flags, s);
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
-    if (!run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
+    if (!run_seq(h, h->g_step[n_on ? 1 : 0][h->dense], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
 
     /* one readback: counters, events, error bits, polling iterations and
@@ -1035,7 +1047,7 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         cudaEventRecord(sl.ev0, s);
         long long k0 = sevc_kernel_launches;
         h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
-        bool ran = run_seq(h, h->g_step[n_on ? 1 : 0], [&] { enqueue_step(h, n_on > 0); });
+        bool ran = run_seq(h, h->g_step[n_on ? 1 : 0][h->dense], [&] { enqueue_step(h, n_on > 0); });
         h->force_direct = false;
         if (!ran) {
             st = SEVC_ERR_CUDA;

@@ -123,11 +123,12 @@ void launch_two_three_first(const DevMesh &m, const DevScratch &x, cudaStream_t 
 /* The sparse phases (k_tail): all of them, the position update, the counts
  * and the summary in one launch for meshes that tail_whole accepts; else the
  * removals and the flips, each with the edits of its list fix-up, and the
- * position update with the rest of the flips' fix-up. */
+ * position update with the rest of the flips' fix-up.  dense: the events of
+ * both are applied over the whole GPU (two launches more each). */
 bool tail_whole(const DevMesh &m);
 void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s);
-void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s);
-void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
+void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, bool dense, cudaStream_t s);
+void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, bool dense, cudaStream_t s);
 void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s);
 void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s);
 

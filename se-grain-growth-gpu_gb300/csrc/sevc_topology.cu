@@ -1536,7 +1536,9 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
  *   TAIL_END     the list fix-ups (:262-266, :294), position update (:314),
  *                counts (:317-325), step summary
  * On a large mesh TAIL_REMOVE and TAIL_FLIP are launches of their own and
- * the fix-ups run on the whole GPU behind each (k_edit).
+ * the fix-ups run on the whole GPU behind each (k_edit).  TAIL_SPREAD: each
+ * ends at its reservations, and k_apply and k_deferred behind it take the
+ * events (see launch_tail_removals).
  *
  * What bounds it: nothing but the chain of its phases, each a handful of
  * dependent loads.  As ~25 kernels (programmatic dependent launch between
@@ -1544,7 +1546,7 @@ __device__ void two_three_loop(const DevMesh &m, const DevScratch &x, const Team
  * cluster barrier costs well under a microsecond.  16 blocks of 512 are the
  * largest cluster; with a warp per event that is 256 events at once. */
 constexpr int TAIL_WHOLE_NV = 64 * 1024;
-enum { TAIL_REMOVE = 1, TAIL_FLIP = 2, TAIL_END = 4 };
+enum { TAIL_REMOVE = 1, TAIL_FLIP = 2, TAIL_END = 4, TAIL_SPREAD = 8 };
 template <int PART>
 __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, PollGrid pg, int cap, double dt, double eps,
                                                   int *summary)
@@ -1574,7 +1576,7 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
             if (T.tid == 0) *x.n_ehits = 0;          /* the grains a 2x3 pass left with three sides */
             T.sync();
         }
-        const int nc = na > 0 ? *x.n_c : 0;
+        const int nc = na > 0 && !(PART & TAIL_SPREAD) ? *x.n_c : 0;
         if (nc > 0) {
             remove_apply(m, x, T, x.list_c, nc);
             T.sync();
@@ -1598,6 +1600,7 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
     }
     if ((PART & TAIL_FLIP) && na > 0) {
         flip_reserve(m, x, T, x.list_a, na);
+        if (PART & TAIL_SPREAD) return;
         T.sync();
         flip_apply(m, x, T, x.list_a, na, eps);
         T.sync();
@@ -1622,6 +1625,32 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(DevMesh m, DevScratch x, Poll
         T.sync();
         pack_summary(m, x, summary, T.tid, T.n);
     }
+}
+
+/* The events behind their reservations, over the whole GPU: those that hold
+ * their records, a warp each, then (one cluster) the deferred ones.  For steps
+ * of many events (see DENSE_EVENTS): the cluster's 256 warps take 10,400
+ * removals and 12,700 flips in rounds, 760 and 600 us with their fix-ups, and
+ * such a step of 256 meshes (1.28M grains) went from 3.13 ms to 2.36. */
+constexpr int APPLY_TPB = 256, APPLY_BLOCKS = 2 * WL_BLOCKS;
+template <bool FLIPS>
+__global__ void __launch_bounds__(APPLY_TPB) k_apply(DevMesh m, DevScratch x, double eps)
+{
+    griddep_wait();
+    const Team T;
+    if (FLIPS) flip_apply(m, x, T, x.list_a, *x.n_a, eps);
+    else remove_apply(m, x, T, x.list_c, *x.n_c);
+}
+template <bool FLIPS>
+__global__ void __launch_bounds__(TAIL_TPB) k_deferred(DevMesh m, DevScratch x, double eps)
+{
+    griddep_wait();
+    const Team T;
+    /* without candidates n_ehits still counts the 2x3 loop's list */
+    const int nd = *x.n_a > 0 ? *x.n_ehits : 0;
+    if (nd == 0) return;
+    if (FLIPS) run_deferred(m, x, T, nd, m.boff, [&](int b, int) { flip_warp(m, b, eps, T.lane); });
+    else run_deferred(m, x, T, nd, m.goff, [&](int g, int inst) { remove_warp(m, g, inst, T.lane); });
 }
 
 /* edit_grains over the whole GPU, after the removals (REMOVED) or the
@@ -1659,12 +1688,11 @@ __global__ void k_fill_instance_ids(DevMesh m)
         m.ginst[g] = lower_bound_i(m.goff, m.ninst + 1, g + 1) - 1;
 }
 
-/* k_tail<PART> as one cluster, after the previous kernel of the stream (or
- * without programmatic serialisation, see launch_dep) */
-template <int PART>
-void launch_tail_part(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s)
+/* k as one cluster, after the previous kernel of the stream (or without
+ * programmatic serialisation, see launch_dep) */
+template <typename... P, typename... A>
+void launch_cluster(void (*k)(P...), cudaStream_t s, A &&...args)
 {
-    auto k = k_tail<PART>;
     cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1681,7 +1709,12 @@ void launch_tail_part(const DevMesh &m, const DevScratch &x, const StepParams &p
     if (sevc_pdl_skip > 0) sevc_pdl_skip--;
     cfg.numAttrs = plain ? 1 : 2;
     COUNT_LAUNCHES(1);
-    cudaLaunchKernelEx(&cfg, k, m, x, poll_grid(p), cap, p.dt, p.eps, summary);
+    cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(args)...);
+}
+template <int PART>
+void launch_tail_part(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, int *summary, cudaStream_t s)
+{
+    launch_cluster(k_tail<PART>, s, m, x, poll_grid(p), cap, p.dt, p.eps, summary);
 }
 
 } // namespace
@@ -1707,14 +1740,26 @@ void launch_tail_whole(const DevMesh &m, const DevScratch &x, const StepParams &
 {
     launch_tail_part<TAIL_REMOVE | TAIL_FLIP | TAIL_END>(m, x, p, cap, summary, s);
 }
-void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, cudaStream_t s)
+void launch_tail_removals(const DevMesh &m, const DevScratch &x, const StepParams &p, int cap, bool dense, cudaStream_t s)
 {
-    launch_tail_part<TAIL_REMOVE>(m, x, p, cap, nullptr, s);
+    if (dense) {
+        launch_tail_part<TAIL_REMOVE | TAIL_SPREAD>(m, x, p, cap, nullptr, s);
+        launch_dep(k_apply<false>, APPLY_BLOCKS, APPLY_TPB, s, m, x, p.eps);
+        launch_cluster(k_deferred<false>, s, m, x, p.eps);
+    } else {
+        launch_tail_part<TAIL_REMOVE>(m, x, p, cap, nullptr, s);
+    }
     launch_dep(k_edit<true>, WL_BLOCKS, EDIT_TPB, s, m, x);
 }
-void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
+void launch_tail_flips(const DevMesh &m, const DevScratch &x, const StepParams &p, bool dense, cudaStream_t s)
 {
-    launch_tail_part<TAIL_FLIP>(m, x, p, 0, nullptr, s);
+    if (dense) {
+        launch_tail_part<TAIL_FLIP | TAIL_SPREAD>(m, x, p, 0, nullptr, s);
+        launch_dep(k_apply<true>, APPLY_BLOCKS, APPLY_TPB, s, m, x, p.eps);
+        launch_cluster(k_deferred<true>, s, m, x, p.eps);
+    } else {
+        launch_tail_part<TAIL_FLIP>(m, x, p, 0, nullptr, s);
+    }
     launch_dep(k_edit<false>, WL_BLOCKS, EDIT_TPB, s, m, x);
 }
 void launch_update_positions(const DevMesh &m, double dt, cudaStream_t s)
