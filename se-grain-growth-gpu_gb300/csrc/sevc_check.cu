@@ -372,11 +372,11 @@ void launch_check(const DevMesh &m, int *out, cudaStream_t s)
     if (bb + vb + gb > 0) COUNT_LAUNCHES(1), k_check<<<bb + vb + gb, TPB, 0, s>>>(m, bb, vb, out);
 }
 
-void launch_export(const DevMesh &m, const sevc_mesh_host &o, int part, cudaStream_t s)
+cudaError_t launch_export(const DevMesh &m, const sevc_mesh_host &o, int part, cudaStream_t s)
 {
     size_t n = (size_t)m.nv + m.nb;
     size_t g = (n + TPB - 1) / TPB;
-    COUNT_LAUNCHES(1), k_export<<<(unsigned)(g < 8 * 152 ? (g ? g : 1) : 8 * 152), TPB, 0, s>>>(m, o, part);
+    return launch_status(k_export, (unsigned)(g < 8 * 152 ? (g ? g : 1) : 8 * 152), TPB, 0, s, m, o, part);
 }
 
 void launch_digest(const DevMesh &m, unsigned long long *out, cudaStream_t s)

@@ -489,7 +489,11 @@ bool graphs_on(const sevc_handle *h)
  * enqueue it directly. */
 template <class F> bool run_seq(sevc_handle *h, StepGraph &g, F &&enqueue)
 {
-    if (!graphs_on(h)) { enqueue(); return true; }
+    if (!graphs_on(h)) {
+        cudaGetLastError();   /* what an earlier call left behind is not these launches' */
+        enqueue();
+        return cuda_ok(cudaGetLastError(), "launch");
+    }
     if (!g.exec) {
         long long k0 = sevc_kernel_launches;
         cudaGraph_t graph = nullptr;
@@ -938,7 +942,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     h->h_flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && h->n % o.snap_gap == 0);
     h->h_flags[2] = batch ? 0 : mg;   /* a batch does not stop at min_grains */
     h->h_flags[3] = h->curr_n_grains;
-    launch_set_flags(x, h->h_flags, s);
+    if (!cuda_ok(launch_set_flags(x, h->h_flags, s), "step flags")) return SEVC_ERR_CUDA;
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
     if (!run_seq(h, h->g_step[n_on ? 1 : 0][h->dense], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
@@ -946,8 +950,8 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     /* one readback: counters, events, error bits, polling iterations and
      * 2x3 counts of every instance */
     int *hb = h->h_big;
-    launch_read_out(x.summary, hb, (int)(summary_bytes(h) / sizeof(int)), s);
-    if (!cuda_ok(cudaGetLastError(), "readback") || !cuda_ok(cudaStreamSynchronize(s), "readback sync"))
+    if (!cuda_ok(launch_read_out(x.summary, hb, (int)(summary_bytes(h) / sizeof(int)), s), "readback") ||
+        !cuda_ok(cudaStreamSynchronize(s), "readback sync"))
         return SEVC_ERR_CUDA;
     float ms = 0;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
@@ -1043,7 +1047,10 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
             st = SEVC_ERR_CUDA;
             break;
         }
-        launch_set_flags(x, sl.flags, s);
+        if (!cuda_ok(launch_set_flags(x, sl.flags, s), "step flags")) {
+            st = SEVC_ERR_CUDA;
+            break;
+        }
         cudaEventRecord(sl.ev0, s);
         long long k0 = sevc_kernel_launches;
         h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
@@ -1064,8 +1071,7 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
             st = SEVC_ERR_CUDA;
             break;
         }
-        launch_read_out(x.summary, sl.big, (int)(summary_bytes(h) / sizeof(int)), s);
-        if (!cuda_ok(cudaGetLastError(), "readback") ||
+        if (!cuda_ok(launch_read_out(x.summary, sl.big, (int)(summary_bytes(h) / sizeof(int)), s), "readback") ||
             !cuda_ok(cudaEventRecord(sl.done, s), "event")) {
             st = SEVC_ERR_CUDA;
             break;
@@ -1125,16 +1131,17 @@ sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *o)
         /* the device writes the caller's arrays, the grains' (60% of the
          * bytes) while the host maps the pages of the others */
         const int n = SEVC_HOST_FIELDS, ngf = SEVC_HOST_GRAIN_FIELDS;
+        bool sent;
         if (bytes[0] < (size_t)16 << 20) {
             sevc_host_touch(n, ptr, bytes);
-            launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s);
+            sent = cuda_ok(launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s), "export");
         } else {
             sevc_host_touch(ngf, ptr, bytes);
-            launch_export(h->m, d, EXPORT_GRAINS, s);
+            sent = cuda_ok(launch_export(h->m, d, EXPORT_GRAINS, s), "export");
             sevc_host_touch(n - ngf, ptr + ngf, bytes + ngf);
-            launch_export(h->m, d, EXPORT_REST, s);
+            sent = cuda_ok(launch_export(h->m, d, EXPORT_REST, s), "export") && sent;
         }
-        return cuda_ok(cudaGetLastError(), "export") && cuda_ok(cudaStreamSynchronize(s), "sync") ? SEVC_OK : SEVC_ERR_CUDA;
+        return cuda_ok(cudaStreamSynchronize(s), "sync") && sent ? SEVC_OK : SEVC_ERR_CUDA;
     }
     /* else through device memory in the same layout */
     size_t off[SEVC_HOST_FIELDS], total = 0;
@@ -1142,8 +1149,7 @@ sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *o)
     char *dev = nullptr;
     if (!cuda_ok(cudaMalloc(&dev, total), "cudaMalloc")) return SEVC_ERR_CUDA;
     sevc_host_relocate(&d, dev, off);
-    launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s);
-    bool ok = cuda_ok(cudaGetLastError(), "export");
+    bool ok = cuda_ok(launch_export(h->m, d, EXPORT_GRAINS | EXPORT_REST, s), "export");
     for (int f = 0; f < SEVC_HOST_FIELDS && ok; f++)
         ok = cuda_ok(cudaMemcpyAsync(ptr[f], dev + off[f], bytes[f], cudaMemcpyDeviceToHost, s), "download");
     ok = cuda_ok(cudaStreamSynchronize(s), "sync") && ok;

@@ -974,14 +974,14 @@ void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaSt
     launch_dep(k_pack_summary, g < 152 ? g : 152, TPB, s, m, x, out);
 }
 
-void launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s)
+cudaError_t launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s)
 {
-    COUNT_LAUNCHES(1), k_set_flags<<<1, 1, 0, s>>>(x.flags, flags[1], flags[2], flags[3]);
+    return launch_status(k_set_flags, 1, 1, 0, s, x.flags, flags[1], flags[2], flags[3]);
 }
-void launch_read_out(const int *from, int *host, int n, cudaStream_t s)
+cudaError_t launch_read_out(const int *from, int *host, int n, cudaStream_t s)
 {
     int g = nblk(n);
-    COUNT_LAUNCHES(1), k_read_out<<<g < 16 ? g : 16, TPB, 0, s>>>(from, host, n);
+    return launch_status(k_read_out, g < 16 ? g : 16, TPB, 0, s, from, host, n);
 }
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s)
 {

@@ -108,8 +108,8 @@ void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 /* the host's part of the output decision, flags[1..3], into x.flags; and n
  * ints into pinned host memory, both in stream order */
-void launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s);
-void launch_read_out(const int *from, int *host, int n, cudaStream_t s);
+cudaError_t launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s);
+cudaError_t launch_read_out(const int *from, int *host, int n, cudaStream_t s);
 /* counters | events | error bits | polling iterations | 2x3 counts | output decision, into out */
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s);
 
@@ -135,7 +135,7 @@ void launch_fill_instance_ids(const DevMesh &m, cudaStream_t s);
 /* The mesh in the layout of sevc_mesh_host, written by the device through
  * pointers it can store to.  part: EXPORT_GRAINS, EXPORT_REST or both. */
 enum { EXPORT_GRAINS = 1, EXPORT_REST = 2 };
-void launch_export(const DevMesh &m, const sevc_mesh_host &o, int part, cudaStream_t s);
+cudaError_t launch_export(const DevMesh &m, const sevc_mesh_host &o, int part, cudaStream_t s);
 
 /* check_data on the device (sevc_check.cu): violations counted into *out */
 void launch_check(const DevMesh &m, int *out, cudaStream_t s);
@@ -200,6 +200,21 @@ extern long long sevc_kernel_launches;
  * serialisation attribute (a kernel with two predecessors) */
 extern thread_local int sevc_pdl_skip;
 #define COUNT_LAUNCHES(k) (sevc_kernel_launches += (k))
+
+/* Launch and return the launch's own status.  (cudaGetLastError after a
+ * launch also returns what any earlier failed call of this thread, of this
+ * library or not, left behind.) */
+template <typename... P, typename... A>
+inline cudaError_t launch_status(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    COUNT_LAUNCHES(1);
+    return cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(args)...);
+}
 
 /* Launch with programmatic dependent launch allowed: the grid may be
  * scheduled while the previous kernel of the stream drains, which hides
