@@ -688,13 +688,17 @@ static int hist_threads(const DevMesh &m, int nbins)
     return T;
 }
 size_t stat_doubles(int nbins) { return (size_t)2 * 152 * (nbins > NSTAT ? nbins : NSTAT); }
-void launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *part, double *hist,
-                      cudaStream_t s)
+cudaError_t launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *part,
+                             double *hist, cudaStream_t s)
 {
     const int T = hist_threads(m, nbins);
     const size_t smem = (size_t)T * nbins * 8;
-    cudaFuncSetAttribute(k_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    COUNT_LAUNCHES(1), k_hist<<<stat_blocks(m.ng, T), TPB, smem, s>>>(m, nbins, T, amax, sc, nnorm, part, hist);
+    /* the attribute belongs to the kernel, for every handle and thread: always
+     * the largest any launch takes (1024 bins), never this one's size, under
+     * which another thread's launch would be refused */
+    cudaError_t e = cudaFuncSetAttribute(k_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * 1024 * 8);
+    if (e != cudaSuccess) return e;
+    return launch_status(k_hist, stat_blocks(m.ng, T), TPB, smem, s, m, nbins, T, amax, sc, nnorm, part, hist);
 }
 
 void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, double nnorm, const double *dldh,

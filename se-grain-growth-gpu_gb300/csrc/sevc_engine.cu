@@ -1429,8 +1429,9 @@ sevc_status sevc_area_histogram(sevc_handle *h, int nbins, double amax, double *
     if (!h || nbins < 1 || nbins > 1024 || !(amax > 0) || !hist) return SEVC_ERR_ARG;
     if (!stat_scratch(h, nbins)) return SEVC_ERR_CUDA;
     double nnorm = h->curr_n_grains, sc = nnorm / (h->ninst * h->opt.domain_bound * h->opt.domain_bound);
-    launch_histogram(h->m, nbins, amax, sc, nnorm, h->stat + 1024, h->stat, h->stream);
-    if (!stat_read(h, nbins)) return SEVC_ERR_CUDA;
+    if (!cuda_ok(launch_histogram(h->m, nbins, amax, sc, nnorm, h->stat + 1024, h->stat, h->stream), "histogram") ||
+        !stat_read(h, nbins))
+        return SEVC_ERR_CUDA;
     memcpy(hist, h->h_stat, nbins * 8);
     return SEVC_OK;
 }

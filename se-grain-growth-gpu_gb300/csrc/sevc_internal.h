@@ -174,8 +174,8 @@ void launch_adjoint_signs(const DevMesh &m, const TapeRecord &first, size_t byte
 /* soft histogram of a_g = |A_g| sc over nbins bins of [0, amax), divided by
  * nnorm; part: stat_doubles(nbins) doubles of scratch */
 size_t stat_doubles(int nbins);
-void launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *part, double *hist,
-                      cudaStream_t s);
+cudaError_t launch_histogram(const DevMesh &m, int nbins, double amax, double sc, double nnorm, double *part,
+                             double *hist, cudaStream_t s);
 /* lam = d(sum_k dldh_k h_k)/dx at the current state; zero_sum: see
  * k_hist_grad_area */
 void launch_hist_seed(const DevMesh &m, int nbins, double amax, double sc, double nnorm, const double *dldh,
