@@ -438,24 +438,26 @@ bool stat_read(sevc_handle *h, int nout)
     return cuda_ok(cudaMemcpyAsync(h->h_stat, h->stat, nout * 8, cudaMemcpyDeviceToHost, h->stream), "readback") &&
            cuda_ok(cudaStreamSynchronize(h->stream), "sync");
 }
-/* a device copy of the whole block as it is at this point of the stream */
-void *tape_copy(sevc_handle *h)
+/* whether a checkpoint of the tape is due after the step that goes in now,
+ * `ahead` steps before it still unfinished */
+bool tape_due(const sevc_handle *h, int ahead)
 {
-    void *ck = nullptr;
-    if (!cuda_ok(cudaMalloc(&ck, h->dbytes), "cudaMalloc checkpoint")) return nullptr;
-    if (!cuda_ok(cudaMemcpyAsync(ck, h->dblock, h->dbytes, cudaMemcpyDeviceToDevice, h->stream), "checkpoint")) {
-        cudaFree(ck);
-        return nullptr;
-    }
-    return ck;
+    return h->tape.every > 0 && !h->tape.replaying && (h->tape.nsteps + ahead + 1) % h->tape.every == 0;
 }
-/* ck (or, if null, a copy taken now) becomes the tape's next checkpoint */
-bool tape_checkpoint(sevc_handle *h, void *ck = nullptr)
+/* memory for a checkpoint: taken before its step goes in, so that a step
+ * never runs whose checkpoint finds none */
+bool tape_room(const sevc_handle *h, void **ck) { return cuda_ok(cudaMalloc(ck, h->dbytes), "cudaMalloc checkpoint"); }
+/* the whole block as it is at this point of the stream into ck */
+bool tape_copy(sevc_handle *h, void *ck)
 {
-    if (!ck && !(ck = tape_copy(h))) return false;
+    return cuda_ok(cudaMemcpyAsync(ck, h->dblock, h->dbytes, cudaMemcpyDeviceToDevice, h->stream), "checkpoint");
+}
+/* ck becomes the tape's next checkpoint, of the run state as it is now */
+void tape_checkpoint(sevc_handle *h, void *&ck)
+{
     h->tape.ckpt.push_back(ck);
     h->tape.runs.push_back(save_run(h));
-    return true;
+    ck = nullptr;
 }
 void tape_free(sevc_handle *h)
 {
@@ -644,9 +646,10 @@ size_t summary_bytes(const sevc_handle *h)
  * iterations and 2x3 counts of every instance; h_on: the instances that
  * attempted a nucleation) into the run state and `info`; then n++ and
  * t = n dt (src/main.cu:388-391).  loc carries n, t and the attempt flag of
- * the step; ckpt a tape checkpoint already copied after it. */
+ * the step; ckpt a tape checkpoint copied after it (null if none was due),
+ * which the tape takes over unless the step failed. */
 sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms, int launches,
-                        sevc_step_info loc, sevc_step_info *info, void *ckpt = nullptr)
+                        sevc_step_info loc, sevc_step_info *info, void *&ckpt)
 {
     const sevc_options &o = h->opt;
     const int I = h->ninst;
@@ -727,7 +730,7 @@ sevc_status finish_step(sevc_handle *h, const int *hb, const int *h_on, float ms
     sevc_status st = err_bits_to_status(hb[o_err]);
     if (!st && h->tape.every > 0 && !h->tape.replaying) {
         h->tape.nsteps++;
-        if (h->tape.nsteps % h->tape.every == 0 && !tape_checkpoint(h, ckpt)) return SEVC_ERR_CUDA;
+        if (ckpt) tape_checkpoint(h, ckpt);
     }
     return st;
 }
@@ -923,6 +926,8 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     memset(&loc, 0, sizeof loc);
     loc.n = h->n;
     loc.t = h->t;
+    struct Room { void *p = nullptr; ~Room() { if (p) cudaFree(p); } } ckpt;
+    if (tape_due(h, 0) && !tape_room(h, &ckpt.p)) return SEVC_ERR_CUDA;
     long long launches0 = sevc_kernel_launches;
     cudaEventRecord(h->ev0, s);
     int n_on = 0;                                                                                  /* :137-141 */
@@ -946,6 +951,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
     if (!run_seq(h, h->g_step[n_on ? 1 : 0][h->dense], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
+    if (ckpt.p && !tape_copy(h, ckpt.p)) return SEVC_ERR_CUDA;
 
     /* one readback: counters, events, error bits, polling iterations and
      * 2x3 counts of every instance */
@@ -957,7 +963,7 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     if (h->profiling) prof_collect(h);
     int launches = (int)(sevc_kernel_launches - launches0);
-    return finish_step(h, hb, h->h_on, ms, launches, loc, info);
+    return finish_step(h, hb, h->h_on, ms, launches, loc, info, ckpt.p);
 }
 
 } // extern "C"
@@ -977,9 +983,11 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
     if (!pipe) {
         for (int k = 0; k < nsteps; k++) {
             sevc_step_info inf;
+            const int n0 = h->n;
             if (hooks) hooks->before(k);
             sevc_status st = sevc_step(h, &inf);
             if (hooks) hooks->after(k);
+            if (h->n == n0) return st;         /* the step was not taken */
             if (infos) infos[k] = inf;
             if (done) *done = k + 1;
             if (st) return st;
@@ -999,6 +1007,7 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         h->rslot_ready = true;
     }
     int launched = 0, finished = 0;
+    bool step_failed = false;
     sevc_status st = SEVC_OK;
     auto finish_one = [&]() -> sevc_status {
         sevc_handle::RunSlot &sl = h->rslot[finished % 2];
@@ -1007,7 +1016,6 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         cudaEventElapsedTime(&ms, sl.ev0, sl.ev1);
         sevc_step_info inf;
         sevc_status r = finish_step(h, sl.big, sl.on, ms, (int)sl.launches, sl.loc, &inf, sl.ckpt);
-        sl.ckpt = nullptr;
         if (infos) infos[finished] = inf;
         finished++;
         if (done) *done = finished;
@@ -1026,9 +1034,14 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
             for (int i = 0; i < I; i++) can_launch = can_launch && h->iallow[i];
         if (!can_launch) {
             st = finish_one();
+            step_failed = st != SEVC_OK;
             continue;
         }
         sevc_handle::RunSlot &sl = h->rslot[launched % 2];
+        if (tape_due(h, launched - finished) && !tape_room(h, &sl.ckpt)) {
+            st = SEVC_ERR_CUDA;
+            break;
+        }
         memset(&sl.loc, 0, sizeof sl.loc);
         sl.loc.n = nk;
         sl.loc.t = nk * o.dt;
@@ -1065,9 +1078,7 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         if (hooks) hooks->after(launched);
         /* a checkpoint of the tape due after this step is copied here, before
          * the next step goes in; finish_step adds it to the tape */
-        sl.ckpt = nullptr;
-        if (h->tape.every > 0 && !h->tape.replaying && (h->tape.nsteps + (launched - finished) + 1) % h->tape.every == 0 &&
-            !(sl.ckpt = tape_copy(h))) {
+        if (sl.ckpt && !tape_copy(h, sl.ckpt)) {
             st = SEVC_ERR_CUDA;
             break;
         }
@@ -1078,7 +1089,13 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         }
         launched++;
     }
-    if (launched > finished) cudaStreamSynchronize(s);   /* after a failure: let the step in flight end */
+    /* the steps in flight behind one that could not go in are counted like the
+     * others; behind a step that failed they end uncounted (the mesh is in an
+     * undefined state) */
+    if (st) {
+        while (!step_failed && finished < launched) step_failed = finish_one() != SEVC_OK;
+        cudaStreamSynchronize(s);
+    }
     for (auto &sl : h->rslot)
         if (sl.ckpt) { cudaFree(sl.ckpt); sl.ckpt = nullptr; }
     return st;
@@ -1098,7 +1115,9 @@ sevc_status sevc_run_steps(sevc_handle *h, int nsteps, int *done, sevc_step_info
     int k = 0;
     sevc_status st = SEVC_OK;
     while (k < nsteps) {
+        const int n0 = h->n;
         st = sevc_step(h, &inf);
+        if (h->n == n0) break;                 /* the step was not taken */
         k++;
         if (st || !inf.keep_going) break;
     }
@@ -1409,12 +1428,19 @@ sevc_status sevc_tape_start(sevc_handle *h, int checkpoint_every)
 {
     if (!h || checkpoint_every < 1) return SEVC_ERR_ARG;
     tape_free(h);
-    h->tape.every = checkpoint_every;
-    if (!cuda_ok(cudaMalloc(&h->tape.separam, (size_t)h->ng * 8), "cudaMalloc tape") ||
-        !cuda_ok(cudaMemcpyAsync(h->tape.separam, h->m.gse, (size_t)h->ng * 8, cudaMemcpyDeviceToDevice, h->stream),
-                 "tape copy"))
+    void *ck = nullptr;
+    const bool ok = cuda_ok(cudaMalloc(&h->tape.separam, (size_t)h->ng * 8), "cudaMalloc tape") &&
+                    cuda_ok(cudaMemcpyAsync(h->tape.separam, h->m.gse, (size_t)h->ng * 8, cudaMemcpyDeviceToDevice,
+                                            h->stream), "tape copy") &&
+                    tape_room(h, &ck) && tape_copy(h, ck);
+    if (!ok) {                   /* no tape */
+        if (ck) cudaFree(ck);
+        tape_free(h);
         return SEVC_ERR_CUDA;
-    return tape_checkpoint(h) ? SEVC_OK : SEVC_ERR_CUDA;
+    }
+    tape_checkpoint(h, ck);
+    h->tape.every = checkpoint_every;
+    return SEVC_OK;
 }
 
 sevc_status sevc_tape_stop(sevc_handle *h)
