@@ -1144,6 +1144,11 @@ sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *o)
     void *ptr[SEVC_HOST_FIELDS];
     size_t bytes[SEVC_HOST_FIELDS];
     sevc_host_fields(&d, ptr, bytes);
+    for (int f = 0; f < SEVC_HOST_FIELDS; f++)
+        if (!ptr[f] && bytes[f]) { sevc_set_error("an array of the host mesh is missing"); return SEVC_ERR_CUDA; }
+    /* nothing is written after an error that ended the context (asked only when
+     * some call failed) */
+    if (cudaPeekAtLastError() != cudaSuccess && !cuda_ok(cudaStreamSynchronize(s), "download")) return SEVC_ERR_CUDA;
     int direct = 0;   /* the device can store to the caller's (pageable) memory */
     cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccess, h->device);
     if (direct && sevc_host_aligned(&d)) {

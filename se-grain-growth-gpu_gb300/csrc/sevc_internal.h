@@ -207,13 +207,11 @@ extern thread_local int sevc_pdl_skip;
 template <typename... P, typename... A>
 inline cudaError_t launch_status(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
     COUNT_LAUNCHES(1);
-    return cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(args)...);
+    return [&](P... p) {
+        void *at[] = { &p... };
+        return cudaLaunchKernel(reinterpret_cast<const void *>(k), grid, block, at, smem, s);
+    }(static_cast<A &&>(args)...);
 }
 
 /* Launch with programmatic dependent launch allowed: the grid may be
