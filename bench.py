@@ -550,7 +550,7 @@ def run_engine(args):
                    "l2": "working set > L2 (129 MB): ~1.4 GB of mesh state per step", **ev_win,
                    "mesh_generation_s": round(gen_s, 1), "wall_s": round(wall, 3),
                    "launch_shapes": {"tpb_vertex": shapes[0], "tpb_boundary": shapes[1], "wide_sides": shapes[2],
-                                     "grain_blocks_per_sm": shapes[3],
+                                     "grains_per_block": 64 if shapes[3] < 6 else "8, 16 or 32 by size",
                                      "picked_by": "sevc_autotune, 10 steps per candidate"},
                    "launch_mode": {"graph": "one CUDA graph per step (loops inside its kernels)",
                                    "hostloops": "as graph (kept for callers that select it)",

@@ -334,9 +334,10 @@ sevc_status sevc_set_graphs(sevc_handle *h, int on);
  * steps from the current state for each candidate block size of the
  * vertex pass (128/256/512) and of the per-boundary passes, each side
  * count from which grains get a warp each in the grain pass (9..11; 12: none
- * below 32), and the grain pass's block shape (4, 5: 64 grains a block; 6,
- * 8: 32), one parameter at a
- * time, keeps the fastest and restores the state.  chosen (4 ints, may be
+ * below 32), and the grain pass's block shape (4: 64 grains a block; 6: 8,
+ * 16 or 32 by the mesh's size), one parameter at a time, keeps the fastest
+ * and restores the state.  (Meshes of up to 12,288 vertices have one block
+ * size of the vertex pass, reported as it stands.)  chosen (4 ints, may be
  * NULL) receives them in that order.  Results never depend on these
  * shapes. */
 sevc_status sevc_autotune(sevc_handle *h, int steps, int *chosen);

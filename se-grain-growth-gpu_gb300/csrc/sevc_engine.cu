@@ -40,6 +40,7 @@ struct StepGraph {
 /* host part of the run state (the device part is the handle's block) */
 struct RunState {
     int n = 0, curr_n_grains = 0;
+    bool dense = false;
     double t = 0, nucleated_area = 0;
     std::vector<int> icurr, iallow;
     std::vector<double> iarea;
@@ -402,6 +403,7 @@ RunState save_run(const sevc_handle *h)
     RunState r;
     r.n = h->n;
     r.curr_n_grains = h->curr_n_grains;
+    r.dense = h->dense;
     r.t = h->t;
     r.nucleated_area = h->nucleated_area;
     r.icurr = h->icurr;
@@ -413,6 +415,7 @@ void load_run(sevc_handle *h, const RunState &r)
 {
     h->n = r.n;
     h->curr_n_grains = r.curr_n_grains;
+    h->dense = r.dense;
     h->t = r.t;
     h->nucleated_area = r.nucleated_area;
     h->icurr = r.icurr;
@@ -1344,9 +1347,20 @@ sevc_status sevc_set_gb_scaling(sevc_handle *h, double s)
     return SEVC_OK;
 }
 
+sevc_status sevc_set_launch_shape(sevc_handle *h, const int *shape)
+{
+    if (!h || !shape) return SEVC_ERR_ARG;
+    for (int k = 0; k < 2; k++)
+        if (shape[k] != 128 && shape[k] != 256 && shape[k] != 512) return SEVC_ERR_ARG;
+    if (shape[2] < 9 || shape[2] > 12 || shape[3] < 4 || shape[3] > 8 || shape[3] == 7) return SEVC_ERR_ARG;
+    h->p.shape = LaunchShape{ shape[0], shape[1], shape[2], shape[3] };
+    drop_graphs(h);
+    return SEVC_OK;
+}
+
 /* Launch-shape autotuner: coordinate search over the vertex-pass block
- * size, the per-boundary block size and the side count from which grains
- * get a warp each, timing `steps` steps (device time) per candidate from
+ * size (where the pass has one), the per-boundary block size, the side count
+ * from which grains get a warp each and the grains of a block, timing `steps` steps (device time) per candidate from
  * the same saved state; the state is restored afterwards, and results do
  * not depend on the shapes. */
 sevc_status sevc_autotune(sevc_handle *h, int steps, int *chosen)
@@ -1374,9 +1388,9 @@ sevc_status sevc_autotune(sevc_handle *h, int steps, int *chosen)
     };
     LaunchShape &sh = h->p.shape;
     int *fields[4] = { &sh.tpb_vertex, &sh.tpb_boundary, &sh.wide_sides, &sh.grain_occ };
-    const std::vector<int> cands[4] = { { 128, 256, 512 }, { 128, 256, 512 }, { 9, 10, 11, 12 }, { 4, 5, 6, 8 } };
+    const std::vector<int> cands[4] = { { 128, 256, 512 }, { 128, 256, 512 }, { 9, 10, 11, 12 }, { 4, 6 } };
     sevc_status st = SEVC_OK;
-    for (int f = 0; f < 4 && !st; f++) {
+    for (int f = vertex_lanes(h->m) ? 1 : 0; f < 4 && !st; f++) {
         int best = *fields[f];
         double best_ms = 1e300;
         for (int v : cands[f]) {

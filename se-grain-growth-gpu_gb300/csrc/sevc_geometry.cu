@@ -932,11 +932,12 @@ void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape 
     else go(k_grain_pass<32, 128, 208>, 32, 128);
 }
 
+bool vertex_lanes(const DevMesh &m) { return m.nv <= VERTEX_LANES_NV; }
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s)
 {
     /* six lanes per vertex: 8 us against 12 at 2,000 grains, 10 against 12 at
      * 5,000, the same at 10,000, 18 against 14 at 20,000 */
-    if (m.nv <= VERTEX_LANES_NV) {
+    if (vertex_lanes(m)) {
         const int g = (m.nv + 19) / 20;               /* four warps of five vertices */
         if (unit_gamma) COUNT_LAUNCHES(1), k_vertex_fd_lanes<true><<<g, 128, 0, s>>>(m, mu);
         else COUNT_LAUNCHES(1), k_vertex_fd_lanes<false><<<g, 128, 0, s>>>(m, mu);

@@ -82,10 +82,10 @@ enum {
 /* launch shapes the autotuner may change (results do not depend on them);
  * the defaults are what it picked on the 1M-grain mesh */
 struct LaunchShape {
-    int tpb_vertex = 128;    /* threads per block of the vertex pass */
+    int tpb_vertex = 128;    /* threads per block of the vertex pass (meshes that vertex_lanes accepts: always 128) */
     int tpb_boundary = 128;  /* of the per-boundary passes (geometry, t_ext) */
     int wide_sides = 12;     /* 9..11: grains of this many sides or more get a warp each; 12: of 32 or more */
-    int grain_occ = 6;       /* grains per block of the grain pass: 64 below 6, else 32 (4, 5, 6, 8) */
+    int grain_occ = 6;       /* grain pass: 4 or 5: 64 grains a block; 6 or 8: 8, 16 or 32 by the mesh's size */
 };
 
 struct StepParams {
@@ -96,12 +96,18 @@ struct StepParams {
     LaunchShape shape;
 };
 
+/* The handle's launch shapes (tpb_vertex, tpb_boundary, wide_sides,
+ * grain_occ), for tests of every shape the autotuner may pick; SEVC_ERR_ARG
+ * for others. */
+extern "C" sevc_status sevc_set_launch_shape(sevc_handle *h, const int *shape);
+
 /* geometry (sevc_geometry.cu) */
 void launch_boundary_geometry(const DevMesh &m, double eps, double scaling, const LaunchShape &sh, cudaStream_t s);
 /* grain pass: areas, moved areas, and the list of 3-sided grains */
 void launch_grain_pass(const DevMesh &m, const DevScratch &x, const LaunchShape &sh, cudaStream_t s);
 /* unit_gamma: every boundary energy is exactly 1 (GB_eps = 0, GB_scaling = 1) */
 void launch_vertex_fd(const DevMesh &m, double mu, bool unit_gamma, const LaunchShape &sh, cudaStream_t s);
+bool vertex_lanes(const DevMesh &m);   /* whether it takes six lanes per vertex */
 void launch_grain_dadt(const DevMesh &m, const DevScratch &x, cudaStream_t s);
 /* also lists the candidates and starts the polling's first comparison */
 void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
