@@ -93,13 +93,20 @@ struct DevMesh {
      * and vstamp / bstamp the step stamp (*stamp, advanced once per step)
      * under which they were saved; an entry with an older stamp is stale
      * and the live value is still the step's starting one.  bexact /
-     * gexact say which values are already exact this step. */
+     * gexact say which values are already exact this step.
+     * A removed grain keeps the area of the step's start (the areas of the
+     * enabled grains are computed again after the removals, src/main.cu:266):
+     * a 2x3 pass that edits a grain first saves it in garea0, and
+     * GEXACT_AREA of gexact says so. */
     double2 *pos0, *vel0;
     int2 *bv0;
     unsigned *vstamp, *bstamp, *stamp;
     uint8_t *bexact, *gexact;
+    double *garea0;
     int *lastblk;        /* arrival counters of last_block, zero between launches */
 };
+
+enum { GEXACT_DADT = 1, GEXACT_AREA = 2 };   /* bits of gexact */
 
 /* per-instance event counters of a step; EVT_CONFLICTS counts the
  * boundaries check_conflictive_boundaries marks (src/topological.h:116

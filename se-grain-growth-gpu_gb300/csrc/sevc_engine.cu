@@ -210,7 +210,7 @@ bool alloc_device(sevc_handle *h)
         { (void **)&m.contrib, V * 48 }, { (void **)&m.venergy, V * 8 }, { (void **)&m.ven, V },
         { (void **)&m.vspd, V * 4 },
         { (void **)&m.vb, V * 16 }, { (void **)&m.vg, V * 16 }, { (void **)&m.vmod, V * 64 },
-        { &x.reserved, V * 4 }, { (void **)&m.vmodmark, V }, { (void **)&m.modlist, V * 4 },
+        { (void **)&m.garea0, std::max(V * 4, G * 8) }, { (void **)&m.vmodmark, V }, { (void **)&m.modlist, V * 4 },
         { (void **)&m.bv, B * 8 }, { (void **)&m.benergy, B * 8 }, { (void **)&m.blen, B * 8 },
         { (void **)&m.btext, B * 8 }, { (void **)&m.ben, B }, { (void **)&m.bcand, B },
         { (void **)&m.bcandbuf, B }, { (void **)&m.bvotes, B * 4 }, { (void **)&m.bconf, B * 4 },

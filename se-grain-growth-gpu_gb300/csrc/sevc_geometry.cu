@@ -738,7 +738,7 @@ __global__ void k_grain_dadt(DevMesh m, const int *flags)
 __device__ void dadt_of(const DevMesh &m, int g)
 {
     m.gdadt[g] = dadt_from(m, g, m.pos, m.vel);
-    m.gexact[g] = 1;
+    m.gexact[g] = GEXACT_DADT;
 }
 
 /* compute_t_ext (src/topological.h:303-334) then label_boundaries

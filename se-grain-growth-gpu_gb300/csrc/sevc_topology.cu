@@ -1370,7 +1370,8 @@ __device__ __noinline__ void settle_boundary(const DevMesh &m, int b) { finalize
  *            belongs only to grains that removal queues), and its list and
  *            vertices are final for the step here; a grain edited by several
  *            fix-ups (2x3 passes, then the removals) is computed again by
- *            each, the last one on the final positions.  The flips' fix-up
+ *            each, the last one on the final positions; one that is removed
+ *            after a 2x3 pass edited it gets its first area back.  The flips' fix-up
  *            comes after the counts and needs none (the next step's grain
  *            pass computes every area).
  * No warp reads another's grain, so nothing separates the three.  three,
@@ -1403,7 +1404,7 @@ __device__ void edit_grains(const DevMesh &m, const Team &T, EditShared<WARPS> &
         }
         if (due) {
             const double d = warp_sum<true>(m, L, n, lane, st);
-            if (lane == 0) { m.gdadt[g] = d; m.gexact[g] = 1; }
+            if (lane == 0) { m.gdadt[g] = d; m.gexact[g] = GEXACT_DADT; }
         }
         if (edit) {
             __syncwarp();
@@ -1423,10 +1424,17 @@ __device__ void edit_grains(const DevMesh &m, const Team &T, EditShared<WARPS> &
         if (queued) {
             if (areas) {
                 const double a = warp_sum<false>(m, edit ? S.Ls[wib] : L, n, lane, 0);
-                if (lane == 0) m.garea[g] = a;
+                if (lane == 0) {
+                    if (n_three && !(m.gexact[g] & GEXACT_AREA)) {   /* a 2x3 pass: see DevMesh */
+                        m.garea0[g] = m.garea[g];
+                        m.gexact[g] |= GEXACT_AREA;
+                    }
+                    m.garea[g] = a;
+                }
             }
             if (lane == 0) m.gfix[g] = 0;            /* clear_grains_fix_state (:1150-1163) */
         }
+        if (w >= nf && lane == 0 && (m.gexact[g] & GEXACT_AREA)) m.garea[g] = m.garea0[g];
         __syncwarp();
     }
     /* the boundaries from the other end of the team, beside the grains */
