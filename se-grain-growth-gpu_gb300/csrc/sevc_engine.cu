@@ -585,8 +585,9 @@ void enqueue_tail(sevc_handle *h)
     DevScratch &x = h->x;
     const StepParams &p = h->p;
     if (!h->profiling) sevc_pdl_skip = 1;   /* joins the dA/dt branch: two predecessors */
-    if (tail_whole(m)) {
-        Prof pr(h, "tail");
+    /* while profiling, small meshes take the split form too: its times are
+     * the phases' (one launch would be one entry) */
+    if (tail_whole(m) && !h->profiling) {
         launch_tail_whole(m, x, p, h->polling_cap, x.summary, s);
         sevc_pdl_skip = 0;
         return;
