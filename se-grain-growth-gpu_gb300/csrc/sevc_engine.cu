@@ -102,7 +102,6 @@ struct sevc_handle {
     int *h_big = nullptr;
     size_t h_big_ints = 0;
     int *h_on = nullptr;   /* per instance: nucleation attempt this step */
-    int *h_flags = nullptr;/* host part of the step's output decision (x.flags) */
     size_t dbytes = 0;     /* size of the device block */
     /* scratch and result of the statistics calls (device) with a pinned
      * readback buffer, kept from the first call on */
@@ -119,7 +118,7 @@ struct sevc_handle {
     /* sevc_run keeps two steps in flight, each with its own pinned upload
      * and readback buffers and its events (allocated on first use) */
     struct RunSlot {
-        int *big = nullptr, *on = nullptr, *flags = nullptr;
+        int *big = nullptr, *on = nullptr;
         cudaEvent_t ev0 = nullptr, ev1 = nullptr, done = nullptr;
         sevc_step_info loc;
         long long launches = 0;
@@ -368,8 +367,7 @@ sevc_status create_from_host(const sevc_options *opt, sevc_hmesh *hm, sevc_handl
     if (!streams_ok || !cuda_ok(cudaMallocHost(&h->h_ctr, 256), "pinned") ||
         !cuda_ok(cudaMallocHost(&h->h_big, h->h_big_ints * sizeof(int)), "pinned") ||
         !cuda_ok(cudaMallocHost(&h->h_on, ninst * sizeof(int)), "pinned") ||
-        !cuda_ok(cudaMallocHost(&h->h_flags, 4 * sizeof(int)), "pinned") || !alloc_device(h) ||
-        !upload(h, hm->m)) {
+        !alloc_device(h) || !upload(h, hm->m)) {
         sevc_destroy(h);
         return SEVC_ERR_CUDA;
     }
@@ -888,11 +886,9 @@ void sevc_destroy(sevc_handle *h)
     if (h->h_ctr) cudaFreeHost(h->h_ctr);
     if (h->h_big) cudaFreeHost(h->h_big);
     if (h->h_on) cudaFreeHost(h->h_on);
-    if (h->h_flags) cudaFreeHost(h->h_flags);
     for (auto &sl : h->rslot) {
         if (sl.big) cudaFreeHost(sl.big);
         if (sl.on) cudaFreeHost(sl.on);
-        if (sl.flags) cudaFreeHost(sl.flags);
         if (sl.ev0) cudaEventDestroy(sl.ev0);
         if (sl.ev1) cudaEventDestroy(sl.ev1);
         if (sl.done) cudaEventDestroy(sl.done);
@@ -948,10 +944,9 @@ sevc_status sevc_step(sevc_handle *h, sevc_step_info *info)
     /* host part of the output decision (k_two_three_first): steps that can
      * export, long steps and exact_all */
     int mg = o.min_grains;
-    h->h_flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && h->n % o.snap_gap == 0);
-    h->h_flags[2] = batch ? 0 : mg;   /* a batch does not stop at min_grains */
-    h->h_flags[3] = h->curr_n_grains;
-    if (!cuda_ok(launch_set_flags(x, h->h_flags, s), "step flags")) return SEVC_ERR_CUDA;
+    const int full = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && h->n % o.snap_gap == 0);
+    /* a batch does not stop at min_grains */
+    if (!cuda_ok(launch_set_flags(x, full, batch ? 0 : mg, h->curr_n_grains, s), "step flags")) return SEVC_ERR_CUDA;
     h->force_direct = n_on > 0 && (bool)h->tape.after_nucleation;
     if (!run_seq(h, h->g_step[n_on ? 1 : 0][h->dense], [&] { enqueue_step(h, n_on > 0); })) return SEVC_ERR_CUDA;
     cudaEventRecord(h->ev1, s);
@@ -1004,7 +999,7 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
         for (auto &sl : h->rslot)
             if (!cuda_ok(cudaMallocHost(&sl.big, h->h_big_ints * sizeof(int)), "pinned") ||
                 !cuda_ok(cudaMallocHost(&sl.on, I * sizeof(int)), "pinned") ||
-                !cuda_ok(cudaMallocHost(&sl.flags, 4 * sizeof(int)), "pinned") || !cuda_ok(cudaEventCreate(&sl.ev0), "event") ||
+                !cuda_ok(cudaEventCreate(&sl.ev0), "event") ||
                 !cuda_ok(cudaEventCreate(&sl.ev1), "event") ||
                 !cuda_ok(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming), "event"))
                 return SEVC_ERR_CUDA;
@@ -1056,15 +1051,14 @@ sevc_status run_steps_core(sevc_handle *h, int nsteps, sevc_step_info *infos, in
             n_on += sl.on[i];
         }
         sl.loc.nucleation_attempted = n_on > 0;
-        sl.flags[1] = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && nk % o.snap_gap == 0);
-        sl.flags[2] = batch ? 0 : mg;
-        sl.flags[3] = h->curr_n_grains;   /* read only when min_grains > 0: not here */
         if (hooks) hooks->before(launched);
         if (n_on && !cuda_ok(cudaMemcpyAsync(x.nucl_on, sl.on, I * sizeof(int), cudaMemcpyHostToDevice, s), "upload")) {
             st = SEVC_ERR_CUDA;
             break;
         }
-        if (!cuda_ok(launch_set_flags(x, sl.flags, s), "step flags")) {
+        /* the grain count is read only when min_grains > 0: not here */
+        const int full = h->exact_all || o.dt >= 100 || (o.snap_gap > 0 && nk % o.snap_gap == 0);
+        if (!cuda_ok(launch_set_flags(x, full, batch ? 0 : mg, h->curr_n_grains, s), "step flags")) {
             st = SEVC_ERR_CUDA;
             break;
         }

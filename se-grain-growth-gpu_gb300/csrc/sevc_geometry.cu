@@ -975,9 +975,9 @@ void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaSt
     launch_dep(k_pack_summary, g < 152 ? g : 152, TPB, s, m, x, out);
 }
 
-cudaError_t launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s)
+cudaError_t launch_set_flags(const DevScratch &x, int full, int min_grains, int grains, cudaStream_t s)
 {
-    return launch_status(k_set_flags, 1, 1, 0, s, x.flags, flags[1], flags[2], flags[3]);
+    return launch_status(k_set_flags, 1, 1, 0, s, x.flags, full, min_grains, grains);
 }
 cudaError_t launch_read_out(const int *from, int *host, int n, cudaStream_t s)
 {

@@ -114,7 +114,7 @@ void launch_text_label(const DevMesh &m, const DevScratch &x, const StepParams &
 void launch_counts(const DevMesh &m, const DevScratch &x, const StepParams &p, cudaStream_t s);
 /* the host's part of the output decision, flags[1..3], into x.flags; and n
  * ints into pinned host memory, both in stream order */
-cudaError_t launch_set_flags(const DevScratch &x, const int *flags, cudaStream_t s);
+cudaError_t launch_set_flags(const DevScratch &x, int full, int min_grains, int grains, cudaStream_t s);
 cudaError_t launch_read_out(const int *from, int *host, int n, cudaStream_t s);
 /* counters | events | error bits | polling iterations | 2x3 counts | output decision, into out */
 void launch_pack_summary(const DevMesh &m, const DevScratch &x, int *out, cudaStream_t s);
