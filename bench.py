@@ -400,14 +400,14 @@ KERNEL_BYTES = {
 # k_vertex_fd under profiles/); traffic grows with the units processed, so
 # a full launch is scaled by its units.
 NCU_TRAFFIC_PER_UNIT = {
-    "grain_fd": (45.263e6 + 1.599e6) / 200000,
+    "grain_fd": (45.738e6 + 2.222e6) / 200000,
     "vertex_fd": (50.058e6 + 1.700e6) / 400000,
 }
 # FP64 pipe activity of the same captures (of elapsed cycles)
-NCU_FP64_ACTIVE = {"grain_fd": 0.555, "vertex_fd": 0.684}
+NCU_FP64_ACTIVE = {"grain_fd": 0.534, "vertex_fd": 0.684}
 # DADD + DMUL + DFMA thread instructions per unit, ncu counters on the
 # 200K-grain mesh (the FP64 instruction summary kept with the profiles)
-NCU_FP64_INST_PER_UNIT = {"grain_fd": 22.010e6 / 200000, "vertex_fd": 24.405e6 / 400000}
+NCU_FP64_INST_PER_UNIT = {"grain_fd": 21.810e6 / 200000, "vertex_fd": 24.405e6 / 400000}
 
 
 def run_engine(args):

@@ -158,7 +158,8 @@ sevc_status sevc_export_text(sevc_handle *h, const char *path, double time);
  * writer produces. */
 sevc_status sevc_write_snapshot(const sevc_mesh_host *mesh, const sevc_options *opt, const char *path, double time);
 /* device_to_host, src/translation.h:184-199 (without freeing anything):
- * copy the mesh into caller-owned arrays sized like sevc_mesh_sizes. */
+ * copy the mesh into caller-owned arrays sized like sevc_mesh_sizes.  A
+ * missing (NULL) array is refused (SEVC_ERR_CUDA) with nothing written. */
 sevc_status sevc_get_state(sevc_handle *h, sevc_mesh_host *out);
 sevc_status sevc_mesh_sizes(const sevc_handle *h, int *nv, int *nb, int *ng);
 /* check_data, src/utils.h:85-336: number of violated invariants (>= 0),
@@ -288,7 +289,9 @@ sevc_status sevc_set_stored_energy(sevc_handle *h, const double *se /* ng values
  * replayed random draws).  Discrete decisions carry no gradient, and a
  * nucleated grain's stored energy (0) is not a parameter.
  * Memory: one copy of the device state per checkpoint plus about 600 bytes
- * per grain per step of one segment. */
+ * per grain per step of one segment.  A step whose checkpoint finds no
+ * memory is not taken (SEVC_ERR_CUDA); the tape and the steps before it
+ * stand. */
 sevc_status sevc_tape_start(sevc_handle *h, int checkpoint_every);
 sevc_status sevc_tape_stop(sevc_handle *h);
 /* Smoothed histogram of normalised grain areas a = |A| N / (domain area)
@@ -343,7 +346,8 @@ sevc_status sevc_set_graphs(sevc_handle *h, int on);
 sevc_status sevc_autotune(sevc_handle *h, int steps, int *chosen);
 
 /* Per-kernel device time accumulated while profiling is on (CUDA events
- * around each launch on the handle's stream). */
+ * around each launch on the handle's stream; small meshes are stepped in
+ * the form of large ones meanwhile, so that the phases are apart). */
 sevc_status sevc_set_profiling(sevc_handle *h, int on);
 sevc_status sevc_get_profile(sevc_handle *h, int max_entries, char (*names)[48], double *ms,
                              int64_t *launches, int *n_entries);

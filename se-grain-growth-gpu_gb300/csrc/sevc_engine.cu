@@ -5,8 +5,9 @@
  * The step follows src/main.cu:120-394 of the reference phase by phase;
  * the kernels live in sevc_geometry.cu, sevc_topology.cu and
  * sevc_nucleation.cu.  All work of a handle is enqueued on its own CUDA
- * stream; the host reads back only small counters (polling convergence,
- * 2x3 counts, the step summary).
+ * stream (branches of a step on two side streams joined inside it); the
+ * loops of a step run in its kernels, and the host reads back one packed
+ * summary per step.
  */
 #include "sevc_internal.h"
 #include "sevc_host.h"

@@ -1,6 +1,7 @@
 /*
  * Geometry and kinetics kernels of one time step (src/calculus.h and
- * src/topological.h:303-353 of the reference), one thread per entity.
+ * src/topological.h:303-353 of the reference): blocks of grains in the
+ * grain pass, one thread or six lanes per vertex, one thread per boundary.
  *
  * The finite-difference velocity (src/calculus.h:19-73,143-154) is split
  * in two passes so that no thread re-reads another grain's polygon:
@@ -73,7 +74,7 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  *
  * What bounds it: the FP64 pipe (2 thread-operations per clock and SM, of
  * which independent chains reach 84%) together with the latency of the
- * phases below.  The certificate leaves 111 FP64 operations per grain (234
+ * phases below.  The certificate leaves 109 FP64 operations per grain (234
  * when the chains are recomputed): the integer pipe forms the exact
  * differences, and the product of the stored energy with an area difference
  * (mul_diff).  Forming the shoelace products on the integer pipe as well
@@ -98,7 +99,7 @@ __device__ __forceinline__ void put_contrib(const DevMesh &m, int g, int v, doub
  * outside the domain or + eps in the next binade.
  *
  * Measured (GB300): 1M grains 0.368 ms, FP64 pipe active 69% of the
- * cycles, 21 of 32 lanes per FP64 instruction (slots of different s or p in
+ * cycles, 22 of 32 lanes per FP64 instruction (slots of different s or p in
  * one warp); 2,000 grains 15 us.  The form before it (a grain per thread,
  * polygon in registers, one unrolled body per side count, side-count order
  * of the whole mesh first, warp-per-grain kernel for 11 sides and more)
